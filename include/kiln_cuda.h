@@ -312,7 +312,7 @@ KC_API int kc_qweight_create(kc_ctx_t ctx, const uint32_t* w, const void* scales
                              int32_t out_features, int32_t in_features, int32_t bits,
                              int32_t group_size, int32_t on_device, kc_qweight_t* out);
 KC_API void kc_qweight_free(kc_qweight_t w);
-/* y[m, out] (bf16, device) = x[m, in] (bf16, device) · dequant(W)ᵀ. */
+/* y[m, out] (bf16, device) = x[m, in] (bf16, device, 16-byte aligned) · dequant(W)ᵀ. */
 KC_API int kc_quantized_matmul(kc_ctx_t ctx, kc_qweight_t w, const void* x_dev, int32_t m,
                                void* y_dev);
 
@@ -361,7 +361,8 @@ KC_API int kc_rms_norm(kc_ctx_t ctx, const void* x_dev, const void* weight_dev, 
  * Replaces PagedKv::gather + fast::scaled_dot_product_attention
  * (paged.rs:191-225, nn.rs:800-817) and the Metal kernels of
  * crates/kiln-engine/src/paged_attn.rs:59-303. softcap = 0 disables capping;
- * window = 0 is global. out: bf16 [n, num_heads*head_dim]. */
+ * window = 0 is global. out: bf16 [n, num_heads*head_dim]. Synchronous (like kc_rope_kv_write below): the context keeps
+ * the call's metadata buffers and workspace for the next one, up to 64 MB. */
 KC_API int kc_paged_attention(kc_ctx_t ctx, kc_kv_t kv, int32_t layer, const void* q_dev,
                               int32_t n, int32_t num_heads, const kc_seq_step* seqs,
                               int32_t n_seqs, float scale, float softcap, int32_t window,

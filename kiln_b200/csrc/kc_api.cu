@@ -71,12 +71,17 @@ extern "C" int64_t kc_live_objects(void) { return g_live.load(); }
 // handles
 // ---------------------------------------------------------------------------
 
+struct kc_model;
+
 struct kc_ctx {
   int device = 0;
   int sm_count = 148;
   cudaStream_t stream = nullptr;
-  uint32_t* status = nullptr;  // device status word
-  uint32_t* status_host = nullptr;  // pinned copy, filled by the copy that precedes a synchronisation
+  // Status word: pinned host memory mapped into the device's address space. A kernel writes it only when one of its
+  // bounded waits gives up, so the host reads it after a synchronisation without a copy in the stream.
+  uint32_t* status = nullptr;             // the device's address of it
+  volatile uint32_t* status_host = nullptr;
+  kc_model* op = nullptr;                 // metadata and workspace of the single-op entry points (op_shell)
   ncclComm_t comm = nullptr;
   int tp_rank = 0, tp_world = 1;
   // launch accounting and optional per-class timing (kc_profile_*)
@@ -206,14 +211,16 @@ struct kc_model {
   cudaEvent_t meta_ev[kStaging] = {nullptr, nullptr, nullptr, nullptr};
   int meta_next = 0;
   // verify results
-  uint32_t* row_tokens = nullptr; int32_t *n_committed = nullptr, *n_accepted = nullptr; uint32_t* committed = nullptr;
+  uint32_t* row_tokens = nullptr; uint32_t* committed = nullptr;
   uint8_t* result_host = nullptr;      // pinned
   // pipelined decode: launch k keeps its sampled tokens in slot k % 2 until launch k + 2 reuses it
   uint32_t* pipe_tokens[2] = {nullptr, nullptr};   // device [max_seqs]
-  uint32_t* pipe_host[2] = {nullptr, nullptr};     // pinned [max_seqs + 1]: tokens, then the device status word
+  uint32_t* pipe_host[2] = {nullptr, nullptr};     // pinned [max_seqs], written by the sampling kernel
   cudaEvent_t pipe_ev[2] = {nullptr, nullptr};
   int pipe_n[2] = {0, 0};
   uint64_t pipe_ticket = 0;                        // of the most recent launch; 0 = none yet
+  uint32_t pipe_bad = 0;                           // status of a bounded wait that gave up in a launch up to pipe_bad_upto
+  uint64_t pipe_bad_upto = 0;
 };
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -255,15 +262,14 @@ extern "C" int kc_ctx_create(int device, kc_ctx_t* out) {
   c->device = device;
   c->sm_count = prop.multiProcessorCount;
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&c->status, sizeof(uint32_t)) != cudaSuccess ||
-      cudaMallocHost(&c->status_host, sizeof(uint32_t)) != cudaSuccess ||
-      cudaMemsetAsync(c->status, 0, sizeof(uint32_t), c->stream) != cudaSuccess) {
+      cudaHostAlloc((void**)&c->status_host, sizeof(uint32_t), cudaHostAllocMapped) != cudaSuccess ||
+      cudaHostGetDevicePointer((void**)&c->status, (void*)c->status_host, 0) != cudaSuccess) {
     if (c->stream) cudaStreamDestroy(c->stream);
-    cudaFree(c->status);
-    if (c->status_host) cudaFreeHost(c->status_host);
+    if (c->status_host) cudaFreeHost((void*)c->status_host);
     delete c;
     return fail(KC_ERR_CUDA, "kc_ctx_create: stream/status allocation failed");
   }
+  *c->status_host = 0;
   cudaEventCreate(&c->step_a);
   cudaEventCreate(&c->step_b);
   g_live++;
@@ -274,6 +280,8 @@ extern "C" int kc_ctx_create(int device, kc_ctx_t* out) {
   *out = c;
   return KC_OK;
 }
+
+static void free_op_shell(kc_ctx* c);
 
 extern "C" void kc_ctx_destroy(kc_ctx_t c) {
   if (!c) return;
@@ -288,24 +296,19 @@ extern "C" void kc_ctx_destroy(kc_ctx_t c) {
   cudaEventDestroy(c->step_a);
   cudaEventDestroy(c->step_b);
   if (c->comm) ncclCommDestroy(c->comm);
-  cudaFree(c->status);
-  cudaFreeHost(c->status_host);
+  free_op_shell(c);
+  cudaFreeHost((void*)c->status_host);
   cudaStreamDestroy(c->stream);
   delete c;
   g_live--;
 }
 
-// Queues the copy of the status word into the context's pinned word; the caller synchronises the stream and then
-// calls status_verdict. A bounded wait that gave up therefore never passes as success: every entry point that
+// Read after a synchronisation. A bounded wait that gave up never passes as success: every entry point that
 // synchronises returns KC_ERR_TIMEOUT when a kernel of the queue before it abandoned its work.
-static cudaError_t status_fetch(kc_ctx* c) {
-  return cudaMemcpyAsync(c->status_host, c->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
-}
 static int status_verdict(kc_ctx* c, const char* where) {
   const uint32_t st = *c->status_host;
   if (!st) return KC_OK;
   *c->status_host = 0;
-  cudaMemsetAsync(c->status, 0, sizeof(uint32_t), c->stream);
   return fail(KC_ERR_TIMEOUT, "%s: device status 0x%x: a bounded wait gave up (kernel 0x%x, wait %u); the results of the "
               "calls since the last synchronisation are not valid", where, st, st & 0xff00u, st & 0xffu);
 }
@@ -313,7 +316,6 @@ static int status_verdict(kc_ctx* c, const char* where) {
 extern "C" int kc_sync(kc_ctx_t c) {
   if (!c) return fail(KC_ERR_INVALID, "kc_sync: ctx is NULL");
   CK(cudaSetDevice(c->device));
-  CK(status_fetch(c));
   CK(cudaStreamSynchronize(c->stream));
   return status_verdict(c, "kc_sync");
 }
@@ -323,7 +325,6 @@ extern "C" void* kc_ctx_stream(kc_ctx_t c) { return c ? (void*)c->stream : nullp
 extern "C" int kc_device_status(kc_ctx_t c, uint32_t* status) {
   if (!c || !status) return fail(KC_ERR_INVALID, "kc_device_status: NULL argument");
   CK(cudaSetDevice(c->device));
-  CK(status_fetch(c));
   CK(cudaStreamSynchronize(c->stream));
   *status = *c->status_host;
   return status_verdict(c, "kc_device_status");
@@ -601,12 +602,11 @@ extern "C" int kc_quantized_matmul(kc_ctx_t c, kc_qweight_t q, const void* x_dev
   if ((uintptr_t)x_dev % 16) return fail(KC_ERR_INVALID, "kc_quantized_matmul: x must be 16-byte aligned");
   if (q->ctx != c) return fail(KC_ERR_INVALID, "kc_quantized_matmul: the weight was created on another context");
   CK(cudaSetDevice(c->device));
-  // x must be readable for round_up(m, 16) rows; rows past m may hold anything.
-  const int rows = (m + 15) & ~15;
-  if (q->op_ptr != x_dev || q->op_rows != rows) {
+  // The tensor map ends at row m: the rows that pad a launch to a multiple of 16 are filled with zeros by the copy.
+  if (q->op_ptr != x_dev || q->op_rows != m) {
     const char* terr = "";
-    if (!act_operand_init(&q->op, (const bf16*)x_dev, rows, q->w.K, &terr)) return fail(KC_ERR_CUDA, "kc_quantized_matmul: %s", terr);
-    q->op_ptr = x_dev; q->op_rows = rows;
+    if (!act_operand_init(&q->op, (const bf16*)x_dev, m, q->w.K, &terr)) return fail(KC_ERR_CUDA, "kc_quantized_matmul: %s", terr);
+    q->op_ptr = x_dev; q->op_rows = m;
   }
   RC(run_qlinear(c, q->w, q->op, m, (bf16*)y_dev, q->w.N, q->partial));
   return KC_OK;
@@ -812,7 +812,7 @@ void free_model(kc_model* m) {
     if (m->meta_host[i]) cudaFreeHost(m->meta_host[i]);
     if (m->meta_ev[i]) cudaEventDestroy(m->meta_ev[i]);
   }
-  cudaFree(m->row_tokens); cudaFree(m->n_committed); cudaFree(m->n_accepted); cudaFree(m->committed);
+  cudaFree(m->row_tokens); cudaFree(m->committed);
   if (m->result_host) cudaFreeHost(m->result_host);
   for (int i = 0; i < 2; ++i) {
     cudaFree(m->pipe_tokens[i]);
@@ -981,14 +981,12 @@ extern "C" int kc_model_load(kc_ctx_t c, const kc_model_desc* desc, const kc_ten
   {
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = cudaMalloc(&m->row_tokens, R * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&m->n_committed, (size_t)m->max_seqs * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&m->n_accepted, (size_t)m->max_seqs * 4);
     if (e == cudaSuccess) e = cudaMalloc(&m->committed, R * 4);
     if (e == cudaSuccess) e = cudaMallocHost(&m->result_host, R * 4 + (size_t)m->max_seqs * 8 + 64);
     for (int i = 0; i < kc_model::kStaging && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&m->meta_ev[i], cudaEventDisableTiming);
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
       e = cudaMalloc(&m->pipe_tokens[i], (size_t)m->max_seqs * 4);
-      if (e == cudaSuccess) e = cudaMallocHost(&m->pipe_host[i], ((size_t)m->max_seqs + 1) * 4);
+      if (e == cudaSuccess) e = cudaMallocHost(&m->pipe_host[i], (size_t)m->max_seqs * 4);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->pipe_ev[i], cudaEventDisableTiming);
     }
     if (e != cudaSuccess) LOAD_FAIL(fail(KC_ERR_OOM, "kc_model_load: result buffers: %s", cudaGetErrorString(e)));
@@ -1238,10 +1236,10 @@ bf16* tp_out_buffer(kc_model* m) {
 }
 
 // The forward proper. tokens_dev: n u32 on the device (normally the metadata arena's copy).
-// greedy_out (optional, device): where a single sampled row's raw arg-max goes when the head's reduction can produce
+// greedy_out (optional, device; greedy_host: a pinned copy of it): where a single sampled row's raw arg-max goes when the head's reduction can produce
 // it itself (*greedy_done = true then; otherwise the caller samples from the logits as usual).
 int run_forward(kc_model* m, kc_kv* kv, const uint32_t* tokens_dev, const StepPlan& p, bool want_logits, uint32_t* greedy_out = nullptr,
-                bool* greedy_done = nullptr) {
+                bool* greedy_done = nullptr, uint32_t* greedy_host = nullptr) {
   kc_ctx* c = m->ctx;
   const kc_model_desc& d = m->d;
   const int n = p.n, H = d.hidden_size, D = d.head_dim;
@@ -1308,7 +1306,7 @@ int run_forward(kc_model* m, kc_kv* kv, const uint32_t* tokens_dev, const StepPl
     if (streams(m->head) && greedy_out && p.n_sampled == 1 && m->argmax_scratch && !(gemma && d.final_logit_softcapping > 0.f)) {
       LAUNCH(c, KC_PROF_GEMM, 1, qlinear_stream(m->head, m->hs, m->head.K, 1, m->partial, c->status, c->stream));
       LAUNCH(c, KC_PROF_SAMPLE, 1, qlinear_reduce_argmax(m->partial, qlinear_stream_pieces(m->head), d.vocab_size, m->logits, m->argmax_scratch,
-                                                         greedy_out, c->stream));
+                                                         greedy_out, greedy_host, c->stream));
       if (greedy_done) *greedy_done = true;
     }
     else if (streams(m->head)) RC(run_stream(c, m->head, m->hs, p.n_sampled, m->logits, d.vocab_size, m->partial, nullptr));
@@ -1436,20 +1434,17 @@ extern "C" int kc_verify_step(kc_model_t m, kc_kv_t kv, const uint32_t* token_id
   if ((rc = upload_meta(m, kv, token_ids, seqs, p, c->step_a))) return rc;
   if ((rc = run_forward(m, kv, reinterpret_cast<const uint32_t*>(m->meta_dev + p.lay.tokens), p, true))) return rc;
   if (p.n_sampled > 0) {
-    LAUNCH(c, KC_PROF_SAMPLE, 1, launch_greedy_rows(m->logits, p.n_sampled, m->d.vocab_size, 1, m->row_tokens, c->stream));
+    // The results go straight into the pinned result buffer (a few hundred bytes of posted writes): no copies follow.
+    uint8_t* hb = m->result_host;
+    const size_t o1 = align_up((size_t)p.n_sampled * 4, 16), o2 = o1 + align_up((size_t)n_seqs * 4, 16);
+    LAUNCH(c, KC_PROF_SAMPLE, 1, launch_greedy_rows(m->logits, p.n_sampled, m->d.vocab_size, 1, m->row_tokens, c->stream, (uint32_t*)hb));
     // max_commit = 0: the committed list is row_tokens[row_off .. row_off + n_committed), no second copy needed
     LAUNCH(c, KC_PROF_SAMPLE, 1, launch_verify_accept(m->row_tokens, reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.v_row_off),
                             reinterpret_cast<const uint32_t*>(m->meta_dev + p.lay.v_draft),
                             reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.v_draft_off),
                             reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.v_draft_len), n_seqs, 0, m->committed,
-                            m->n_committed, m->n_accepted, c->stream));
-    uint8_t* hb = m->result_host;
-    const size_t o1 = align_up((size_t)p.n_sampled * 4, 16), o2 = o1 + align_up((size_t)n_seqs * 4, 16);
-    CK(cudaMemcpyAsync(hb, m->row_tokens, (size_t)p.n_sampled * 4, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(hb + o1, m->n_committed, (size_t)n_seqs * 4, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(hb + o2, m->n_accepted, (size_t)n_seqs * 4, cudaMemcpyDeviceToHost, c->stream));
-    CK(status_fetch(c));
-    CK(cudaEventRecord(c->step_b, c->stream));
+                            (int32_t*)(hb + o1), (int32_t*)(hb + o2), c->stream));
+      CK(cudaEventRecord(c->step_b, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     cudaEventElapsedTime(&c->last_step_ms, c->step_a, c->step_b);
     RC(status_verdict(c, "kc_verify_step"));
@@ -1457,8 +1452,7 @@ extern "C" int kc_verify_step(kc_model_t m, kc_kv_t kv, const uint32_t* token_id
     if (n_committed_out) memcpy(n_committed_out, hb + o1, (size_t)n_seqs * 4);
     if (n_accepted_out) memcpy(n_accepted_out, hb + o2, (size_t)n_seqs * 4);
   } else {
-    CK(status_fetch(c));
-    CK(cudaEventRecord(c->step_b, c->stream));
+      CK(cudaEventRecord(c->step_b, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     cudaEventElapsedTime(&c->last_step_ms, c->step_a, c->step_b);
     RC(status_verdict(c, "kc_verify_step"));
@@ -1486,11 +1480,10 @@ extern "C" int kc_draft_chain(kc_model_t m, kc_kv_t kv, uint32_t first_token, in
     if ((rc = upload_meta(m, kv, &tok, &s, p))) return rc;
     const uint32_t* tokens_dev = j == 0 ? reinterpret_cast<const uint32_t*>(m->meta_dev + p.lay.tokens) : m->row_tokens + (j - 1);
     bool sampled = false;
-    if ((rc = run_forward(m, kv, tokens_dev, p, true, m->row_tokens + j, &sampled))) return rc;
-    if (!sampled) LAUNCH(c, KC_PROF_SAMPLE, 1, launch_greedy_rows(m->logits, 1, m->d.vocab_size, 0, m->row_tokens + j, c->stream));
+    uint32_t* token_host = reinterpret_cast<uint32_t*>(m->result_host) + j;   // pinned: no copy back at the end
+    if ((rc = run_forward(m, kv, tokens_dev, p, true, m->row_tokens + j, &sampled, token_host))) return rc;
+    if (!sampled) LAUNCH(c, KC_PROF_SAMPLE, 1, launch_greedy_rows(m->logits, 1, m->d.vocab_size, 0, m->row_tokens + j, c->stream, token_host));
   }
-  CK(cudaMemcpyAsync(m->result_host, m->row_tokens, (size_t)gamma * 4, cudaMemcpyDeviceToHost, c->stream));
-  CK(status_fetch(c));
   CK(cudaStreamSynchronize(c->stream));
   RC(status_verdict(c, "kc_draft_chain"));
   memcpy(proposal_out, m->result_host, (size_t)gamma * 4);
@@ -1537,9 +1530,7 @@ extern "C" int kc_decode_launch(kc_model_t m, kc_kv_t kv, const uint32_t* token_
   if ((rc = run_forward(m, kv, tokens_dev, p, true))) return rc;
   const uint64_t ticket = m->pipe_ticket + 1;
   const int slot = (int)(ticket % 2);
-  LAUNCH(c, KC_PROF_SAMPLE, 1, launch_greedy_rows(m->logits, n_seqs, m->d.vocab_size, 1, m->pipe_tokens[slot], c->stream));
-  CK(cudaMemcpyAsync(m->pipe_host[slot], m->pipe_tokens[slot], (size_t)n_seqs * 4, cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(m->pipe_host[slot] + m->max_seqs, c->status, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream));
+  LAUNCH(c, KC_PROF_SAMPLE, 1, launch_greedy_rows(m->logits, n_seqs, m->d.vocab_size, 1, m->pipe_tokens[slot], c->stream, m->pipe_host[slot]));
   CK(cudaEventRecord(m->pipe_ev[slot], c->stream));
   m->pipe_ticket = ticket;
   m->pipe_n[slot] = n_seqs;
@@ -1557,9 +1548,12 @@ extern "C" int kc_decode_collect(kc_model_t m, uint64_t ticket, uint32_t* row_to
   kc_ctx* c = m->ctx;
   CK(cudaSetDevice(c->device));
   CK(cudaEventSynchronize(m->pipe_ev[slot]));
-  const uint32_t st = m->pipe_host[slot][m->max_seqs];
-  if (st) {
-    cudaMemsetAsync(c->status, 0, sizeof(uint32_t), c->stream);
+  // The status word is the context's: a wait that gave up in the launch behind this one shows here as well. Every
+  // launch queued so far is then reported as failed, whichever of them it was.
+  const uint32_t now = *c->status_host;
+  if (now) { *c->status_host = 0; m->pipe_bad = now; m->pipe_bad_upto = m->pipe_ticket; }
+  if (m->pipe_bad && ticket <= m->pipe_bad_upto) {
+    const uint32_t st = m->pipe_bad;
     return fail(KC_ERR_TIMEOUT, "kc_decode_collect: device status 0x%x: a bounded wait gave up (kernel 0x%x, wait %u); the tokens of "
                 "this launch and of any launch fed from it are not valid", st, st & 0xff00u, st & 0xffu);
   }
@@ -1571,19 +1565,43 @@ extern "C" int kc_decode_collect(kc_model_t m, uint64_t ticket, uint32_t* row_to
 // single ops over a caller-described step
 // ---------------------------------------------------------------------------
 
-// A throw-away model shell that owns only step metadata and the attention workspace,
-// so the single-op entry points share upload_meta / attn_params with the forward.
+// A model shell that owns only step metadata and the attention workspace, so the single-op entry points share
+// upload_meta / attn_params with the forward. It belongs to the context and is kept from call to call: making and
+// freeing its events, pinned buffers and device memory took about 700 us of a call whose kernels take 25. What a large
+// call made it grow to is given back at the end of that call (op_shell_done); a context is used from one host thread.
+constexpr size_t OP_KEEP_BYTES = (size_t)64 << 20;
+
 static int op_shell(kc_ctx* c, kc_kv* kv, int num_heads, int n, int n_seqs, kc_model** out) {
-  kc_model* m = new kc_model;
-  m->ctx = c;
+  if (!c->op) {
+    kc_model* s = new kc_model;
+    s->ctx = c;
+    for (int i = 0; i < kc_model::kStaging; ++i)
+      if (cudaEventCreateWithFlags(&s->meta_ev[i], cudaEventDisableTiming) != cudaSuccess) { free_model(s); return fail(KC_ERR_CUDA, "event"); }
+    c->op = s;
+  }
+  kc_model* m = c->op;
   m->d.num_layers = kv->layers; m->d.head_dim = kv->head_dim; m->d.num_heads = num_heads; m->d.num_kv_heads = kv->kv_heads;
   m->d.vocab_size = 0x7fffffff; m->d.hidden_size = 0; m->d.max_step_tokens = n; m->d.tp_world = 1;
   m->Hq = num_heads; m->Hkv = kv->kv_heads;
   m->max_rows = n; m->max_seqs = n_seqs; m->logit_rows = n;
-  for (int i = 0; i < kc_model::kStaging; ++i)
-    if (cudaEventCreateWithFlags(&m->meta_ev[i], cudaEventDisableTiming) != cudaSuccess) { free_model(m); return fail(KC_ERR_CUDA, "event"); }
   *out = m;
   return KC_OK;
+}
+static void free_op_shell(kc_ctx* c) {
+  if (c->op) free_model(c->op);
+  c->op = nullptr;
+}
+// Waits for the op and, if everything before it went well (rc == KC_OK), reports what the device says.
+static int op_shell_done(kc_ctx* c, int rc, const char* where) {
+  cudaError_t e = cudaStreamSynchronize(c->stream);
+  if (c->op->attn_ws_bytes > OP_KEEP_BYTES || c->op->meta_cap > OP_KEEP_BYTES) {
+    std::string keep = g_err;
+    free_op_shell(c);
+    g_err = keep;
+  }
+  if (rc) return rc;
+  if (e != cudaSuccess) return fail(KC_ERR_CUDA, "%s: %s", where, cudaGetErrorString(e));
+  return status_verdict(c, where);
 }
 
 extern "C" int kc_paged_attention(kc_ctx_t c, kc_kv_t kv, int32_t layer, const void* q_dev, int32_t n, int32_t num_heads,
@@ -1609,11 +1627,7 @@ extern "C" int kc_paged_attention(kc_ctx_t c, kc_kv_t kv, int32_t layer, const v
       return KC_OK;
     }();
   }
-  cudaStreamSynchronize(c->stream);
-  std::string keep = g_err;
-  free_model(m);
-  g_err = keep;
-  return rc;
+  return op_shell_done(c, rc, "kc_paged_attention");
 }
 
 extern "C" int kc_rope_kv_write(kc_ctx_t c, kc_kv_t kv, int32_t layer, const void* qkv_dev, const void* qkv_bias_dev,
@@ -1637,9 +1651,5 @@ extern "C" int kc_rope_kv_write(kc_ctx_t c, kc_kv_t kv, int32_t layer, const voi
                                          kv->pool, (bf16*)q_out_dev, c->stream);
     if (e != cudaSuccess) rc = fail(KC_ERR_CUDA, "kc_rope_kv_write: %s", cudaGetErrorString(e));
   }
-  cudaStreamSynchronize(c->stream);
-  std::string keep = g_err;
-  free_model(m);
-  g_err = keep;
-  return rc;
+  return op_shell_done(c, rc, "kc_rope_kv_write");
 }

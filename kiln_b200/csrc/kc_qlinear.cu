@@ -189,8 +189,10 @@ static const CUtensorMap* act_operand_rows_map(const ActOperand* op, int m_pad) 
 bool act_operand_init(ActOperand* op, const bf16* ptr, int rows, int K, const char** err) {
   op->ptr = ptr; op->rows = rows; op->K = K; op->rows_map_n = 0;
   if (K % QL_KB) { *err = "activation width must be a multiple of 64"; return false; }
-  if (!make_tmap_bf16_2d(&op->map16, ptr, K, rows, QL_KB, 16, err)) return false;
-  if (!make_tmap_bf16_2d(&op->map64, ptr, K, rows, QL_KB, 64, err)) return false;
+  // the first launch's map is encoded here so that a geometry the driver refuses is reported at binding
+  const int m_pad = std::min(256, (rows + 15) & ~15);
+  if (!make_tmap_bf16_2d(&op->rows_map, ptr, K, rows, QL_KB, m_pad, err)) return false;
+  op->rows_map_n = m_pad;
   return true;
 }
 
@@ -730,7 +732,7 @@ static int plan_row_cap(int nt, uint32_t raw_stride) {
 cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   const QWeight& w = *l.w;
   if (l.M < 1 || l.M > QL_MAX_M) return cudaErrorInvalidValue;
-  if (l.row0 % 16 || l.row0 + ((l.M + 15) & ~15) > l.x->rows) return cudaErrorInvalidValue;
+  if (l.row0 % 16 || l.row0 + l.M > l.x->rows) return cudaErrorInvalidValue;   // rows past the operand's end read as zeros
   const int nt = plan_tiles_per_cta(w, w.sm_count);
   const int cap = plan_row_cap(nt, w.record_bytes);
   if (cap == 0) return cudaErrorInvalidValue;
@@ -1362,7 +1364,7 @@ __global__ void qlinear_reduce_kernel(const float* __restrict__ partial, int spl
 // CTA followed by one counter word that is zero between launches (the last CTA resets it).
 __global__ void __launch_bounds__(256) qlinear_reduce_argmax_kernel(const float* __restrict__ partial, int splits, int N,
                                                                     bf16* __restrict__ y, float* __restrict__ scratch,
-                                                                    uint32_t* __restrict__ token) {
+                                                                    uint32_t* __restrict__ token, uint32_t* __restrict__ token_host) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float s_v[8];
@@ -1414,16 +1416,19 @@ __global__ void __launch_bounds__(256) qlinear_reduce_argmax_kernel(const float*
   __syncthreads();   // s_v / s_i are reused
   reduce_block();
   if (threadIdx.x == 0) {
-    *token = (uint32_t)best_i < (uint32_t)N ? (uint32_t)best_i : 0u;   // a row of NaNs has no maximum
+    const uint32_t tok = (uint32_t)best_i < (uint32_t)N ? (uint32_t)best_i : 0u;   // a row of NaNs has no maximum
+    *token = tok;
+    if (token_host) *token_host = tok;
     *counter = 0u;
   }
 }
 
 int qlinear_reduce_argmax_ctas(int N) { return std::max(1, std::min((N + 511) / 512, 296)); }
 
-cudaError_t qlinear_reduce_argmax(const float* partial, int splits, int N, bf16* y, float* scratch, uint32_t* token, cudaStream_t s) {
+cudaError_t qlinear_reduce_argmax(const float* partial, int splits, int N, bf16* y, float* scratch, uint32_t* token, uint32_t* token_host,
+                                  cudaStream_t s) {
   if (!partial || !y || !scratch || !token || splits < 1 || N < 1) return cudaErrorInvalidValue;
-  return launch_k(qlinear_reduce_argmax_kernel, dim3(qlinear_reduce_argmax_ctas(N)), dim3(256), 0, s, partial, splits, N, y, scratch, token);
+  return launch_k(qlinear_reduce_argmax_kernel, dim3(qlinear_reduce_argmax_ctas(N)), dim3(256), 0, s, partial, splits, N, y, scratch, token, token_host);
 }
 
 cudaError_t qlinear_reduce_splits(const float* partial, int splits, int M, int N, bf16* y, int ldy,

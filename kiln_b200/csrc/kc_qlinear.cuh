@@ -46,15 +46,13 @@ struct QWeight {
   size_t mlx_bytes() const { return (size_t)N * K * bits / 8 + (size_t)2 * N * (K / group) * 2; }
 };
 
-// Activation operand: a bf16 [rows, K] row-major device buffer plus the two
-// tensor maps (16-row and 64-row boxes of 64 features, 128-byte swizzle) the
-// TMA loads use.
+// Activation operand: a bf16 [rows, K] row-major device buffer plus the tensor
+// map (box of 64 features x a launch's rows, 128-byte swizzle) the TMA loads
+// use; rows of a box past the end of the buffer are filled with zeros.
 struct ActOperand {
   const bf16* ptr = nullptr;
-  int rows = 0;  // allocated rows (multiple of 16)
+  int rows = 0;  // rows of the buffer
   int K = 0;
-  CUtensorMap map16;
-  CUtensorMap map64;
   mutable CUtensorMap rows_map;   // box of rows_map_n rows: one TMA operation per k-block while the row count is stable
   mutable int rows_map_n = 0;
 };
@@ -115,9 +113,10 @@ cudaError_t qlinear_gemv(const QWeight& w, const bf16* x, int ldx, int M, float*
                          const QvGatedInput* gated = nullptr);
 
 // One row: y[n] = bf16(sum over pieces of partial[k][n]) and *token = arg-max of that row (lowest index on ties), in
-// one launch. scratch: 2 * qlinear_reduce_argmax_ctas(N) floats followed by one zeroed 32-bit counter (left zero).
+// one launch (token_host, optional: pinned host memory that gets the token as well). scratch: 2 * qlinear_reduce_argmax_ctas(N) floats followed by one zeroed 32-bit counter (left zero).
 int qlinear_reduce_argmax_ctas(int N);
-cudaError_t qlinear_reduce_argmax(const float* partial, int splits, int N, bf16* y, float* scratch, uint32_t* token, cudaStream_t s);
+cudaError_t qlinear_reduce_argmax(const float* partial, int splits, int N, bf16* y, float* scratch, uint32_t* token, uint32_t* token_host,
+                                  cudaStream_t s);
 
 // out[m, n] = bf16(sum over splits of partial[s][m][n]) in split order.
 cudaError_t qlinear_reduce_splits(const float* partial, int splits, int M, int N, bf16* y, int ldy,

@@ -25,7 +25,8 @@ __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
 // logits into ties — hence the explicit lowest-index rule.
 // normalize == 0: argmax of the raw row (crates/kiln-models/src/draft.rs:379-381).
 __global__ void __launch_bounds__(1024)
-greedy_rows_kernel(const bf16* __restrict__ logits, int vocab, int normalize, uint32_t* __restrict__ tokens) {
+greedy_rows_kernel(const bf16* __restrict__ logits, int vocab, int normalize, uint32_t* __restrict__ tokens,
+                   uint32_t* __restrict__ tokens_host) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float red_m[32];
@@ -113,7 +114,11 @@ greedy_rows_kernel(const bf16* __restrict__ logits, int vocab, int normalize, ui
       ArgMax b2{__shfl_xor_sync(0xffffffffu, best.v, o), __shfl_xor_sync(0xffffffffu, best.i, o)};
       best = better(best, b2);
     }
-    if (lane == 0) tokens[blockIdx.x] = (uint32_t)(best.i == 0x7fffffff ? 0 : best.i);
+    if (lane == 0) {
+      const uint32_t tok = (uint32_t)(best.i == 0x7fffffff ? 0 : best.i);
+      tokens[blockIdx.x] = tok;
+      if (tokens_host) tokens_host[blockIdx.x] = tok;
+    }
   }
 }
 
@@ -166,9 +171,9 @@ cudaError_t launch_feed_tokens(uint32_t* tokens, const int32_t* feed, const uint
 }
 
 cudaError_t launch_greedy_rows(const bf16* logits, int rows, int vocab, int normalize, uint32_t* tokens,
-                               cudaStream_t s) {
+                               cudaStream_t s, uint32_t* tokens_host) {
   if (rows <= 0) return cudaSuccess;
-  return launch_k(greedy_rows_kernel, dim3(rows), dim3(1024), 0, s, logits, vocab, normalize, tokens);
+  return launch_k(greedy_rows_kernel, dim3(rows), dim3(1024), 0, s, logits, vocab, normalize, tokens, tokens_host);
 }
 
 cudaError_t launch_verify_accept(const uint32_t* row_tokens, const int32_t* seq_row_offsets, const uint32_t* draft,
