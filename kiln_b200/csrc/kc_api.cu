@@ -580,6 +580,7 @@ extern "C" int kc_qweight_create(kc_ctx_t c, const uint32_t* w, const void* scal
     if (need) e = cudaMalloc(&q->partial, need * sizeof(float));
   }
   cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess) e = qweight_finish(&q->w);
   cudaFree(dw); cudaFree(ds); cudaFree(db);
   if (e != cudaSuccess) { qweight_free(&q->w); delete q; return fail(KC_ERR_CUDA, "kc_qweight_create: %s", cudaGetErrorString(e)); }
   g_live++;
@@ -729,6 +730,7 @@ int build_linear(kc_model* m, TensorIndex& idx, const std::vector<Part>& parts, 
   cudaError_t e = qweight_build(out, (const uint32_t*)dw, (const bf16*)ds, (const bf16*)db, (int)N, K, bits, group,
                                 c->sm_count, c->stream);
   cudaStreamSynchronize(c->stream);
+  if (e == cudaSuccess) e = qweight_finish(out);
   cudaFree(dw); cudaFree(ds); cudaFree(db);
   if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? KC_ERR_OOM : KC_ERR_CUDA, "re-tiling %s: %s", parts[0].prefix.c_str(), cudaGetErrorString(e));
   m->weight_bytes += (int64_t)out->mlx_bytes();

@@ -27,10 +27,13 @@ namespace kc {
 // Re-tiling
 // ---------------------------------------------------------------------------
 
+// Scales below this limit can be multiplied by 2^129 (4-bit) or 2^133 (8-bit) within bf16: see dequant_pairs.
+__host__ __device__ constexpr float ql_scale_limit(int bits) { return bits == 4 ? 0.5f : 0.03125f; }
+
 __global__ void qweight_retile_kernel(uint8_t* __restrict__ records, const uint32_t* __restrict__ w,
                                       const bf16* __restrict__ scales, const bf16* __restrict__ biases,
                                       int N, int K, int bits, int group, int n_tiles, int kblocks,
-                                      int gpk, uint32_t packed_bytes, uint32_t record_bytes) {
+                                      int gpk, uint32_t packed_bytes, uint32_t record_bytes, int* __restrict__ wide) {
   const int words_per_row_kb = QL_KB * bits / 32;  // 8 (w4) or 16 (w8)
   const int words_per_rec = QL_TILE_N * words_per_row_kb;
   const int sb_per_rec = QL_TILE_N * gpk;
@@ -63,7 +66,8 @@ __global__ void qweight_retile_kernel(uint8_t* __restrict__ records, const uint3
         }
         v = o;
       }
-      reinterpret_cast<uint32_t*>(base)[e] = v;
+      // 16-byte chunk c / 4 of row r: chunk-major, so that neighbouring rows' chunks are neighbours in shared memory
+      reinterpret_cast<uint32_t*>(base)[((c >> 2) * QL_TILE_N + r) * 4 + (c & 3)] = v;
     } else {
       const int e2 = e - words_per_rec;
       const int r = e2 / gpk, gi = e2 % gpk;
@@ -73,6 +77,7 @@ __global__ void qweight_retile_kernel(uint8_t* __restrict__ records, const uint3
         const int g = (kb * QL_KB + gi * group) / group;
         sb.x = scales[(long long)n * groups_per_row + g];
         sb.y = biases[(long long)n * groups_per_row + g];
+        if (!(fabsf(__bfloat162float(sb.x)) < ql_scale_limit(bits))) *wide = 1;
       }
       reinterpret_cast<bf162*>(base + packed_bytes)[e2] = sb;
     }
@@ -99,18 +104,26 @@ cudaError_t qweight_build(QWeight* out, const uint32_t* w, const bf16* scales, c
   q.record_bytes = q.packed_bytes + QL_TILE_N * q.gpk * 4;
   q.splits = qlinear_plan_splits(q.n_tiles, q.kblocks, sm_count);
   q.sm_count = sm_count;
-  cudaError_t e = cudaMalloc(&q.records, q.bytes());
+  // one allocation: the records, then a flag that the re-tiling raises
+  cudaError_t e = cudaMalloc(&q.records, q.bytes() + 16);
   if (e != cudaSuccess) return e;
+  q.wide = reinterpret_cast<int*>(q.records + q.bytes());
+  e = cudaMemsetAsync(q.wide, 0, 16, s);
+  if (e != cudaSuccess) { cudaFree(q.records); return e; }
   const long long total = (long long)(q.bytes() / 4);
   const int threads = 256;
   const int blocks = (int)std::min<long long>((total + threads - 1) / threads, 148LL * 16);
   qweight_retile_kernel<<<blocks, threads, 0, s>>>(q.records, w, scales, biases, N, K, bits, group,
                                                    q.n_tiles, q.kblocks, q.gpk, q.packed_bytes,
-                                                   q.record_bytes);
+                                                   q.record_bytes, q.wide);
   e = cudaGetLastError();
   if (e != cudaSuccess) { cudaFree(q.records); return e; }
   *out = q;
   return cudaSuccess;
+}
+
+cudaError_t qweight_finish(QWeight* w) {
+  return cudaMemcpy(&w->wide_scale, w->wide, sizeof(int), cudaMemcpyDeviceToHost);
 }
 
 void qweight_free(QWeight* w) {
@@ -197,45 +210,80 @@ bool act_operand_init(ActOperand* op, const bf16* ptr, int rows, int K, const ch
 }
 
 // ---------------------------------------------------------------------------
-// Dequantisation of one 8-element chunk -> 8 bf16 (16 bytes)
+// Dequantisation of one weight row of one k-block: 64 values -> 32 bf16 pairs, w = bf16(q * scale + bias), one rounding.
+//
+// The dequantisers' instruction issue is what bounds a launch of few rows, so the integers become bf16 operands of the
+// multiply-add without a conversion: the bf16 with bit pattern N < 256 is N * 2^-133 (subnormals and the first binade
+// have the same spacing), so a nibble masked into bits 4..7 of a half-word IS q * 2^-129 and a byte in bits 0..7 IS
+// q * 2^-133. One fused multiply-add with the scale times 2^129 (2^133: exact, a power of two) gives q * scale + bias
+// rounded once — the value that converting q first gives. 11 instructions for 8 weights instead of 15 (4 bits), 2 for
+// 2 instead of 7 (8 bits). The scaled scale must stay below 2^128: a weight with a scale of ql_scale_limit or more
+// (its `wide` flag, raised when it is re-tiled) takes the conversion.
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ uint4 dequant8_w4(uint32_t u, bf162 sb) {
-  const bf162 s2 = __bfloat162bfloat162(sb.x);
-  const bf162 b2 = __bfloat162bfloat162(sb.y);
-  const bf162 c128 = __floats2bfloat162_rn(128.f, 128.f);
-  // The record's nibble order puts element 2j at bits 4j and element 2j + 1 at bits 16 + 4j. Two masks split the word
-  // into bytes (even nibbles: elements 0, 4, 1, 5; odd nibbles: 2, 6, 3, 7) and a byte permute sets each under 0x43:
-  // 0x4300 | q is the bf16 value 128 + q (exact for q < 128); subtracting 128 is exact.
-  const uint32_t lo = u & 0x0F0F0F0Fu, hi = (u >> 4) & 0x0F0F0F0Fu;
-  uint32_t t[4];
-  t[0] = __byte_perm(lo, 0x43434343u, 0x4240u);   // elements 0, 1
-  t[1] = __byte_perm(hi, 0x43434343u, 0x4240u);   // elements 2, 3
-  t[2] = __byte_perm(lo, 0x43434343u, 0x4341u);   // elements 4, 5
-  t[3] = __byte_perm(hi, 0x43434343u, 0x4341u);   // elements 6, 7
-  uint32_t o[4];
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    bf162 q = __hsub2(*reinterpret_cast<bf162*>(&t[j]), c128);
-    bf162 wv = __hfma2(q, s2, b2);  // one rounding: bf16(q*s + b)
-    o[j] = *reinterpret_cast<uint32_t*>(&wv);
-  }
-  return make_uint4(o[0], o[1], o[2], o[3]);
+__device__ __forceinline__ uint32_t bf2_fma(uint32_t a, bf162 s, bf162 b) {
+  const bf162 r = __hfma2(*reinterpret_cast<const bf162*>(&a), s, b);
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ bf162 bf2_bits(uint32_t u) { return *reinterpret_cast<const bf162*>(&u); }
+// (scale, scale) times 2^129 or 2^133, in two exact steps (neither power of two is a bf16)
+template <int BITS>
+__device__ __forceinline__ bf162 scaled_scale(bf162 sb) {
+  const bf162 s = __hmul2(__bfloat162bfloat162(sb.x), bf2_bits(0x7F007F00u));              // 2^127
+  return __hmul2(s, BITS == 4 ? bf2_bits(0x40804080u) : bf2_bits(0x42804280u));            // 2^2, 2^6
 }
 
-__device__ __forceinline__ uint4 dequant8_w8(uint32_t u0, uint32_t u1, bf162 sb) {
-  const float s = __bfloat162float(sb.x), b = __bfloat162float(sb.y);
-  float f[8];
+// Packed words of a row (chunk c = 16 bytes at row_base + c * QL_TILE_N * 16) -> v[32].
+template <int BITS, int GPK>
+__device__ __forceinline__ void dequant_row(const uint8_t* row_base, const bf162 (&sb)[GPK], uint32_t (&v)[32]) {
+  constexpr int CHUNKS = BITS / 2;
+  bf162 s2[GPK], b2[GPK];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    // byte k under the exponent of 2^23: the float 8388608 + q, minus 2^23 = q exactly.
-    f[k] = __uint_as_float(__byte_perm(u0, 0x4B000000u, 0x7540u | k)) - 8388608.f;
-    f[4 + k] = __uint_as_float(__byte_perm(u1, 0x4B000000u, 0x7540u | k)) - 8388608.f;
+  for (int g = 0; g < GPK; ++g) { s2[g] = scaled_scale<BITS>(sb[g]); b2[g] = __bfloat162bfloat162(sb[g].y); }
+#pragma unroll
+  for (int h = 0; h < CHUNKS; ++h) {
+    const uint4 q = *reinterpret_cast<const uint4*>(row_base + h * (QL_TILE_N * 16));
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    const int g = GPK == 2 ? h * 2 / CHUNKS : 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (BITS == 4) {
+        // the record's nibble order: element 2j at bits 4j, element 2j + 1 at bits 16 + 4j
+        uint32_t* o = v + (h * 4 + c) * 4;
+        o[0] = bf2_fma((w[c] << 4) & 0x00F000F0u, s2[g], b2[g]);
+        o[1] = bf2_fma(w[c] & 0x00F000F0u, s2[g], b2[g]);
+        o[2] = bf2_fma((w[c] >> 4) & 0x00F000F0u, s2[g], b2[g]);
+        o[3] = bf2_fma((w[c] >> 8) & 0x00F000F0u, s2[g], b2[g]);
+      } else {
+        uint32_t* o = v + (h * 4 + c) * 2;
+        o[0] = bf2_fma(__byte_perm(w[c], 0u, 0x4140u), s2[g], b2[g]);
+        o[1] = bf2_fma(__byte_perm(w[c], 0u, 0x4342u), s2[g], b2[g]);
+      }
+    }
   }
-  uint32_t o[4];
+}
+
+// The same for a weight with a scale past the limit: the integers are converted (a byte under the exponent of 2^23 is
+// the float 8388608 + q) and one fp32 multiply-add is rounded to bf16; q * scale has at most 16 bits, so the fp32 sum
+// is rounded at 24 bits and then at 8.
+template <int BITS, int GPK>
+__device__ __forceinline__ void dequant_row_wide(const uint8_t* row_base, const bf162 (&sb)[GPK], uint32_t (&v)[32]) {
+  constexpr int CHUNKS = BITS / 2;
 #pragma unroll
-  for (int j = 0; j < 4; ++j) o[j] = pack_bf162(fmaf(f[2 * j], s, b), fmaf(f[2 * j + 1], s, b));
-  return make_uint4(o[0], o[1], o[2], o[3]);
+  for (int h = 0; h < CHUNKS; ++h) {
+    const uint4 q = *reinterpret_cast<const uint4*>(row_base + h * (QL_TILE_N * 16));
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+    const int g = GPK == 2 ? h * 2 / CHUNKS : 0;
+    const float s = __bfloat162float(sb[g].x), b = __bfloat162float(sb[g].y);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int j = 0; j < 16 / BITS; ++j) {
+        const uint32_t lo = BITS == 4 ? (w[c] >> (4 * j)) & 0xFu : (w[c] >> (16 * j)) & 0xFFu;
+        const uint32_t hi = BITS == 4 ? (w[c] >> (16 + 4 * j)) & 0xFu : (w[c] >> (16 * j + 8)) & 0xFFu;
+        v[(h * 4 + c) * (16 / BITS) + j] = pack_bf162(fmaf((float)lo, s, b), fmaf((float)hi, s, b));
+      }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -292,12 +340,9 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 // ---------------------------------------------------------------------------
 
 constexpr int QL_DQ_WARP0 = 4;         // first dequant/epilogue warp
-constexpr int QL_DQ_GROUPS = 2;        // dequant groups; group g converts k-blocks g, g + G, g + 2G, ...
-constexpr int QL_DQ_GROUP_WARPS = 8;
-constexpr int QL_DQ_GROUP_THREADS = QL_DQ_GROUP_WARPS * 32;
-constexpr int QL_DQ_WARPS = QL_DQ_GROUPS * QL_DQ_GROUP_WARPS;
+constexpr int QL_DQ_GROUPS = 4;        // dequant groups of four warps (the four TMEM lane quarters)
+constexpr int QL_DQ_WARPS = QL_DQ_GROUPS * 4;
 constexpr int QL_THREADS = (QL_DQ_WARP0 + QL_DQ_WARPS) * 32;   // 20 warps
-constexpr int QL_A_BYTES = QL_TILE_N * 128;  // one 128-row A tile of one stage
 constexpr int QL_EPI_STAGE_BYTES = 32 * 32 * 4;   // per-warp transpose buffer of the epilogue
 
 struct QlKernelParams {
@@ -307,12 +352,11 @@ struct QlKernelParams {
   int M, m_pad;          // live rows, rows rounded up to 16
   int row0;              // first activation row
   int splits;
-  int a_stages, r_stages, b_stages;   // b_stages: activation ring of the kernel that keeps its A ring in TMEM
-  uint32_t raw_stride;   // distance between the records of neighbouring tiles in a raw stage (= record_bytes)
-  int b_single;          // 1: the first tensor map's box spans all m_pad rows (one TMA operation per k-block)
+  int a_stages, r_stages, b_stages;   // ring depths: stages in TMEM, k-blocks of records and stages of activations in shared memory
+  int wide;              // a scale of the weight is past ql_scale_limit
   int glu;               // 0, or 1 (silu) / 2 (gelu_approx): the epilogue writes act = activation(gate tile) * up tile
   bf16* act; int ld_act;
-  uint32_t tmem_cols;    // power of two >= max(32, NT * m_pad)
+  uint32_t tmem_cols;    // columns allocated: a power of two
   bf16* y; int ldy;
   float* partial;        // [splits][part_M][N]; this launch writes rows part_row0 .. part_row0 + M
   int part_M, part_row0;
@@ -337,7 +381,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
 // split-K partials, or — when the CTA owns (gate, up) tile pairs — the gated activation.
 template <int NT>
 __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* smem, int warp, int lane, uint32_t tmem_base,
-                                            int tile0, int nt_live, int split) {
+                                            int tile0, int nt_live, int split, bool two_sums) {
   tc_fence_after();
   // every MMA has completed and every copy into the rings has been consumed: the ring memory is free
   float* stage = reinterpret_cast<float*>(smem + (size_t)(warp - QL_DQ_WARP0) * QL_EPI_STAGE_BYTES);
@@ -378,9 +422,15 @@ __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* sm
   } else
   for (int item = eg; item < nt_live * chunks; item += QL_DQ_WARPS / 4) {
     const int t = item / chunks, ch = item - t * chunks;
-    const int col = (NT == 1 ? 0 : t * col_stride) + ch * 32;   // NT == 1: columns are m directly (incl. the 256+ accumulator)
+    const int col = t * col_stride + ch * 32;
     uint32_t v[32];
     tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + col, v);
+    if (NT == 1 && two_sums) {                   // even plus odd k-blocks
+      uint32_t w[32];
+      tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + col + col_stride, w);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
+    }
     __syncwarp();                                // the previous item's reads of the buffer are done
 #pragma unroll
     for (int j = 0; j < 32; ++j) stage[j * 32 + lane] = __uint_as_float(v[j]);   // stage[m][n]
@@ -415,18 +465,23 @@ __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* sm
 
 // ---------------------------------------------------------------------------
 // The kernel. The dequantised weights reach the tensor core through TENSOR MEMORY (tcgen05.mma with the A operand in
-// TMEM), not through shared memory. Measured reason: an M = 128, N = 192 MMA needs 97 cycles when run alone, but a
-// kernel that staged the bf16 weights in shared memory took about 1140 cycles per k-block of eight of them — its 154 KB
-// of shared-memory traffic per k-block (32 KB of bf16 weights written, 32 KB read back by the MMAs, the activation
-// k-block read once per tile, the copies) is what the 128 B/clk shared memory can move in that time. Here a
-// dequantiser thread owns one weight row (= one TMEM lane) of one unit, expands its 64 weights in registers and writes
-// them with one tcgen05.st (column c = weights 2c and 2c + 1), so the MMAs read only the activation k-block from shared
-// memory and the A ring costs no shared memory at all. Units per stage are fixed at two: two tiles of one k-block
-// (NT == 2), or two k-blocks of one tile (NT == 1; a split with an odd number of k-blocks ends with a one-unit
-// stage). NT is free to depend on the row count: it changes which CTA computes an output element, never the order in
-// which that element's k-blocks are accumulated.
+// TMEM), not through shared memory: an M = 128, N = 192 MMA needs 97 cycles when run alone, but a kernel that staged the
+// bf16 weights in shared memory took about 1140 cycles per k-block of eight of them, the time its 154 KB of
+// shared-memory traffic takes. A dequantiser thread owns one weight row (= one TMEM lane) of one UNIT — one 128-row tile
+// of one 64-feature k-block —, expands its 64 weights in registers and writes them with one tcgen05.st (column c =
+// weights 2c and 2c + 1), so the MMAs read only the activation k-block from shared memory.
 //
-// TMEM columns: [NT accumulators of round32(m_pad)] [a_stages x 2 units x 32 columns of bf16 pairs].
+// What bounds it: at few rows (an MMA then takes 46 cycles whatever its N) the dequantisers' instruction issue and the
+// hand-overs; from about 128 rows on the tensor pipe, 4 * N / 2 cycles per unit. Hence: four groups of four warps, each
+// converting every fourth unit on its own; and two accumulators, each with an issuing WARP and a ring of A slots of its
+// own — the CTA's two tiles, or the even and the odd k-blocks of its one tile, summed in the epilogue. A stage is one
+// unit of each. An issuing warp runs its loop converged with one elected lane around the MMAs: with `if (lane == 0)`
+// around the loop the operands of each MMA went through vector registers and eight MMAs took 700 cycles to issue.
+// 28672 x 4096 in 4 bits, 112 CTAs, every launch from HBM: 35.7 us -> 24 us at 1 row, 40.7 -> 37 us at 192 rows.
+//
+// The order in which an element's k-blocks are accumulated is a function of the weight's shape only.
+//
+// TMEM columns: [2 accumulators of round32(m_pad)] [a_stages x 2 units x 32 columns of bf16 pairs].
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t d_hi, uint32_t idesc,
                                              uint32_t accumulate) {
@@ -447,54 +502,55 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
         "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
         "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
       : "memory");
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// A bounded wait of a whole warp; the warp is converged afterwards.
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32_t* status, uint32_t code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
 }
 
 template <int BITS, int GPK, int NT>
 __global__ void __launch_bounds__(QL_THREADS, 1)
 qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKernelParams p) {
-  constexpr int KC = NT == 1 ? 2 : 1;
-  constexpr int UNITS = 2;
-  static_assert(NT * KC == UNITS, "two units per stage");
+  constexpr int KC = NT == 1 ? 2 : 1;                   // k-blocks of a stage; a stage is two units
   constexpr uint32_t PACKED = QL_TILE_N * (QL_KB * BITS / 8);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const int SA = p.a_stages, SB = p.b_stages, RS = p.r_stages;
-  const uint32_t bk_bytes = (uint32_t)p.m_pad * 128u;   // one activation k-block
-  const uint32_t b_stage = KC * bk_bytes;
-  const uint32_t r_stage = UNITS * p.raw_stride;
+  const int SA = p.a_stages, SB = p.b_stages;
+  const uint32_t b_bytes = (uint32_t)p.m_pad * 128u;    // one activation k-block
+  const uint32_t r_stage = NT * p.record_bytes;         // the records of one k-block
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int tile0 = blockIdx.x * NT, split = blockIdx.y;
+  const int nt_live = min(NT, p.n_tiles - tile0);
+  // splits may be uneven: split s takes k-blocks [K s / S, K (s + 1) / S) — a fixed function of the weight's shape
+  const int kb0 = (int)((long long)p.kblocks * split / p.splits);
+  const int nkb = (int)((long long)p.kblocks * (split + 1) / p.splits) - kb0;
+  // Ring depths: a group visits every second stage, and it must meet every fill of the slots it waits on (a wait names a
+  // fill by its parity only), so r_stages is a multiple of 2 * KC k-blocks and a_stages of 2.
+  const int RS = p.r_stages;
+  const uint32_t col_stride = (uint32_t)(p.m_pad + 31) & ~31u;
+  const uint32_t a_col0 = 2 * col_stride;               // first column of the A ring
+
   uint8_t* sB = smem;
-  uint8_t* sR = sB + (size_t)SB * b_stage;
+  uint8_t* sR = sB + (size_t)SB * b_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sR + (size_t)RS * r_stage);
   uint64_t* raw_full = bars;
   uint64_t* raw_empty = raw_full + RS;
   uint64_t* b_full = raw_empty + RS;
   uint64_t* b_empty = b_full + SB;
   uint64_t* a_ready = b_empty + SB;
-  uint64_t* a_empty = a_ready + SA;
-  uint64_t* acc_full = a_empty + SA;
-  uint64_t* turn = acc_full + 1;                        // the two MMA issuers hand the issue order to each other through it
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(turn + 1);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int tile0 = blockIdx.x * NT, split = blockIdx.y;
-  const int nt_live = min(NT, p.n_tiles - tile0);
-  // splits may be uneven: split s takes k-blocks [K s / S, K (s + 1) / S) — a fixed function of the weight's shape
-  const int kb0 = (int)((long long)p.kblocks * split / p.splits);
-  const int nkb = (int)((long long)p.kblocks * (split + 1) / p.splits) - kb0;
-  const int nst = (nkb + KC - 1) / KC;                  // pipeline stages of this CTA
-  const int tail_kc = nkb - (nst - 1) * KC;             // k-blocks of the last stage (1 or KC)
-  const int n_issuers = 1;   // a stage's MMAs are all issued (and its slots released) by one thread
-  const uint32_t col_stride = (uint32_t)(p.m_pad + 31) & ~31u;
-  const uint32_t a_col0 = NT * col_stride;              // first column of the A ring
+  uint64_t* a_empty = a_ready + 2 * SA;                 // [stage][unit], like a_ready
+  uint64_t* acc_full = a_empty + 2 * SA;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
 
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
-    for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], QL_DQ_GROUP_WARPS); }
-    for (int i = 0; i < SB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], n_issuers); }
-    for (int i = 0; i < SA; ++i) { mbar_init(&a_ready[i], QL_DQ_GROUP_WARPS); mbar_init(&a_empty[i], n_issuers); }
-    mbar_init(acc_full, 2);   // both issuing threads commit to it after their last stage
-    mbar_init(turn, 1);
+    for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4 * nt_live); }
+    for (int i = 0; i < SB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], nt_live); }
+    for (int i = 0; i < 2 * SA; ++i) { mbar_init(&a_ready[i], 4); mbar_init(&a_empty[i], 1); }
+    mbar_init(acc_full, NT == 1 ? 2 : nt_live);   // each issuer commits to it after its last MMA
     mbar_fence_init();
   }
   if (warp == 2) {
@@ -508,22 +564,17 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  bool ok = true;
 
   if (warp == 0) {
-    // ---- weight record producer ----
+    // ---- weight record producer: weights depend on no kernel before this one ----
     if (lane == 0) {
       RingPos rp;
-      for (int i = 0; i < nst; ++i, rp.advance(RS)) {
-        if (!mbar_wait(&raw_empty[rp.stage], rp.phase ^ 1, p.status, KC_DEV_QLINEAR | 1)) { ok = false; break; }
-        const int kcs = i == nst - 1 ? tail_kc : KC;
-        mbar_arrive_expect_tx(&raw_full[rp.stage], p.record_bytes * nt_live * kcs);
-#pragma unroll
-        for (int kc = 0; kc < KC; ++kc)
-          if (kc < kcs)
-          bulk_g2s(sR + (size_t)rp.stage * r_stage + (size_t)kc * NT * p.raw_stride,
-                   p.records + (((size_t)(tile0 / QL_TILE_GROUP) * p.kblocks + kb0 + i * KC + kc) * QL_TILE_GROUP + tile0 % QL_TILE_GROUP) * p.record_bytes,
-                   p.record_bytes * nt_live, &raw_full[rp.stage]);
+      const uint8_t* src = p.records + (((size_t)(tile0 / QL_TILE_GROUP) * p.kblocks + kb0) * QL_TILE_GROUP + tile0 % QL_TILE_GROUP) * p.record_bytes;
+      const uint32_t bytes = p.record_bytes * nt_live;
+      for (int i = 0; i < nkb; ++i, rp.advance(RS), src += (size_t)QL_TILE_GROUP * p.record_bytes) {
+        if (!mbar_wait(&raw_empty[rp.stage], rp.phase ^ 1, p.status, KC_DEV_QLINEAR | 1)) break;
+        mbar_arrive_expect_tx(&raw_full[rp.stage], bytes);
+        bulk_g2s(sR + (size_t)rp.stage * r_stage, src, bytes, &raw_full[rp.stage]);
       }
     }
   } else if (warp == 1) {
@@ -531,127 +582,110 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
     if (lane == 0) {
       pdl_wait();
       RingPos bp;
-      for (int i = 0; i < nst; ++i, bp.advance(SB)) {
-        if (!mbar_wait(&b_empty[bp.stage], bp.phase ^ 1, p.status, KC_DEV_QLINEAR | 2)) { ok = false; break; }
-        const int kcs = i == nst - 1 ? tail_kc : KC;
-        mbar_arrive_expect_tx(&b_full[bp.stage], kcs * bk_bytes);
-#pragma unroll
-        for (int kc = 0; kc < KC; ++kc)
-          if (kc < kcs)
-          tma_load_2d(sB + (size_t)bp.stage * b_stage + (size_t)kc * bk_bytes, &map_rows, (kb0 + i * KC + kc) * QL_KB, p.row0,
-                      &b_full[bp.stage]);
+      for (int i = 0; i < nkb; ++i, bp.advance(SB)) {
+        if (!mbar_wait(&b_empty[bp.stage], bp.phase ^ 1, p.status, KC_DEV_QLINEAR | 2)) break;
+        mbar_arrive_expect_tx(&b_full[bp.stage], b_bytes);
+        tma_load_2d(sB + (size_t)bp.stage * b_bytes, &map_rows, (kb0 + i) * QL_KB, p.row0, &b_full[bp.stage]);
       }
     }
-  } else if (warp == 2 || warp == 3) {
-    // ---- MMA issuers: warp 2 takes the even stages, warp 3 the odd ones ----
-    // Two issuing threads take alternate stages (all MMAs of a stage, both tiles): while one issues, the other is
-    // already through the waits, the fence and the descriptor arithmetic of the next stage. The order in which the
-    // MMAs enter the tensor pipe is handed over through `turn`: the issuer of stage i arrives on it after its last
-    // MMA instruction, the issuer of stage i + 1 waits for that before its first.
-    if (lane == 0) {
-      pdl_wait();
-      const int me = warp - 2;
+  } else if (warp < QL_DQ_WARP0) {
+    // ---- MMA issuers: warp 2 + u issues the MMAs of unit u of every stage into accumulator u. The whole warp runs the
+    // loop, one elected lane issues. The two never touch the same accumulator, so nothing orders them to each other.
+    // A barrier test takes about 130 cycles from issue to branch, as long as the issue of four MMAs: the next stage's
+    // barriers are tested before this stage's MMAs issue, and only a stage that was not ready then waits.
+    pdl_wait();
+    const int u = warp - 2;
+    if (NT == 1 || u < nt_live) {
       const uint32_t idesc = umma_idesc_bf16(QL_TILE_N, p.m_pad);
       const uint64_t proto = umma_smem_desc_sw128(0);
-      const uint32_t d_hi = (uint32_t)(proto >> 32), d_lo = (uint32_t)proto;
-      const uint32_t b_lo0 = d_lo | ((smem_u32(sB) >> 4) & 0x3FFF);
-      const uint32_t b_step = b_stage >> 4;
-      RingPos ap, bp;
-      for (int i = 0; i < nst; ++i, ap.advance(SA), bp.advance(SB)) {
-        if ((i & 1) != me) continue;
-        if (!mbar_wait(&a_ready[ap.stage], ap.phase, p.status, KC_DEV_QLINEAR | 3)) { ok = false; break; }
-        if (!mbar_wait(&b_full[bp.stage], bp.phase, p.status, KC_DEV_QLINEAR | 4)) { ok = false; break; }
-        tc_fence_after();   // the A operand was written with tcgen05.st by other threads
-        const uint32_t b_lo = b_lo0 + bp.stage * b_step;
-        const uint32_t a_t = tmem_base + a_col0 + ap.stage * (UNITS * 32);
-        const uint32_t acc = i > 0 ? 1u : 0u;
-        if (i > 0 && !mbar_wait(turn, (uint32_t)(i - 1) & 1u, p.status, KC_DEV_QLINEAR | 8)) { ok = false; break; }
-#pragma unroll
-        for (int u = 0; u < UNITS; ++u) {
-          if ((NT == 2 ? u < nt_live : true) && (NT == 2 || u == 0 || i < nst - 1 || tail_kc == KC)) {
-            const int t = NT == 2 ? u : 0, kc = NT == 2 ? 0 : u;
-            const uint32_t b_u = b_lo + kc * (bk_bytes >> 4);
-#pragma unroll
-            for (int ks = 0; ks < QL_KB / 16; ++ks)
-              umma_bf16_ts(tmem_base + t * col_stride, a_t + u * 32 + 8 * ks, b_u + 2 * ks, d_hi, idesc,
-                           (NT == 1 && u == 1) ? 1u : (ks == 0 ? acc : 1u));
-          }
+      const uint32_t d_hi = (uint32_t)(proto >> 32), b_lo0 = (uint32_t)proto | ((smem_u32(sB) >> 4) & 0x3FFF);
+      const uint32_t d_t = tmem_base + u * col_stride, a_t0 = tmem_base + a_col0 + u * 32;
+      const int n_own = NT == 2 ? nkb : (nkb + 1 - u) / 2;  // k-blocks of this accumulator
+      int as = 0, bs = NT == 2 ? 0 : u;                     // ring positions of the next one
+      uint32_t aphase = 0, bphase = 0, acc = 0;
+      bool ok = true, ready = false;
+      for (int i = 0; i < n_own; ++i) {
+        if (!__all_sync(0xffffffffu, ready)) {
+          ok = warp_wait(&b_full[bs], bphase, p.status, KC_DEV_QLINEAR | 4) &&
+               warp_wait(&a_ready[2 * as + u], aphase, p.status, KC_DEV_QLINEAR | 3);
+          if (!ok) break;
         }
-        mbar_arrive(turn);
-        umma_commit(&a_empty[ap.stage]);
-        umma_commit(&b_empty[bp.stage]);
+        tc_fence_after();   // the A operand was written with tcgen05.st by other threads
+        const uint32_t b_lo = b_lo0 + bs * (b_bytes >> 4), a_t = a_t0 + as * 64;
+        uint64_t *a_done = &a_empty[2 * as + u], *b_done = &b_empty[bs];
+        if (++as == SA) { as = 0; aphase ^= 1u; }
+        bs += KC;
+        if (bs >= SB) { bs -= SB; bphase ^= 1u; }
+        ready = i + 1 < n_own && (mbar_test_wait(&b_full[bs], bphase) & mbar_test_wait(&a_ready[2 * as + u], aphase));
+        if (elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < QL_KB / 16; ++ks)
+            umma_bf16_ts(d_t, a_t + 8 * ks, b_lo + 2 * ks, d_hi, idesc, ks == 0 ? acc : 1u);
+          umma_commit(a_done);
+          umma_commit(b_done);
+        }
+        __syncwarp();
+        acc = 1;
       }
-      umma_commit(acc_full);
+      if (ok && elect_one()) umma_commit(acc_full);
+      __syncwarp();
     }
-  } else {
-    // ---- dequantisers: thread = one weight row (TMEM lane 32 * (warp % 4) + lane) of one unit ----
-    const int td = threadIdx.x - QL_DQ_WARP0 * 32;  // 0..511
-    const int grp = td / QL_DQ_GROUP_THREADS;
-    const int wj = (warp - QL_DQ_WARP0) & 7;        // warp inside the group; (wj & 3) == (warp & 3): the lane quarter
-    const int unit = wj >> 2;
-    const int row = (wj & 3) * 32 + lane;
-    const bool live = NT == 1 || unit < nt_live;
-    const uint32_t raw_off = (uint32_t)unit * p.raw_stride + row * (QL_KB * BITS / 8);
-    const uint32_t sb_off = (uint32_t)unit * p.raw_stride + PACKED + row * GPK * 4;
-    const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-    RingPos rp, ap;
-    for (int g = 0; g < grp; ++g) { rp.advance(RS); ap.advance(SA); }
-    bool released = false;
-    for (int i = grp; i < nst && ok; i += QL_DQ_GROUPS) {
+  } else if (warp >= QL_DQ_WARP0) {
+    // ---- dequantisers: thread = one weight row (TMEM lane 32 * (warp % 4) + lane) of every fourth unit ----
+    // Group g converts unit g & 1 of the stages g >> 1, (g >> 1) + 2, ...
+    const int grp = (warp - QL_DQ_WARP0) >> 2, unit = grp & 1;
+    const int row = (warp & 3) * 32 + lane;
+    const uint32_t a_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + a_col0 + unit * 32;
+    const int tile = NT == 2 ? unit : 0;
+    const uint8_t* row_raw = sR + (size_t)tile * p.record_bytes + row * 16;
+    const uint8_t* row_sb = sR + (size_t)tile * p.record_bytes + PACKED + row * (GPK * 4);
+    int rs = NT == 2 ? grp >> 1 : (grp >> 1) * 2 + unit, as = grp >> 1;   // ring positions of the group's next unit
+    constexpr int R_STEP = 2 * KC;                      // k-blocks between a group's units
+    uint32_t rphase = 0, aphase = 0;
+    const int own = NT == 2 ? (unit < nt_live ? nkb : 0) : (nkb + 1 - unit) / 2;   // units of this accumulator: one per stage
+    bool ok = true, released = false, raw_ready = false;
+    for (int i = grp >> 1; i < own; i += 2) {
       // the first SA stages are dequantised under the tail of the previous kernel; a slot that is being reused is freed
       // by an MMA, which needs activations, which need the previous kernel: the bounded wait for it counts from there
       if (!released && i >= SA) { pdl_wait(); released = true; }
-      ok = __all_sync(0xffffffffu, mbar_wait(&raw_full[rp.stage], rp.phase, p.status, KC_DEV_QLINEAR | 5));
-      if (!ok) break;
-      uint32_t v[32];
-      const bool unit_live = live && (NT == 2 || unit == 0 || i < nst - 1 || tail_kc == KC);
-      if (unit_live) {
-        const uint8_t* rec = sR + (size_t)rp.stage * r_stage;
-        bf162 sb[GPK];
-#pragma unroll
-        for (int g = 0; g < GPK; ++g) sb[g] = *reinterpret_cast<const bf162*>(rec + sb_off + g * 4);
-        if (BITS == 4) {
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const uint4 q = *reinterpret_cast<const uint4*>(rec + raw_off + h * 16);
-            const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const uint4 o = dequant8_w4(w4[c], sb[GPK == 2 ? h : 0]);
-              v[(h * 4 + c) * 4 + 0] = o.x; v[(h * 4 + c) * 4 + 1] = o.y; v[(h * 4 + c) * 4 + 2] = o.z; v[(h * 4 + c) * 4 + 3] = o.w;
-            }
-          }
-        } else {
-#pragma unroll
-          for (int h = 0; h < 4; ++h) {
-            const uint4 q = *reinterpret_cast<const uint4*>(rec + raw_off + h * 16);
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-              const uint4 o = dequant8_w8(c ? q.z : q.x, c ? q.w : q.y, sb[GPK == 2 ? (h >> 1) : 0]);
-              v[(h * 2 + c) * 4 + 0] = o.x; v[(h * 2 + c) * 4 + 1] = o.y; v[(h * 2 + c) * 4 + 2] = o.z; v[(h * 2 + c) * 4 + 3] = o.w;
-            }
-          }
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = 0u;
+      if (!__all_sync(0xffffffffu, raw_ready)) {
+        ok = warp_wait(&raw_full[rs], rphase, p.status, KC_DEV_QLINEAR | 5);
+        if (!ok) break;
       }
+      // the slot's barrier is tested under the arithmetic, the next record's under the store (see the issuers)
+      const bool a_free = mbar_test_wait(&a_empty[2 * as + unit], aphase ^ 1);
+      uint32_t v[32];
+      bf162 sb[GPK];
+      if (GPK == 1) {
+        sb[0] = *reinterpret_cast<const bf162*>(row_sb + (size_t)rs * r_stage);
+      } else {
+        const uint2 s = *reinterpret_cast<const uint2*>(row_sb + (size_t)rs * r_stage);
+        sb[0] = bf2_bits(s.x); sb[GPK - 1] = bf2_bits(s.y);
+      }
+      if (!p.wide) dequant_row<BITS, GPK>(row_raw + (size_t)rs * r_stage, sb, v);
+      else dequant_row_wide<BITS, GPK>(row_raw + (size_t)rs * r_stage, sb, v);
       __syncwarp();
-      if (lane == 0) mbar_arrive(&raw_empty[rp.stage]);   // the record is in registers: its slot can refill
-      ok = __all_sync(0xffffffffu, mbar_wait(&a_empty[ap.stage], ap.phase ^ 1, p.status, KC_DEV_QLINEAR | 6));
-      if (!ok) break;
+      if (lane == 0) mbar_arrive(&raw_empty[rs]);       // the record is in registers: its slot can refill
+      rs += R_STEP;
+      if (rs >= RS) { rs -= RS; rphase ^= 1u; }
+      raw_ready = i + 2 < own && mbar_test_wait(&raw_full[rs], rphase);
+      if (!__all_sync(0xffffffffu, a_free)) {
+        ok = warp_wait(&a_empty[2 * as + unit], aphase ^ 1, p.status, KC_DEV_QLINEAR | 6);
+        if (!ok) break;
+      }
       tc_fence_after();
-      tmem_st32(tmem_base + lane_addr + a_col0 + ap.stage * (UNITS * 32) + unit * 32, v);
+      tmem_st32(a_addr + as * 64, v);
+      tmem_wait_st();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&a_ready[ap.stage]);
-#pragma unroll
-      for (int g = 0; g < QL_DQ_GROUPS; ++g) { rp.advance(RS); ap.advance(SA); }
+      if (lane == 0) mbar_arrive(&a_ready[2 * as + unit]);
+      as += 2;
+      if (as >= SA) { as -= SA; aphase ^= 1u; }
     }
     // ---- epilogue ----
     pdl_wait();   // the stores below may overwrite what an earlier kernel still reads
-    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(acc_full, 0, p.status, KC_DEV_QLINEAR | 7));
-    if (ok) ql_epilogue<NT>(p, smem, warp, lane, tmem_base, tile0, nt_live, split);
+    if (ok) ok = warp_wait(acc_full, 0, p.status, KC_DEV_QLINEAR | 7);
+    if (ok) ql_epilogue<NT>(p, smem, warp, lane, tmem_base, tile0, nt_live, split, nkb > 1);
   }
   __syncwarp();
   tc_fence_before();
@@ -665,26 +699,27 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
 
 // Ring depths and shared memory of one launch geometry; ok == false when it does not fit tensor or shared memory.
 struct TaPlan { bool ok; int sa, sb, rs; uint32_t tmem_cols; size_t smem; };
-static TaPlan plan_ta(int nt, int m_pad, uint32_t raw_stride) {
+static TaPlan plan_ta(int nt, int m_pad, uint32_t record_bytes) {
   TaPlan t{};
-  const int kc = nt == 1 ? 2 : 1;
-  const int col_stride = (m_pad + 31) & ~31;
-  const int acc_cols = nt * col_stride;
-  int sa = (512 - acc_cols) / 64;            // two units of 32 columns per stage
-  if (sa > 4) sa = 4;
+  const int acc_cols = 2 * ((m_pad + 31) & ~31);
+  int sa = std::min(6, (512 - acc_cols) / 64) & ~1;
   if (sa < 2 || m_pad > 256) return t;
   uint32_t cols = 32;
   while ((int)cols < acc_cols + sa * 64) cols <<= 1;
   const size_t budget = (size_t)212 * 1024;
-  const size_t b_stage = (size_t)kc * m_pad * 128;
-  const size_t rstage = (size_t)2 * raw_stride;
-  if (budget < 6 * rstage + 2 * b_stage) return t;
-  const int sb = (int)std::min<size_t>(4, (budget - 6 * rstage) / b_stage);
-  int rs = (int)std::min<size_t>(24, (budget - (size_t)sb * b_stage) / rstage);
-  if (sb < 2 || rs < 3) return t;
+  const size_t b_stage = (size_t)m_pad * 128;
+  const size_t r_stage = (size_t)nt * record_bytes;
+  // activations arrive from L2 (about 2000 cycles): up to 16 k-blocks ahead where they are small, 6 of 192 rows
+  int sb = (int)std::min<size_t>(16, std::max<size_t>(6, (size_t)(64 * 1024) / b_stage));
+  while (sb > 4 && (size_t)sb * b_stage + (nt == 2 ? 6 : 8) * r_stage > budget) --sb;
+  sb &= nt == 1 ? ~1 : ~0;   // one tile per CTA: an issuer takes every second k-block and must meet every fill of its slots
+  if ((size_t)sb * b_stage + 4 * r_stage > budget) return t;
+  // a multiple of the k-blocks between a group's units (see the kernel), so that a slot always serves the same groups
+  int rs = (int)std::min<size_t>(32, (budget - (size_t)sb * b_stage) / r_stage) & (nt == 2 ? ~1 : ~3);
+  if (rs < 4) return t;
   // the epilogue's per-warp transpose buffers reuse the ring memory from its start
-  while ((size_t)sb * b_stage + (size_t)rs * rstage < (size_t)QL_DQ_WARPS * QL_EPI_STAGE_BYTES) ++rs;
-  const size_t smem = 1024 + (size_t)sb * b_stage + (size_t)rs * rstage + (2 * rs + 2 * sb + 2 * sa + 2) * 8 + 16;
+  while ((size_t)sb * b_stage + (size_t)rs * r_stage < (size_t)QL_DQ_WARPS * QL_EPI_STAGE_BYTES) rs += 4;
+  const size_t smem = 1024 + (size_t)sb * b_stage + (size_t)rs * r_stage + (2 * rs + 2 * sb + 4 * sa + 1) * 8 + 16;
   if (smem > 227 * 1024) return t;
   t.ok = true; t.sa = sa; t.sb = sb; t.rs = rs; t.tmem_cols = cols; t.smem = smem;
   return t;
@@ -693,7 +728,7 @@ static TaPlan plan_ta(int nt, int m_pad, uint32_t raw_stride) {
 template <int BITS, int GPK, int NT>
 static cudaError_t launch_umma_ta(const QLinearLaunch& l, QlKernelParams& p, cudaStream_t s) {
   const QWeight& w = *l.w;
-  const TaPlan t = plan_ta(NT, p.m_pad, p.raw_stride);
+  const TaPlan t = plan_ta(NT, p.m_pad, p.record_bytes);
   if (!t.ok) return cudaErrorInvalidValue;   // the caller sized the row chunk with plan_ta
   p.tmem_cols = t.tmem_cols;
   p.a_stages = t.sa; p.b_stages = t.sb; p.r_stages = t.rs;
@@ -704,7 +739,6 @@ static cudaError_t launch_umma_ta(const QLinearLaunch& l, QlKernelParams& p, cud
   }
   const CUtensorMap* rows = act_operand_rows_map(l.x, p.m_pad);
   if (!rows) return cudaErrorInvalidValue;
-  p.b_single = 1;
   dim3 grid((w.n_tiles + NT - 1) / NT, w.splits);
   return launch_k(qlinear_umma_ta_kernel<BITS, GPK, NT>, grid, dim3(QL_THREADS), t.smem, s, *rows, p);
 }
@@ -722,10 +756,10 @@ static int plan_tiles_per_cta(const QWeight& w, int sm_count) {
 
 // The most rows one launch of this weight takes: what the accumulators (two tiles: 192 columns each, one tile: 256)
 // and the rings of the weight's record size leave room for.
-static int plan_row_cap(int nt, uint32_t raw_stride) {
+static int plan_row_cap(int nt, uint32_t record_bytes) {
   static const int caps[] = {256, 192, 128, 64, 32, 16};
   for (int c : caps)
-    if (plan_ta(nt, c, raw_stride).ok) return c;
+    if (plan_ta(nt, c, record_bytes).ok) return c;
   return 0;
 }
 
@@ -749,7 +783,7 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
     p.N = w.N; p.n_tiles = w.n_tiles; p.kblocks = w.kblocks;
     p.M = std::min(per, l.M - r0); p.m_pad = (p.M + 15) & ~15; p.row0 = l.row0 + r0;
     p.splits = w.splits;
-    p.raw_stride = w.record_bytes;
+    p.wide = w.wide_scale;
     p.y = l.y; p.ldy = l.ldy; p.partial = l.partial; p.part_M = l.M; p.part_row0 = r0; p.status = l.status;
     p.glu = glu ? l.glu : 0; p.act = l.act; p.ld_act = l.ld_act;
     cudaError_t e;
@@ -845,11 +879,18 @@ __device__ __forceinline__ void qg_raw_pairs(const uint32_t* u, uint32_t (&e)[4]
   }
 }
 
+// Byte offset in a record of the 8 features 8 t .. 8 t + 7 of a row's first 32-feature half: with 16-byte chunks
+// chunk-major, the four lanes of a 4-bit row read one chunk and those of an 8-bit row two.
+template <int BITS>
+__device__ __forceinline__ uint32_t lane_offset(int row, int t) {
+  return BITS == 4 ? (uint32_t)row * 16 + t * 4 : (uint32_t)((t >> 1) * QL_TILE_N + row) * 16 + (t & 1) * 8;
+}
+
 template <int BITS, int GPK>
 __global__ void __launch_bounds__(QG_THREADS, QG_CTAS_PER_SM) qlinear_stream_kernel(const QgParams p) {
   constexpr int ROW_BYTES = QL_KB * BITS / 8;          // bytes of one weight row in one k-block: 32 or 64
   constexpr int PACKED = QL_TILE_N * ROW_BYTES;
-  constexpr int HALF_BYTES = ROW_BYTES / 2;            // one 32-feature half of a row
+  constexpr int HALF_BYTES = QL_TILE_N * ROW_BYTES / 2;   // one 32-feature half of all rows (chunk-major order)
   constexpr int LANE_WORDS = BITS / 4;                 // 32-bit words holding the lane's 8 features of a half
   constexpr int NT = QL_TILE_GROUP;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -957,7 +998,7 @@ __global__ void __launch_bounds__(QG_THREADS, QG_CTAS_PER_SM) qlinear_stream_ker
         acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
       }
     };
-    const uint32_t lane_off = (uint32_t)r0 * ROW_BYTES + t * (4 * LANE_WORDS);
+    const uint32_t lane_off = lane_offset<BITS>(r0, t);
     const uint32_t sb_off = PACKED + (uint32_t)r0 * GPK * 4;
     // the activation fragment and the row sums of a unit are fetched one unit ahead
     uint4 xa[2], xa_next[2];
@@ -989,7 +1030,7 @@ __global__ void __launch_bounds__(QG_THREADS, QG_CTAS_PER_SM) qlinear_stream_ker
         for (int h = 0; h < 2; ++h)
 #pragma unroll
           for (int r = 0; r < 2; ++r) {
-            const uint8_t* src = rec + lane_off + r * 8 * ROW_BYTES + h * HALF_BYTES;
+            const uint8_t* src = rec + lane_off + r * 8 * 16 + h * HALF_BYTES;
             if (LANE_WORDS == 1) u[h][r][0] = *reinterpret_cast<const uint32_t*>(src);
             else { const uint2 v = *reinterpret_cast<const uint2*>(src); u[h][r][0] = v.x; u[h][r][LANE_WORDS - 1] = v.y; }
           }
@@ -1112,7 +1153,7 @@ template <int BITS, int GPK>
 __global__ void __launch_bounds__(QV_THREADS) qlinear_gemv_kernel(const QvParams p) {
   constexpr int ROW_BYTES = QL_KB * BITS / 8;
   constexpr int PACKED = QL_TILE_N * ROW_BYTES;
-  constexpr int HALF_BYTES = ROW_BYTES / 2;
+  constexpr int HALF_BYTES = QL_TILE_N * ROW_BYTES / 2;
   constexpr int LANE_WORDS = BITS / 4;
   constexpr int RB = BITS == 4 ? 4 : 2;               // records whose loads and MMA chains overlap
   extern __shared__ __align__(128) uint8_t smem[];
@@ -1182,7 +1223,7 @@ __global__ void __launch_bounds__(QV_THREADS) qlinear_gemv_kernel(const QvParams
   __syncthreads();
   const int g = lane >> 2, t = lane & 3;
   const int r0 = warp * 16 + g;
-  const uint32_t lane_off = (uint32_t)r0 * ROW_BYTES + t * (4 * LANE_WORDS);
+  const uint32_t lane_off = lane_offset<BITS>(r0, t);
   const uint32_t sb_off = PACKED + (uint32_t)r0 * GPK * 4;
   const bf16* xrow = xs + (size_t)g * row_elems + 8 * t;
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
@@ -1210,7 +1251,7 @@ __global__ void __launch_bounds__(QV_THREADS) qlinear_gemv_kernel(const QvParams
       for (int h = 0; h < 2; ++h)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const uint8_t* src = rc + lane_off + r * 8 * ROW_BYTES + h * HALF_BYTES;
+          const uint8_t* src = rc + lane_off + r * 8 * 16 + h * HALF_BYTES;
           if (LANE_WORDS == 1) u[i][h][r][0] = *reinterpret_cast<const uint32_t*>(src);
           else { const uint2 v = *reinterpret_cast<const uint2*>(src); u[i][h][r][0] = v.x; u[i][h][r][LANE_WORDS - 1] = v.y; }
         }

@@ -9,7 +9,7 @@
 // needs for one k-block is ONE contiguous, 16-byte aligned run that a single
 // bulk copy brings into shared memory:
 //
-//   record(tile t, kblock kb) = packed[128 rows][64*bits/8 bytes]   (stored in the order [t / 4][kb][t % 4])
+//   record(tile t, kblock kb) = packed[64*bits/128 chunks][128 rows][16 bytes]   (stored in the order [t / 4][kb][t % 4])
 //                             ++ sb[128 rows][gpk] as bf162 (scale, bias)
 //
 // with 128 output rows per tile, 64 input features per k-block and gpk =
@@ -41,6 +41,8 @@ struct QWeight {
   uint32_t record_bytes = 0;
   int splits = 1;              // fixed function of (N, K): never of M
   int sm_count = 148;
+  int* wide = nullptr;         // device flag of the re-tiling (inside the records' allocation)
+  int wide_scale = 0;          // its value, read once at load: a scale is too large for the conversion-free dequantisation
   size_t bytes() const { return (size_t)((n_tiles + QL_TILE_GROUP - 1) / QL_TILE_GROUP) * QL_TILE_GROUP * kblocks * record_bytes; }
   // Algorithmic bytes of the mlx tensors this weight was built from.
   size_t mlx_bytes() const { return (size_t)N * K * bits / 8 + (size_t)2 * N * (K / group) * 2; }
@@ -81,8 +83,10 @@ struct QLinearLaunch {
 int qlinear_plan_splits(int n_tiles, int kblocks, int sm_count);
 
 // Re-tile on the device. w/scales/biases are device pointers in mlx layout.
+// The caller reads the weight's flag with qweight_finish once the stream has run.
 cudaError_t qweight_build(QWeight* out, const uint32_t* w, const bf16* scales, const bf16* biases,
                           int N, int K, int bits, int group, int sm_count, cudaStream_t s);
+cudaError_t qweight_finish(QWeight* w);
 void qweight_free(QWeight* w);
 
 // Creates the tensor maps of an activation buffer. Returns false (and sets

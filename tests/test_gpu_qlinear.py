@@ -181,3 +181,39 @@ def test_stream_lane_rows_do_not_depend_on_row_count(ctx):
     assert torch.equal(one.view(torch.int16), full[5:6].view(torch.int16))
     with pytest.raises(api.KcError, match="m = 9"):
         qw.matmul_stream(acts(9, 4096, 9).cuda())
+
+
+@pytest.mark.parametrize("n,k,bits,group,m,gain", [
+    (26700, 192, 4, 64, 33, 1.0),     # 209 tiles, two per CTA: the last CTA owns one; three k-blocks
+    (26700, 64, 8, 64, 192, 1.0),     # one k-block: the second issuer has nothing to do
+    (384, 1088, 4, 32, 256, 1.0),     # one tile per CTA, 256 rows, splits of 8 and 9 k-blocks: stages with one k-block
+    (384, 1088, 8, 32, 177, 1.0),     # 8-bit, rows past the activations' end inside the last group of 16
+    (300, 512, 4, 64, 20, 200.0),     # scales of 0.5 and more: integers converted before the multiply-add
+    (300, 512, 8, 64, 20, 300.0),     # the same for 8 bits (scales of 1/32 and more)
+    (300, 512, 4, 64, 20, 1e-30),     # scales near the smallest normal numbers
+])
+def test_stage_edges_and_scale_range(ctx, n, k, bits, group, m, gain):
+    """The places where the pipeline's stages end unevenly, and the range of scales on both sides of the one where the
+    dequantisation changes form. Bound: the GEMM's bar for outputs of order one; with another gain the outputs scale
+    with it, so the inputs are scaled back by a power of two and the same bar holds."""
+    g = torch.Generator().manual_seed(31)
+    w = torch.empty(n, k).normal_(0, 0.02 * gain, generator=g)
+    p, s, b = quantize_affine(w, bits, group)
+    if gain > 1:
+        assert float(s.float().max()) >= (0.5 if bits == 4 else 0.03125)
+    if gain < 1e-20:
+        s = (s.float() * 0 + 2.0 ** -110).to(torch.bfloat16)      # the quantiser's floor is far above such a gain
+        b = (b.float().sign() * 2.0 ** -108).to(torch.bfloat16)
+        shift = 2.0 ** 108
+    else:
+        shift = 2.0 ** -int(torch.log2(torch.tensor(gain)).round())
+    x = (acts(m, k, 32).float() * shift).to(torch.bfloat16)
+    O.set_weight_class(1)
+    want = O.quantized_matmul(x, p, s, b, bits, group)
+    O.set_weight_class(0)
+    qw = api.QuantizedWeight(ctx, p.cuda(), s.cuda(), b.cuda(), bits, group)
+    got = qw.matmul(x.cuda()).cpu()
+    assert parity(f"qlinear {n}x{k} w{bits}g{group} rows {m} gain {gain:g}", got, want, MAX_ABS, MIN_COS)
+    one = qw.matmul(x[m - 1:].cuda()).cpu()
+    assert torch.equal(one.view(torch.int16), got[m - 1:].view(torch.int16))
+    assert ctx.device_status() == 0
