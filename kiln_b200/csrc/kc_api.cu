@@ -29,13 +29,6 @@
 
 using namespace kc;
 
-namespace kc {
-bool make_tmap_bf16_2d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint32_t box_inner,
-                       uint32_t box_outer, const char** err);
-bool make_tmap_kv_4d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t plane_rows, uint64_t planes,
-                     const char** err);
-}
-
 // ---------------------------------------------------------------------------
 // errors, live counter
 // ---------------------------------------------------------------------------
@@ -129,8 +122,8 @@ struct kc_kv {
   bf16* pool = nullptr;        // [layers][2][num_blocks][kv_heads][block_size][head_dim]
   size_t block_elems = 0;      // kv_heads * block_size * head_dim
   size_t bytes = 0;
-  CUtensorMap map;             // all pool rows x head_dim, box {64, 16}, 128-byte swizzle; or, with map4d, the 4-D
-  bool map4d = false;          // map whose box is the K and the V tile of a layer (make_tmap_kv_4d)
+  CUtensorMap map;             // all pool rows x head_dim, box {64, 8}, 128-byte swizzle; or, with map5d, the 5-D
+  bool map5d = false;          // map whose box is 16 keys of K and V of a layer (make_tmap_kv_5d)
 };
 
 struct kc_qweight {
@@ -159,7 +152,7 @@ struct Layer {
 
 // Per-step metadata, packed on the host and copied to the device in one transfer.
 struct MetaLayout {
-  size_t tokens, token_pos, kv_slot, sampled, tables, work, v_row_off, v_draft_off, v_draft_len, v_draft, feed, total;
+  size_t tokens, token_pos, kv_slot, sampled, tables, units, v_row_off, v_draft_off, v_draft_len, v_draft, feed, total;
 };
 
 struct kc_model {
@@ -190,6 +183,8 @@ struct kc_model {
   float* argmax_scratch = nullptr;     // per-CTA bests + counter of the fused reduction / arg-max of a streamed head
   float* partial_gu = nullptr;         // gate_up's fp32 partials while a gated down projection reads them (stream lane on)
   float* attn_ws = nullptr; size_t attn_ws_bytes = 0;
+  CUtensorMap q_map, q_map_small;      // query maps of q_map_ptr [q_map_rows tokens], boxes of q_map_box and ATT_SMALL_TOKENS tokens
+  const void* q_map_ptr = nullptr; int q_map_box = 0, q_map_rows = 0, q_map_gqa = 0;
   float* tp_buf = nullptr;             // fp32 staging for the tensor-parallel all-reduce
   // Tensor-parallel exchange over peer memory (kc_tp_export / kc_tp_attach): the o_proj / down_proj output of exchange e
   // goes to tp_out[e & 1]; tp_flags[r] = the last exchange rank r has published. peer_* = every rank's buffers as
@@ -408,11 +403,11 @@ extern "C" int kc_kv_create(kc_ctx_t c, int32_t layers, int32_t kv_heads, int32_
   if (e != cudaSuccess) { delete kv; return fail(KC_ERR_OOM, "kc_kv_create: %zu bytes: %s", kv->bytes, cudaGetErrorString(e)); }
   e = cudaMemsetAsync(kv->pool, 0, kv->bytes, c->stream);
   const char* terr = "";
-  if (e == cudaSuccess && !getenv("KILN_KV_MAP_2D")) {   // KILN_KV_MAP_2D=1 keeps the 2-D map (4 operations per tile pair)
+  if (e == cudaSuccess && !getenv("KILN_KV_MAP_2D")) {   // KILN_KV_MAP_2D=1 keeps the 2-D map
     const char* e4 = "";
-    kv->map4d = make_tmap_kv_4d(&kv->map, kv->pool, head_dim, (uint64_t)num_blocks * kv_heads * block_size, (uint64_t)layers * 2, &e4);
+    kv->map5d = make_tmap_kv_5d(&kv->map, kv->pool, head_dim, (uint64_t)num_blocks * kv_heads * block_size, (uint64_t)layers * 2, &e4);
   }
-  if (e != cudaSuccess || (!kv->map4d && !make_tmap_bf16_2d(&kv->map, kv->pool, head_dim, rows, 64, 16, &terr))) {
+  if (e != cudaSuccess || (!kv->map5d && !make_tmap_kv_2d(&kv->map, kv->pool, head_dim, rows, &terr))) {
     cudaFree(kv->pool); delete kv;
     return fail(KC_ERR_CUDA, "kc_kv_create: %s", e != cudaSuccess ? cudaGetErrorString(e) : terr);
   }
@@ -1030,10 +1025,46 @@ constexpr int KC_TP_HANDLES = 3;   // per rank: tp_out[0], tp_out[1], tp_flags
 namespace {
 
 struct StepPlan {
-  int n = 0, n_seqs = 0, n_sampled = 0, max_blocks = 0, n_work = 0, tokens_per_item = 1, max_chunks = 1;
+  int n = 0, n_seqs = 0, n_sampled = 0, max_blocks = 0, tokens_per_item = 1, max_chunks = 1;
   int max_len = 1;
+  bool whole = false;              // attention units hold all chunks of their rows
+  std::vector<AttnUnit> units;
   MetaLayout lay{};
 };
+
+// The step's attention units: items of up to tokens_per_item tokens of a sequence, each as one unit over all its chunks,
+// longest first, or as one unit per chunk, whole chunks first.
+void plan_attention(StepPlan* p, const kc_seq_step* seqs, int head_dim, int kv_heads, int sm_count) {
+  std::vector<AttnUnit>& items = p->units;
+  items.clear();
+  int row = 0;
+  for (int i = 0; i < p->n_seqs; ++i) {
+    const kc_seq_step& s = seqs[i];
+    for (int t = 0; t < s.len; t += p->tokens_per_item) {
+      AttnUnit u{};
+      u.seq = i; u.tok0 = row + t; u.ntok = std::min(p->tokens_per_item, s.len - t); u.pos0 = s.offset + t;
+      u.chunk0 = 0; u.chunk1 = (u.pos0 + u.ntok - 1) / ATT_CHUNK + 1;
+      u.small = p->tokens_per_item > ATT_SMALL_TOKENS && u.ntok <= ATT_SMALL_TOKENS ? 1 : 0;
+      items.push_back(u);
+    }
+    row += s.len;
+  }
+  std::stable_sort(items.begin(), items.end(), [](const AttnUnit& a, const AttnUnit& b) { return a.pos0 + a.ntok > b.pos0 + b.ntok; });
+  std::vector<int> tiles(items.size());
+  for (size_t i = 0; i < items.size(); ++i) tiles[i] = (items[i].pos0 + items[i].ntok + 127) / 128;
+  p->whole = attn_whole(head_dim, tiles.data(), (int)items.size(), kv_heads, sm_count);
+  if (p->whole) return;
+  std::vector<AttnUnit> full, rest;
+  for (const AttnUnit& u : items)
+    for (int c = 0; c < u.chunk1; ++c) {
+      AttnUnit v = u;
+      v.chunk0 = c; v.chunk1 = c + 1;
+      (c + 1 < u.chunk1 ? full : rest).push_back(v);
+    }
+  std::stable_sort(rest.begin(), rest.end(), [](const AttnUnit& a, const AttnUnit& b) { return (a.pos0 + a.ntok - 1) % ATT_CHUNK > (b.pos0 + b.ntok - 1) % ATT_CHUNK; });
+  full.insert(full.end(), rest.begin(), rest.end());
+  items.swap(full);
+}
 
 int validate_step(kc_model* m, kc_kv* kv, const uint32_t* token_ids, int32_t n, const kc_seq_step* seqs, int32_t n_seqs,
                   int32_t pad_rows, StepPlan* plan) {
@@ -1072,20 +1103,20 @@ int validate_step(kc_model* m, kc_kv* kv, const uint32_t* token_ids, int32_t n, 
   if (p.n_sampled > m->logit_rows) return fail(KC_ERR_INVALID, "step samples %d rows; at most %d", p.n_sampled, m->logit_rows);
   const int gqa = m->d.num_heads / m->d.num_kv_heads;
   p.tokens_per_item = attn_tokens_per_item(gqa, p.max_len);
-  for (int i = 0; i < n_seqs; ++i) p.n_work += (seqs[i].len + p.tokens_per_item - 1) / p.tokens_per_item;
   p.max_chunks = (max_ctx + ATT_CHUNK - 1) / ATT_CHUNK;
+  plan_attention(&p, seqs, m->d.head_dim, m->Hkv, m->ctx->sm_count);
   MetaLayout& L = p.lay;
   size_t at = 0;
   auto put = [&](size_t bytes) { size_t o = at; at = align_up(at + bytes, 16); return o; };
   L.tokens = put((size_t)n * 4); L.token_pos = put((size_t)n * 4); L.kv_slot = put((size_t)n * 4);
   L.sampled = put((size_t)std::max(1, p.n_sampled) * 4);
   L.tables = put((size_t)n_seqs * p.max_blocks * 4);
-  L.work = put((size_t)p.n_work * 16);
+  L.units = put(p.units.size() * sizeof(AttnUnit));
   L.v_row_off = put((size_t)n_seqs * 4); L.v_draft_off = put((size_t)n_seqs * 4); L.v_draft_len = put((size_t)n_seqs * 4);
   L.v_draft = put((size_t)n * 4);
   L.feed = put((size_t)n * 4);
   L.total = at;
-  *plan = p;
+  *plan = std::move(p);
   return KC_OK;
 }
 
@@ -1114,7 +1145,7 @@ int upload_meta(kc_model* m, kc_kv* kv, const uint32_t* token_ids, const kc_seq_
   int32_t* slotv = reinterpret_cast<int32_t*>(hbuf + L.kv_slot);
   int32_t* sampled = reinterpret_cast<int32_t*>(hbuf + L.sampled);
   int32_t* tables = reinterpret_cast<int32_t*>(hbuf + L.tables);
-  int32_t* work = reinterpret_cast<int32_t*>(hbuf + L.work);
+  memcpy(hbuf + L.units, p.units.data(), p.units.size() * sizeof(AttnUnit));
   int32_t* v_row = reinterpret_cast<int32_t*>(hbuf + L.v_row_off);
   int32_t* v_doff = reinterpret_cast<int32_t*>(hbuf + L.v_draft_off);
   int32_t* v_dlen = reinterpret_cast<int32_t*>(hbuf + L.v_draft_len);
@@ -1122,7 +1153,7 @@ int upload_meta(kc_model* m, kc_kv* kv, const uint32_t* token_ids, const kc_seq_
   memcpy(tokens, token_ids, (size_t)p.n * 4);
   if (feed) memcpy(hbuf + L.feed, feed, (size_t)p.n * 4);
   const int BS = kv->block_size;
-  int row = 0, srow = 0, w = 0, dat = 0;
+  int row = 0, srow = 0, dat = 0;
   for (int i = 0; i < p.n_seqs; ++i) {
     const kc_seq_step& s = seqs[i];
     for (int b = 0; b < p.max_blocks; ++b) tables[(size_t)i * p.max_blocks + b] = b < s.n_blocks ? (int32_t)s.blocks[b] : 0;
@@ -1130,11 +1161,6 @@ int upload_meta(kc_model* m, kc_kv* kv, const uint32_t* token_ids, const kc_seq_
       const int pp = s.offset + t;
       pos[row + t] = pp;
       slotv[row + t] = (int32_t)s.blocks[pp / BS] * BS + pp % BS;   // WriteRun derivation, engine.rs:2757-2769
-    }
-    for (int t = 0; t < s.len; t += p.tokens_per_item) {
-      work[4 * w + 0] = i; work[4 * w + 1] = row + t; work[4 * w + 2] = std::min(p.tokens_per_item, s.len - t);
-      work[4 * w + 3] = s.offset + t;
-      ++w;
     }
     // trailing sample_rows positions (nn.rs:1367-1372)
     v_row[i] = srow; v_doff[i] = dat; v_dlen[i] = s.sample_rows - 1;   // -1: nothing sampled
@@ -1150,6 +1176,7 @@ int upload_meta(kc_model* m, kc_kv* kv, const uint32_t* token_ids, const kc_seq_
 }
 
 int ensure_attn_ws(kc_model* m, const StepPlan& p) {
+  if (p.whole) return KC_OK;   // no partials
   const size_t rows = (size_t)p.n * m->Hq * p.max_chunks;
   const size_t need = rows * m->d.head_dim * 4 + rows * 8 + 256;
   if (need > m->attn_ws_bytes) {
@@ -1171,18 +1198,32 @@ AttnParams attn_params(kc_model* m, kc_kv* kv, const StepPlan& p, int layer, con
   a.part_o = m->attn_ws;
   a.part_ml = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(m->attn_ws) + align_up(rows * m->d.head_dim * 4, 256));
   a.block_tables = reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.tables);
-  a.work = reinterpret_cast<const int4*>(m->meta_dev + p.lay.work);
+  a.units = reinterpret_cast<const AttnUnit*>(m->meta_dev + p.lay.units);
+  a.n_units = (int)p.units.size();
   a.token_pos = reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.token_pos);
   a.status = m->ctx->status;
   a.max_blocks = p.max_blocks;
   a.Hq = Hq; a.Hkv = kv->kv_heads; a.gqa = Hq / kv->kv_heads;
   a.layer = layer; a.NB = kv->num_blocks; a.BS = kv->block_size;
-  a.max_chunks = p.max_chunks; a.chunk_lo_grid = 0;
-  a.single_chunk = p.max_chunks == 1 ? 1 : 0;
+  a.max_chunks = p.max_chunks;
+  a.whole = p.whole ? 1 : 0; a.single = p.max_chunks == 1 ? 1 : 0;
   a.scale = scale; a.softcap = softcap; a.window = window;
-  a.pool = kv->pool;
-  a.kv4d = kv->map4d ? 1 : 0;
+  a.q_tokens = p.tokens_per_item;
+  a.kv5d = kv->map5d ? 1 : 0;
   return a;
+}
+// Kernels one attention call of this plan launches.
+int attn_launches(const StepPlan& p) { return p.whole || p.max_chunks == 1 ? 1 : 2; }
+
+// The query maps of a buffer of `rows` tokens: encoded again only when the buffer or a step's item size changes.
+int ensure_q_maps(kc_model* m, const bf16* q, int rows, int Hq, int gqa, const StepPlan& p) {
+  if (m->q_map_ptr == q && m->q_map_rows == rows && m->q_map_box == p.tokens_per_item && m->q_map_gqa == gqa) return KC_OK;
+  const char* err = "";
+  const int D = m->d.head_dim, small = std::min(p.tokens_per_item, ATT_SMALL_TOKENS);
+  if (!make_tmap_q(&m->q_map, q, rows, Hq, gqa, D, p.tokens_per_item, &err) || !make_tmap_q(&m->q_map_small, q, rows, Hq, gqa, D, small, &err))
+    return fail(KC_ERR_CUDA, "attention queries: %s", err);
+  m->q_map_ptr = q; m->q_map_rows = rows; m->q_map_box = p.tokens_per_item; m->q_map_gqa = gqa;
+  return KC_OK;
 }
 
 // Brings every tensor-parallel rank's bf16 [n, H] sublayer output to every rank: out[r] = rank r's rows. The SUM is
@@ -1250,6 +1291,7 @@ int run_forward(kc_model* m, kc_kv* kv, const uint32_t* tokens_dev, const StepPl
   const int32_t* kv_slot = reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.kv_slot);
   int rc;
   if ((rc = ensure_attn_ws(m, p))) return rc;
+  if ((rc = ensure_q_maps(m, m->q_rot, m->max_rows, m->Hq, m->Hq / m->Hkv, p))) return rc;
   const bool stream = m->stream_lane && n <= QL_STREAM_MAX_M && d.tp_world <= 1;
   // Per weight: the streaming kernel pays for itself from about 24 MB of records on (8B-class layers, every head); below
   // that the launch is latency-bound either way and the consumer would only have more partial pieces to sum. A
@@ -1270,7 +1312,7 @@ int run_forward(kc_model* m, kc_kv* kv, const uint32_t* tokens_dev, const StepPl
                             kv->num_blocks, kv->block_size, kv->pool, m->q_rot, c->stream));
     const int window = (d.sliding_window > 0 && (l % 2 == 0)) ? d.sliding_window : 0;
     AttnParams a = attn_params(m, kv, p, l, m->q_rot, m->attn, m->attn_scale, gemma ? d.attn_logit_softcapping : 0.f, window, m->Hq);
-    LAUNCH(c, KC_PROF_ATTN, a.single_chunk ? 1 : 2, paged_attention(kv->map, a, D, p.tokens_per_item, p.n_work, p.max_chunks, n, c->stream));
+    LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, D, n, c->sm_count, c->stream));
     if (streams(L.o)) RC(run_stream(c, L.o, m->attn, n, m->proj, H, m->partial, &so));
     else if (small(L.o)) RC(run_gemv(c, L.o, m->attn, n, m->proj, H, m->partial, &so));
     else RC(run_qlinear(c, L.o, m->op_attn, n, d.tp_world > 1 ? tp_out_buffer(m) : m->proj, H, m->partial, d.tp_world > 1 ? nullptr : &so));
@@ -1584,6 +1626,7 @@ static int op_shell(kc_ctx* c, kc_kv* kv, int num_heads, int n, int n_seqs, kc_m
   kc_model* m = c->op;
   m->d.num_layers = kv->layers; m->d.head_dim = kv->head_dim; m->d.num_heads = num_heads; m->d.num_kv_heads = kv->kv_heads;
   m->d.vocab_size = 0x7fffffff; m->d.hidden_size = 0; m->d.max_step_tokens = n; m->d.tp_world = 1;
+  m->q_map_ptr = nullptr;   // head counts and head size may differ from the last call's
   m->Hq = num_heads; m->Hkv = kv->kv_heads;
   m->max_rows = n; m->max_seqs = n_seqs; m->logit_rows = n;
   *out = m;
@@ -1622,10 +1665,11 @@ extern "C" int kc_paged_attention(kc_ctx_t c, kc_kv_t kv, int32_t layer, const v
   rc = validate_step(m, kv, ids.data(), n, seqs, n_seqs, 0, &p);
   if (!rc) rc = upload_meta(m, kv, ids.data(), seqs, p);
   if (!rc) rc = ensure_attn_ws(m, p);
+  if (!rc) rc = ensure_q_maps(m, (const bf16*)q_dev, n, num_heads, num_heads / kv->kv_heads, p);
   if (!rc) {
     AttnParams a = attn_params(m, kv, p, layer, (const bf16*)q_dev, (bf16*)out_dev, scale, softcap, window, num_heads);
     rc = [&]() -> int {
-      LAUNCH(c, KC_PROF_ATTN, a.single_chunk ? 1 : 2, paged_attention(kv->map, a, kv->head_dim, p.tokens_per_item, p.n_work, p.max_chunks, n, c->stream));
+      LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, kv->head_dim, n, c->sm_count, c->stream));
       return KC_OK;
     }();
   }

@@ -4,370 +4,502 @@
 // (crates/kiln-engine/src/paged.rs:191-225; crates/kiln-models/src/nn.rs:800-817)
 // and its decode-only Metal kernels (crates/kiln-engine/src/paged_attn.rs:59-303):
 // token i of kv-head h is read at pool[tbl[i / BS], h, i % BS, :] (paged_attn.rs:95-99),
-// never copied. Scores use the reference's algebra — fp32 scores, fp32 online
-// softmax with exp(max - new_max) rescaling, output o / sum (paged_attn.rs:106-153);
-// the causal predicate is bottom-right aligned: query at absolute position p
-// sees keys 0..p. Gemma-2's softcap (nn.rs:527-534) and a sliding window are
+// never copied. Scores use the reference's algebra — fp32 scores, fp32 online softmax
+// (paged_attn.rs:106-153); the causal predicate is bottom-right aligned: query at absolute
+// position p sees keys 0..p. Gemma-2's softcap (nn.rs:527-534) and a sliding window are
 // optional.
 //
-// Partition geometry is a function of absolute key position only: keys are cut
-// into chunks of ATT_CHUNK, a chunk into 16-key tiles, tile t of a chunk belongs
-// to key-split t % KS, splits and chunks are merged in index order. A query
-// row's result therefore does not depend on how many other rows (of its own
-// sequence or of others) share the launch.
+// Both contractions run on tcgen05: S = Q K^T with Q and K in shared memory, O += P V with P in tensor
+// memory (written over S) and V in shared memory. One warp-wide lane = one query row (token x head of
+// the kv head's group), up to 128 rows of one sequence per unit, so K/V bytes cross HBM once per
+// (sequence, kv head, 128 rows).
 //
-// One CTA = (chunk, kv head, work item); a work item is up to MT*16/gqa
-// consecutive tokens of one sequence, so the CTA's MT*16 query rows (token x
-// head-in-group) all read the same K/V tiles: K/V bytes cross HBM once per
-// (sequence, kv head). K/V tiles arrive by TMA (cp.async.bulk.tensor, 128-byte
-// swizzle) through an mbarrier ring; QK^T and PV run on mma.sync m16n8k16.
+// What a row sees is a function of its own position only, so its bits do not depend on how many other rows share the
+// launch: keys are cut into chunks of ATT_CHUNK at absolute positions and a chunk into tiles; a chunk's sums start from
+// nothing, and the chunks of a row are merged one after the other in index order (merge_chunk) — by the kernel itself
+// where a unit holds all chunks of its rows, by the combine kernel where the chunks of an item are units of their own.
+//
+// Roles (12 warps, one CTA per SM, units taken grid-stride so that K/V tiles of the next unit arrive under the last one):
+//   warp 0      TMA: queries of a unit, K/V tiles through a ring
+//   warp 1      issues the MMAs: QK of tile i + 1 before PV of tile i
+//   warps 4-7   softmax, one row per thread: S -> P, rescaling O when a row's maximum moved
+//   warps 8-11  a finished chunk's O: store the partial, or merge it into the row and store the row
 #include "kc_attn.cuh"
 
+#include "kc_umma.cuh"
+
 #include <algorithm>
+#include <vector>
 
 namespace kc {
 
 namespace {
 
-// A multiple of every key-split count, so one ring slot is always drained by the same
-// consumer warps and each warp meets a slot's barrier phases strictly in order.
-constexpr int ATT_STAGES = 8;
-constexpr int ATT_MINB = 3;   // CTAs per SM the compiler must leave room for (head_dim <= 128, at most 32 query rows)
-
-__device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
-}
-__device__ __forceinline__ void mma16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void named_bar_sync(int id, int threads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
-}
-
-// Key-splits per chunk. A constant (never a function of how many query rows the CTA
-// holds): the split a key tile belongs to, and so the merge order a row sees, must be the
-// same in a one-token decode launch and in a verify launch.
-template <int MT> struct KeySplit { static constexpr int value = 2; };
-static_assert(KeySplit<1>::value > 1, "the partial kernel finishes single-chunk rows in its key-split merge");
-
-// Shared memory: [stages][K tile | V tile] (1024-aligned, swizzled by TMA),
-// then the Q rows (padded), then barriers. The K/V ring is reused for the
-// cross-split merge after the main loop.
-template <int D, int MT>
-struct AttnSmem {
-  static constexpr int KS = KeySplit<MT>::value;
-  static constexpr int CW = MT * KS;                 // consumer warps
-  static constexpr int TILE_BYTES = 16 * D * 2;      // one K (or V) tile
-  static constexpr int STAGE_BYTES = 2 * TILE_BYTES;
-  static constexpr int Q_LD = D * 2 + 16;            // bytes per Q row incl. pad
-  static constexpr int Q_BYTES = MT * 16 * Q_LD;
-  static constexpr int RING = ATT_STAGES * STAGE_BYTES;
-  static constexpr int MERGE = KS > 1 ? KS * MT * 16 * (D + 4) * 4 : 0;
-  static constexpr int RING_BYTES = RING > MERGE ? RING : MERGE;
-  static constexpr int TOTAL = 1024 + RING_BYTES + Q_BYTES + 2 * ATT_STAGES * 8 + 64;
+constexpr int ATT_THREADS = 12 * 32;
+template <int D>
+struct AttnShape {
+  static constexpr int TK = D == 256 ? 64 : 128;      // keys per tile
+  static constexpr int SLABS = D / 64;
+  static constexpr int GROUP_BYTES = 2 * SLABS * 1024; // 8 keys: K slabs, then V slabs, [8][128 B] each
+  static constexpr int TILE_BYTES = TK / 8 * GROUP_BYTES;
+  static constexpr int RING = D == 64 ? 6 : D == 128 ? 3 : 2;
+  static constexpr int Q_BYTES = SLABS * ATT_ROWS * 128;
+  static constexpr int O_BUFS = D == 256 ? 1 : 2;
+  static constexpr int TMEM_O = 256;                   // columns: S0 at 0, S1 at TK, O from 256
+  static constexpr int TMEM_COLS = 512;
+  static constexpr int TILES_PER_CHUNK = ATT_CHUNK / TK;
+  static constexpr int SMEM = RING * TILE_BYTES + Q_BYTES + 2 * ATT_ROWS * 8 + 32 * 8;
+  static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
 };
 
-template <int D, int MT>
-__global__ void __launch_bounds__((MT * KeySplit<MT>::value + 1) * 32, (D <= 128 && MT <= 2) ? ATT_MINB : 1)
-attn_partial_kernel(const __grid_constant__ CUtensorMap kvmap, const AttnParams p) {
-  using S = AttnSmem<D, MT>;
-  constexpr int KS = S::KS;
-  constexpr int CW = S::CW;
-  constexpr int NT_D = D / 8;   // PV n-tiles
-  constexpr int KSTEPS = D / 16;
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 
+// Adds a chunk (o scaled by 2^-m, sum l) to what a row has accumulated: the weights of one merge.
+struct MergeW { float a, b, m; };
+__device__ __forceinline__ MergeW merge_weights(float m_acc, float m_chunk) {
+  MergeW w;
+  w.m = fmaxf(m_acc, m_chunk);
+  w.a = m_acc == -INFINITY ? 0.f : ex2(m_acc - w.m);
+  w.b = m_chunk == -INFINITY ? 0.f : ex2(m_chunk - w.m);
+  return w;
+}
+__device__ __forceinline__ float merge_value(float acc, float v, const MergeW& w) { return __fmaf_rn(v, w.b, __fmul_rn(acc, w.a)); }
+__device__ __forceinline__ float row_scale(float l) { return l == 0.f ? 1.f : __frcp_rn(l); }
+
+// The tiles of one unit in order, as every role walks them.
+struct UnitTiles {
+  int seq, tok0, ntok, pos0, small, rows, pos_max, wlo;
+  int c, c1, t, t1, keys;       // chunk, end of chunks, tile, end of tiles of the chunk, keys of the chunk
+  __device__ __forceinline__ void open(const AttnParams& p, int unit, int tk) {
+    const int4 a = *reinterpret_cast<const int4*>(&p.units[unit]);
+    const int4 b = *(reinterpret_cast<const int4*>(&p.units[unit]) + 1);
+    seq = a.x; tok0 = a.y; ntok = a.z; pos0 = a.w;
+    c = b.x; c1 = b.y; small = b.z;
+    rows = ntok * p.gqa;
+    pos_max = pos0 + ntok - 1;
+    wlo = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;    // first key that any row of the unit sees
+    c = max(c, wlo / ATT_CHUNK);
+    chunk(tk);
+  }
+  __device__ __forceinline__ void chunk(int tk) {
+    keys = min(ATT_CHUNK, pos_max + 1 - c * ATT_CHUNK);
+    t = max(0, wlo - c * ATT_CHUNK) / tk;
+    t1 = (keys + tk - 1) / tk;
+  }
+  __device__ __forceinline__ bool live() const { return c < c1; }
+  __device__ __forceinline__ bool last() const { return t == t1 - 1; }
+  __device__ __forceinline__ int first_tile(int tk) const { return max(0, wlo - c * ATT_CHUNK) / tk; }
+  __device__ __forceinline__ int key0(int tk) const { return c * ATT_CHUNK + t * tk; }
+  // 16-key blocks of the tile that hold a key of the sequence
+  __device__ __forceinline__ int blocks(int tk) const { return (min(tk, keys - t * tk) + 15) >> 4; }
+  __device__ __forceinline__ void next(int tk) {
+    if (++t == t1) { if (++c < c1) chunk(tk); }
+  }
+};
+
+// The r-th unit of a CTA: forth and back over the CTAs, so that with units in falling order of length every CTA gets about
+// the same number of tiles (attn_whole counts them the same way). -1: no more.
+__host__ __device__ __forceinline__ int unit_index(int r, int cta, int ctas, int total) {
+  const int i = r * ctas + ((r & 1) ? ctas - 1 - cta : cta);
+  return i < total ? i : -1;
+}
+
+template <int D, bool WHOLE>
+__global__ void __launch_bounds__(ATT_THREADS, 1)
+attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ CUtensorMap qmap,
+            const __grid_constant__ CUtensorMap qmap_small, const AttnParams p) {
+  using S = AttnShape<D>;
+  constexpr int TK = S::TK;
+  extern __shared__ __align__(1024) uint8_t ring[];   // no static shared memory: the dynamic part starts on its boundary
+  uint8_t* sQ = ring + S::RING * S::TILE_BYTES;
+  float2* stat = reinterpret_cast<float2*>(sQ + S::Q_BYTES);          // [2][ATT_ROWS] (m, l) of a finished chunk
+  uint64_t* bars = reinterpret_cast<uint64_t*>(stat + 2 * ATT_ROWS);
+  uint64_t* kv_full = bars;
+  uint64_t* kv_empty = kv_full + S::RING;
+  uint64_t* q_full = kv_empty + S::RING;
+  uint64_t* q_empty = q_full + 1;
+  uint64_t* s_ready = q_empty + 1;      // [2] scores of a tile are in S[tile & 1]
+  uint64_t* p_ready = s_ready + 2;      // [2] its probabilities are
+  uint64_t* pv_done = p_ready + 2;      // [2] they have been multiplied
+  uint64_t* stat_full = pv_done + 2;    // [2] (m, l) of a chunk; with the last PV of the chunk its O is complete
+  uint64_t* o_full = stat_full + 2;
+  uint64_t* o_empty = o_full + 2;       // [2] O and (m, l) have been read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_empty + 2);
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   pdl_launch_dependents();
-  pdl_wait();   // everything below reads step data (work items, q, block tables, this layer's K/V rows)
-  const int chunk = p.chunk_lo_grid + blockIdx.x;
-  const int kvh = blockIdx.y;
-  const int4 wk = p.work[blockIdx.z];   // {seq, first token row in the step, tokens, position of first token}
-  const int seq = wk.x, tok0 = wk.y, qlen = wk.z, pos0 = wk.w;
-  const int pos_max = pos0 + qlen - 1;
-  const int c_hi = pos_max / ATT_CHUNK;
-  int c_lo = 0;
-  if (p.window > 0) c_lo = max(0, pos0 - p.window + 1) / ATT_CHUNK;
-  if (chunk > c_hi || chunk < c_lo) return;
-
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* ring = smem;
-  uint8_t* sQ = ring + S::RING_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(sQ + S::Q_BYTES);
-  uint64_t* empty = full + ATT_STAGES;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int gqa = p.gqa;
-  const int rows = qlen * gqa;                 // live query rows of this CTA
-  const int key_base = chunk * ATT_CHUNK;
-  const int keys_here = min(ATT_CHUNK, pos_max + 1 - key_base);
-  const int ntiles = (keys_here + 15) >> 4;
-
   if (threadIdx.x == 0) {
-    for (int i = 0; i < ATT_STAGES; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], MT); }
+    for (int i = 0; i < S::RING; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
+    mbar_init(q_full, 1); mbar_init(q_empty, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s_ready[i], 1); mbar_init(&p_ready[i], 4); mbar_init(&pv_done[i], 1);
+      mbar_init(&stat_full[i], 4); mbar_init(&o_full[i], 1); mbar_init(&o_empty[i], 4);
+    }
     mbar_fence_init();
   }
-  __syncthreads();
-  // The producer starts on the K/V tiles at once; the consumer warps stage Q meanwhile (its load latency then hides
-  // under that of the first tiles). Row r = token (r / gqa), head-in-group (r % gqa); dead rows are zero.
-  if (warp < CW) {
-    const int chunks_per_row = D / 8;
-    for (int i = threadIdx.x; i < MT * 16 * chunks_per_row; i += CW * 32) {
-      const int r = i / chunks_per_row, ch = i % chunks_per_row;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (r < rows) {
-        const int t = r / gqa, hg = r % gqa;
-        v = *reinterpret_cast<const uint4*>(p.q + ((size_t)(tok0 + t) * p.Hq + kvh * gqa + hg) * D + ch * 8);
-      }
-      *reinterpret_cast<uint4*>(sQ + r * S::Q_LD + ch * 16) = v;
-    }
-    named_bar_sync(1, CW * 32);
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(S::TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  if (warp == 0 && lane == 0) { tma_prefetch_desc(&kvmap); tma_prefetch_desc(&qmap); tma_prefetch_desc(&qmap_small); }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  pdl_wait();   // everything below reads step data (units, q, block tables, this layer's K/V rows)
 
-  if (warp == CW) {
-    // ---- producer: one TMA per K+V tile pair (4-D map), or one per 64-feature slab of a K or V tile (2-D map). The chunk's block-table entries (at most
-    //      ATT_CHUNK / 16 = 32) are fetched once, one per lane, so the per-tile loop has no global load in it ----
-    if (lane == 0) tma_prefetch_desc(&kvmap);
-    const int32_t* tbl = p.block_tables + (size_t)seq * p.max_blocks;
-    const int blk0 = key_base / p.BS;
-    const int nblk = (keys_here + p.BS - 1) / p.BS;
-    const int my_blk = lane < nblk ? tbl[blk0 + lane] : 0;   // block_size is a power of two >= 16: chunks start on block edges
-    bool alive = true;                                        // lane 0 only: false after a bounded wait gave up
-    for (int t = 0; t < ntiles; ++t) {
-      const int st = t & (ATT_STAGES - 1); const uint32_t ph = (t / ATT_STAGES) & 1;   // ATT_STAGES is a power of two
-      const int koff = t * 16;
-      const int blk = __shfl_sync(0xffffffffu, my_blk, koff / p.BS);
-      if (lane == 0 && alive) {
-        alive = mbar_wait(&empty[st], ph ^ 1, p.status, KC_DEV_ATTN | 1);
-        if (!alive) continue;
-        const int in_blk = (key_base + koff) % p.BS;
-        const long long rowK = ((((long long)p.layer * 2 + 0) * p.NB + blk) * p.Hkv + kvh) * p.BS + in_blk;
-        const long long rowV = ((((long long)p.layer * 2 + 1) * p.NB + blk) * p.Hkv + kvh) * p.BS + in_blk;
-        mbar_arrive_expect_tx(&full[st], S::STAGE_BYTES);
-        uint8_t* dst = ring + (size_t)st * S::STAGE_BYTES;
-        if (p.kv4d) {
-          // one operation: K slabs then V slabs, the layout of the loads below
-          tma_load_4d(dst, &kvmap, 0, (blk * p.Hkv + kvh) * p.BS + in_blk, 0, p.layer * 2, &full[st]);
-        } else {
-#pragma unroll
-          for (int h = 0; h < D / 64; ++h) {
-            tma_load_2d(dst + h * 2048, &kvmap, h * 64, (int)rowK, &full[st]);
-            tma_load_2d(dst + S::TILE_BYTES + h * 2048, &kvmap, h * 64, (int)rowV, &full[st]);
+  const int total = p.n_units * p.Hkv;
+  if (warp == 0) {
+    // ---- TMA producer. A chunk's block-table entries (at most ATT_CHUNK / 16 = 32) are fetched once, one per lane ----
+    RingPos kv;
+    uint32_t qphase = 0;
+    bool ok = true;
+    for (int r = 0, w; ok && r * (int)gridDim.x < total; ++r) {
+      if ((w = unit_index(r, blockIdx.x, gridDim.x, total)) < 0) break;
+      UnitTiles u;
+      const int kvh = w % p.Hkv;
+      u.open(p, w / p.Hkv, TK);
+      if (!u.live()) continue;
+      ok = warp_wait(q_empty, qphase ^ 1, p.status, KC_DEV_ATTN | 1);
+      if (!ok) break;
+      qphase ^= 1;
+      if (lane == 0) {
+        const int tokens = u.small ? ATT_SMALL_TOKENS : p.q_tokens;
+        mbar_arrive_expect_tx(q_full, S::SLABS * tokens * p.gqa * 128);
+        for (int s = 0; s < S::SLABS; ++s)
+          tma_load_5d(sQ + s * ATT_ROWS * 128, u.small ? &qmap_small : &qmap, 0, 0, s, kvh, u.tok0, q_full);
+      }
+      const int32_t* tbl = p.block_tables + (size_t)u.seq * p.max_blocks;
+      int loaded_c = -1, my_blk = 0;
+      for (; u.live() && ok; u.next(TK)) {
+        if (u.c != loaded_c) {
+          loaded_c = u.c;
+          const int nblk = (u.keys + p.BS - 1) / p.BS;
+          my_blk = lane < nblk ? tbl[u.c * (ATT_CHUNK / p.BS) + lane] : 0;   // block_size is a power of two >= 16: chunks start on block edges
+        }
+        const int nb = u.blocks(TK);
+        ok = warp_wait(&kv_empty[kv.stage], kv.phase ^ 1, p.status, KC_DEV_ATTN | 2);
+        if (!ok) break;
+        if (lane == 0) mbar_arrive_expect_tx(&kv_full[kv.stage], nb * 2 * S::GROUP_BYTES);
+        uint8_t* dst = ring + (size_t)kv.stage * S::TILE_BYTES;
+        for (int b = 0; b < nb; ++b) {
+          const int koff = u.t * TK + b * 16;
+          const int blk = __shfl_sync(0xffffffffu, my_blk, koff / p.BS);
+          const int row = (blk * p.Hkv + kvh) * p.BS + koff % p.BS;   // of a plane
+          if (lane == 0) {
+            if (p.kv5d) {
+              tma_load_5d(dst + b * 2 * S::GROUP_BYTES, &kvmap, 0, 0, 0, p.layer * 2, row >> 3, &kv_full[kv.stage]);
+            } else {
+              for (int g = 0; g < 2; ++g)
+                for (int pl = 0; pl < 2; ++pl)
+                  for (int s = 0; s < S::SLABS; ++s)
+                    tma_load_2d(dst + (b * 2 + g) * S::GROUP_BYTES + (pl * S::SLABS + s) * 1024, &kvmap, s * 64,
+                                (int)((long long)(p.layer * 2 + pl) * p.NB * p.Hkv * p.BS) + row + g * 8, &kv_full[kv.stage]);
+            }
           }
         }
+        __syncwarp();
+        kv.advance(S::RING);
       }
     }
-    __syncwarp();
-  } else {
-    // ---- consumers: warp (mt, ks) owns query rows 16*mt.. and tiles t % KS == ks ----
-    const int mt = warp / KS, ks = warp % KS;
-    const int g = lane >> 2, tq = lane & 3;
-    const int r_lo = mt * 16 + g, r_hi = r_lo + 8;
-    // Absolute position of each of this thread's two rows; -1 = dead row.
-    const int p_lo = r_lo < rows ? pos0 + r_lo / gqa : -1;
-    const int p_hi = r_hi < rows ? pos0 + r_hi / gqa : -1;
-    const int w_lo = (p.window > 0 && p_lo >= 0) ? p_lo - p.window : -1;  // keys <= w are outside the window
-    const int w_hi = (p.window > 0 && p_hi >= 0) ? p_hi - p.window : -1;
-
-    float o[NT_D][4];
-#pragma unroll
-    for (int i = 0; i < NT_D; ++i) { o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f; }
-    float m_lo = -INFINITY, m_hi = -INFINITY, l_lo = 0.f, l_hi = 0.f;
-
-    const uint32_t q_base = smem_u32(sQ) + (mt * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * S::Q_LD + (lane >> 4) * 16;
+  } else if (warp == 1) {
+    // ---- MMA issuer: converged, one elected lane around the MMAs ----
+    const uint64_t qd = umma_smem_desc(smem_u32(sQ), 1024);
+    const uint64_t kd = umma_smem_desc(smem_u32(ring), S::GROUP_BYTES);
+    const uint64_t vd = umma_smem_desc(smem_u32(ring) + S::SLABS * 1024, S::GROUP_BYTES, 1024);
+    const uint32_t q_hi = (uint32_t)(qd >> 32), k_hi = (uint32_t)(kd >> 32), v_hi = (uint32_t)(vd >> 32);
+    const uint32_t idesc_pv = umma_idesc_bf16(ATT_ROWS, D, true);
+    RingPos kv;
+    int tile = 0;                 // tiles issued by this CTA so far (S buffer = tile & 1)
+    int chunks = 0;               // chunks begun (O buffer)
+    uint32_t qphase = 0;
     bool ok = true;
-    for (int t = ks; t < ntiles; t += KS) {
-      const int st = t & (ATT_STAGES - 1); const uint32_t ph = (t / ATT_STAGES) & 1;
-      ok = __all_sync(0xffffffffu, mbar_wait(&full[st], ph, p.status, KC_DEV_ATTN | 2));
-      if (!ok) break;
-      const uint32_t kt = smem_u32(ring + (size_t)st * S::STAGE_BYTES);
-      const uint32_t vt = kt + S::TILE_BYTES;
-
-      // S = Q K^T for 16 rows x 16 keys
-      float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-#pragma unroll
-      for (int kk = 0; kk < KSTEPS; ++kk) {
-        uint32_t a[4], b[4];
-        ldsm_x4(a, q_base + kk * 32);
-        {
-          const int mi = lane >> 3;
-          const int key = (mi >> 1) * 8 + (lane & 7);
-          const int c = (kk & 3) * 2 + (mi & 1);
-          ldsm_x4(b, kt + (kk >> 2) * 2048 + key * 128 + ((c ^ (key & 7)) << 4));
-        }
-        mma16816(s[0], a, b[0], b[1]);
-        mma16816(s[1], a, b[2], b[3]);
+    // the tile whose PV is still to be issued
+    bool pend = false, pend_first = false, pend_last = false;
+    int pend_nb = 0, pend_stage = 0, pend_tile = 0, pend_chunk = 0;
+    auto issue_pv = [&]() {
+      const int sb = pend_tile & 1, ob = S::O_BUFS == 2 ? pend_chunk & 1 : 0;
+      if (pend_first) {
+        // the O buffer's previous chunk has been read
+        const int use = S::O_BUFS == 2 ? pend_chunk >> 1 : pend_chunk;
+        ok = ok && warp_wait(&o_empty[ob], (use & 1) ^ 1, p.status, KC_DEV_ATTN | 3);
       }
-
-      // scale, softcap, mask -> log2-domain scores
-      const int key0 = key_base + t * 16;
-      float tmax_lo = -INFINITY, tmax_hi = -INFINITY;
-      bool v[2][4];
-      // Every key of the tile is visible to every live row (the rows' positions start at pos0), no window, no softcap:
-      // the same arithmetic without the per-element predicates. Dead rows then carry finite garbage nobody stores.
-      if (p.window == 0 && p.softcap == 0.f && key0 + 15 <= pos0) {
-#pragma unroll
-        for (int nt = 0; nt < 2; ++nt) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            float x = s[nt][j] * p.scale;
-            x *= 1.4426950408889634f;
-            v[nt][j] = true;
-            s[nt][j] = x;
-            if (j >= 2) tmax_hi = fmaxf(tmax_hi, x); else tmax_lo = fmaxf(tmax_lo, x);
-          }
-        }
-      } else
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int key = key0 + nt * 8 + 2 * tq + (j & 1);
-          const bool hi = j >= 2;
-          const int lim = hi ? p_hi : p_lo;
-          const int wlim = hi ? w_hi : w_lo;
-          float x = s[nt][j] * p.scale;
-          if (p.softcap > 0.f) x = p.softcap * tanhf(x / p.softcap);
-          x *= 1.4426950408889634f;
-          const bool valid = key <= lim && key > wlim;
-          v[nt][j] = valid;
-          s[nt][j] = x;
-          if (valid) { if (hi) tmax_hi = fmaxf(tmax_hi, x); else tmax_lo = fmaxf(tmax_lo, x); }
-        }
-      }
-      tmax_lo = fmaxf(tmax_lo, __shfl_xor_sync(0xffffffffu, tmax_lo, 1));
-      tmax_lo = fmaxf(tmax_lo, __shfl_xor_sync(0xffffffffu, tmax_lo, 2));
-      tmax_hi = fmaxf(tmax_hi, __shfl_xor_sync(0xffffffffu, tmax_hi, 1));
-      tmax_hi = fmaxf(tmax_hi, __shfl_xor_sync(0xffffffffu, tmax_hi, 2));
-      const float mn_lo = fmaxf(m_lo, tmax_lo), mn_hi = fmaxf(m_hi, tmax_hi);
-      const float al_lo = (mn_lo == -INFINITY) ? 1.f : exp2f(m_lo - mn_lo);
-      const float al_hi = (mn_hi == -INFINITY) ? 1.f : exp2f(m_hi - mn_hi);
-      m_lo = mn_lo; m_hi = mn_hi;
-      float ps_lo = 0.f, ps_hi = 0.f;
-#pragma unroll
-      for (int nt = 0; nt < 2; ++nt) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const bool hi = j >= 2;
-          const float pv = v[nt][j] ? exp2f(s[nt][j] - (hi ? mn_hi : mn_lo)) : 0.f;
-          s[nt][j] = pv;
-          if (hi) ps_hi += pv; else ps_lo += pv;
-        }
-      }
-      l_lo = l_lo * al_lo + ps_lo;
-      l_hi = l_hi * al_hi + ps_hi;
-      uint32_t pa[4];
-      pa[0] = pack_bf162(s[0][0], s[0][1]);
-      pa[1] = pack_bf162(s[0][2], s[0][3]);
-      pa[2] = pack_bf162(s[1][0], s[1][1]);
-      pa[3] = pack_bf162(s[1][2], s[1][3]);
-
-      // O = O * alpha + P V. Multiplying by exactly 1 changes no bit, so the rescale is skipped when no row of
-      // the warp moved its maximum (the common case once the running maximum has settled).
-      if (!__all_sync(0xffffffffu, al_lo == 1.f && al_hi == 1.f)) {
-#pragma unroll
-        for (int dn = 0; dn < NT_D; ++dn) { o[dn][0] *= al_lo; o[dn][1] *= al_lo; o[dn][2] *= al_hi; o[dn][3] *= al_hi; }
-      }
-#pragma unroll
-      for (int dn = 0; dn < NT_D; dn += 2) {
-        uint32_t b[4];
-        const int mi = lane >> 3;
-        const int key = (mi & 1) * 8 + (lane & 7);
-        const int cg = dn + (mi >> 1);         // 8-feature chunk index over D
-        const int c = cg & 7;
-        ldsm_x4_t(b, vt + (cg >> 3) * 2048 + key * 128 + ((c ^ (key & 7)) << 4));
-        mma16816(o[dn], pa, b[0], b[1]);
-        mma16816(o[dn + 1], pa, b[2], b[3]);
+      ok = ok && warp_wait(&p_ready[sb], (pend_tile >> 1) & 1, p.status, KC_DEV_ATTN | 4);
+      if (!ok) return;
+      tc_fence_after();
+      const uint32_t v_lo = (uint32_t)vd + pend_stage * (S::TILE_BYTES >> 4);
+      const uint32_t o = tmem + S::TMEM_O + ob * D, a = tmem + sb * TK;
+      if (elect_one()) {
+        for (int b = 0; b < pend_nb; ++b)
+          umma_bf16_ts(o, a + b * 8, v_lo + b * (2 * S::GROUP_BYTES >> 4), v_hi, idesc_pv, pend_first && b == 0 ? 0u : 1u);
+        umma_commit(&pv_done[sb]);
+        umma_commit(&kv_empty[pend_stage]);
+        if (pend_last) umma_commit(&o_full[ob]);
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[st]);
-    }
-
-    // Row sums live spread over the quad.
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 1);
-    l_lo += __shfl_xor_sync(0xffffffffu, l_lo, 2);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 1);
-    l_hi += __shfl_xor_sync(0xffffffffu, l_hi, 2);
-
-    if (KS > 1) {
-      // Merge the key-splits of each row group in split order through shared memory.
-      named_bar_sync(1, CW * 32);   // every consumer is done with the K/V ring
-      float* mg = reinterpret_cast<float*>(ring);
-      constexpr int RS = D + 4;     // floats per row record: o[D], m, l, pad (keeps rows 16-byte aligned)
-      float* rec_lo = mg + ((size_t)(ks * MT * 16) + r_lo) * RS;
-      float* rec_hi = mg + ((size_t)(ks * MT * 16) + r_hi) * RS;
-#pragma unroll
-      for (int dn = 0; dn < NT_D; ++dn) {
-        *reinterpret_cast<float2*>(rec_lo + dn * 8 + 2 * tq) = make_float2(o[dn][0], o[dn][1]);
-        *reinterpret_cast<float2*>(rec_hi + dn * 8 + 2 * tq) = make_float2(o[dn][2], o[dn][3]);
-      }
-      if (tq == 0) { rec_lo[D] = m_lo; rec_lo[D + 1] = l_lo; rec_hi[D] = m_hi; rec_hi[D + 1] = l_hi; }
-      named_bar_sync(1, CW * 32);
-      if (ks == 0 && ok) {
-        // warp (mt, 0) merges rows 16*mt..16*mt+15: two lanes per row, half of D each.
-        const int r = mt * 16 + (lane >> 1);
-        if (r < rows) {
-          float mmax = -INFINITY;
-          for (int k = 0; k < KS; ++k) mmax = fmaxf(mmax, mg[((size_t)(k * MT * 16) + r) * RS + D]);
-          float wgt[KS]; float lsum = 0.f;
-          for (int k = 0; k < KS; ++k) {
-            const float mk = mg[((size_t)(k * MT * 16) + r) * RS + D];
-            wgt[k] = (mk == -INFINITY) ? 0.f : exp2f(mk - mmax);
-            lsum += wgt[k] * mg[((size_t)(k * MT * 16) + r) * RS + D + 1];
-          }
-          const int t = r / gqa, hg = r % gqa;
-          const size_t prow = ((size_t)(tok0 + t) * p.Hq + kvh * gqa + hg) * p.max_chunks + chunk;
-          float* po = p.part_o + prow * D;
-          // When no sequence of the step reaches past the first chunk, the chunk merge is the identity (weight
-          // exp2(m - m) = 1) followed by the division: the row is finished here, with the arithmetic the combine
-          // kernel would have applied to it, and that launch is skipped.
-          bf16* fo = p.out + prow * D;   // max_chunks == 1 and chunk == 0 then: prow is the output row
-          const int d0 = (lane & 1) * (D / 2);
-          for (int d = d0; d < d0 + D / 2; d += 4) {
-            float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int k = 0; k < KS; ++k) {
-              const float4 x = *reinterpret_cast<const float4*>(mg + ((size_t)(k * MT * 16) + r) * RS + d);
-              acc.x += wgt[k] * x.x; acc.y += wgt[k] * x.y; acc.z += wgt[k] * x.z; acc.w += wgt[k] * x.w;
-            }
-            if (p.single_chunk) {
-              // 0 + x: what the combine kernel's accumulation from zero yields (a -0 becomes +0 there too)
-              acc.x = 0.f + acc.x; acc.y = 0.f + acc.y; acc.z = 0.f + acc.z; acc.w = 0.f + acc.w;
-              if (lsum != 0.f) { acc.x = acc.x / lsum; acc.y = acc.y / lsum; acc.z = acc.z / lsum; acc.w = acc.w / lsum; }
-              *reinterpret_cast<uint2*>(fo + d) = make_uint2(pack_bf162(acc.x, acc.y), pack_bf162(acc.z, acc.w));
-            } else {
-              *reinterpret_cast<float4*>(po + d) = acc;
-            }
-          }
-          if ((lane & 1) == 0 && !p.single_chunk) p.part_ml[prow] = make_float2(mmax, lsum);
+      pend = false;
+    };
+    for (int r = 0, w; ok && r * (int)gridDim.x < total; ++r) {
+      if ((w = unit_index(r, blockIdx.x, gridDim.x, total)) < 0) break;
+      UnitTiles u;
+      u.open(p, w / p.Hkv, TK);
+      if (!u.live()) continue;
+      bool first_of_unit = true;
+      for (; u.live() && ok;) {
+        // QK of this tile goes ahead of the pending PV when its operands are there; else the PV is issued first
+        bool ready = mbar_test_wait(&kv_full[kv.stage], kv.phase) && (!first_of_unit || mbar_test_wait(q_full, qphase));
+        ready = __all_sync(0xffffffffu, ready);
+        if (!ready && pend) { issue_pv(); if (!ok) break; }
+        if (first_of_unit) {
+          ok = warp_wait(q_full, qphase, p.status, KC_DEV_ATTN | 5);
+          if (!ok) break;
+          qphase ^= 1;
         }
-      }
-    } else if (ok) {
-      const int rr[2] = {r_lo, r_hi};
+        ok = warp_wait(&kv_full[kv.stage], kv.phase, p.status, KC_DEV_ATTN | 6);
+        if (!ok) break;
+        first_of_unit = false;
+        tc_fence_after();
+        const int nb = u.blocks(TK), sb = tile & 1;
+        const bool first = u.t == u.first_tile(TK), last = u.last();
+        const uint32_t k_lo = (uint32_t)kd + kv.stage * (S::TILE_BYTES >> 4);
+        const uint32_t idesc = umma_idesc_bf16(ATT_ROWS, nb * 16);
+        const int stage = kv.stage;
+        const int chunk = chunks;
+        if (last) ++chunks;
+        u.next(TK);
+        const bool unit_done = !u.live();
+        if (elect_one()) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = rr[h];
-        if (r < rows) {
-          const int t = r / gqa, hg = r % gqa;
-          const size_t prow = ((size_t)(tok0 + t) * p.Hq + kvh * gqa + hg) * p.max_chunks + chunk;
-          float* po = p.part_o + prow * D;
-#pragma unroll
-          for (int dn = 0; dn < NT_D; ++dn)
-            *reinterpret_cast<float2*>(po + dn * 8 + 2 * tq) = make_float2(o[dn][2 * h], o[dn][2 * h + 1]);
-          if (tq == 0) p.part_ml[prow] = make_float2(h ? m_hi : m_lo, h ? l_hi : l_lo);
+          for (int ks = 0; ks < D / 16; ++ks)
+            umma_bf16_ss(tmem + sb * TK, (uint32_t)qd + (ks >> 2) * (ATT_ROWS * 128 >> 4) + (ks & 3) * 2, q_hi,
+                         k_lo + (ks >> 2) * (1024 >> 4) + (ks & 3) * 2, k_hi, idesc, ks == 0 ? 0u : 1u);
+          umma_commit(&s_ready[sb]);
+          if (unit_done) umma_commit(q_empty);
         }
+        __syncwarp();
+        if (pend) issue_pv();
+        pend = true; pend_first = first; pend_last = last; pend_nb = nb; pend_stage = stage; pend_tile = tile; pend_chunk = chunk;
+        ++tile;
+        kv.advance(S::RING);
       }
     }
+    if (ok && pend) issue_pv();
+  } else if (warp >= 4 && warp < 8) {
+    // ---- softmax: thread = query row 32 * (warp & 3) + lane ----
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    const float scale_log2 = p.scale * 1.4426950408889634f;
+    const float cap2 = p.softcap > 0.f ? 2.f * 1.4426950408889634f * p.scale / p.softcap : 0.f;   // exp2 argument of e^(2 x / cap)
+    const float cap_log2 = p.softcap * 1.4426950408889634f;
+    int tile = 0, chunks = 0;
+    bool ok = true;
+    for (int r = 0, w; ok && r * (int)gridDim.x < total; ++r) {
+      if ((w = unit_index(r, blockIdx.x, gridDim.x, total)) < 0) break;
+      UnitTiles u;
+      u.open(p, w / p.Hkv, TK);
+      if (!u.live()) continue;
+      const bool warp_live = quarter * 32 < u.rows;
+      const int pos = u.pos0 + min(row / p.gqa, u.ntok - 1);      // dead rows of a live warp compute the last token's row
+      const int w_excl = p.window > 0 ? pos - p.window : -1;       // keys <= this are outside the window
+      float m = -INFINITY, l = 0.f;
+      for (; u.live() && ok; u.next(TK), ++tile) {
+        const int sb = tile & 1;
+        const bool first = u.t == u.first_tile(TK), last = u.last();
+        ok = warp_wait(&s_ready[sb], (tile >> 1) & 1, p.status, KC_DEV_ATTN | 7);
+        if (!ok) break;
+        if (first) { m = -INFINITY; l = 0.f; }
+        if (warp_live) {
+          tc_fence_after();
+          const uint32_t s_addr = tmem + lane_addr + sb * TK;
+          const int nb = u.blocks(TK), key0 = u.key0(TK);
+          uint32_t v[TK];
+#pragma unroll
+          for (int c = 0; c < TK / 32; ++c) tmem_ld32_issue(s_addr + c * 32, v + c * 32);   // columns past 16 nb hold an older tile's scores: masked below
+          tmem_wait_ld();
+          const bool capped = p.softcap > 0.f;
+          if (capped) {
+            // cap * tanh(x / cap) in log2 units: cap * (1 - 2 / (e^(2 x / cap) + 1)), accurate to about 1e-7 of cap
+#pragma unroll
+            for (int j = 0; j < TK; ++j) {
+              const float e = ex2(fminf(__uint_as_float(v[j]) * cap2, 120.f));
+              v[j] = __float_as_uint(cap_log2 - 2.f * cap_log2 * rcp_approx(e + 1.f));
+            }
+          }
+          const float mul = capped ? 1.f : scale_log2;
+          // every key of the tile is visible to every row of the unit: the same arithmetic without the predicates
+          if (!(nb * 16 == TK && key0 + TK - 1 <= u.pos0 && (p.window == 0 || key0 > u.pos_max - p.window))) {
+#pragma unroll
+            for (int j = 0; j < TK; ++j) {
+              const int key = key0 + j;
+              if (key > pos || key <= w_excl) v[j] = 0xff800000u;   // -inf
+            }
+          }
+          float t0 = -INFINITY, t1 = -INFINITY, t2 = -INFINITY, t3 = -INFINITY;
+#pragma unroll
+          for (int j = 0; j < TK; j += 4) {
+            t0 = fmaxf(t0, __uint_as_float(v[j]));     t1 = fmaxf(t1, __uint_as_float(v[j + 1]));
+            t2 = fmaxf(t2, __uint_as_float(v[j + 2])); t3 = fmaxf(t3, __uint_as_float(v[j + 3]));
+          }
+          const float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)) * mul;
+          float alpha = 1.f;
+          // The reference is the running maximum itself, not one that lags behind it by a few powers of two (which would
+          // spare most rescales): the key with the most weight then has p = 1, which bf16 holds exactly.
+          if (tmax > m) { alpha = ex2(m - tmax); m = tmax; }   // from -inf: alpha = 0
+          const float ref = m == -INFINITY ? 0.f : m;
+          float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll
+          for (int j = 0; j < TK; j += 4) {
+            const float p0 = ex2(__fmaf_rn(__uint_as_float(v[j]), mul, -ref)), p1 = ex2(__fmaf_rn(__uint_as_float(v[j + 1]), mul, -ref));
+            const float p2 = ex2(__fmaf_rn(__uint_as_float(v[j + 2]), mul, -ref)), p3 = ex2(__fmaf_rn(__uint_as_float(v[j + 3]), mul, -ref));
+            a0 += p0; a1 += p1; a2 += p2; a3 += p3;
+            v[j / 2] = pack_bf162(p0, p1);
+            v[j / 2 + 1] = pack_bf162(p2, p3);
+          }
+          l = __fmaf_rn(l, alpha, (a0 + a1) + (a2 + a3));
+#pragma unroll
+          for (int c = 0; c < TK / 64; ++c) tmem_st32(s_addr + c * 32, v + c * 32);
+          if (!first && !__all_sync(0xffffffffu, alpha == 1.f)) {
+            // a row's maximum moved: what O holds of it is rescaled once the previous tile's product is in
+            const int pt = tile - 1;
+            ok = warp_wait(&pv_done[pt & 1], (pt >> 1) & 1, p.status, KC_DEV_ATTN | 8);
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t o_addr = tmem + lane_addr + S::TMEM_O + (S::O_BUFS == 2 ? (chunks & 1) * D : 0);
+#pragma unroll 1
+            for (int c = 0; c < D / 64; ++c) {
+              uint32_t o[64];
+              tmem_ld32_issue(o_addr + c * 64, o);
+              tmem_ld32_issue(o_addr + c * 64 + 32, o + 32);
+              tmem_wait_ld();
+#pragma unroll
+              for (int j = 0; j < 64; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * alpha);
+              tmem_st32(o_addr + c * 64, o);
+              tmem_st32(o_addr + c * 64 + 32, o + 32);
+            }
+          }
+          tmem_wait_st();
+          tc_fence_before();
+        }
+        if (last) {
+          const int cb = chunks & 1;
+          // (m, l) of the chunk two before this one has been read (with one O buffer the wait is implied by that buffer's)
+          ok = warp_wait(&o_empty[S::O_BUFS == 2 ? cb : 0], S::O_BUFS == 2 ? ((chunks >> 1) & 1) ^ 1 : (chunks & 1) ^ 1, p.status, KC_DEV_ATTN | 9);
+          if (!ok) break;
+          stat[cb * ATT_ROWS + row] = make_float2(m, l);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&stat_full[cb]);
+          ++chunks;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_ready[sb]);
+      }
+    }
+  } else if (warp >= 8) {
+    // ---- a finished chunk: thread = query row ----
+    const int quarter = warp & 3, row = quarter * 32 + lane;
+    const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    int chunks = 0;
+    bool ok = true;
+    constexpr int ACC = WHOLE ? D : 1;
+    float acc[ACC];
+    for (int r = 0, w; ok && r * (int)gridDim.x < total; ++r) {
+      if ((w = unit_index(r, blockIdx.x, gridDim.x, total)) < 0) break;
+      UnitTiles u;
+      const int kvh = w % p.Hkv;
+      u.open(p, w / p.Hkv, TK);
+      if (!u.live()) continue;
+      const bool warp_live = quarter * 32 < u.rows, row_live = row < u.rows;
+      const int t = row / p.gqa;
+      const size_t orow = (size_t)(u.tok0 + t) * p.Hq + kvh * p.gqa + (row - t * p.gqa);
+      float macc = -INFINITY, lacc = 0.f;
+      if (WHOLE) {
+#pragma unroll
+        for (int j = 0; j < ACC; ++j) acc[j] = 0.f;
+      }
+      for (; u.c < u.c1 && ok; ++u.c, ++chunks) {
+        const int cb = chunks & 1, ob = S::O_BUFS == 2 ? cb : 0;
+        const uint32_t oph = S::O_BUFS == 2 ? (chunks >> 1) & 1 : chunks & 1;
+        ok = warp_wait(&stat_full[cb], (chunks >> 1) & 1, p.status, KC_DEV_ATTN | 10) && warp_wait(&o_full[ob], oph, p.status, KC_DEV_ATTN | 11);
+        if (!ok) break;
+        if (warp_live) {
+          tc_fence_after();
+          const float2 ml = stat[cb * ATT_ROWS + row];
+          const uint32_t o_addr = tmem + lane_addr + S::TMEM_O + ob * D;
+          if (WHOLE) {
+            const MergeW mw = merge_weights(macc, ml.x);
+            macc = mw.m;
+            lacc = merge_value(lacc, ml.y, mw);
+#pragma unroll
+            for (int c = 0; c < D / 32; ++c) {
+              uint32_t o[32];
+              tmem_ld32(o_addr + c * 32, o);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) acc[(c * 32 + j) % ACC] = merge_value(acc[(c * 32 + j) % ACC], __uint_as_float(o[j]), mw);
+            }
+          } else {
+            const size_t prow = orow * p.max_chunks + u.c;
+            float* po = p.part_o + prow * D;
+            if (row_live && !p.single) p.part_ml[prow] = ml;
+            const float inv = row_scale(ml.y);
+#pragma unroll 1
+            for (int c = 0; c < D / 32; ++c) {
+              uint32_t o[32];
+              tmem_ld32(o_addr + c * 32, o);
+              if (row_live && p.single) {
+                // the row's only chunk: merging it into nothing changes no bit, so the row is finished here
+                bf16* out = p.out + orow * D + c * 32;
+#pragma unroll
+                for (int j = 0; j < 32; j += 8) {
+                  uint32_t q[4];
+#pragma unroll
+                  for (int k = 0; k < 4; ++k)
+                    q[k] = pack_bf162(__fmul_rn(__uint_as_float(o[j + 2 * k]), inv), __fmul_rn(__uint_as_float(o[j + 2 * k + 1]), inv));
+                  *reinterpret_cast<uint4*>(out + j) = make_uint4(q[0], q[1], q[2], q[3]);
+                }
+              } else if (row_live) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4)
+                  *reinterpret_cast<uint4*>(po + c * 32 + j) = make_uint4(o[j], o[j + 1], o[j + 2], o[j + 3]);
+              }
+            }
+          }
+          tc_fence_before();
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&o_empty[ob]);
+      }
+      if (WHOLE && ok && row_live) {
+        const float inv = row_scale(lacc);
+        bf16* out = p.out + orow * D;
+#pragma unroll
+        for (int j = 0; j < ACC; j += 8)
+          *reinterpret_cast<uint4*>(out + j) =
+              make_uint4(pack_bf162(__fmul_rn(acc[j % ACC], inv), __fmul_rn(acc[(j + 1) % ACC], inv)), pack_bf162(__fmul_rn(acc[(j + 2) % ACC], inv), __fmul_rn(acc[(j + 3) % ACC], inv)),
+                         pack_bf162(__fmul_rn(acc[(j + 4) % ACC], inv), __fmul_rn(acc[(j + 5) % ACC], inv)), pack_bf162(__fmul_rn(acc[(j + 6) % ACC], inv), __fmul_rn(acc[(j + 7) % ACC], inv)));
+      }
+      __syncwarp();
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 2) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(S::TMEM_COLS) : "memory");
   }
 }
 
-// out[token, head, :] = sum_c w_c o_c / sum_c w_c l_c over the row's own chunks, in chunk order.
+// The chunks of a row merged in index order: the arithmetic of a whole-row unit (merge_weights, merge_value) over the
+// stored partials. Chunks are taken eight at a time with all of a batch's loads issued before the first use.
 template <int D>
 __global__ void attn_combine_kernel(const AttnParams p, int n_rows) {
   pdl_launch_dependents();
@@ -380,22 +512,12 @@ __global__ void attn_combine_kernel(const AttnParams p, int n_rows) {
   const int c_hi = pos / ATT_CHUNK;
   const int c_lo = p.window > 0 ? max(0, pos - p.window + 1) / ATT_CHUNK : 0;
   const float2* ml = p.part_ml + (size_t)row * p.max_chunks;
-  // Chunks are taken eight at a time with all of a batch's loads issued before the first use: the arithmetic and its
-  // order are those of a chunk-by-chunk loop, the kernel's duration is two round trips to L2 instead of two per chunk.
   constexpr int CB = 8;
-  float mmax = -INFINITY;
-  for (int c0 = c_lo; c0 <= c_hi; c0 += CB) {
-    float2 v[CB];
-#pragma unroll
-    for (int j = 0; j < CB; ++j) v[j] = c0 + j <= c_hi ? ml[c0 + j] : make_float2(-INFINITY, 0.f);
-#pragma unroll
-    for (int j = 0; j < CB; ++j) mmax = fmaxf(mmax, v[j].x);
-  }
   constexpr int PER = D / 32;
   float acc[PER];
 #pragma unroll
   for (int i = 0; i < PER; ++i) acc[i] = 0.f;
-  float lsum = 0.f;
+  float macc = -INFINITY, lacc = 0.f;
   for (int c0 = c_lo; c0 <= c_hi; c0 += CB) {
     float2 v[CB];
     float po[CB][PER];
@@ -418,41 +540,47 @@ __global__ void attn_combine_kernel(const AttnParams p, int n_rows) {
 #pragma unroll
     for (int j = 0; j < CB; ++j) {
       if (c0 + j <= c_hi) {
-        const float w = (v[j].x == -INFINITY) ? 0.f : exp2f(v[j].x - mmax);
-        lsum += w * v[j].y;
+        const MergeW mw = merge_weights(macc, v[j].x);
+        macc = mw.m;
+        lacc = merge_value(lacc, v[j].y, mw);
 #pragma unroll
-        for (int i = 0; i < PER; ++i) acc[i] += w * po[j][i];
+        for (int i = 0; i < PER; ++i) acc[i] = merge_value(acc[i], po[j][i], mw);
       }
     }
   }
+  const float inv = row_scale(lacc);
   bf16* out = p.out + (size_t)row * D + lane * PER;
+  if (PER == 2) {
+    *reinterpret_cast<uint32_t*>(out) = pack_bf162(__fmul_rn(acc[0], inv), __fmul_rn(acc[PER - 1], inv));
+  } else {
 #pragma unroll
-  for (int i = 0; i < PER; ++i) out[i] = __float2bfloat16_rn(lsum == 0.f ? acc[i] : acc[i] / lsum);
+    for (int i = 0; i < PER; i += 4)
+      *reinterpret_cast<uint2*>(out + i) = make_uint2(pack_bf162(__fmul_rn(acc[i], inv), __fmul_rn(acc[(i + 1) % PER], inv)),
+                                                      pack_bf162(__fmul_rn(acc[(i + 2) % PER], inv), __fmul_rn(acc[(i + 3) % PER], inv)));
+  }
 }
 
-template <int D, int MT>
-cudaError_t launch_partial(const CUtensorMap& map, const AttnParams& p, int n_work, int grid_chunks, cudaStream_t s) {
-  using S = AttnSmem<D, MT>;
+template <int D, bool WHOLE>
+cudaError_t launch_attn(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, int sm_count, cudaStream_t s) {
+  using S = AttnShape<D>;
   static DeviceOnce configured;   // the attribute belongs to the device's copy of the kernel
   if (configured.first_on_current_device()) {
-    cudaError_t e = cudaFuncSetAttribute(attn_partial_kernel<D, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(attn_kernel<D, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
     if (e != cudaSuccess) { configured.forget_current_device(); return e; }
   }
-  dim3 grid(grid_chunks, p.Hkv, n_work);
-  return launch_k(attn_partial_kernel<D, MT>, grid, dim3((S::CW + 1) * 32), S::TOTAL, s, map, p);
+  const int grid = std::min(p.n_units * p.Hkv, sm_count);
+  return launch_k(attn_kernel<D, WHOLE>, dim3(grid), dim3(ATT_THREADS), S::SMEM, s, map, q, q_small, p);
 }
 
 template <int D>
-cudaError_t launch_d(const CUtensorMap& map, const AttnParams& p, int mt, int n_work, int grid_chunks, int n_tokens,
+cudaError_t launch_d(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, int n_tokens, int sm_count,
                      cudaStream_t s) {
-  cudaError_t e;
-  switch (mt) {
-    case 1: e = launch_partial<D, 1>(map, p, n_work, grid_chunks, s); break;
-    case 2: e = launch_partial<D, 2>(map, p, n_work, grid_chunks, s); break;
-    case 3: e = launch_partial<D, 3>(map, p, n_work, grid_chunks, s); break;
-    default: e = launch_partial<D, 4>(map, p, n_work, grid_chunks, s); break;
+  if (p.whole) {
+    if constexpr (D <= 128) return launch_attn<D, true>(map, q, q_small, p, sm_count, s);
+    else return cudaErrorInvalidValue;
   }
-  if (e != cudaSuccess || p.single_chunk) return e;
+  cudaError_t e = launch_attn<D, false>(map, q, q_small, p, sm_count, s);
+  if (e != cudaSuccess || p.single) return e;
   const int n_rows = n_tokens * p.Hq;
   return launch_k(attn_combine_kernel<D>, dim3((n_rows + 7) / 8), dim3(256), 0, s, p, n_rows);
 }
@@ -460,20 +588,59 @@ cudaError_t launch_d(const CUtensorMap& map, const AttnParams& p, int mt, int n_
 }  // namespace
 
 int attn_tokens_per_item(int gqa, int max_len) {
-  // Largest token count whose rows fit 64 (MT <= 4); capped by the longest segment.
-  int t = std::max(1, 64 / gqa);
-  return std::min(t, std::max(1, max_len));
+  return std::min(std::max(1, ATT_ROWS / gqa), std::max(1, max_len));
 }
 
-cudaError_t paged_attention(const CUtensorMap& kvmap, const AttnParams& p, int head_dim, int tokens_per_item,
-                            int n_work, int grid_chunks, int n_tokens, cudaStream_t s) {
-  const int rows = tokens_per_item * p.gqa;
-  const int mt = (rows + 15) / 16;
-  if (mt < 1 || mt > 4) return cudaErrorInvalidValue;
+bool attn_whole(int head_dim, const int* item_tiles, int n_items, int kv_heads, int sm_count) {
+  if (head_dim > 128) return false;   // a thread of the last role holds a row of the output in registers
+  const int total = n_items * kv_heads, ctas = std::min(total, sm_count);
+  long long sum = 0, most = 0;
+  for (int i = 0; i < n_items; ++i) sum += (long long)item_tiles[i] * kv_heads;
+  std::vector<int> load(ctas, 0);
+  for (int r = 0; r * ctas < total; ++r)
+    for (int c = 0; c < ctas; ++c) {
+      const int w = unit_index(r, c, ctas, total);
+      if (w >= 0) load[c] += item_tiles[w / kv_heads];
+    }
+  for (int c = 0; c < ctas; ++c) most = std::max<long long>(most, load[c]);
+  // Whole rows save the partials' round trip through memory and the combine launch (about a tenth of a step of 32 long
+  // sequences); units of one chunk, 4 tiles, are for steps whose items leave SMs idle for longer than that.
+  return most <= 4 || most * sm_count * 4 <= sum * 5;
+}
+
+// Queries [n_tokens][Hkv][gqa][D] as {64 features, gqa, slabs, Hkv, tokens}: one operation brings a slab of up to 128
+// rows in (token, head) order. Tokens past the end read as zeros.
+bool make_tmap_q(CUtensorMap* map, const bf16* q, int n_tokens, int Hq, int gqa, int head_dim, int box_tokens, const char** err) {
+  const uint64_t D = head_dim, dims[5] = {64, (uint64_t)gqa, D / 64, (uint64_t)(Hq / gqa), (uint64_t)n_tokens};
+  const uint64_t strides[4] = {D * 2, 128, (uint64_t)gqa * D * 2, (uint64_t)Hq * D * 2};
+  const uint32_t box[5] = {64, (uint32_t)gqa, 1, 1, (uint32_t)box_tokens};
+  return encode_tmap_bf16(map, 5, q, dims, strides, box, err);
+}
+
+// K/V pools as a 5-D tensor {64 features, 8 rows, head_dim / 64 slabs, planes, plane_rows / 8} with box {64, 8, slabs, 2, 2}:
+// ONE operation brings 16 keys of K and V of a layer (plane 2 * layer and the next) as two groups of 8 keys, each with
+// its K slabs and then its V slabs of [8][128 B], 128-byte swizzle. Groups of 8 rows at one constant stride are what a
+// tensor-core operand of many 16-key blocks needs, wherever the block table scatters them. The slab stride (128 B) is
+// smaller than the row stride, which the encoder may refuse: the caller then keeps the 2-D map (8 rows x 64 features).
+bool make_tmap_kv_5d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t plane_rows, uint64_t planes, const char** err) {
+  const uint64_t D = head_dim, dims[5] = {64, 8, D / 64, planes, plane_rows / 8};
+  const uint64_t strides[4] = {D * 2, 128, plane_rows * D * 2, 8 * D * 2};
+  const uint32_t box[5] = {64, 8, head_dim / 64, 2, 2};
+  return encode_tmap_bf16(map, 5, pool, dims, strides, box, err);
+}
+bool make_tmap_kv_2d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t rows, const char** err) {
+  const uint64_t dims[2] = {head_dim, rows}, strides[1] = {(uint64_t)head_dim * 2};
+  const uint32_t box[2] = {64, 8};
+  return encode_tmap_bf16(map, 2, pool, dims, strides, box, err);
+}
+
+cudaError_t paged_attention(const CUtensorMap& kvmap, const CUtensorMap& qmap, const CUtensorMap& qmap_small, const AttnParams& p,
+                            int head_dim, int n_tokens, int sm_count, cudaStream_t s) {
+  if (p.gqa < 1 || p.gqa * p.q_tokens > ATT_ROWS || p.n_units < 1) return cudaErrorInvalidValue;
   switch (head_dim) {
-    case 64: return launch_d<64>(kvmap, p, mt, n_work, grid_chunks, n_tokens, s);
-    case 128: return launch_d<128>(kvmap, p, mt, n_work, grid_chunks, n_tokens, s);
-    case 256: return launch_d<256>(kvmap, p, mt, n_work, grid_chunks, n_tokens, s);
+    case 64: return launch_d<64>(kvmap, qmap, qmap_small, p, n_tokens, sm_count, s);
+    case 128: return launch_d<128>(kvmap, qmap, qmap_small, p, n_tokens, sm_count, s);
+    case 256: return launch_d<256>(kvmap, qmap, qmap_small, p, n_tokens, sm_count, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -7,10 +7,16 @@ namespace kc {
 
 // Keys per chunk. Chunks are cut at absolute key positions, so the partition a
 // query row sees depends only on its own position.
-#ifndef ATT_CHUNK_KEYS
-#define ATT_CHUNK_KEYS 512
-#endif
-constexpr int ATT_CHUNK = ATT_CHUNK_KEYS;
+constexpr int ATT_CHUNK = 512;
+constexpr int ATT_ROWS = 128;   // query rows (token x head of the group) of one work item: the lanes of tensor memory
+
+// One unit of work for every kv head: consecutive tokens of one sequence against the chunks [chunk0, chunk1).
+struct AttnUnit {
+  int seq, tok0, ntok, pos0;    // sequence, first token row in the step, tokens, absolute position of the first
+  int chunk0, chunk1;
+  int small, pad;               // 1: at most ATT_SMALL_TOKENS tokens (the query map with the small box)
+};
+constexpr int ATT_SMALL_TOKENS = 8;
 
 struct AttnParams {
   const bf16* q;               // [n_tokens, Hq, D] post-RoPE
@@ -18,28 +24,36 @@ struct AttnParams {
   float* part_o;               // [n_tokens * Hq][max_chunks][D]  un-normalised partial outputs
   float2* part_ml;             // [n_tokens * Hq][max_chunks]     (running max in log2 units, sum)
   const int32_t* block_tables; // [n_seqs][max_blocks]
-  const int4* work;            // [n_work] {seq, first token row, tokens, absolute position of first token}
+  const AttnUnit* units;       // [n_units]
+  int n_units;
   const int32_t* token_pos;    // [n_tokens] absolute position of each token row
   uint32_t* status;
   int max_blocks;
   int Hq, Hkv, gqa;
   int layer, NB, BS;
   int max_chunks;
-  int single_chunk;            // 1: max_chunks == 1, the partial kernel writes `out` itself and no combine kernel follows
-  int chunk_lo_grid;           // chunk index of blockIdx.x == 0
+  int whole;                   // 1: every unit holds all chunks of its rows: the kernel writes `out`, no combine kernel follows
+  int single;                  // 1: no row of the step has a second chunk (max_chunks == 1): no combine kernel either
   float scale;                 // softmax scale (applied to fp32 scores)
   float softcap;               // 0 = off
   int window;                  // 0 = global
-  const bf16* pool;            // K/V pools: [layers][2][NB][Hkv][BS][head_dim]
-  int kv4d;                    // kvmap is the 4-D map (one operation per K+V tile pair) instead of the 2-D one
+  int q_tokens;                // tokens in the box of the large query map
+  int kv5d;                    // kvmap is the 5-D map (one operation per 16 keys of K and V) instead of the 2-D one
 };
 
-// Tokens of one sequence that share a CTA (their rows x gqa must fit 64 rows).
+// Tokens of one sequence that share a CTA (their rows x gqa must fit ATT_ROWS).
 int attn_tokens_per_item(int gqa, int max_len);
+// Whether units of whole rows (all chunks of an item in one unit) keep the SMs about as busy as units of single chunks:
+// item_tiles = tiles of 128 keys of each item, in the order of the units.
+bool attn_whole(int head_dim, const int* item_tiles, int n_items, int kv_heads, int sm_count);
 
-// kvmap: 2-D tensor map over all pool rows ([layers*2*NB*Hkv*BS, D] bf16, box {64, 16}, 128-byte swizzle), or, with
-// p.kv4d, the 4-D map of make_tmap_kv_4d. n_work CTAs in z, grid_chunks in x.
-cudaError_t paged_attention(const CUtensorMap& kvmap, const AttnParams& p, int head_dim, int tokens_per_item,
-                            int n_work, int grid_chunks, int n_tokens, cudaStream_t s);
+// Query maps over [n_tokens, Hq, D] (5-D: 64 features, heads of a group, slabs, groups, tokens).
+bool make_tmap_q(CUtensorMap* map, const bf16* q, int n_tokens, int Hq, int gqa, int head_dim, int box_tokens, const char** err);
+// K/V pools [planes = layers * 2][plane_rows = NB * Hkv * BS][head_dim]: see kc_attn.cu.
+bool make_tmap_kv_5d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t plane_rows, uint64_t planes, const char** err);
+bool make_tmap_kv_2d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t rows, const char** err);
+
+cudaError_t paged_attention(const CUtensorMap& kvmap, const CUtensorMap& qmap, const CUtensorMap& qmap_small, const AttnParams& p,
+                            int head_dim, int n_tokens, int sm_count, cudaStream_t s);
 
 }  // namespace kc

@@ -148,15 +148,18 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* t
       "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(y)
       : "memory");
 }
-// 4-D tiled TMA load (no multicast): coordinates {x = innermost, y, z, w}; x * element size a multiple of 16 bytes.
-__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* tmap, int32_t x, int32_t y, int32_t z,
-                                            int32_t w, uint64_t* bar) {
+// 5-D tiled TMA load (no multicast).
+__device__ __forceinline__ void tma_load_5d(void* smem_dst, const CUtensorMap* tmap, int32_t x, int32_t y, int32_t z,
+                                            int32_t w, int32_t v, uint64_t* bar) {
   asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];" ::
+      "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::
           "r"(smem_u32(smem_dst)),
-      "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+      "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(w), "r"(v)
       : "memory");
 }
+// Encodes a tiled map of `rank` <= 5 dimensions over bf16 elements, 128-byte swizzle; strides in bytes, of dimensions 1 ..
+bool encode_tmap_bf16(CUtensorMap* map, int rank, const void* ptr, const uint64_t* dims, const uint64_t* strides,
+                      const uint32_t* box, const char** err);
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }

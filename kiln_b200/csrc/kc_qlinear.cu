@@ -15,6 +15,7 @@
 // and still reproduce the bits of a one-row decode. Launches of more rows than one accumulator set holds are cut
 // into row chunks, each its own launch over the same weights: rows are independent, so no bit changes.
 #include "kc_qlinear.cuh"
+#include "kc_umma.cuh"
 
 #include <algorithm>
 #include <cstdio>
@@ -153,39 +154,27 @@ static EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-bool make_tmap_bf16_2d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer,
-                       uint32_t box_inner, uint32_t box_outer, const char** err) {
+bool encode_tmap_bf16(CUtensorMap* map, int rank, const void* ptr, const uint64_t* dims, const uint64_t* strides,
+                      const uint32_t* box, const char** err) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) { *err = "cuTensorMapEncodeTiled entry point unavailable"; return false; }
-  cuuint64_t dims[2] = {inner, outer};
-  cuuint64_t strides[1] = {inner * sizeof(bf16)};
-  cuuint32_t box[2] = {box_inner, box_outer};
-  cuuint32_t estr[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box,
-                  estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  cuuint64_t d[5], st[4];
+  cuuint32_t b[5], estr[5];
+  for (int i = 0; i < rank; ++i) { d[i] = dims[i]; b[i] = box[i]; estr[i] = 1; }
+  for (int i = 0; i + 1 < rank; ++i) st[i] = strides[i];
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(ptr), d, st, b, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  rank > 2 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) { *err = "cuTensorMapEncodeTiled rejected the tensor geometry"; return false; }
   return true;
 }
 
-// K/V pools [planes = layers * 2][plane_rows = NB * Hkv * BS][head_dim] bf16 as a 4-D tensor
-// {64 features, plane_rows, head_dim / 64 slabs, planes} with box {64, 16, head_dim / 64, 2}: ONE operation brings the
-// 16-key K tile and the V tile of a layer (plane 2 * layer and the next), each as head_dim / 64 slabs of [16][128 B]
-// with the 128-byte swizzle — the shared-memory image of 2 * head_dim / 64 separate 2-D loads. The slab stride
-// (128 B) is smaller than the row stride, which the encoder may refuse: the caller then keeps the 2-D map.
-bool make_tmap_kv_4d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t plane_rows, uint64_t planes,
-                     const char** err) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) { *err = "cuTensorMapEncodeTiled entry point unavailable"; return false; }
-  cuuint64_t dims[4] = {64, plane_rows, head_dim / 64, planes};
-  cuuint64_t strides[3] = {head_dim * sizeof(bf16), 128, plane_rows * head_dim * sizeof(bf16)};
-  cuuint32_t box[4] = {64, 16, head_dim / 64, 2};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(pool), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);   // head_dim >= 128: a key's row is 256 B or more, both slabs of it in one L2 fill
-  if (r != CUDA_SUCCESS) { *err = "cuTensorMapEncodeTiled rejected the 4-D K/V geometry"; return false; }
-  return true;
+static bool make_tmap_bf16_2d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer,
+                              uint32_t box_inner, uint32_t box_outer, const char** err) {
+  const uint64_t dims[2] = {inner, outer}, strides[1] = {inner * sizeof(bf16)};
+  const uint32_t box[2] = {box_inner, box_outer};
+  return encode_tmap_bf16(map, 2, ptr, dims, strides, box, err);
 }
 
 // The map whose box covers `m_pad` rows (<= 256), so that one TMA operation brings a whole activation k-block.
@@ -287,43 +276,9 @@ __device__ __forceinline__ void dequant_row_wide(const uint8_t* row_base, const 
 }
 
 // ---------------------------------------------------------------------------
-// tcgen05 helpers
+// tcgen05 helpers (the others are in kc_umma.cuh)
 // ---------------------------------------------------------------------------
 
-__device__ __forceinline__ uint64_t umma_smem_desc_sw128(uint32_t smem_addr) {
-  // K-major, 128-byte swizzle: rows of 128 bytes, 8-row groups 1024 bytes apart.
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);       // start address
-  d |= (uint64_t)1 << 16;                           // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;                 // stride byte offset between 8-row groups
-  d |= (uint64_t)1 << 46;                           // descriptor version (Blackwell)
-  d |= (uint64_t)2 << 61;                           // SWIZZLE_128B
-  return d;
-}
-
-__device__ __forceinline__ uint32_t umma_idesc_bf16(int m, int n) {
-  // kind::f16 takes A and B of the SAME 16-bit type: an f16 A against a bf16 B is an illegal instruction.
-  uint32_t d = 0;
-  d |= 1u << 4;                    // D format f32
-  d |= 1u << 7;                    // A format bf16
-  d |= 1u << 10;                   // B format bf16
-  // a_major (bit 15) = b_major (bit 16) = 0: both K-major
-  d |= (uint32_t)(n >> 3) << 17;   // N
-  d |= (uint32_t)(m >> 4) << 24;   // M
-  return d;
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                   smem_u32(bar))
-               : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
@@ -362,19 +317,6 @@ struct QlKernelParams {
   int part_M, part_row0;
   uint32_t* status;
 };
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 
 // The epilogue shared by the GEMM kernels: every epilogue warp drains its TMEM lane quarter, 32 columns (rows of the
 // step) at a time, transposes through a private 4 KB shared buffer and stores row-contiguous vectors: bf16 y, fp32
@@ -483,34 +425,6 @@ __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* sm
 //
 // TMEM columns: [2 accumulators of round32(m_pad)] [a_stages x 2 units x 32 columns of bf16 pairs].
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_lo, uint32_t d_hi, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "setp.ne.b32 p, %5, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "r"(b_lo), "r"(d_hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
-      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
-// A bounded wait of a whole warp; the warp is converged afterwards.
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, uint32_t* status, uint32_t code) {
-  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, status, code));
-}
-
 template <int BITS, int GPK, int NT>
 __global__ void __launch_bounds__(QL_THREADS, 1)
 qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKernelParams p) {
@@ -597,7 +511,7 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
     const int u = warp - 2;
     if (NT == 1 || u < nt_live) {
       const uint32_t idesc = umma_idesc_bf16(QL_TILE_N, p.m_pad);
-      const uint64_t proto = umma_smem_desc_sw128(0);
+      const uint64_t proto = umma_smem_desc(0, 1024);
       const uint32_t d_hi = (uint32_t)(proto >> 32), b_lo0 = (uint32_t)proto | ((smem_u32(sB) >> 4) & 0x3FFF);
       const uint32_t d_t = tmem_base + u * col_stride, a_t0 = tmem_base + a_col0 + u * 32;
       const int n_own = NT == 2 ? nkb : (nkb + 1 - u) / 2;  // k-blocks of this accumulator
