@@ -478,11 +478,12 @@ extern "C" int kc_kv_write_block(kc_kv_t kv, uint32_t block, const void* src, si
 static int run_qlinear(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, bf16* y, int ldy, float* partial,
                        SublayerOut* fused = nullptr) {
   const bool defer = fused && w.splits > 1 && M <= QL_MAX_M;
-  for (int row0 = 0; row0 < M; row0 += QL_MAX_M) {
+  const int slab = qlinear_slab_rows(w, M);
+  for (int row0 = 0; row0 < M; row0 += slab) {
     QLinearLaunch l;
-    l.w = &w; l.x = &x; l.row0 = row0; l.M = std::min(QL_MAX_M, M - row0);
+    l.w = &w; l.x = &x; l.row0 = row0; l.M = std::min(slab, M - row0);
     l.y = y; l.ldy = ldy; l.partial = partial; l.status = c->status;
-    LAUNCH(c, KC_PROF_GEMM, qlinear_launches(w, l.M), qlinear_umma(l, c->stream));
+    LAUNCH(c, KC_PROF_GEMM, 1, qlinear_umma(l, c->stream));
     if (w.splits > 1 && !defer)
       LAUNCH(c, KC_PROF_GEMM_REDUCE, 1, qlinear_reduce_splits(partial, w.splits, l.M, w.N, y + (size_t)row0 * ldy, ldy, c->stream));
   }
@@ -495,14 +496,15 @@ static int run_qlinear(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, 
 // interleaved [M, 2F] product and run the element-wise kernel on it. Both ways round at the same points.
 static int run_gated(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, bf16* gu, int F, int gelu, bool interleaved,
                      bf16* act, float* partial) {
-  for (int row0 = 0; row0 < M; row0 += QL_MAX_M) {
-    const int rows = std::min(QL_MAX_M, M - row0);
+  const int slab = qlinear_slab_rows(w, M);
+  for (int row0 = 0; row0 < M; row0 += slab) {
+    const int rows = std::min(slab, M - row0);
     int done = 0;
     QLinearLaunch l;
     l.w = &w; l.x = &x; l.row0 = row0; l.M = rows;
     l.y = gu; l.ldy = 2 * F; l.partial = partial; l.status = c->status;
     if (interleaved) { l.glu = gelu ? 2 : 1; l.act = act; l.ld_act = F; l.glu_done = &done; }
-    LAUNCH(c, KC_PROF_GEMM, qlinear_launches(w, rows), qlinear_umma(l, c->stream));
+    LAUNCH(c, KC_PROF_GEMM, 1, qlinear_umma(l, c->stream));
     if (done) continue;
     if (w.splits > 1)
       LAUNCH(c, KC_PROF_GEMM_REDUCE, 1, qlinear_reduce_splits(partial, w.splits, rows, w.N, gu + (size_t)row0 * 2 * F, 2 * F, c->stream));

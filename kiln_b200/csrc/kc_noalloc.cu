@@ -79,13 +79,14 @@ extern "C" int kc_quantized_matmul_static(kc_ctx_t c, kc_qweight_t q, const void
     return api_fail(KC_ERR_CUDA, msg);
   }
   bf16* y = (bf16*)y_dev;
-  for (int row0 = 0; row0 < m; row0 += QL_MAX_M) {
+  const int rows = qlinear_slab_rows(w, m);
+  for (int row0 = 0; row0 < m; row0 += rows) {
     QLinearLaunch l;
-    l.w = &w; l.x = &op; l.row0 = row0; l.M = (m - row0) < QL_MAX_M ? (m - row0) : QL_MAX_M;
+    l.w = &w; l.x = &op; l.row0 = row0; l.M = (m - row0) < rows ? (m - row0) : rows;
     l.y = y; l.ldy = w.N; l.partial = scratch; l.status = cv.status;
     // launches are counted once they are queued; this entry point takes no part in kc_profile_* timing
     e = qlinear_umma(l, cv.stream);
-    if (e == cudaSuccess) ctx_count_launches(c, 0, qlinear_launches(w, l.M));
+    if (e == cudaSuccess) ctx_count_launches(c, 0, 1);
     if (e == cudaSuccess && w.splits > 1) {
       e = qlinear_reduce_splits(scratch, w.splits, l.M, w.N, y + (size_t)row0 * w.N, w.N, cv.stream);
       if (e == cudaSuccess) ctx_count_launches(c, 1, 1);

@@ -12,8 +12,8 @@
 // The accumulator D[n, m] lives in TMEM: lane = weight row n, column = activation row m.
 // Every output element depends only on its own activation row and on a k order
 // fixed by (N, K), which is what lets verify rows share a step with other rows
-// and still reproduce the bits of a one-row decode. Launches of more rows than one accumulator set holds are cut
-// into row chunks, each its own launch over the same weights: rows are independent, so no bit changes.
+// and still reproduce the bits of a one-row decode. More rows than one accumulator set holds are cut into chunks of
+// rows (blockIdx.z): rows are independent, so no bit changes.
 #include "kc_qlinear.cuh"
 #include "kc_umma.cuh"
 
@@ -304,7 +304,7 @@ struct QlKernelParams {
   const uint8_t* records;
   uint32_t record_bytes;
   int N, n_tiles, kblocks;
-  int M, m_pad;          // live rows, rows rounded up to 16
+  int M, m_pad;          // live rows of the launch; rows of a chunk (blockIdx.z), a multiple of 16
   int row0;              // first activation row
   int splits;
   int a_stages, r_stages, b_stages;   // ring depths: stages in TMEM, k-blocks of records and stages of activations in shared memory
@@ -313,8 +313,7 @@ struct QlKernelParams {
   bf16* act; int ld_act;
   uint32_t tmem_cols;    // columns allocated: a power of two
   bf16* y; int ldy;
-  float* partial;        // [splits][part_M][N]; this launch writes rows part_row0 .. part_row0 + M
-  int part_M, part_row0;
+  float* partial;        // [splits][M][N]
   uint32_t* status;
 };
 
@@ -323,7 +322,7 @@ struct QlKernelParams {
 // split-K partials, or — when the CTA owns (gate, up) tile pairs — the gated activation.
 template <int NT>
 __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* smem, int warp, int lane, uint32_t tmem_base,
-                                            int tile0, int nt_live, int split, bool two_sums) {
+                                            int tile0, int nt_live, int split, int chunk0, bool two_sums) {
   tc_fence_after();
   // every MMA has completed and every copy into the rings has been consumed: the ring memory is free
   float* stage = reinterpret_cast<float*>(smem + (size_t)(warp - QL_DQ_WARP0) * QL_EPI_STAGE_BYTES);
@@ -354,7 +353,7 @@ __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* sm
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int mr = 4 * k + mr0;
-        const int m = ch * 16 + mr;
+        const int m = chunk0 + ch * 16 + mr;
         if (m >= p.M) continue;
         const float4 v4 = *reinterpret_cast<const float4*>(stage + mr * 32 + nl);
         *reinterpret_cast<uint2*>(p.act + (size_t)(p.row0 + m) * p.ld_act + f) =
@@ -381,8 +380,8 @@ __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* sm
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       const int mr = 4 * k + mr0;
-      const int m = ch * 32 + mr;
-      if (m >= p.M || n >= p.N) continue;
+      const int mc = ch * 32 + mr, m = chunk0 + mc;
+      if (mc >= p.m_pad || m >= p.M || n >= p.N) continue;
       const float4 f = *reinterpret_cast<const float4*>(stage + mr * 32 + nl);
       if (p.splits == 1) {
         bf16* dst = p.y + (size_t)(p.row0 + m) * p.ldy + n;
@@ -393,7 +392,7 @@ __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* sm
           for (int c = 0; c < 4 && n + c < p.N; ++c) dst[c] = __float2bfloat16_rn(e[c]);
         }
       } else {
-        float* dst = p.partial + ((size_t)split * p.part_M + p.part_row0 + m) * p.N + n;
+        float* dst = p.partial + ((size_t)split * p.M + m) * p.N + n;
         if (vec_ok && n + 3 < p.N) {
           *reinterpret_cast<float4*>(dst) = f;
         } else {
@@ -436,7 +435,7 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
   const uint32_t b_bytes = (uint32_t)p.m_pad * 128u;    // one activation k-block
   const uint32_t r_stage = NT * p.record_bytes;         // the records of one k-block
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const int tile0 = blockIdx.x * NT, split = blockIdx.y;
+  const int tile0 = blockIdx.x * NT, split = blockIdx.y, chunk0 = blockIdx.z * p.m_pad;
   const int nt_live = min(NT, p.n_tiles - tile0);
   // splits may be uneven: split s takes k-blocks [K s / S, K (s + 1) / S) — a fixed function of the weight's shape
   const int kb0 = (int)((long long)p.kblocks * split / p.splits);
@@ -499,7 +498,7 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
       for (int i = 0; i < nkb; ++i, bp.advance(SB)) {
         if (!mbar_wait(&b_empty[bp.stage], bp.phase ^ 1, p.status, KC_DEV_QLINEAR | 2)) break;
         mbar_arrive_expect_tx(&b_full[bp.stage], b_bytes);
-        tma_load_2d(sB + (size_t)bp.stage * b_bytes, &map_rows, (kb0 + i) * QL_KB, p.row0, &b_full[bp.stage]);
+        tma_load_2d(sB + (size_t)bp.stage * b_bytes, &map_rows, (kb0 + i) * QL_KB, p.row0 + chunk0, &b_full[bp.stage]);
       }
     }
   } else if (warp < QL_DQ_WARP0) {
@@ -599,7 +598,7 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
     // ---- epilogue ----
     pdl_wait();   // the stores below may overwrite what an earlier kernel still reads
     if (ok) ok = warp_wait(acc_full, 0, p.status, KC_DEV_QLINEAR | 7);
-    if (ok) ql_epilogue<NT>(p, smem, warp, lane, tmem_base, tile0, nt_live, split, nkb > 1);
+    if (ok) ql_epilogue<NT>(p, smem, warp, lane, tmem_base, tile0, nt_live, split, chunk0, nkb > 1);
   }
   __syncwarp();
   tc_fence_before();
@@ -653,7 +652,7 @@ static cudaError_t launch_umma_ta(const QLinearLaunch& l, QlKernelParams& p, cud
   }
   const CUtensorMap* rows = act_operand_rows_map(l.x, p.m_pad);
   if (!rows) return cudaErrorInvalidValue;
-  dim3 grid((w.n_tiles + NT - 1) / NT, w.splits);
+  dim3 grid((w.n_tiles + NT - 1) / NT, w.splits, (p.M + p.m_pad - 1) / p.m_pad);
   return launch_k(qlinear_umma_ta_kernel<BITS, GPK, NT>, grid, dim3(QL_THREADS), t.smem, s, *rows, p);
 }
 
@@ -668,8 +667,8 @@ static int plan_tiles_per_cta(const QWeight& w, int sm_count) {
   return ((w.n_tiles + 1) / 2) * w.splits * 10 >= sm_count * 7 ? 2 : 1;
 }
 
-// The most rows one launch of this weight takes: what the accumulators (two tiles: 192 columns each, one tile: 256)
-// and the rings of the weight's record size leave room for.
+// The most rows one CTA takes: what the accumulators (two tiles: 192 columns each, one tile: 256) and the rings of the
+// weight's record size leave room for.
 static int plan_row_cap(int nt, uint32_t record_bytes) {
   static const int caps[] = {256, 192, 128, 64, 32, 16};
   for (int c : caps)
@@ -677,9 +676,28 @@ static int plan_row_cap(int nt, uint32_t record_bytes) {
   return 0;
 }
 
+// Rows of a chunk (one CTA's share of the rows) for M rows. All chunks are one launch, CTAs of the next filling the SMs
+// that the last wave of one leaves idle; the chunk size is the one whose waves take the least time, counted in MMA
+// cycles: a unit of 128 x 64 weights takes 2 cycles per row, not less than 184, and a CTA about 6000 around them.
+// 28672 x 4096, 2048 rows: 13 chunks of 160 rows are 10 waves, 368 us; 11 chunks of 192, a launch each, took 450.
+static int plan_chunk_rows(const QWeight& w, int nt, int cap, int M) {
+  const int ctas = ((w.n_tiles + nt - 1) / nt) * w.splits;
+  const long long units = (long long)w.kblocks * nt / w.splits;
+  int best = 0;
+  long long best_cost = 0;
+  for (int chunks = (M + cap - 1) / cap; best == 0 || chunks * 96 <= M; ++chunks) {
+    const int per = ((M + chunks - 1) / chunks + 15) & ~15;
+    const int n = (M + per - 1) / per;
+    const long long waves = ((long long)ctas * n + w.sm_count - 1) / w.sm_count;
+    const long long cost = waves * (units * std::max(184, 2 * per) + 6000);
+    if (best == 0 || cost < best_cost) { best = per; best_cost = cost; }
+  }
+  return best;
+}
+
 cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   const QWeight& w = *l.w;
-  if (l.M < 1 || l.M > QL_MAX_M) return cudaErrorInvalidValue;
+  if (l.M < 1 || l.M > qlinear_slab_rows(w, l.M)) return cudaErrorInvalidValue;
   if (l.row0 % 16 || l.row0 + l.M > l.x->rows) return cudaErrorInvalidValue;   // rows past the operand's end read as zeros
   const int nt = plan_tiles_per_cta(w, w.sm_count);
   const int cap = plan_row_cap(nt, w.record_bytes);
@@ -688,30 +706,16 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   const bool glu = l.glu && nt == 2 && w.splits == 1 && (w.n_tiles & 1) == 0 && (w.N % (2 * QL_TILE_N)) == 0 && l.act &&
                    (l.ld_act & 3) == 0 && (reinterpret_cast<uintptr_t>(l.act) & 7) == 0;
   if (l.glu_done) *l.glu_done = glu ? 1 : 0;
-  // equal row chunks (multiples of 16 rows): fewer accumulator columns per chunk leave more A stages
-  const int chunks = (l.M + cap - 1) / cap;
-  const int per = (((l.M + chunks - 1) / chunks) + 15) & ~15;
-  for (int r0 = 0; r0 < l.M; r0 += per) {
-    QlKernelParams p;
-    p.records = w.records; p.record_bytes = w.record_bytes;
-    p.N = w.N; p.n_tiles = w.n_tiles; p.kblocks = w.kblocks;
-    p.M = std::min(per, l.M - r0); p.m_pad = (p.M + 15) & ~15; p.row0 = l.row0 + r0;
-    p.splits = w.splits;
-    p.wide = w.wide_scale;
-    p.y = l.y; p.ldy = l.ldy; p.partial = l.partial; p.part_M = l.M; p.part_row0 = r0; p.status = l.status;
-    p.glu = glu ? l.glu : 0; p.act = l.act; p.ld_act = l.ld_act;
-    cudaError_t e;
-    if (w.bits == 4) e = w.gpk == 2 ? launch_umma_nt<4, 2>(l, p, nt, s) : launch_umma_nt<4, 1>(l, p, nt, s);
-    else e = w.gpk == 2 ? launch_umma_nt<8, 2>(l, p, nt, s) : launch_umma_nt<8, 1>(l, p, nt, s);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
-}
-
-int qlinear_launches(const QWeight& w, int M) {
-  const int nt = plan_tiles_per_cta(w, w.sm_count);
-  const int cap = plan_row_cap(nt, w.record_bytes);
-  return cap ? (M + cap - 1) / cap : 0;
+  QlKernelParams p;
+  p.records = w.records; p.record_bytes = w.record_bytes;
+  p.N = w.N; p.n_tiles = w.n_tiles; p.kblocks = w.kblocks;
+  p.M = l.M; p.m_pad = plan_chunk_rows(w, nt, cap, l.M); p.row0 = l.row0;
+  p.splits = w.splits;
+  p.wide = w.wide_scale;
+  p.y = l.y; p.ldy = l.ldy; p.partial = l.partial; p.status = l.status;
+  p.glu = glu ? l.glu : 0; p.act = l.act; p.ld_act = l.ld_act;
+  if (w.bits == 4) return w.gpk == 2 ? launch_umma_nt<4, 2>(l, p, nt, s) : launch_umma_nt<4, 1>(l, p, nt, s);
+  return w.gpk == 2 ? launch_umma_nt<8, 2>(l, p, nt, s) : launch_umma_nt<8, 1>(l, p, nt, s);
 }
 
 // ---------------------------------------------------------------------------

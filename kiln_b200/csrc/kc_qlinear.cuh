@@ -28,7 +28,7 @@ namespace kc {
 
 constexpr int QL_TILE_N = 128;  // output features per tile = UMMA M
 constexpr int QL_KB = 64;       // input features per k-block = one 128-byte swizzle row of bf16
-constexpr int QL_MAX_M = 512;   // activation rows per qlinear_umma call (one slab of the split-K workspace)
+constexpr int QL_MAX_M = 512;   // activation rows of one slab of the split-K workspace
 constexpr size_t QL_STREAM_MIN_BYTES = (size_t)24 << 20;  // records of a weight from which a model's small steps stream it
 constexpr int QL_STREAM_MAX_M = 8;  // activation rows the weight-streaming lane takes (the 8 columns of one mma.sync)
 constexpr int QL_TILE_GROUP = 4;  // tiles whose records are interleaved per k-block (the most one CTA owns)
@@ -63,7 +63,7 @@ struct QLinearLaunch {
   const QWeight* w;
   const ActOperand* x;
   int row0;         // first activation row of this launch (x, y and partial are indexed from it)
-  int M;            // live activation rows, 1..QL_MAX_M
+  int M;            // live activation rows, at most qlinear_slab_rows
   bf16* y;          // [M, ldy] bf16 when the weight has splits == 1 (else unused)
   int ldy;
   float* partial;   // [splits][M][N] fp32 workspace when splits > 1 (rows relative to row0)
@@ -93,11 +93,10 @@ void qweight_free(QWeight* w);
 // *err) if the driver entry point is unavailable or rejects the geometry.
 bool act_operand_init(ActOperand* op, const bf16* ptr, int rows, int K, const char** err);
 
-// The GEMM (tcgen05 + TMEM + TMA). Returns a CUDA error. A launch of more rows than the accumulators hold (192 with
-// two weight tiles per CTA, 256 with one) is issued as several kernels over equal row chunks.
+// The GEMM (tcgen05 + TMEM + TMA). Returns a CUDA error. One launch, whatever the number of rows.
 cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s);
-// Kernels qlinear_umma issues for M rows of this weight.
-int qlinear_launches(const QWeight& w, int M);
+// Rows that one call takes out of M: the workspace of a weight that is split along K holds QL_MAX_M.
+inline int qlinear_slab_rows(const QWeight& w, int M) { return w.splits > 1 && M > QL_MAX_M ? QL_MAX_M : M; }
 
 // The weight-streaming lane for at most QL_STREAM_MAX_M rows: x bf16 [M, ldx] against dequant(W)^T, left as fp32
 // partials [qlinear_stream_pieces(w)][M][N] that the caller's consumer kernel (or qlinear_reduce_splits) sums in index

@@ -217,3 +217,21 @@ def test_stage_edges_and_scale_range(ctx, n, k, bits, group, m, gain):
     one = qw.matmul(x[m - 1:].cuda()).cpu()
     assert torch.equal(one.view(torch.int16), got[m - 1:].view(torch.int16))
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("n,k,bits,group,m", [
+    (26700, 320, 4, 64, 193),     # two tiles per CTA, two chunks, the last accumulator tile missing
+    (26700, 192, 4, 128, 1001),   # a last chunk of fewer rows than the others
+    (384, 1088, 4, 32, 257),      # one tile per CTA, split along K
+    (300, 512, 8, 64, 700),       # more rows than a slab of the split-K workspace
+])
+def test_row_chunks_carry_the_bits_of_few_rows(ctx, n, k, bits, group, m):
+    """Rows are cut into chunks by a rule on the shape: a row's bits are those it has in a launch of its own."""
+    p, s, b = make(n, k, bits, group, 41)
+    qw = api.QuantizedWeight(ctx, p.cuda(), s.cuda(), b.cuda(), bits, group)
+    x = acts(m, k, 42).cuda()
+    full = qw.matmul(x).cpu()
+    for r0, r1 in ((0, 1), (90, 131), (m - 70, m), (m - 1, m)):
+        part = qw.matmul(x[r0:r1].contiguous()).cpu()
+        assert torch.equal(part.view(torch.int16), full[r0:r1].view(torch.int16)), f"rows {r0}..{r1}"
+    assert ctx.device_status() == 0
