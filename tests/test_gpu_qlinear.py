@@ -221,7 +221,7 @@ def test_stage_edges_and_scale_range(ctx, n, k, bits, group, m, gain):
 
 @pytest.mark.parametrize("n,k,bits,group,m", [
     (26700, 320, 4, 64, 193),     # two tiles per CTA, two chunks, the last accumulator tile missing
-    (26700, 192, 4, 128, 1001),   # a last chunk of fewer rows than the others
+    (26700, 384, 4, 128, 1001),   # a last chunk of fewer rows than the others
     (384, 1088, 4, 32, 257),      # one tile per CTA, split along K
     (300, 512, 8, 64, 700),       # more rows than a slab of the split-K workspace
 ])
