@@ -424,16 +424,16 @@ __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* sm
 //
 // TMEM columns: [2 accumulators of round32(m_pad)] [a_stages x 2 units x 32 columns of bf16 pairs].
 // ---------------------------------------------------------------------------
-template <int BITS, int GPK, int NT>
+template <int BITS, int GPK, int NT, int P>
 __global__ void __launch_bounds__(QL_THREADS, 1)
 qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKernelParams p) {
-  constexpr int KC = NT == 1 ? 2 : 1;                   // k-blocks of a stage; a stage is two units
+  constexpr int KC = NT == 1 ? 2 : 1;                   // slots of records and activations in a stage (see below)
   constexpr uint32_t PACKED = QL_TILE_N * (QL_KB * BITS / 8);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const int SA = p.a_stages, SB = p.b_stages;
   const uint32_t b_bytes = (uint32_t)p.m_pad * 128u;    // one activation k-block
-  const uint32_t r_stage = NT * p.record_bytes;         // the records of one k-block
+  const uint32_t r_bytes = NT * p.record_bytes;         // the records of one k-block
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int tile0 = blockIdx.x * NT, split = blockIdx.y, chunk0 = blockIdx.z * p.m_pad;
   const int nt_live = min(NT, p.n_tiles - tile0);
@@ -443,12 +443,18 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
   // Ring depths: a group visits every second stage, and it must meet every fill of the slots it waits on (a wait names a
   // fill by its parity only), so r_stages is a multiple of 2 * KC k-blocks and a_stages of 2.
   const int RS = p.r_stages;
+  // A slot holds the P k-blocks of one unit per tile: two tiles: slot n has k-blocks P n ..; one tile: slot 2 j + u has
+  // k-blocks 2 P j + u, 2 P j + u + 2, .. of accumulator u. own(u): k-blocks of accumulator u.
+  auto own = [&](int u) { return NT == 2 ? nkb : (nkb + 1 - u) / 2; };
+  const int n_slots = NT == 2 ? (nkb + P - 1) / P : (own(0) + P - 1) / P + (own(1) + P - 1) / P;
+  auto slot_kb = [&](int n) { return NT == 2 ? P * n : 2 * P * (n >> 1) + (n & 1); };
+  auto slot_live = [&](int n) { return NT == 2 ? min(P, nkb - P * n) : min(P, own(n & 1) - P * (n >> 1)); };
   const uint32_t col_stride = (uint32_t)(p.m_pad + 31) & ~31u;
   const uint32_t a_col0 = 2 * col_stride;               // first column of the A ring
 
   uint8_t* sB = smem;
-  uint8_t* sR = sB + (size_t)SB * b_bytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sR + (size_t)RS * r_stage);
+  uint8_t* sR = sB + (size_t)SB * P * b_bytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sR + (size_t)RS * P * r_bytes);
   uint64_t* raw_full = bars;
   uint64_t* raw_empty = raw_full + RS;
   uint64_t* b_full = raw_empty + RS;
@@ -484,10 +490,15 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
       RingPos rp;
       const uint8_t* src = p.records + (((size_t)(tile0 / QL_TILE_GROUP) * p.kblocks + kb0) * QL_TILE_GROUP + tile0 % QL_TILE_GROUP) * p.record_bytes;
       const uint32_t bytes = p.record_bytes * nt_live;
-      for (int i = 0; i < nkb; ++i, rp.advance(RS), src += (size_t)QL_TILE_GROUP * p.record_bytes) {
+      const size_t kb_pitch = (size_t)QL_TILE_GROUP * p.record_bytes;
+      for (int i = 0; i < n_slots; ++i, rp.advance(RS)) {
         if (!mbar_wait(&raw_empty[rp.stage], rp.phase ^ 1, p.status, KC_DEV_QLINEAR | 1)) break;
-        mbar_arrive_expect_tx(&raw_full[rp.stage], bytes);
-        bulk_g2s(sR + (size_t)rp.stage * r_stage, src, bytes, &raw_full[rp.stage]);
+        const int live = slot_live(i);
+        const uint8_t* from = src + slot_kb(i) * kb_pitch;
+        mbar_arrive_expect_tx(&raw_full[rp.stage], bytes * live);
+#pragma unroll
+        for (int q = 0; q < P; ++q)
+          if (q < live) bulk_g2s(sR + (size_t)(rp.stage * P + q) * r_bytes, from + q * KC * kb_pitch, bytes, &raw_full[rp.stage]);
       }
     }
   } else if (warp == 1) {
@@ -495,10 +506,14 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
     if (lane == 0) {
       pdl_wait();
       RingPos bp;
-      for (int i = 0; i < nkb; ++i, bp.advance(SB)) {
+      for (int i = 0; i < n_slots; ++i, bp.advance(SB)) {
         if (!mbar_wait(&b_empty[bp.stage], bp.phase ^ 1, p.status, KC_DEV_QLINEAR | 2)) break;
-        mbar_arrive_expect_tx(&b_full[bp.stage], b_bytes);
-        tma_load_2d(sB + (size_t)bp.stage * b_bytes, &map_rows, (kb0 + i) * QL_KB, p.row0 + chunk0, &b_full[bp.stage]);
+        const int live = slot_live(i), kb = kb0 + slot_kb(i);
+        mbar_arrive_expect_tx(&b_full[bp.stage], b_bytes * live);
+#pragma unroll
+        for (int q = 0; q < P; ++q)
+          if (q < live)
+            tma_load_2d(sB + (size_t)(bp.stage * P + q) * b_bytes, &map_rows, (kb + q * KC) * QL_KB, p.row0 + chunk0, &b_full[bp.stage]);
       }
     }
   } else if (warp < QL_DQ_WARP0) {
@@ -512,8 +527,8 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
       const uint32_t idesc = umma_idesc_bf16(QL_TILE_N, p.m_pad);
       const uint64_t proto = umma_smem_desc(0, 1024);
       const uint32_t d_hi = (uint32_t)(proto >> 32), b_lo0 = (uint32_t)proto | ((smem_u32(sB) >> 4) & 0x3FFF);
-      const uint32_t d_t = tmem_base + u * col_stride, a_t0 = tmem_base + a_col0 + u * 32;
-      const int n_own = NT == 2 ? nkb : (nkb + 1 - u) / 2;  // k-blocks of this accumulator
+      const uint32_t d_t = tmem_base + u * col_stride, a_t0 = tmem_base + a_col0 + u * 32 * P;
+      const int left0 = own(u), n_own = (left0 + P - 1) / P;   // k-blocks and units of this accumulator
       int as = 0, bs = NT == 2 ? 0 : u;                     // ring positions of the next one
       uint32_t aphase = 0, bphase = 0, acc = 0;
       bool ok = true, ready = false;
@@ -524,16 +539,21 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
           if (!ok) break;
         }
         tc_fence_after();   // the A operand was written with tcgen05.st by other threads
-        const uint32_t b_lo = b_lo0 + bs * (b_bytes >> 4), a_t = a_t0 + as * 64;
+        const uint32_t b_lo = b_lo0 + bs * P * (b_bytes >> 4), a_t = a_t0 + as * (64 * P);
         uint64_t *a_done = &a_empty[2 * as + u], *b_done = &b_empty[bs];
         if (++as == SA) { as = 0; aphase ^= 1u; }
         bs += KC;
         if (bs >= SB) { bs -= SB; bphase ^= 1u; }
         ready = i + 1 < n_own && (mbar_test_wait(&b_full[bs], bphase) & mbar_test_wait(&a_ready[2 * as + u], aphase));
+        const int live = left0 - P * i;
         if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < QL_KB / 16; ++ks)
-            umma_bf16_ts(d_t, a_t + 8 * ks, b_lo + 2 * ks, d_hi, idesc, ks == 0 ? acc : 1u);
+          for (int q = 0; q < P; ++q) {
+            if (q > 0 && q >= live) break;
+#pragma unroll
+            for (int ks = 0; ks < QL_KB / 16; ++ks)
+              umma_bf16_ts(d_t, a_t + 32 * q + 8 * ks, b_lo + q * (b_bytes >> 4) + 2 * ks, d_hi, idesc, q == 0 && ks == 0 ? acc : 1u);
+          }
           umma_commit(a_done);
           umma_commit(b_done);
         }
@@ -548,16 +568,16 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
     // Group g converts unit g & 1 of the stages g >> 1, (g >> 1) + 2, ...
     const int grp = (warp - QL_DQ_WARP0) >> 2, unit = grp & 1;
     const int row = (warp & 3) * 32 + lane;
-    const uint32_t a_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + a_col0 + unit * 32;
+    const uint32_t a_addr = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + a_col0 + unit * 32 * P;
     const int tile = NT == 2 ? unit : 0;
     const uint8_t* row_raw = sR + (size_t)tile * p.record_bytes + row * 16;
     const uint8_t* row_sb = sR + (size_t)tile * p.record_bytes + PACKED + row * (GPK * 4);
     int rs = NT == 2 ? grp >> 1 : (grp >> 1) * 2 + unit, as = grp >> 1;   // ring positions of the group's next unit
-    constexpr int R_STEP = 2 * KC;                      // k-blocks between a group's units
+    constexpr int R_STEP = 2 * KC;                      // slots between a group's units
     uint32_t rphase = 0, aphase = 0;
-    const int own = NT == 2 ? (unit < nt_live ? nkb : 0) : (nkb + 1 - unit) / 2;   // units of this accumulator: one per stage
+    const int left0 = NT == 2 && unit >= nt_live ? 0 : own(unit), units = (left0 + P - 1) / P;   // units: one per stage
     bool ok = true, released = false, raw_ready = false;
-    for (int i = grp >> 1; i < own; i += 2) {
+    for (int i = grp >> 1; i < units; i += 2) {
       // the first SA stages are dequantised under the tail of the previous kernel; a slot that is being reused is freed
       // by an MMA, which needs activations, which need the previous kernel: the bounded wait for it counts from there
       if (!released && i >= SA) { pdl_wait(); released = true; }
@@ -567,27 +587,35 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
       }
       // the slot's barrier is tested under the arithmetic, the next record's under the store (see the issuers)
       const bool a_free = mbar_test_wait(&a_empty[2 * as + unit], aphase ^ 1);
-      uint32_t v[32];
-      bf162 sb[GPK];
-      if (GPK == 1) {
-        sb[0] = *reinterpret_cast<const bf162*>(row_sb + (size_t)rs * r_stage);
-      } else {
-        const uint2 s = *reinterpret_cast<const uint2*>(row_sb + (size_t)rs * r_stage);
-        sb[0] = bf2_bits(s.x); sb[GPK - 1] = bf2_bits(s.y);
+      const uint32_t a_slot = a_addr + as * (64 * P);
+      const int live = left0 - P * i;
+#pragma unroll
+      for (int q = 0; q < P; ++q) {
+        if (q > 0 && q >= live) break;
+        const size_t at = (size_t)(rs * P + q) * r_bytes;
+        uint32_t v[32];
+        bf162 sb[GPK];
+        if (GPK == 1) {
+          sb[0] = *reinterpret_cast<const bf162*>(row_sb + at);
+        } else {
+          const uint2 s = *reinterpret_cast<const uint2*>(row_sb + at);
+          sb[0] = bf2_bits(s.x); sb[GPK - 1] = bf2_bits(s.y);
+        }
+        if (!p.wide) dequant_row<BITS, GPK>(row_raw + at, sb, v);
+        else dequant_row_wide<BITS, GPK>(row_raw + at, sb, v);
+        if (q == 0) {
+          if (!__all_sync(0xffffffffu, a_free)) ok = warp_wait(&a_empty[2 * as + unit], aphase ^ 1, p.status, KC_DEV_QLINEAR | 6);
+          if (!ok) break;
+          tc_fence_after();
+        }
+        tmem_st32(a_slot + 32 * q, v);
       }
-      if (!p.wide) dequant_row<BITS, GPK>(row_raw + (size_t)rs * r_stage, sb, v);
-      else dequant_row_wide<BITS, GPK>(row_raw + (size_t)rs * r_stage, sb, v);
+      if (!ok) break;
       __syncwarp();
-      if (lane == 0) mbar_arrive(&raw_empty[rs]);       // the record is in registers: its slot can refill
+      if (lane == 0) mbar_arrive(&raw_empty[rs]);       // the records are in registers: their slot can refill
       rs += R_STEP;
       if (rs >= RS) { rs -= RS; rphase ^= 1u; }
-      raw_ready = i + 2 < own && mbar_test_wait(&raw_full[rs], rphase);
-      if (!__all_sync(0xffffffffu, a_free)) {
-        ok = warp_wait(&a_empty[2 * as + unit], aphase ^ 1, p.status, KC_DEV_QLINEAR | 6);
-        if (!ok) break;
-      }
-      tc_fence_after();
-      tmem_st32(a_addr + as * 64, v);
+      raw_ready = i + 2 < units && mbar_test_wait(&raw_full[rs], rphase);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -612,18 +640,18 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
 
 // Ring depths and shared memory of one launch geometry; ok == false when it does not fit tensor or shared memory.
 struct TaPlan { bool ok; int sa, sb, rs; uint32_t tmem_cols; size_t smem; };
-static TaPlan plan_ta(int nt, int m_pad, uint32_t record_bytes) {
+static TaPlan plan_ta(int nt, int per, int m_pad, uint32_t record_bytes) {
   TaPlan t{};
   const int acc_cols = 2 * ((m_pad + 31) & ~31);
-  int sa = std::min(6, (512 - acc_cols) / 64) & ~1;
+  int sa = std::min(6 / per, (512 - acc_cols) / (64 * per)) & ~1;
   if (sa < 2 || m_pad > 256) return t;
   uint32_t cols = 32;
-  while ((int)cols < acc_cols + sa * 64) cols <<= 1;
+  while ((int)cols < acc_cols + sa * 64 * per) cols <<= 1;
   const size_t budget = (size_t)212 * 1024;
-  const size_t b_stage = (size_t)m_pad * 128;
-  const size_t r_stage = (size_t)nt * record_bytes;
+  const size_t b_stage = (size_t)per * m_pad * 128;
+  const size_t r_stage = (size_t)per * nt * record_bytes;
   // activations arrive from L2 (about 2000 cycles): up to 16 k-blocks ahead where they are small, 6 of 192 rows
-  int sb = (int)std::min<size_t>(16, std::max<size_t>(6, (size_t)(64 * 1024) / b_stage));
+  int sb = (int)std::min<size_t>(16 / per, std::max<size_t>(per == 1 ? 6 : 4, (size_t)(64 * 1024) / b_stage));
   while (sb > 4 && (size_t)sb * b_stage + (nt == 2 ? 6 : 8) * r_stage > budget) --sb;
   sb &= nt == 1 ? ~1 : ~0;   // one tile per CTA: an issuer takes every second k-block and must meet every fill of its slots
   if ((size_t)sb * b_stage + 4 * r_stage > budget) return t;
@@ -638,27 +666,29 @@ static TaPlan plan_ta(int nt, int m_pad, uint32_t record_bytes) {
   return t;
 }
 
-template <int BITS, int GPK, int NT>
+template <int BITS, int GPK, int NT, int P>
 static cudaError_t launch_umma_ta(const QLinearLaunch& l, QlKernelParams& p, cudaStream_t s) {
   const QWeight& w = *l.w;
-  const TaPlan t = plan_ta(NT, p.m_pad, p.record_bytes);
+  const TaPlan t = plan_ta(NT, P, p.m_pad, p.record_bytes);
   if (!t.ok) return cudaErrorInvalidValue;   // the caller sized the row chunk with plan_ta
   p.tmem_cols = t.tmem_cols;
   p.a_stages = t.sa; p.b_stages = t.sb; p.r_stages = t.rs;
   static DeviceOnce configured;   // the attribute belongs to the device's copy of the kernel
   if (configured.first_on_current_device()) {
-    cudaError_t e = cudaFuncSetAttribute(qlinear_umma_ta_kernel<BITS, GPK, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(qlinear_umma_ta_kernel<BITS, GPK, NT, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) { configured.forget_current_device(); return e; }
   }
   const CUtensorMap* rows = act_operand_rows_map(l.x, p.m_pad);
   if (!rows) return cudaErrorInvalidValue;
   dim3 grid((w.n_tiles + NT - 1) / NT, w.splits, (p.M + p.m_pad - 1) / p.m_pad);
-  return launch_k(qlinear_umma_ta_kernel<BITS, GPK, NT>, grid, dim3(QL_THREADS), t.smem, s, *rows, p);
+  return launch_k(qlinear_umma_ta_kernel<BITS, GPK, NT, P>, grid, dim3(QL_THREADS), t.smem, s, *rows, p);
 }
 
 template <int BITS, int GPK>
 static cudaError_t launch_umma_nt(const QLinearLaunch& l, QlKernelParams& p, int nt, cudaStream_t s) {
-  return nt == 2 ? launch_umma_ta<BITS, GPK, 2>(l, p, s) : launch_umma_ta<BITS, GPK, 1>(l, p, s);
+  if (plan_ta(nt, 2, p.m_pad, p.record_bytes).ok)
+    return nt == 2 ? launch_umma_ta<BITS, GPK, 2, 2>(l, p, s) : launch_umma_ta<BITS, GPK, 1, 2>(l, p, s);
+  return nt == 2 ? launch_umma_ta<BITS, GPK, 2, 1>(l, p, s) : launch_umma_ta<BITS, GPK, 1, 1>(l, p, s);
 }
 
 // Weight tiles per CTA: two when the grid then still has about 0.7 CTAs per SM (measured: 112 CTAs of two tiles beat
@@ -672,7 +702,7 @@ static int plan_tiles_per_cta(const QWeight& w, int sm_count) {
 static int plan_row_cap(int nt, uint32_t record_bytes) {
   static const int caps[] = {256, 192, 128, 64, 32, 16};
   for (int c : caps)
-    if (plan_ta(nt, c, record_bytes).ok) return c;
+    if (plan_ta(nt, 1, c, record_bytes).ok) return c;
   return 0;
 }
 
