@@ -63,6 +63,17 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
+// tanh(y). 1 - 2 / (e^(2 y) + 1) is good to 1e-7 of ONE, so where y is small the Taylor series to y^9 takes its place
+// (the next term is 1e-8 of y): a relative error of 6e-7 at most.
+__device__ __forceinline__ float softcap_unit(float y) {
+  const float y2 = y * y;
+  const float far = __fmaf_rn(-2.f, rcp_approx(ex2(fminf(y * 2.8853900817779268f, 120.f)) + 1.f), 1.f);
+  float c = __fmaf_rn(y2, 62.f / 2835.f, -17.f / 315.f);
+  c = __fmaf_rn(y2, c, 2.f / 15.f);
+  c = __fmaf_rn(y2, c, -1.f / 3.f);
+  return y2 < 0.0625f ? __fmaf_rn(y * y2, c, y) : far;
+}
+
 // Adds a chunk (o scaled by 2^-m, sum l) to what a row has accumulated: the weights of one merge.
 struct MergeW { float a, b, m; };
 __device__ __forceinline__ MergeW merge_weights(float m_acc, float m_chunk) {
@@ -155,20 +166,28 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  pdl_wait();   // everything below reads step data (units, q, block tables, this layer's K/V rows)
+  // Units and block tables reach the device before the step's first kernel and no kernel writes them, so the roles read
+  // them under the tail of the kernel before this one; q, K and V are loaded after pdl_wait.
 
   const int total = p.n_units * p.Hkv;
   if (warp == 0) {
     // ---- TMA producer. A chunk's block-table entries (at most ATT_CHUNK / 16 = 32) are fetched once, one per lane ----
     RingPos kv;
     uint32_t qphase = 0;
-    bool ok = true;
+    bool ok = true, waited = false;
     for (int r = 0, w; ok && r * (int)gridDim.x < total; ++r) {
       if ((w = unit_index(r, blockIdx.x, gridDim.x, total)) < 0) break;
       UnitTiles u;
       const int kvh = w % p.Hkv;
       u.open(p, w / p.Hkv, TK);
       if (!u.live()) continue;
+      const int32_t* tbl = p.block_tables + (size_t)u.seq * p.max_blocks;
+      const int bs_log2 = 31 - __clz(p.BS);
+      auto entries = [&]() {   // of the chunk. block_size is a power of two >= 16: chunks start on block edges
+        return lane < (u.keys + p.BS - 1) >> bs_log2 ? tbl[u.c * (ATT_CHUNK >> bs_log2) + lane] : 0;
+      };
+      int my_blk = entries(), loaded_c = u.c;
+      if (!waited) { pdl_wait(); waited = true; }
       ok = warp_wait(q_empty, qphase ^ 1, p.status, KC_DEV_ATTN | 1);
       if (!ok) break;
       qphase ^= 1;
@@ -178,33 +197,29 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
         for (int s = 0; s < S::SLABS; ++s)
           tma_load_5d(sQ + s * ATT_ROWS * 128, u.small ? &qmap_small : &qmap, 0, 0, s, kvh, u.tok0, q_full);
       }
-      const int32_t* tbl = p.block_tables + (size_t)u.seq * p.max_blocks;
-      int loaded_c = -1, my_blk = 0;
       for (; u.live() && ok; u.next(TK)) {
-        if (u.c != loaded_c) {
-          loaded_c = u.c;
-          const int nblk = (u.keys + p.BS - 1) / p.BS;
-          my_blk = lane < nblk ? tbl[u.c * (ATT_CHUNK / p.BS) + lane] : 0;   // block_size is a power of two >= 16: chunks start on block edges
-        }
+        if (u.c != loaded_c) { loaded_c = u.c; my_blk = entries(); }
         const int nb = u.blocks(TK);
         ok = warp_wait(&kv_empty[kv.stage], kv.phase ^ 1, p.status, KC_DEV_ATTN | 2);
         if (!ok) break;
         if (lane == 0) mbar_arrive_expect_tx(&kv_full[kv.stage], nb * 2 * S::GROUP_BYTES);
         uint8_t* dst = ring + (size_t)kv.stage * S::TILE_BYTES;
-        for (int b = 0; b < nb; ++b) {
-          const int koff = u.t * TK + b * 16;
-          const int blk = __shfl_sync(0xffffffffu, my_blk, koff / p.BS);
-          const int row = (blk * p.Hkv + kvh) * p.BS + koff % p.BS;   // of a plane
-          if (lane == 0) {
-            if (p.kv5d) {
-              tma_load_5d(dst + b * 2 * S::GROUP_BYTES, &kvmap, 0, 0, 0, p.layer * 2, row >> 3, &kv_full[kv.stage]);
-            } else {
-              for (int g = 0; g < 2; ++g)
-                for (int pl = 0; pl < 2; ++pl)
-                  for (int s = 0; s < S::SLABS; ++s)
-                    tma_load_2d(dst + (b * 2 + g) * S::GROUP_BYTES + (pl * S::SLABS + s) * 1024, &kvmap, s * 64,
-                                (int)((long long)(p.layer * 2 + pl) * p.NB * p.Hkv * p.BS) + row + g * 8, &kv_full[kv.stage]);
-            }
+        __syncwarp();   // the byte count is announced
+        // A lane issues the 16-key block of its index. One lane issuing them in turn, with a division by the block size
+        // each, took 340 cycles a block, 2800 of a tile's 3600: the bound of every step, whatever its rows.
+        const int koff = u.t * TK + lane * 16;
+        const int blk = __shfl_sync(0xffffffffu, my_blk, (koff >> bs_log2) & 31);
+        const int row = (blk * p.Hkv + kvh) * p.BS + (koff & (p.BS - 1));   // of a plane
+        if (lane < nb) {
+          uint8_t* to = dst + lane * 2 * S::GROUP_BYTES;
+          if (p.kv5d) {
+            tma_load_5d(to, &kvmap, 0, 0, 0, p.layer * 2, row >> 3, &kv_full[kv.stage]);
+          } else {
+            for (int g = 0; g < 2; ++g)
+              for (int pl = 0; pl < 2; ++pl)
+                for (int s = 0; s < S::SLABS; ++s)
+                  tma_load_2d(to + g * S::GROUP_BYTES + (pl * S::SLABS + s) * 1024, &kvmap, s * 64,
+                              (int)((long long)(p.layer * 2 + pl) * p.NB * p.Hkv * p.BS) + row + g * 8, &kv_full[kv.stage]);
           }
         }
         __syncwarp();
@@ -298,7 +313,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const float scale_log2 = p.scale * 1.4426950408889634f;
-    const float cap2 = p.softcap > 0.f ? 2.f * 1.4426950408889634f * p.scale / p.softcap : 0.f;   // exp2 argument of e^(2 x / cap)
+    const float cap_arg = p.softcap > 0.f ? p.scale / p.softcap : 0.f;
     const float cap_log2 = p.softcap * 1.4426950408889634f;
     int tile = 0, chunks = 0;
     bool ok = true;
@@ -321,53 +336,70 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
           tc_fence_after();
           const uint32_t s_addr = tmem + lane_addr + sb * TK;
           const int nb = u.blocks(TK), key0 = u.key0(TK);
-          uint32_t v[TK];
-#pragma unroll
-          for (int c = 0; c < TK / 32; ++c) tmem_ld32_issue(s_addr + c * 32, v + c * 32);   // columns past 16 nb hold an older tile's scores: masked below
-          tmem_wait_ld();
-          const bool capped = p.softcap > 0.f;
-          if (capped) {
-            // cap * tanh(x / cap) in log2 units: cap * (1 - 2 / (e^(2 x / cap) + 1)), accurate to about 1e-7 of cap
-#pragma unroll
-            for (int j = 0; j < TK; ++j) {
-              const float e = ex2(fminf(__uint_as_float(v[j]) * cap2, 120.f));
-              v[j] = __float_as_uint(cap_log2 - 2.f * cap_log2 * rcp_approx(e + 1.f));
-            }
-          }
-          const float mul = capped ? 1.f : scale_log2;
+          // columns of the tile that this row does not see: j > hi or j < lo. Columns past 16 nb hold an older tile's scores.
+          const int hi = pos - key0, lo = w_excl - key0 + 1;
           // every key of the tile is visible to every row of the unit: the same arithmetic without the predicates
-          if (!(nb * 16 == TK && key0 + TK - 1 <= u.pos0 && (p.window == 0 || key0 > u.pos_max - p.window))) {
+          const bool edge = !(nb * 16 == TK && key0 + TK - 1 <= u.pos0 && (p.window == 0 || key0 > u.pos_max - p.window));
+          auto load = [&](int c, uint32_t (&v)[64]) {
+            tmem_ld32_issue(s_addr + c * 64, v);
+            tmem_ld32_issue(s_addr + c * 64 + 32, v + 32);
+            tmem_wait_ld();
+            if (edge) {
 #pragma unroll
-            for (int j = 0; j < TK; ++j) {
-              const int key = key0 + j;
-              if (key > pos || key <= w_excl) v[j] = 0xff800000u;   // -inf
+              for (int j = 0; j < 64; ++j)
+                if (c * 64 + j > hi || c * 64 + j < lo) v[j] = 0xff800000u;   // -inf
+            }
+          };
+          // Two loops over 64 columns, each reading the scores from tensor memory: the same time as one pass over a row of
+          // 128 registers, in a third of the code. About 2100 cycles a tile: 330 the maximum, 1550 the exponentials (of
+          // which 1024 are the special-function unit's, a warp being alone on its scheduler).
+          float t0 = -INFINITY, t1 = -INFINITY, t2 = -INFINITY, t3 = -INFINITY;
+#pragma unroll 1
+          for (int c = 0; c < TK / 64; ++c) {
+            uint32_t v[64];
+            load(c, v);
+#pragma unroll
+            for (int j = 0; j < 64; j += 4) {
+              t0 = fmaxf(t0, __uint_as_float(v[j]));     t1 = fmaxf(t1, __uint_as_float(v[j + 1]));
+              t2 = fmaxf(t2, __uint_as_float(v[j + 2])); t3 = fmaxf(t3, __uint_as_float(v[j + 3]));
             }
           }
-          float t0 = -INFINITY, t1 = -INFINITY, t2 = -INFINITY, t3 = -INFINITY;
-#pragma unroll
-          for (int j = 0; j < TK; j += 4) {
-            t0 = fmaxf(t0, __uint_as_float(v[j]));     t1 = fmaxf(t1, __uint_as_float(v[j + 1]));
-            t2 = fmaxf(t2, __uint_as_float(v[j + 2])); t3 = fmaxf(t3, __uint_as_float(v[j + 3]));
-          }
-          const float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)) * mul;
+          const bool capped = p.softcap > 0.f;
+          const float mul = capped ? cap_log2 : scale_log2;
+          float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3));
+          if (capped && tmax > -INFINITY) tmax = softcap_unit(tmax * cap_arg);   // grows with the score
+          tmax *= mul;
           float alpha = 1.f;
           // The reference is the running maximum itself, not one that lags behind it by a few powers of two (which would
           // spare most rescales): the key with the most weight then has p = 1, which bf16 holds exactly.
           if (tmax > m) { alpha = ex2(m - tmax); m = tmax; }   // from -inf: alpha = 0
           const float ref = m == -INFINITY ? 0.f : m;
           float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+#pragma unroll 1
+          for (int c = 0; c < TK / 64; ++c) {
+            uint32_t v[64];
+            load(c, v);
+            if (capped) {
 #pragma unroll
-          for (int j = 0; j < TK; j += 4) {
-            const float p0 = ex2(__fmaf_rn(__uint_as_float(v[j]), mul, -ref)), p1 = ex2(__fmaf_rn(__uint_as_float(v[j + 1]), mul, -ref));
-            const float p2 = ex2(__fmaf_rn(__uint_as_float(v[j + 2]), mul, -ref)), p3 = ex2(__fmaf_rn(__uint_as_float(v[j + 3]), mul, -ref));
-            a0 += p0; a1 += p1; a2 += p2; a3 += p3;
-            v[j / 2] = pack_bf162(p0, p1);
-            v[j / 2 + 1] = pack_bf162(p2, p3);
+              for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(softcap_unit(__uint_as_float(v[j]) * cap_arg));
+              if (edge) {   // -inf has become -1
+#pragma unroll
+                for (int j = 0; j < 64; ++j)
+                  if (c * 64 + j > hi || c * 64 + j < lo) v[j] = 0xff800000u;
+              }
+            }
+#pragma unroll
+            for (int j = 0; j < 64; j += 4) {
+              const float p0 = ex2(__fmaf_rn(__uint_as_float(v[j]), mul, -ref)), p1 = ex2(__fmaf_rn(__uint_as_float(v[j + 1]), mul, -ref));
+              const float p2 = ex2(__fmaf_rn(__uint_as_float(v[j + 2]), mul, -ref)), p3 = ex2(__fmaf_rn(__uint_as_float(v[j + 3]), mul, -ref));
+              a0 += p0; a1 += p1; a2 += p2; a3 += p3;
+              v[j / 2] = pack_bf162(p0, p1);
+              v[j / 2 + 1] = pack_bf162(p2, p3);
+            }
+            tmem_st32(s_addr + c * 32, v);   // over scores that have been read
           }
           l = __fmaf_rn(l, alpha, (a0 + a1) + (a2 + a3));
-#pragma unroll
-          for (int c = 0; c < TK / 64; ++c) tmem_st32(s_addr + c * 32, v + c * 32);
-          if (!first && !__all_sync(0xffffffffu, alpha == 1.f)) {
+          if (!first && !__all_sync(0xffffffffu, alpha == 1.f || row >= u.rows)) {
             // a row's maximum moved: what O holds of it is rescaled once the previous tile's product is in
             const int pt = tile - 1;
             ok = warp_wait(&pv_done[pt & 1], (pt >> 1) & 1, p.status, KC_DEV_ATTN | 8);
@@ -405,6 +437,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     }
   } else if (warp >= 8) {
     // ---- a finished chunk: thread = query row ----
+    pdl_wait();   // the stores below may overwrite what an earlier kernel still reads
     const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     int chunks = 0;

@@ -256,10 +256,13 @@ add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __re
                        const int32_t* __restrict__ row_map, float eps, bf16* __restrict__ h_out,
                        bf16* __restrict__ normed) {
   if (!y.peers) pdl_launch_dependents();
-  pdl_wait();
-  if (y.peers) { tp_wait(y); pdl_launch_dependents(); }
   constexpr int H = 2048 * CPT;
   __shared__ float red[32];
+  uint4 wraw[CPT];   // a weight depends on no kernel: it arrives under the tail of the one before this
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) wraw[c] = w_out ? *reinterpret_cast<const uint4*>(w_out + (c * 256 + threadIdx.x) * 8) : make_uint4(0, 0, 0, 0);
+  pdl_wait();
+  if (y.peers) { tp_wait(y); pdl_launch_dependents(); }
   const int row = blockIdx.x;
   const size_t src = row_map ? row_map[row] : row;
   const bf16* xr = x + src * H;
@@ -315,8 +318,9 @@ add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __re
     const int i = (c * 256 + threadIdx.x) * 8;
     if (h_out) store8_bf16(h_out + (size_t)row * H + i, v[c]);
     if (w_out) {
-      float wv[8], o[8];
-      load8_bf16(w_out + i, wv);
+      const float2 w0 = unpack_bf162(wraw[c].x), w1 = unpack_bf162(wraw[c].y), w2 = unpack_bf162(wraw[c].z), w3 = unpack_bf162(wraw[c].w);
+      const float wv[8] = {w0.x, w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y};
+      float o[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) o[k] = wv[k] * (v[c][k] * inv);
       store8_bf16(normed + (size_t)row * H + i, o);
