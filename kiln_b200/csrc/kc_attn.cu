@@ -63,15 +63,40 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-// tanh(y). 1 - 2 / (e^(2 y) + 1) is good to 1e-7 of ONE, so where y is small the Taylor series to y^9 takes its place
-// (the next term is 1e-8 of y): a relative error of 6e-7 at most.
+// Two fp32 operations an instruction.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
+// tanh(y) for small y: the Taylor series to y^9 (below a quarter the next term is 1e-8 of y). y2 = y * y.
+__device__ __forceinline__ float2 softcap_series(float2 y, float2 y2) {
+  float2 c = fma2(y2, make_float2(62.f / 2835.f, 62.f / 2835.f), make_float2(-17.f / 315.f, -17.f / 315.f));
+  c = fma2(y2, c, make_float2(2.f / 15.f, 2.f / 15.f));
+  c = fma2(y2, c, make_float2(-1.f / 3.f, -1.f / 3.f));
+  return fma2(mul2(y, y2), c, y);
+}
+// tanh(y). 1 - 2 / (e^(2 y) + 1) is good to 1e-7 of ONE, so below a quarter the series takes its place: a relative error of
+// 6e-7 at most.
 __device__ __forceinline__ float softcap_unit(float y) {
   const float y2 = y * y;
   const float far = __fmaf_rn(-2.f, rcp_approx(ex2(fminf(y * 2.8853900817779268f, 120.f)) + 1.f), 1.f);
-  float c = __fmaf_rn(y2, 62.f / 2835.f, -17.f / 315.f);
-  c = __fmaf_rn(y2, c, 2.f / 15.f);
-  c = __fmaf_rn(y2, c, -1.f / 3.f);
-  return y2 < 0.0625f ? __fmaf_rn(y * y2, c, y) : far;
+  return y2 < 0.0625f ? softcap_series(make_float2(y, y), make_float2(y2, y2)).x : far;
 }
 
 // Adds a chunk (o scaled by 2^-m, sum l) to what a row has accumulated: the weights of one merge.
@@ -340,65 +365,66 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
           const int hi = pos - key0, lo = w_excl - key0 + 1;
           // every key of the tile is visible to every row of the unit: the same arithmetic without the predicates
           const bool edge = !(nb * 16 == TK && key0 + TK - 1 <= u.pos0 && (p.window == 0 || key0 > u.pos_max - p.window));
-          auto load = [&](int c, uint32_t (&v)[64]) {
-            tmem_ld32_issue(s_addr + c * 64, v);
-            tmem_ld32_issue(s_addr + c * 64 + 32, v + 32);
-            tmem_wait_ld();
-            if (edge) {
+          uint32_t v[TK];
 #pragma unroll
-              for (int j = 0; j < 64; ++j)
-                if (c * 64 + j > hi || c * 64 + j < lo) v[j] = 0xff800000u;   // -inf
-            }
+          for (int c = 0; c < TK / 32; ++c) tmem_ld32_issue(s_addr + c * 32, v + c * 32);
+          tmem_wait_ld();
+          auto mask = [&]() {
+#pragma unroll
+            for (int j = 0; j < TK; ++j)
+              if (j > hi || j < lo) v[j] = 0xff800000u;   // -inf
           };
-          // Two loops over 64 columns, each reading the scores from tensor memory: the same time as one pass over a row of
-          // 128 registers, in a third of the code. About 2100 cycles a tile: 330 the maximum, 1550 the exponentials (of
-          // which 1024 are the special-function unit's, a warp being alone on its scheduler).
+          if (edge) mask();
           float t0 = -INFINITY, t1 = -INFINITY, t2 = -INFINITY, t3 = -INFINITY;
-#pragma unroll 1
-          for (int c = 0; c < TK / 64; ++c) {
-            uint32_t v[64];
-            load(c, v);
 #pragma unroll
-            for (int j = 0; j < 64; j += 4) {
-              t0 = fmaxf(t0, __uint_as_float(v[j]));     t1 = fmaxf(t1, __uint_as_float(v[j + 1]));
-              t2 = fmaxf(t2, __uint_as_float(v[j + 2])); t3 = fmaxf(t3, __uint_as_float(v[j + 3]));
-            }
+          for (int j = 0; j < TK; j += 4) {
+            t0 = fmaxf(t0, __uint_as_float(v[j]));     t1 = fmaxf(t1, __uint_as_float(v[j + 1]));
+            t2 = fmaxf(t2, __uint_as_float(v[j + 2])); t3 = fmaxf(t3, __uint_as_float(v[j + 3]));
           }
-          const bool capped = p.softcap > 0.f;
-          const float mul = capped ? cap_log2 : scale_log2;
-          float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3));
-          if (capped && tmax > -INFINITY) tmax = softcap_unit(tmax * cap_arg);   // grows with the score
+          float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)), mul = scale_log2;
+          if (p.softcap > 0.f) {
+            mul = cap_log2;
+            // Most tiles hold no score past a quarter of the cap: the series alone, two at a time and without the
+            // special-function unit, which the exponentials below keep busy. An element's value is the same on both sides.
+            float b0 = INFINITY, b1 = INFINITY;
+#pragma unroll
+            for (int j = 0; j < TK; j += 2) { b0 = fminf(b0, __uint_as_float(v[j])); b1 = fminf(b1, __uint_as_float(v[j + 1])); }
+            const float reach = fmaxf(tmax, -fminf(b0, b1)) * cap_arg;
+            if (!edge && __all_sync(0xffffffffu, reach < 0.2499f)) {
+              const float2 arg = make_float2(cap_arg, cap_arg);
+#pragma unroll
+              for (int j = 0; j < TK; j += 2) {
+                const float2 y = mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg), y2 = mul2(y, y);
+                const float2 r = softcap_series(y, y2);
+                v[j] = __float_as_uint(r.x); v[j + 1] = __float_as_uint(r.y);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < TK; ++j) v[j] = __float_as_uint(softcap_unit(__uint_as_float(v[j]) * cap_arg));
+              if (edge) mask();   // -inf has become -1
+            }
+            if (tmax > -INFINITY) tmax = softcap_unit(tmax * cap_arg);   // grows with the score
+          }
           tmax *= mul;
           float alpha = 1.f;
           // The reference is the running maximum itself, not one that lags behind it by a few powers of two (which would
           // spare most rescales): the key with the most weight then has p = 1, which bf16 holds exactly.
           if (tmax > m) { alpha = ex2(m - tmax); m = tmax; }   // from -inf: alpha = 0
           const float ref = m == -INFINITY ? 0.f : m;
-          float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-#pragma unroll 1
-          for (int c = 0; c < TK / 64; ++c) {
-            uint32_t v[64];
-            load(c, v);
-            if (capped) {
+          const float2 muls = make_float2(mul, mul), refs = make_float2(-ref, -ref);
+          float2 s0 = make_float2(0.f, 0.f), s1 = s0;
 #pragma unroll
-              for (int j = 0; j < 64; ++j) v[j] = __float_as_uint(softcap_unit(__uint_as_float(v[j]) * cap_arg));
-              if (edge) {   // -inf has become -1
-#pragma unroll
-                for (int j = 0; j < 64; ++j)
-                  if (c * 64 + j > hi || c * 64 + j < lo) v[j] = 0xff800000u;
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < 64; j += 4) {
-              const float p0 = ex2(__fmaf_rn(__uint_as_float(v[j]), mul, -ref)), p1 = ex2(__fmaf_rn(__uint_as_float(v[j + 1]), mul, -ref));
-              const float p2 = ex2(__fmaf_rn(__uint_as_float(v[j + 2]), mul, -ref)), p3 = ex2(__fmaf_rn(__uint_as_float(v[j + 3]), mul, -ref));
-              a0 += p0; a1 += p1; a2 += p2; a3 += p3;
-              v[j / 2] = pack_bf162(p0, p1);
-              v[j / 2 + 1] = pack_bf162(p2, p3);
-            }
-            tmem_st32(s_addr + c * 32, v);   // over scores that have been read
+          for (int j = 0; j < TK; j += 4) {
+            float2 e = fma2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), muls, refs);
+            float2 f = fma2(make_float2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), muls, refs);
+            e.x = ex2(e.x); e.y = ex2(e.y); f.x = ex2(f.x); f.y = ex2(f.y);
+            s0 = add2(s0, e); s1 = add2(s1, f);
+            v[j / 2] = pack_bf162(e.x, e.y);
+            v[j / 2 + 1] = pack_bf162(f.x, f.y);
           }
-          l = __fmaf_rn(l, alpha, (a0 + a1) + (a2 + a3));
+#pragma unroll
+          for (int c = 0; c < TK / 64; ++c) tmem_st32(s_addr + c * 32, v + c * 32);
+          l = __fmaf_rn(l, alpha, (s0.x + s0.y) + (s1.x + s1.y));
           if (!first && !__all_sync(0xffffffffu, alpha == 1.f || row >= u.rows)) {
             // a row's maximum moved: what O holds of it is rescaled once the previous tile's product is in
             const int pt = tile - 1;
