@@ -375,11 +375,14 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
               if (j > hi || j < lo) v[j] = 0xff800000u;   // -inf
           };
           if (edge) mask();
+          // three operands an instruction
           float t0 = -INFINITY, t1 = -INFINITY, t2 = -INFINITY, t3 = -INFINITY;
 #pragma unroll
-          for (int j = 0; j < TK; j += 4) {
-            t0 = fmaxf(t0, __uint_as_float(v[j]));     t1 = fmaxf(t1, __uint_as_float(v[j + 1]));
-            t2 = fmaxf(t2, __uint_as_float(v[j + 2])); t3 = fmaxf(t3, __uint_as_float(v[j + 3]));
+          for (int j = 0; j < TK; j += 8) {
+            t0 = fmaxf(t0, fmaxf(__uint_as_float(v[j]), __uint_as_float(v[j + 1])));
+            t1 = fmaxf(t1, fmaxf(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])));
+            t2 = fmaxf(t2, fmaxf(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5])));
+            t3 = fmaxf(t3, fmaxf(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7])));
           }
           float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)), mul = scale_log2;
           if (p.softcap > 0.f) {

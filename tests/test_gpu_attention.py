@@ -133,3 +133,47 @@ def test_one_operation_per_tile_pair_matches_the_slab_loads(ctx, monkeypatch, hd
         b = api.paged_attention(ctx, kv2, layer, q, seqs, hd ** -0.5).cpu()
         assert torch.equal(a.view(torch.int16), b.view(torch.int16)), f"layer {layer}"
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("hd,heads,kvh,softcap,window", [(128, 8, 4, 0.0, 0), (64, 16, 4, 0.0, 700), (128, 8, 8, 30.0, 0)])
+def test_units_of_whole_rows_carry_the_bits_of_single_chunks(ctx, hd, heads, kvh, softcap, window):
+    """Many long sequences in one step: a unit holds all chunks of its rows and merges them itself. One sequence alone: a
+    unit per chunk, merged by the combine kernel. Same bits, with lengths on both sides of tile and chunk edges."""
+    rng = np.random.default_rng(3)
+    lens = [511, 512, 513, 1023, 1024, 1151, 1537] + [int(v) for v in rng.integers(600, 1600, 73)]
+    bs, rows = 16, 3
+    nb = sum((n + rows + bs - 1) // bs for n in lens)
+    kv = api.PagedKv(ctx, api.KvSpec(1, kvh, hd, nb, bs))
+    data = outlier_values((64, kv.bytes_per_block() // 2), 51)
+    for b in range(64):
+        kv.write_block_bytes(b, data[b].view(torch.uint8).numpy().tobytes())
+    for b in range(64, nb):
+        kv.copy_block(b % 61, b)
+    seqs = build_seqs([(rows, n) for n in lens], bs, nb, 52)
+    q = outlier_values((rows * len(lens), heads, hd), 53).cuda()
+    scale = hd ** -0.5
+    batched = api.paged_attention(ctx, kv, 0, q, seqs, scale, softcap, window).cpu()
+    for i, s in enumerate(seqs[:12]):
+        one = api.paged_attention(ctx, kv, 0, q[rows * i: rows * (i + 1)].contiguous(), [s], scale, softcap, window).cpu()
+        assert torch.equal(one.view(torch.int16), batched[rows * i: rows * (i + 1)].view(torch.int16)), f"sequence {i}"
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("gain", [0.05, 1.0, 20.0])
+def test_softcap_on_both_sides_of_the_series(ctx, gain):
+    """Scores far below, around and beyond the cap against fp64. Bound: probabilities and output are rounded to bf16 (2^-9
+    each, of outputs of order one); the cap itself adds under 1e-5."""
+    hd, heads, kvh, bs, n = 128, 4, 1, 16, 300
+    kv = api.PagedKv(ctx, api.KvSpec(1, kvh, hd, 20, bs))
+    g = torch.Generator().manual_seed(61)
+    k = torch.empty(19 * bs, hd).normal_(generator=g).to(torch.bfloat16)
+    v = torch.empty(19 * bs, hd).normal_(generator=g).to(torch.bfloat16)
+    for b in range(19):
+        kv.write_block_bytes(b, torch.cat([k[b * bs: (b + 1) * bs].reshape(-1), v[b * bs: (b + 1) * bs].reshape(-1)]).view(torch.uint8).numpy().tobytes())
+    q = (torch.empty(2, heads, hd).normal_(generator=g) * gain).to(torch.bfloat16)
+    got = api.paged_attention(ctx, kv, 0, q.cuda(), [api.SeqStep(2, n, 2, list(range(19)))], hd ** -0.5, 5.0, 0).cpu().double()
+    for t in range(2):
+        x = q[t].double() @ k[: n + t + 1].double().T * hd ** -0.5
+        want = torch.softmax(5.0 * torch.tanh(x / 5.0), -1) @ v[: n + t + 1].double()
+        assert float((got.reshape(2, heads, hd)[t] - want).abs().max()) < 2 ** -8 * max(1.0, float(want.abs().max()))
+    assert ctx.device_status() == 0
