@@ -84,19 +84,24 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
   return r;
 }
 
-// tanh(y) for small y: the Taylor series to y^9 (below a quarter the next term is 1e-8 of y). y2 = y * y.
-__device__ __forceinline__ float2 softcap_series(float2 y, float2 y2) {
-  float2 c = fma2(y2, make_float2(62.f / 2835.f, 62.f / 2835.f), make_float2(-17.f / 315.f, -17.f / 315.f));
-  c = fma2(y2, c, make_float2(2.f / 15.f, 2.f / 15.f));
-  c = fma2(y2, c, make_float2(-1.f / 3.f, -1.f / 3.f));
-  return fma2(mul2(y, y2), c, y);
+// tanh(y) for |y| < sqrt(SOFTCAP_NEAR): the convergent y (y^6 + 378 y^4 + 17325 y^2 + 135135) / (28 y^6 + 3150 y^4 + 62370 y^2
+// + 135135) of its continued fraction, a relative error of 3e-7 at most, one special-function operation an element.
+constexpr float SOFTCAP_NEAR = 5.f;
+__device__ __forceinline__ float2 softcap_near(float2 y) {
+  auto both = [](float x) { return make_float2(x, x); };
+  const float2 y2 = mul2(y, y);
+  float2 n = add2(y2, both(378.f));
+  n = fma2(n, y2, both(17325.f));
+  n = fma2(n, y2, both(135135.f));
+  float2 d = fma2(y2, both(28.f), both(3150.f));
+  d = fma2(d, y2, both(62370.f));
+  d = fma2(d, y2, both(135135.f));
+  return mul2(mul2(y, n), make_float2(rcp_approx(d.x), rcp_approx(d.y)));
 }
-// tanh(y). 1 - 2 / (e^(2 y) + 1) is good to 1e-7 of ONE, so below a quarter the series takes its place: a relative error of
-// 6e-7 at most.
-__device__ __forceinline__ float softcap_unit(float y) {
-  const float y2 = y * y;
+// tanh(y) anywhere: further out 1 - 2 / (e^(2 y) + 1), good to 1e-7.
+__device__ __forceinline__ float softcap_any(float y, float near) {
   const float far = __fmaf_rn(-2.f, rcp_approx(ex2(fminf(y * 2.8853900817779268f, 120.f)) + 1.f), 1.f);
-  return y2 < 0.0625f ? softcap_series(make_float2(y, y), make_float2(y2, y2)).x : far;
+  return y * y < SOFTCAP_NEAR ? near : far;
 }
 
 // Adds a chunk (o scaled by 2^-m, sum l) to what a row has accumulated: the weights of one merge.
@@ -387,26 +392,30 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
           float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)), mul = scale_log2;
           if (p.softcap > 0.f) {
             mul = cap_log2;
-            // Most tiles hold no score past a quarter of the cap: the series alone, two at a time and without the
-            // special-function unit, which the exponentials below keep busy. An element's value is the same on both sides.
+            // A tile with no score past 2.2 caps takes the fraction alone, two elements at a time; an element's value is the
+            // same on both sides.
             float b0 = INFINITY, b1 = INFINITY;
 #pragma unroll
             for (int j = 0; j < TK; j += 2) { b0 = fminf(b0, __uint_as_float(v[j])); b1 = fminf(b1, __uint_as_float(v[j + 1])); }
             const float reach = fmaxf(tmax, -fminf(b0, b1)) * cap_arg;
-            if (!edge && __all_sync(0xffffffffu, reach < 0.2499f)) {
-              const float2 arg = make_float2(cap_arg, cap_arg);
+            const bool all_near = __all_sync(0xffffffffu, reach < 2.23f);   // false where a mask has left -inf
+            const float2 arg = make_float2(cap_arg, cap_arg);
+            if (all_near) {
 #pragma unroll
               for (int j = 0; j < TK; j += 2) {
-                const float2 y = mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg), y2 = mul2(y, y);
-                const float2 r = softcap_series(y, y2);
+                const float2 r = softcap_near(mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg));
                 v[j] = __float_as_uint(r.x); v[j + 1] = __float_as_uint(r.y);
               }
             } else {
 #pragma unroll
-              for (int j = 0; j < TK; ++j) v[j] = __float_as_uint(softcap_unit(__uint_as_float(v[j]) * cap_arg));
+              for (int j = 0; j < TK; j += 2) {
+                const float2 y = mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg);
+                const float2 r = softcap_near(y);
+                v[j] = __float_as_uint(softcap_any(y.x, r.x)); v[j + 1] = __float_as_uint(softcap_any(y.y, r.y));
+              }
               if (edge) mask();   // -inf has become -1
             }
-            if (tmax > -INFINITY) tmax = softcap_unit(tmax * cap_arg);   // grows with the score
+            if (tmax > -INFINITY) { tmax *= cap_arg; tmax = softcap_any(tmax, softcap_near(make_float2(tmax, tmax)).x); }   // grows with the score
           }
           tmax *= mul;
           float alpha = 1.f;
