@@ -24,6 +24,11 @@
 //   warp 1      issues the MMAs: QK of tile i + 1 before PV of tile i
 //   warps 4-7   softmax, one row per thread: S -> P, rescaling O when a row's maximum moved
 //   warps 8-11  a finished chunk's O: store the partial, or merge it into the row and store the row
+//
+// What bounds it: per 128-key tile of head size 128, HBM takes 2800 cycles of an SM's share, a softmax warp about 2400
+// (scores and maximum 430, 128 exponentials 1300, of which 1024 the special-function unit's, stores 280, next tile 375),
+// the MMAs 1024. Against one mma.sync warp per 16 query rows with a combine launch: 32 sequences of 1438 keys and 6 rows
+// 69.1 -> 55.8 us; prefill of 2048 tokens after 2048 on the 8B model 64.9 -> 43.2 ms, its attention now 140 us a layer.
 #include "kc_attn.cuh"
 
 #include "kc_umma.cuh"
@@ -674,8 +679,9 @@ bool attn_whole(int head_dim, const int* item_tiles, int n_items, int kv_heads, 
       if (w >= 0) load[c] += item_tiles[w / kv_heads];
     }
   for (int c = 0; c < ctas; ++c) most = std::max<long long>(most, load[c]);
-  // Whole rows save the partials' round trip through memory and the combine launch (about a tenth of a step of 32 long
-  // sequences); units of one chunk, 4 tiles, are for steps whose items leave SMs idle for longer than that.
+  // Four tiles are one chunk: nothing to split. Whole rows save the partials' round trip through memory and the combine
+  // launch (about a tenth of a step of 32 long sequences); units of one chunk are for steps whose items leave SMs idle
+  // for longer than that.
   return most <= 4 || most * sm_count * 4 <= sum * 5;
 }
 
