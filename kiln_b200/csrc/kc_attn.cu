@@ -403,7 +403,8 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
 #pragma unroll
             for (int j = 0; j < TK; j += 2) { b0 = fminf(b0, __uint_as_float(v[j])); b1 = fminf(b1, __uint_as_float(v[j + 1])); }
             const float reach = fmaxf(tmax, -fminf(b0, b1)) * cap_arg;
-            const bool all_near = __all_sync(0xffffffffu, reach < 2.23f);   // false where a mask has left -inf
+            // false where a mask has left -inf; rows past the unit's hold whatever shared memory held and have no say
+            const bool all_near = __all_sync(0xffffffffu, reach < 2.23f || row >= u.rows);
             const float2 arg = make_float2(cap_arg, cap_arg);
             if (all_near) {
 #pragma unroll
