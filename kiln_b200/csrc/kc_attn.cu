@@ -348,8 +348,13 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
     const float scale_log2 = p.scale * 1.4426950408889634f;
-    const float cap_arg = p.softcap > 0.f ? p.scale / p.softcap : 0.f;
+    const bool capped = p.softcap > 0.f;
+    const float cap_arg = capped ? p.scale / p.softcap : 0.f;
     const float cap_log2 = p.softcap * 1.4426950408889634f;
+    // The scale goes into the multiplier of the exponent, behind mask and maximum: right for a positive one only (a
+    // masked -inf times 0 is NaN, times a negative scale +inf). With any other scale, and with factors that leave the
+    // range of fp32, the scores are scaled and capped where they lie first.
+    const bool folded = p.scale > 0.f && scale_log2 < INFINITY && (!capped || (cap_arg > 0.f && cap_arg < INFINITY && cap_log2 < INFINITY));
     int tile = 0, chunks = 0;
     bool ok = true;
     for (int r = 0, w; ok && r * (int)gridDim.x < total; ++r) {
@@ -375,6 +380,21 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
           const int hi = pos - key0, lo = w_excl - key0 + 1;
           // every key of the tile is visible to every row of the unit: the same arithmetic without the predicates
           const bool edge = !(nb * 16 == TK && key0 + TK - 1 <= u.pos0 && (p.window == 0 || key0 > u.pos_max - p.window));
+          if (!folded) {
+#pragma unroll 1
+            for (int c = 0; c < TK / 32; ++c) {
+              uint32_t x[32];
+              tmem_ld32(s_addr + c * 32, x);
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                float f = __uint_as_float(x[j]) * p.scale;
+                if (capped) f = p.softcap * tanhf(f / p.softcap);
+                x[j] = __float_as_uint(f);
+              }
+              tmem_st32(s_addr + c * 32, x);
+            }
+            tmem_wait_st();
+          }
           uint32_t v[TK];
 #pragma unroll
           for (int c = 0; c < TK / 32; ++c) tmem_ld32_issue(s_addr + c * 32, v + c * 32);
@@ -394,8 +414,8 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
             t2 = fmaxf(t2, fmaxf(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5])));
             t3 = fmaxf(t3, fmaxf(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7])));
           }
-          float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)), mul = scale_log2;
-          if (p.softcap > 0.f) {
+          float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)), mul = folded ? scale_log2 : 1.4426950408889634f;
+          if (capped && folded) {
             mul = cap_log2;
             // A tile with no score past 2.2 caps takes the fraction alone, two elements at a time; an element's value is the
             // same on both sides.

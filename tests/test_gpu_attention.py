@@ -177,3 +177,27 @@ def test_softcap_over_its_range(ctx, gain):
         want = torch.softmax(5.0 * torch.tanh(x / 5.0), -1) @ v[: n + t + 1].double()
         assert float((got.reshape(2, heads, hd)[t] - want).abs().max()) < 2 ** -8 * max(1.0, float(want.abs().max()))
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.125, -4.0, 1e-3])
+@pytest.mark.parametrize("hd,softcap,window", [(64, 0.0, 0), (128, 5.0, 0), (256, 3.0, 40)])
+def test_any_scale(ctx, scale, hd, softcap, window):
+    """Scales that turn the order of the scores round or make them all equal, against fp64, with keys on both sides of the
+    mask in the last tile. Bound: the test above's."""
+    heads, kvh, bs, n, rows = 4, 1, 16, 300, 3
+    kv = api.PagedKv(ctx, api.KvSpec(1, kvh, hd, 20, bs))
+    g = torch.Generator().manual_seed(71)
+    k = torch.empty(19 * bs, hd).normal_(generator=g).to(torch.bfloat16)
+    v = torch.empty(19 * bs, hd).normal_(generator=g).to(torch.bfloat16)
+    for b in range(19):
+        kv.write_block_bytes(b, torch.cat([k[b * bs: (b + 1) * bs].reshape(-1), v[b * bs: (b + 1) * bs].reshape(-1)]).view(torch.uint8).numpy().tobytes())
+    q = torch.empty(rows, heads, hd).normal_(generator=g).to(torch.bfloat16)
+    got = api.paged_attention(ctx, kv, 0, q.cuda(), [api.SeqStep(rows, n, rows, list(range(19)))], scale, softcap, window).cpu().double()
+    for t in range(rows):
+        first = max(0, n + t - window + 1) if window else 0
+        x = q[t].double() @ k[first: n + t + 1].double().T * scale
+        if softcap:
+            x = softcap * torch.tanh(x / softcap)
+        want = torch.softmax(x, -1) @ v[first: n + t + 1].double()
+        assert float((got.reshape(rows, heads, hd)[t] - want).abs().max()) < 2 ** -8 * max(1.0, float(want.abs().max()))
+    assert ctx.device_status() == 0
