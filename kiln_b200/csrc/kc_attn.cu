@@ -103,9 +103,9 @@ __device__ __forceinline__ float2 softcap_near(float2 y) {
   d = fma2(d, y2, both(135135.f));
   return mul2(mul2(y, n), make_float2(rcp_approx(d.x), rcp_approx(d.y)));
 }
-// tanh(y) anywhere: further out 1 - 2 / (e^(2 y) + 1), good to 1e-7.
+// tanh(y) anywhere: further out 1 - 2 / (e^(2 y) + 1), good to 1e-7; 1 and -1 at the infinities, NaN stays NaN.
 __device__ __forceinline__ float softcap_any(float y, float near) {
-  const float far = __fmaf_rn(-2.f, rcp_approx(ex2(fminf(y * 2.8853900817779268f, 120.f)) + 1.f), 1.f);
+  const float far = __fmaf_rn(-2.f, rcp_approx(ex2(y * 2.8853900817779268f) + 1.f), 1.f);
   return y * y < SOFTCAP_NEAR ? near : far;
 }
 
@@ -441,7 +441,8 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
               }
               if (edge) mask();   // -inf has become -1
             }
-            if (tmax > -INFINITY) { tmax *= cap_arg; tmax = softcap_any(tmax, softcap_near(make_float2(tmax, tmax)).x); }   // grows with the score
+            const bool seen = !edge || (hi >= 0 && lo < TK && lo <= hi);   // any key: a score of -inf is a key of weight e^-cap
+            if (seen) { tmax *= cap_arg; tmax = softcap_any(tmax, softcap_near(make_float2(tmax, tmax)).x); }   // grows with the score
           }
           tmax *= mul;
           float alpha = 1.f;

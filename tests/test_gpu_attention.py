@@ -201,3 +201,37 @@ def test_any_scale(ctx, scale, hd, softcap, window):
         want = torch.softmax(x, -1) @ v[first: n + t + 1].double()
         assert float((got.reshape(rows, heads, hd)[t] - want).abs().max()) < 2 ** -8 * max(1.0, float(want.abs().max()))
     assert ctx.device_status() == 0
+
+
+def test_softcap_of_scores_that_are_not_finite(ctx):
+    """Under the cap an infinite score is plus or minus the cap, also where every key that a row sees has one; a NaN score
+    makes the rows NaN that see it, and no other."""
+    hd, heads, kvh, bs, n, cap = 64, 2, 1, 16, 180, 4.0
+    g = torch.Generator().manual_seed(81)
+    k = torch.empty(12 * bs, hd).normal_(generator=g) * 6
+    v = torch.empty(12 * bs, hd).normal_(generator=g).to(torch.bfloat16)
+    k[40], k[50] = 3e38, -3e38
+    k[140:144] = -3e38
+    k[182] = float("nan")
+    k = k.to(torch.bfloat16)
+    kv = api.PagedKv(ctx, api.KvSpec(1, kvh, hd, 12, bs))
+    for b in range(12):
+        kv.write_block_bytes(b, torch.cat([k[b * bs: (b + 1) * bs].reshape(-1), v[b * bs: (b + 1) * bs].reshape(-1)]).view(torch.uint8).numpy().tobytes())
+    q = (torch.empty(5, heads, hd).uniform_(0.5, 1.5, generator=g)).to(torch.bfloat16)
+
+    def check(offset, rows, window):
+        got = api.paged_attention(ctx, kv, 0, q[:rows].cuda(), [api.SeqStep(rows, offset, rows, list(range(12)))], hd ** -0.5, cap, window)
+        got = got.cpu().double().reshape(rows, heads, hd)
+        for t in range(rows):
+            first = max(0, offset + t - window + 1) if window else 0
+            x = torch.nan_to_num(q[t].double() @ k[first: offset + t + 1].double().T, nan=float("nan")) * hd ** -0.5
+            x = torch.where(x.abs() > 1e38, x.sign() * float("inf"), x)          # sums of fp32 products beyond its range
+            want = torch.softmax(cap * torch.tanh(x / cap), -1) @ v[first: offset + t + 1].double()
+            if offset + t >= 182:
+                assert bool(torch.isnan(got[t]).all())
+            else:
+                assert float((got[t] - want).abs().max()) < 2 ** -8 * max(1.0, float(want.abs().max()))
+
+    check(n, 5, 0)      # rows 0 and 1 before the NaN, 2 .. 4 from it on
+    check(143, 3, 4)    # row 0 sees four keys of score -inf and no other
+    assert ctx.device_status() == 0
