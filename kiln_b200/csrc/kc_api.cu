@@ -71,7 +71,8 @@ struct kc_ctx {
   int sm_count = 148;
   cudaStream_t stream = nullptr;
   // Status word: pinned host memory mapped into the device's address space. A kernel writes it only when one of its
-  // bounded waits gives up, so the host reads it after a synchronisation without a copy in the stream.
+  // bounded waits gives up, so the host reads it after a synchronisation without a copy in the stream. A pipelined
+  // launch, which is collected without one, keeps a copy of its own (kc_decode_launch).
   uint32_t* status = nullptr;             // the device's address of it
   volatile uint32_t* status_host = nullptr;
   kc_model* op = nullptr;                 // metadata and workspace of the single-op entry points (op_shell)
@@ -210,12 +211,10 @@ struct kc_model {
   uint8_t* result_host = nullptr;      // pinned
   // pipelined decode: launch k keeps its sampled tokens in slot k % 2 until launch k + 2 reuses it
   uint32_t* pipe_tokens[2] = {nullptr, nullptr};   // device [max_seqs]
-  uint32_t* pipe_host[2] = {nullptr, nullptr};     // pinned [max_seqs], written by the sampling kernel
+  uint32_t* pipe_host[2] = {nullptr, nullptr};     // pinned [max_seqs + 1], written by the sampling kernel: tokens, status word
   cudaEvent_t pipe_ev[2] = {nullptr, nullptr};
   int pipe_n[2] = {0, 0};
   uint64_t pipe_ticket = 0;                        // of the most recent launch; 0 = none yet
-  uint32_t pipe_bad = 0;                           // status of a bounded wait that gave up in a launch up to pipe_bad_upto
-  uint64_t pipe_bad_upto = 0;
 };
 
 static size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -985,7 +984,7 @@ extern "C" int kc_model_load(kc_ctx_t c, const kc_model_desc* desc, const kc_ten
     for (int i = 0; i < kc_model::kStaging && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&m->meta_ev[i], cudaEventDisableTiming);
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) {
       e = cudaMalloc(&m->pipe_tokens[i], (size_t)m->max_seqs * 4);
-      if (e == cudaSuccess) e = cudaMallocHost(&m->pipe_host[i], (size_t)m->max_seqs * 4);
+      if (e == cudaSuccess) e = cudaMallocHost(&m->pipe_host[i], ((size_t)m->max_seqs + 1) * 4);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&m->pipe_ev[i], cudaEventDisableTiming);
     }
     if (e != cudaSuccess) LOAD_FAIL(fail(KC_ERR_OOM, "kc_model_load: result buffers: %s", cudaGetErrorString(e)));
@@ -1576,7 +1575,8 @@ extern "C" int kc_decode_launch(kc_model_t m, kc_kv_t kv, const uint32_t* token_
   if ((rc = run_forward(m, kv, tokens_dev, p, true))) return rc;
   const uint64_t ticket = m->pipe_ticket + 1;
   const int slot = (int)(ticket % 2);
-  LAUNCH(c, KC_PROF_SAMPLE, 1, launch_greedy_rows(m->logits, n_seqs, m->d.vocab_size, 1, m->pipe_tokens[slot], c->stream, m->pipe_host[slot]));
+  LAUNCH(c, KC_PROF_SAMPLE, 1, launch_greedy_rows(m->logits, n_seqs, m->d.vocab_size, 1, m->pipe_tokens[slot], c->stream, m->pipe_host[slot],
+                                                 c->status, m->pipe_host[slot] + m->max_seqs));
   CK(cudaEventRecord(m->pipe_ev[slot], c->stream));
   m->pipe_ticket = ticket;
   m->pipe_n[slot] = n_seqs;
@@ -1594,12 +1594,12 @@ extern "C" int kc_decode_collect(kc_model_t m, uint64_t ticket, uint32_t* row_to
   kc_ctx* c = m->ctx;
   CK(cudaSetDevice(c->device));
   CK(cudaEventSynchronize(m->pipe_ev[slot]));
-  // The status word is the context's: a wait that gave up in the launch behind this one shows here as well. Every
-  // launch queued so far is then reported as failed, whichever of them it was.
-  const uint32_t now = *c->status_host;
-  if (now) { *c->status_host = 0; m->pipe_bad = now; m->pipe_bad_upto = m->pipe_ticket; }
-  if (m->pipe_bad && ticket <= m->pipe_bad_upto) {
-    const uint32_t st = m->pipe_bad;
+  // The launch's own copy of the status word, taken in stream order: what another call has read and cleared since is
+  // still in it, what a launch behind this one left is not. The word itself is cleared in stream order too, so that the
+  // launches already behind this one, which may be fed from it, have it in their copies.
+  const uint32_t st = m->pipe_host[slot][m->max_seqs];
+  if (st) {
+    CK(cudaMemsetAsync(c->status, 0, sizeof(uint32_t), c->stream));
     return fail(KC_ERR_TIMEOUT, "kc_decode_collect: device status 0x%x: a bounded wait gave up (kernel 0x%x, wait %u); the tokens of "
                 "this launch and of any launch fed from it are not valid", st, st & 0xff00u, st & 0xffu);
   }

@@ -80,9 +80,11 @@ cudaError_t launch_copy_block(bf16* pool, int layers, int NB, size_t block_elems
                               cudaStream_t s);
 
 // Greedy token per logits row; see kc_greedy_rows in kiln_cuda.h. tokens_host (optional): pinned host memory that gets
-// the same tokens.
+// the same tokens. status_copy (optional): pinned host memory that gets what *status holds once everything before this
+// kernel in the stream has run.
 cudaError_t launch_greedy_rows(const bf16* logits, int rows, int vocab, int normalize, uint32_t* tokens,
-                               cudaStream_t s, uint32_t* tokens_host = nullptr);
+                               cudaStream_t s, uint32_t* tokens_host = nullptr, const uint32_t* status = nullptr,
+                               uint32_t* status_copy = nullptr);
 // tokens[i] = prev[feed[i]] where feed[i] >= 0: the device-side token feedback of kc_decode_launch.
 cudaError_t launch_feed_tokens(uint32_t* tokens, const int32_t* feed, const uint32_t* prev, int n, int prev_n, cudaStream_t s);
 // The settle walk per verify segment; see kc_verify_accept in kiln_cuda.h.

@@ -26,9 +26,11 @@ __device__ __forceinline__ ArgMax better(ArgMax a, ArgMax b) {
 // normalize == 0: argmax of the raw row (crates/kiln-models/src/draft.rs:379-381).
 __global__ void __launch_bounds__(1024)
 greedy_rows_kernel(const bf16* __restrict__ logits, int vocab, int normalize, uint32_t* __restrict__ tokens,
-                   uint32_t* __restrict__ tokens_host) {
+                   uint32_t* __restrict__ tokens_host, const volatile uint32_t* status, uint32_t* __restrict__ status_copy) {
   pdl_launch_dependents();
   pdl_wait();
+  const bool notes = status_copy && blockIdx.x == 0 && threadIdx.x == 0;
+  const uint32_t st = notes ? *status : 0u;   // host memory: on its way under the passes below
   __shared__ float red_m[32];
   __shared__ double red_s[32];
   __shared__ ArgMax red_a[32];
@@ -118,6 +120,7 @@ greedy_rows_kernel(const bf16* __restrict__ logits, int vocab, int normalize, ui
       const uint32_t tok = (uint32_t)(best.i == 0x7fffffff ? 0 : best.i);
       tokens[blockIdx.x] = tok;
       if (tokens_host) tokens_host[blockIdx.x] = tok;
+      if (notes) *status_copy = st;
     }
   }
 }
@@ -171,9 +174,9 @@ cudaError_t launch_feed_tokens(uint32_t* tokens, const int32_t* feed, const uint
 }
 
 cudaError_t launch_greedy_rows(const bf16* logits, int rows, int vocab, int normalize, uint32_t* tokens,
-                               cudaStream_t s, uint32_t* tokens_host) {
+                               cudaStream_t s, uint32_t* tokens_host, const uint32_t* status, uint32_t* status_copy) {
   if (rows <= 0) return cudaSuccess;
-  return launch_k(greedy_rows_kernel, dim3(rows), dim3(1024), 0, s, logits, vocab, normalize, tokens, tokens_host);
+  return launch_k(greedy_rows_kernel, dim3(rows), dim3(1024), 0, s, logits, vocab, normalize, tokens, tokens_host, status, status_copy);
 }
 
 cudaError_t launch_verify_accept(const uint32_t* row_tokens, const int32_t* seq_row_offsets, const uint32_t* draft,
