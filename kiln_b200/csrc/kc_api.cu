@@ -1313,7 +1313,7 @@ int run_forward(kc_model* m, kc_kv* kv, const uint32_t* tokens_dev, const StepPl
                             kv->num_blocks, kv->block_size, kv->pool, m->q_rot, c->stream));
     const int window = (d.sliding_window > 0 && (l % 2 == 0)) ? d.sliding_window : 0;
     AttnParams a = attn_params(m, kv, p, l, m->q_rot, m->attn, m->attn_scale, gemma ? d.attn_logit_softcapping : 0.f, window, m->Hq);
-    LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, D, n, c->sm_count, c->stream));
+    LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, false, D, n, c->sm_count, c->stream));
     if (streams(L.o)) RC(run_stream(c, L.o, m->attn, n, m->proj, H, m->partial, &so));
     else if (small(L.o)) RC(run_gemv(c, L.o, m->attn, n, m->proj, H, m->partial, &so));
     else RC(run_qlinear(c, L.o, m->op_attn, n, d.tp_world > 1 ? tp_out_buffer(m) : m->proj, H, m->partial, d.tp_world > 1 ? nullptr : &so));
@@ -1671,7 +1671,7 @@ extern "C" int kc_paged_attention(kc_ctx_t c, kc_kv_t kv, int32_t layer, const v
   if (!rc) {
     AttnParams a = attn_params(m, kv, p, layer, (const bf16*)q_dev, (bf16*)out_dev, scale, softcap, window, num_heads);
     rc = [&]() -> int {
-      LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, kv->head_dim, n, c->sm_count, c->stream));
+      LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, true, kv->head_dim, n, c->sm_count, c->stream));
       return KC_OK;
     }();
   }

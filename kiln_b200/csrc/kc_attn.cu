@@ -201,8 +201,10 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  // Units and block tables reach the device before the step's first kernel and no kernel writes them, so the roles read
-  // them under the tail of the kernel before this one; q, K and V are loaded after pdl_wait.
+  // Units and block tables reach the device before a step's first kernel and no kernel writes them, so in a step the roles
+  // read them under the tail of the kernel before this one; where this kernel is the first one behind their copy it is
+  // launched in plain stream order (paged_attention). q, K and V are loaded after pdl_wait, and every role is past it
+  // before its first bounded wait: the time that the kernel before this one takes does not count against the limit.
 
   const int total = p.n_units * p.Hkv;
   if (warp == 0) {
@@ -273,6 +275,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     int chunks = 0;               // chunks begun (O buffer)
     uint32_t qphase = 0;
     bool ok = true;
+    bool waited = false;
     // the tile whose PV is still to be issued
     bool pend = false, pend_first = false, pend_last = false;
     int pend_nb = 0, pend_stage = 0, pend_tile = 0, pend_chunk = 0;
@@ -303,6 +306,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
       UnitTiles u;
       u.open(p, w / p.Hkv, TK);
       if (!u.live()) continue;
+      if (!waited) { pdl_wait(); waited = true; }
       bool first_of_unit = true;
       for (; u.live() && ok;) {
         // QK of this tile goes ahead of the pending PV when its operands are there; else the PV is issued first
@@ -356,12 +360,13 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     // range of fp32, the scores are scaled and capped where they lie first.
     const bool folded = p.scale > 0.f && scale_log2 < INFINITY && (!capped || (cap_arg > 0.f && cap_arg < INFINITY && cap_log2 < INFINITY));
     int tile = 0, chunks = 0;
-    bool ok = true;
+    bool ok = true, waited = false;
     for (int r = 0, w; ok && r * (int)gridDim.x < total; ++r) {
       if ((w = unit_index(r, blockIdx.x, gridDim.x, total)) < 0) break;
       UnitTiles u;
       u.open(p, w / p.Hkv, TK);
       if (!u.live()) continue;
+      if (!waited) { pdl_wait(); waited = true; }
       const bool warp_live = quarter * 32 < u.rows;
       const int pos = u.pos0 + min(row / p.gqa, u.ntok - 1);      // dead rows of a live warp compute the last token's row
       const int w_excl = p.window > 0 ? pos - p.window : -1;       // keys <= this are outside the window
@@ -659,7 +664,8 @@ __global__ void attn_combine_kernel(const AttnParams p, int n_rows) {
 }
 
 template <int D, bool WHOLE>
-cudaError_t launch_attn(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, int sm_count, cudaStream_t s) {
+cudaError_t launch_attn(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, bool in_order, int sm_count,
+                        cudaStream_t s) {
   using S = AttnShape<D>;
   static DeviceOnce configured;   // the attribute belongs to the device's copy of the kernel
   if (configured.first_on_current_device()) {
@@ -667,17 +673,17 @@ cudaError_t launch_attn(const CUtensorMap& map, const CUtensorMap& q, const CUte
     if (e != cudaSuccess) { configured.forget_current_device(); return e; }
   }
   const int grid = std::min(p.n_units * p.Hkv, sm_count);
-  return launch_k(attn_kernel<D, WHOLE>, dim3(grid), dim3(ATT_THREADS), S::SMEM, s, map, q, q_small, p);
+  return launch_k_opt(!in_order, attn_kernel<D, WHOLE>, dim3(grid), dim3(ATT_THREADS), S::SMEM, s, map, q, q_small, p);
 }
 
 template <int D>
-cudaError_t launch_d(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, int n_tokens, int sm_count,
-                     cudaStream_t s) {
+cudaError_t launch_d(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, bool in_order,
+                     int n_tokens, int sm_count, cudaStream_t s) {
   if (p.whole) {
-    if constexpr (D <= 128) return launch_attn<D, true>(map, q, q_small, p, sm_count, s);
+    if constexpr (D <= 128) return launch_attn<D, true>(map, q, q_small, p, in_order, sm_count, s);
     else return cudaErrorInvalidValue;
   }
-  cudaError_t e = launch_attn<D, false>(map, q, q_small, p, sm_count, s);
+  cudaError_t e = launch_attn<D, false>(map, q, q_small, p, in_order, sm_count, s);
   if (e != cudaSuccess || p.single) return e;
   const int n_rows = n_tokens * p.Hq;
   return launch_k(attn_combine_kernel<D>, dim3((n_rows + 7) / 8), dim3(256), 0, s, p, n_rows);
@@ -734,12 +740,12 @@ bool make_tmap_kv_2d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint
 }
 
 cudaError_t paged_attention(const CUtensorMap& kvmap, const CUtensorMap& qmap, const CUtensorMap& qmap_small, const AttnParams& p,
-                            int head_dim, int n_tokens, int sm_count, cudaStream_t s) {
+                            bool in_order, int head_dim, int n_tokens, int sm_count, cudaStream_t s) {
   if (p.gqa < 1 || p.gqa * p.q_tokens > ATT_ROWS || p.n_units < 1) return cudaErrorInvalidValue;
   switch (head_dim) {
-    case 64: return launch_d<64>(kvmap, qmap, qmap_small, p, n_tokens, sm_count, s);
-    case 128: return launch_d<128>(kvmap, qmap, qmap_small, p, n_tokens, sm_count, s);
-    case 256: return launch_d<256>(kvmap, qmap, qmap_small, p, n_tokens, sm_count, s);
+    case 64: return launch_d<64>(kvmap, qmap, qmap_small, p, in_order, n_tokens, sm_count, s);
+    case 128: return launch_d<128>(kvmap, qmap, qmap_small, p, in_order, n_tokens, sm_count, s);
+    case 256: return launch_d<256>(kvmap, qmap, qmap_small, p, in_order, n_tokens, sm_count, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -53,7 +53,9 @@ bool make_tmap_q(CUtensorMap* map, const bf16* q, int n_tokens, int Hq, int gqa,
 bool make_tmap_kv_5d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t plane_rows, uint64_t planes, const char** err);
 bool make_tmap_kv_2d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t rows, const char** err);
 
+// in_order: the work before this call in the stream is not one of a step's kernels (the copy of units and block tables, a
+// caller's own work): the first kernel is then launched behind it in plain stream order.
 cudaError_t paged_attention(const CUtensorMap& kvmap, const CUtensorMap& qmap, const CUtensorMap& qmap_small, const AttnParams& p,
-                            int head_dim, int n_tokens, int sm_count, cudaStream_t s);
+                            bool in_order, int head_dim, int n_tokens, int sm_count, cudaStream_t s);
 
 }  // namespace kc

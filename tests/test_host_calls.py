@@ -1,0 +1,65 @@
+"""What the library asks of the CUDA runtime, call by call, against a stand-in for it (fake_cudart.cpp): the order and kind
+of launches, failures of allocations, limits of a launch. Needs no GPU; each test is a process of its own."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+
+PRELUDE = """
+import ctypes as C
+from kiln_b200 import _lib as L
+fake = C.CDLL(None)
+fake.fake_calls.restype = C.c_char_p
+fake.fake_fail_above.argtypes = [C.c_size_t]
+lib = C.CDLL(str(L.LIB_PATH))
+for name, (res, args) in L._SIGNATURES.items():
+    f = getattr(lib, name)
+    f.restype, f.argtypes = res, args
+def ok(rc):
+    assert rc == 0, lib.kc_last_error()
+def calls():
+    out = fake.fake_calls().decode().splitlines()
+    fake.fake_reset()
+    return out
+ctx = C.c_void_p()
+ok(lib.kc_ctx_create(0, C.byref(ctx)))
+kv = C.c_void_p()
+ok(lib.kc_kv_create(ctx, 1, 2, 64, 80, 16, L.KC_BF16, C.byref(kv)))
+room = C.create_string_buffer(1 << 20)
+at = (C.addressof(room) + 255) // 256 * 256
+table = (C.c_uint32 * 80)(*range(80))
+def attention(lens, out=at, heads=4):
+    seqs = (L.KcSeqStep * len(lens))(*[L.KcSeqStep(n, off, n, -(-(n + off) // 16), table) for n, off in lens])
+    return lib.kc_paged_attention(ctx, kv, 0, at, sum(n for n, _ in lens), heads, seqs, len(lens), 0.125, 0.0, 0, out)
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    so = tmp_path_factory.mktemp("fake") / "fake_cudart.so"
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-I/usr/local/cuda/include", "-o", str(so), str(ROOT / "tests" / "fake_cudart.cpp")], check=True)
+    return so
+
+
+def run(fake, code):
+    r = subprocess.run([sys.executable, "-c", PRELUDE + code], cwd=ROOT, env={**os.environ, "LD_PRELOAD": str(fake), "PYTHONPATH": str(ROOT)},
+                       capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_attention_waits_for_its_metadata(fake):
+    """The kernel behind the copy of a call's metadata reads it before it waits for the kernel ahead of it: it must be
+    ordered behind the copy. The kernel that merges the chunks may start early."""
+    run(fake, """
+for lens in ([(3, 40)], [(1, 1000)]):       # one launch; chunks and the kernel that merges them
+    fake.fake_reset()
+    ok(attention(lens))
+    seen = [c for c in calls() if c.startswith(("copy", "launch"))]
+    assert seen[:2] == ["copy", "launch in order"], seen
+    assert seen[2:] in ([], ["launch early"]), seen
+assert seen[2:] == ["launch early"], seen
+""")
