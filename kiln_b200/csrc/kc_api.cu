@@ -640,7 +640,7 @@ extern "C" int kc_rms_norm(kc_ctx_t c, const void* x_dev, const void* weight_dev
   if (rows < 1 || dim < 2 || dim % 2 || dim > 12288) return fail(KC_ERR_INVALID, "kc_rms_norm: [%d, %d]", rows, dim);
   CK(cudaSetDevice(c->device));
   LAUNCH(c, KC_PROF_ROWWISE, 1, launch_add_rmsnorm((const bf16*)x_dev, SublayerOut::none(), nullptr, (const bf16*)weight_dev, nullptr, rows, dim, eps, nullptr,
-                        (bf16*)y_dev, c->stream));
+                        (bf16*)y_dev, c->stream, true));
   return KC_OK;
 }
 

@@ -258,7 +258,7 @@ add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __re
   if (!y.peers) pdl_launch_dependents();
   constexpr int H = 2048 * CPT;
   __shared__ float red[32];
-  uint4 wraw[CPT];   // a weight depends on no kernel: it arrives under the tail of the one before this
+  uint4 wraw[CPT];   // a model's weight depends on no kernel: it arrives under the tail of the one before this
 #pragma unroll
   for (int c = 0; c < CPT; ++c) wraw[c] = w_out ? *reinterpret_cast<const uint4*>(w_out + (c * 256 + threadIdx.x) * 8) : make_uint4(0, 0, 0, 0);
   pdl_wait();
@@ -519,11 +519,11 @@ static RowSource row_source(const SublayerOut& y) {
 
 cudaError_t launch_add_rmsnorm(const bf16* x, const SublayerOut& y, const bf16* w_pre, const bf16* w_out,
                                const int32_t* row_map, int rows, int H, float eps, bf16* h_out, bf16* normed,
-                               cudaStream_t s) {
+                               cudaStream_t s, bool in_order) {
   if (rows <= 0) return cudaSuccess;
   if (H % 8) return cudaErrorInvalidValue;
   const bool aligned = !y.part || ((reinterpret_cast<uintptr_t>(y.part) & 15) == 0 && (y.ld & 3) == 0 && (y.split_stride & 3) == 0);
-  const bool early = y.rank_y == nullptr;   // per-rank inputs arrive from a collective: see launch_k_opt
+  const bool early = y.rank_y == nullptr && !in_order;   // per-rank inputs arrive from a collective: see launch_k_opt
   if (!w_pre && aligned) {
     if (H == 2048) return launch_k_opt(early, add_rmsnorm_reg_kernel<1>, dim3(rows), dim3(256), 0, s, x, row_source(y), w_out, row_map, eps, h_out, normed);
     if (H == 4096) return launch_k_opt(early, add_rmsnorm_reg_kernel<2>, dim3(rows), dim3(256), 0, s, x, row_source(y), w_out, row_map, eps, h_out, normed);

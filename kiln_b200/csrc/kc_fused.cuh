@@ -54,10 +54,12 @@ struct SublayerOut {
 };
 
 // h = y ? bf16(x + (w_pre ? rms_norm(y, w_pre) : y)) : x ; normed = w_out ? rms_norm(h, w_out) : unused.
-// row_map (optional) picks the input rows. h_out / normed may be null when not wanted.
+// row_map (optional) picks the input rows. h_out / normed may be null when not wanted. The weight is read before the
+// kernel ahead has finished; in_order: a kernel ahead may write it (it is a caller's, not a model's), so this one is
+// launched behind it in plain stream order.
 cudaError_t launch_add_rmsnorm(const bf16* x, const SublayerOut& y, const bf16* w_pre, const bf16* w_out,
                                const int32_t* row_map, int rows, int H, float eps, bf16* h_out, bf16* normed,
-                               cudaStream_t s);
+                               cudaStream_t s, bool in_order = false);
 
 cudaError_t launch_rope_kv_write(const SublayerOut& qkv, const bf16* bias, const float* inv_freq, const int32_t* token_pos,
                                  const int32_t* kv_slot, int n, int Hq, int Hkv, int D, int traditional, int layer,

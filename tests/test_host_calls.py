@@ -63,3 +63,13 @@ for lens in ([(3, 40)], [(1, 1000)]):       # one launch; chunks and the kernel 
     assert seen[2:] in ([], ["launch early"]), seen
 assert seen[2:] == ["launch early"], seen
 """)
+
+
+@pytest.mark.parametrize("dim", [1024, 2048, 4096, 8192])
+def test_rms_norm_waits_for_its_weight(fake, dim):
+    """The weight is read before the kernel ahead has finished, and a caller's weight may be what that kernel writes."""
+    run(fake, f"""
+fake.fake_reset()
+ok(lib.kc_rms_norm(ctx, at, at, 2, {dim}, 1e-5, at))
+assert calls() == ["launch in order"]
+""")
