@@ -1131,6 +1131,7 @@ int upload_meta(kc_model* m, kc_kv* kv, const uint32_t* token_ids, const kc_seq_
   if (L.total > m->meta_cap) {
     CK(cudaStreamSynchronize(c->stream));
     const size_t cap = align_up(std::max<size_t>(L.total * 2, 1 << 16), 4096);
+    m->meta_cap = 0;   // until the new buffers are all there: a call after a failed allocation starts from nothing
     cudaFree(m->meta_dev); m->meta_dev = nullptr;
     for (int i = 0; i < kc_model::kStaging; ++i) { if (m->meta_host[i]) cudaFreeHost(m->meta_host[i]); m->meta_host[i] = nullptr; }
     CK(cudaMalloc(&m->meta_dev, cap));

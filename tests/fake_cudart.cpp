@@ -14,15 +14,16 @@ namespace {
 std::mutex mu;
 std::string calls;
 size_t fail_above = ~size_t(0);
+bool fail_host_only = false;
 
 void note(const char* what) {
   std::lock_guard<std::mutex> lk(mu);
   calls += what;
   calls += '\n';
 }
-cudaError_t alloc(void** p, size_t n, const char* what) {
-  note(what);
-  if (n > fail_above) return cudaErrorMemoryAllocation;
+cudaError_t alloc(void** p, size_t n, bool host) {
+  note(host ? "host" : "malloc");
+  if (n > fail_above && (host || !fail_host_only)) return cudaErrorMemoryAllocation;
   *p = aligned_alloc(256, (n + 255) / 256 * 256 + 256);
   return *p ? cudaSuccess : cudaErrorMemoryAllocation;
 }
@@ -34,11 +35,12 @@ CUresult encode(CUtensorMap*, ...) { return CUDA_SUCCESS; }
 // what the tests call
 EXPORT const char* fake_calls() { return calls.c_str(); }
 EXPORT void fake_reset() { std::lock_guard<std::mutex> lk(mu); calls.clear(); }
-EXPORT void fake_fail_above(size_t bytes) { fail_above = bytes; }   // allocations larger than this fail
+EXPORT void fake_fail_above(size_t bytes) { fail_above = bytes; }         // allocations larger than this fail
+EXPORT void fake_fail_host_only(int on) { fail_host_only = on != 0; }     // ... of pinned memory only
 
-EXPORT cudaError_t cudaMalloc(void** p, size_t n) { return alloc(p, n, "malloc"); }
-EXPORT cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return alloc(p, n, "host"); }
-EXPORT cudaError_t cudaMallocHost(void** p, size_t n) { return alloc(p, n, "host"); }
+EXPORT cudaError_t cudaMalloc(void** p, size_t n) { return alloc(p, n, false); }
+EXPORT cudaError_t cudaHostAlloc(void** p, size_t n, unsigned) { return alloc(p, n, true); }
+EXPORT cudaError_t cudaMallocHost(void** p, size_t n) { return alloc(p, n, true); }
 EXPORT cudaError_t cudaFree(void* p) { note("free"); free(p); return cudaSuccess; }
 EXPORT cudaError_t cudaFreeHost(void* p) { note("free"); free(p); return cudaSuccess; }
 EXPORT cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) { *d = h; return cudaSuccess; }

@@ -73,3 +73,19 @@ fake.fake_reset()
 ok(lib.kc_rms_norm(ctx, at, at, 2, {dim}, 1e-5, at))
 assert calls() == ["launch in order"]
 """)
+
+
+@pytest.mark.parametrize("device", [True, False])
+def test_a_call_after_a_failed_allocation(fake, device):
+    """Growing the metadata arena gives the old one up first. Where the new one cannot be had, the next call has to make one
+    of its own size: with the device's memory at its end, or the pinned memory's (the failure is in the second allocation)."""
+    run(fake, f"""
+ok(attention([(3, 40)]))
+fake.fake_fail_above(1 << 16)
+if not {device}: fake.fake_fail_host_only(1)
+assert attention([(1, 1200)] * 600, heads=2) == L.KC_ERR_OOM
+fake.fake_fail_above(2 ** 62)
+fake.fake_reset()
+ok(attention([(3, 40)]))
+assert calls().count("copy") == 1
+""")
