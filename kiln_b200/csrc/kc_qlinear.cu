@@ -252,9 +252,8 @@ __device__ __forceinline__ void dequant_row(const uint8_t* row_base, const bf162
   }
 }
 
-// The same for a weight with a scale past the limit: the integers are converted (a byte under the exponent of 2^23 is
-// the float 8388608 + q) and one fp32 multiply-add is rounded to bf16; q * scale has at most 16 bits, so the fp32 sum
-// is rounded at 24 bits and then at 8.
+// The same for a weight with a scale past the limit: the integers are converted first (exact: at most 8 bits), the
+// multiply-add is the same one with its one rounding.
 template <int BITS, int GPK>
 __device__ __forceinline__ void dequant_row_wide(const uint8_t* row_base, const bf162 (&sb)[GPK], uint32_t (&v)[32]) {
   constexpr int CHUNKS = BITS / 2;
@@ -263,14 +262,14 @@ __device__ __forceinline__ void dequant_row_wide(const uint8_t* row_base, const 
     const uint4 q = *reinterpret_cast<const uint4*>(row_base + h * (QL_TILE_N * 16));
     const uint32_t w[4] = {q.x, q.y, q.z, q.w};
     const int g = GPK == 2 ? h * 2 / CHUNKS : 0;
-    const float s = __bfloat162float(sb[g].x), b = __bfloat162float(sb[g].y);
+    const bf162 s2 = __bfloat162bfloat162(sb[g].x), b2 = __bfloat162bfloat162(sb[g].y);
 #pragma unroll
     for (int c = 0; c < 4; ++c)
 #pragma unroll
       for (int j = 0; j < 16 / BITS; ++j) {
         const uint32_t lo = BITS == 4 ? (w[c] >> (4 * j)) & 0xFu : (w[c] >> (16 * j)) & 0xFFu;
         const uint32_t hi = BITS == 4 ? (w[c] >> (16 + 4 * j)) & 0xFu : (w[c] >> (16 * j + 8)) & 0xFFu;
-        v[(h * 4 + c) * (16 / BITS) + j] = pack_bf162(fmaf((float)lo, s, b), fmaf((float)hi, s, b));
+        v[(h * 4 + c) * (16 / BITS) + j] = bf2_fma(pack_bf162((float)lo, (float)hi), s2, b2);
       }
   }
 }

@@ -235,3 +235,31 @@ def test_row_chunks_carry_the_bits_of_few_rows(ctx, n, k, bits, group, m):
         part = qw.matmul(x[r0:r1].contiguous()).cpu()
         assert torch.equal(part.view(torch.int16), full[r0:r1].view(torch.int16)), f"rows {r0}..{r1}"
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("scale", [129 / 2 ** 10, 129 / 2 ** 8])     # below and above the line where the integers are converted first
+def test_weights_are_rounded_once(ctx, bits, scale):
+    """A weight is q * scale + bias rounded to bf16 once: with a bias far below the last bit of a product that lies half way
+    between two bf16 numbers, a rounding to fp32 in between loses it and the half way goes to the even one. Exact: one-hot
+    rows bring the weights out as they are."""
+    if bits == 8:
+        scale /= 16
+    n, k = 128, 64
+    g = torch.Generator().manual_seed(91)
+    q = torch.randint(0, 2 ** bits, (n, k), generator=g)
+    q[:, 0], q[:, 1] = 3, 5                                            # 3 * 129 and 5 * 129 have 9 and 10 bits: half ways among them
+    per = 32 // bits
+    packed = (q.reshape(n, -1, per) << (torch.arange(per) * bits)).sum(-1)
+    packed = torch.where(packed >= 2 ** 31, packed - 2 ** 32, packed).to(torch.int32)
+    s = torch.full((n, 1), scale).to(torch.bfloat16)
+    b = (torch.where(torch.arange(n) % 2 == 0, 1.0, -1.0) * 2.0 ** -34).reshape(n, 1).to(torch.bfloat16)
+    exact = q.double() * s.double() + b.double()
+    ulp = torch.exp2(torch.floor(torch.log2(exact.abs())) - 7)
+    want = (torch.round(exact / ulp) * ulp).float()                    # half to even, of the exact value
+    via_fp32 = exact.float().to(torch.bfloat16).float()
+    assert not torch.equal(want, via_fp32)                             # the input tells the two apart
+    qw = api.QuantizedWeight(ctx, packed.cuda(), s.cuda(), b.cuda(), bits, 64)
+    got = qw.matmul(torch.eye(k).to(torch.bfloat16).cuda()).cpu().float().T
+    assert torch.equal(got, want)
+    assert ctx.device_status() == 0
