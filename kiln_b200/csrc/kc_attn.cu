@@ -121,6 +121,25 @@ __device__ __forceinline__ MergeW merge_weights(float m_acc, float m_chunk) {
 __device__ __forceinline__ float merge_value(float acc, float v, const MergeW& w) { return __fmaf_rn(v, w.b, __fmul_rn(acc, w.a)); }
 __device__ __forceinline__ float row_scale(float l) { return l == 0.f ? 1.f : __frcp_rn(l); }
 
+// Eight (two, four) bf16 of an output row in one store, or one by one where the caller's output starts off that boundary.
+__device__ __forceinline__ bool row_aligned(const void* p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+template <int N>
+__device__ __forceinline__ void store_row(bf16* out, const uint32_t (&v)[N], bool aligned) {
+  if (!aligned) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      reinterpret_cast<uint16_t*>(out)[2 * i] = (uint16_t)v[i];
+      reinterpret_cast<uint16_t*>(out)[2 * i + 1] = (uint16_t)(v[i] >> 16);
+    }
+  } else if constexpr (N == 4) {
+    *reinterpret_cast<uint4*>(out) = make_uint4(v[0], v[1], v[2], v[3]);
+  } else if constexpr (N == 2) {
+    *reinterpret_cast<uint2*>(out) = make_uint2(v[0], v[1]);
+  } else {
+    *reinterpret_cast<uint32_t*>(out) = v[0];
+  }
+}
+
 // The tiles of one unit in order, as every role walks them.
 struct UnitTiles {
   int seq, tok0, ntok, pos0, small, rows, pos_max, wlo;
@@ -510,6 +529,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     pdl_wait();   // the stores below may overwrite what an earlier kernel still reads
     const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
+    const bool aligned = row_aligned(p.out, 16);
     int chunks = 0;
     bool ok = true;
     constexpr int ACC = WHOLE ? D : 1;
@@ -566,7 +586,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
 #pragma unroll
                   for (int k = 0; k < 4; ++k)
                     q[k] = pack_bf162(__fmul_rn(__uint_as_float(o[j + 2 * k]), inv), __fmul_rn(__uint_as_float(o[j + 2 * k + 1]), inv));
-                  *reinterpret_cast<uint4*>(out + j) = make_uint4(q[0], q[1], q[2], q[3]);
+                  store_row(out + j, q, aligned);
                 }
               } else if (row_live) {
 #pragma unroll
@@ -584,10 +604,12 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
         const float inv = row_scale(lacc);
         bf16* out = p.out + orow * D;
 #pragma unroll
-        for (int j = 0; j < ACC; j += 8)
-          *reinterpret_cast<uint4*>(out + j) =
-              make_uint4(pack_bf162(__fmul_rn(acc[j % ACC], inv), __fmul_rn(acc[(j + 1) % ACC], inv)), pack_bf162(__fmul_rn(acc[(j + 2) % ACC], inv), __fmul_rn(acc[(j + 3) % ACC], inv)),
-                         pack_bf162(__fmul_rn(acc[(j + 4) % ACC], inv), __fmul_rn(acc[(j + 5) % ACC], inv)), pack_bf162(__fmul_rn(acc[(j + 6) % ACC], inv), __fmul_rn(acc[(j + 7) % ACC], inv)));
+        for (int j = 0; j < ACC; j += 8) {
+          uint32_t q[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) q[k] = pack_bf162(__fmul_rn(acc[(j + 2 * k) % ACC], inv), __fmul_rn(acc[(j + 2 * k + 1) % ACC], inv));
+          store_row(out + j, q, aligned);
+        }
       }
       __syncwarp();
     }
@@ -653,14 +675,10 @@ __global__ void attn_combine_kernel(const AttnParams p, int n_rows) {
   }
   const float inv = row_scale(lacc);
   bf16* out = p.out + (size_t)row * D + lane * PER;
-  if (PER == 2) {
-    *reinterpret_cast<uint32_t*>(out) = pack_bf162(__fmul_rn(acc[0], inv), __fmul_rn(acc[PER - 1], inv));
-  } else {
+  uint32_t q[PER / 2];
 #pragma unroll
-    for (int i = 0; i < PER; i += 4)
-      *reinterpret_cast<uint2*>(out + i) = make_uint2(pack_bf162(__fmul_rn(acc[i], inv), __fmul_rn(acc[(i + 1) % PER], inv)),
-                                                      pack_bf162(__fmul_rn(acc[(i + 2) % PER], inv), __fmul_rn(acc[(i + 3) % PER], inv)));
-  }
+  for (int i = 0; i < PER / 2; ++i) q[i] = pack_bf162(__fmul_rn(acc[2 * i], inv), __fmul_rn(acc[2 * i + 1], inv));
+  store_row(out, q, row_aligned(p.out, PER * 2));
 }
 
 template <int D, bool WHOLE>

@@ -235,3 +235,28 @@ def test_softcap_of_scores_that_are_not_finite(ctx):
     check(n, 5, 0)      # rows 0 and 1 before the NaN, 2 .. 4 from it on
     check(143, 3, 4)    # row 0 sees four keys of score -inf and no other
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("hd,batch,offset", [(64, 2, 40), (128, 2, 40), (256, 2, 40), (64, 1, 1300), (128, 1, 1300), (256, 1, 1300), (64, 148, 700), (128, 148, 700)])
+def test_output_off_a_vector_boundary(ctx, hd, batch, offset):
+    """The C entry point writes to any bf16 address: rows of one chunk, chunks merged by the second kernel, whole rows."""
+    import ctypes as C
+    from kiln_b200 import _lib as L
+    heads, kvh, bs, rows = 4, 1, 16, 2
+    need = (offset + rows + bs - 1) // bs
+    kv = api.PagedKv(ctx, api.KvSpec(1, kvh, hd, need, bs))
+    data = outlier_values((need, kv.bytes_per_block() // 2), 95)
+    for b in range(need):
+        kv.write_block_bytes(b, data[b].view(torch.uint8).numpy().tobytes())
+    seqs = [api.SeqStep(rows, offset, rows, list(range(need)))] * batch
+    q = outlier_values((rows * batch, heads, hd), 96).cuda()
+    want = api.paged_attention(ctx, kv, 0, q, seqs, hd ** -0.5)
+    p = api._PackedStep(api.StepBatch([0] * (rows * batch), seqs))
+    for shift in (1, 2, 4):
+        room = torch.full((want.numel() + 16,), 7.0, dtype=torch.bfloat16, device="cuda")
+        torch.cuda.synchronize()
+        api.check(L.lib().kc_paged_attention(ctx._h, kv._h, 0, q.data_ptr(), rows * batch, heads, p.seq_arr, p.n_seqs, hd ** -0.5, 0.0, 0,
+                                             C.c_void_p(room.data_ptr() + 2 * shift)))
+        assert torch.equal(room[shift: shift + want.numel()].view(torch.int16), want.view(-1).view(torch.int16))
+        assert bool((room[:shift] == 7).all()) and bool((room[shift + want.numel():] == 7).all())
+    assert ctx.device_status() == 0
