@@ -260,3 +260,31 @@ def test_output_off_a_vector_boundary(ctx, hd, batch, offset):
         assert torch.equal(room[shift: shift + want.numel()].view(torch.int16), want.view(-1).view(torch.int16))
         assert bool((room[:shift] == 7).all()) and bool((room[shift + want.numel():] == 7).all())
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("hd,batch,offset", [(64, 1, 40), (128, 1, 40), (256, 1, 40), (64, 1, 1300), (128, 1, 1300), (256, 1, 1300), (64, 148, 700), (128, 148, 700)])
+def test_rows_are_divided_by_their_sums(ctx, hd, batch, offset):
+    """Seven keys of equal weight and whole numbers: sums and weights are exact, and the quotients lie half way between two
+    bf16 numbers, where a reciprocal that is rounded before the product shows. In every form a row is finished in: one
+    chunk, chunks merged by the second kernel, whole rows. Values of -0 come out as +0 in each of them."""
+    bs, window = 16, 7
+    need = (offset + 1 + bs - 1) // bs
+    kv = api.PagedKv(ctx, api.KvSpec(1, 1, hd, need, bs))
+    t = torch.arange(hd) % 40 * 2 + 343                          # odd, of 9 bits: the means of seven bf16 numbers
+    v = torch.zeros(need * bs, hd)
+    first = offset - window + 1
+    base = (t - 255) // 6 - ((t - 255) // 6 + 1) % 2             # 255 and six even numbers a little above the mean
+    for j in range(6):
+        v[first + j] = (t + base + 2 * (t - 255 - 6 * base > 2 * j)).float()
+    v[first + 6] = 255
+    assert torch.equal(v[first: first + 7].sum(0), 7.0 * t) and torch.equal(v, v.to(torch.bfloat16).float())
+    want = t.to(torch.bfloat16)
+    v[:, hd - 1] = -0.0
+    want[hd - 1] = 0.0
+    k = torch.zeros(need * bs, hd)
+    for b in range(need):
+        kv.write_block_bytes(b, torch.cat([k[b * bs: (b + 1) * bs].reshape(-1), v[b * bs: (b + 1) * bs].reshape(-1)]).to(torch.bfloat16).view(torch.uint8).numpy().tobytes())
+    seqs = [api.SeqStep(1, offset, 1, list(range(need)))] * batch
+    got = api.paged_attention(ctx, kv, 0, torch.ones(batch, 2, hd, dtype=torch.bfloat16, device="cuda"), seqs, hd ** -0.5, 0.0, window).cpu()
+    assert torch.equal(got.view(batch * 2, hd).view(torch.int16), want.expand(batch * 2, hd).contiguous().view(torch.int16))
+    assert ctx.device_status() == 0
