@@ -193,7 +193,16 @@ __host__ __device__ __forceinline__ int unit_index(int r, int cta, int ctas, int
   return i < total ? i : -1;
 }
 
-template <int D, bool WHOLE>
+// Whether the scale can go into the multiplier of the exponent, behind mask and maximum (FOLDED): right for a positive one
+// only (a masked -inf times 0 is NaN, times a negative scale +inf) whose factors stay in the range of fp32. With any other
+// scale the scores are scaled and capped where they lie first. That is an instantiation of its own: the code for it in the
+// tile loop cost every call 2 to 5 %.
+bool scale_folds(float scale, float softcap) {
+  if (!(scale > 0.f && scale * 1.4426950408889634f < INFINITY)) return false;
+  return !(softcap > 0.f) || (scale / softcap > 0.f && scale / softcap < INFINITY && softcap * 1.4426950408889634f < INFINITY);
+}
+
+template <int D, bool WHOLE, bool FOLDED>
 __global__ void __launch_bounds__(ATT_THREADS, 1)
 attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ CUtensorMap qmap,
             const __grid_constant__ CUtensorMap qmap_small, const AttnParams p) {
@@ -235,9 +244,9 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  // Units and block tables reach the device before a step's first kernel and no kernel writes them, so in a step the roles
-  // read them under the tail of the kernel before this one; where this kernel is the first one behind their copy it is
-  // launched in plain stream order (paged_attention). q, K and V are loaded after pdl_wait, and every role is past it
+  // Units and block tables reach the device before a step's first kernel and no kernel writes them, so in a step the
+  // producer reads them under the tail of the kernel before this one; where this kernel is the first one behind their copy
+  // it is launched in plain stream order (paged_attention). q, K and V are loaded after pdl_wait, and every role is past it
   // before its first bounded wait: the time that the kernel before this one takes does not count against the limit.
 
   const int total = p.n_units * p.Hkv;
@@ -299,6 +308,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     }
   } else if (warp == 1) {
     // ---- MMA issuer: converged, one elected lane around the MMAs ----
+    pdl_wait();
     const uint64_t qd = umma_smem_desc(smem_u32(sQ), 1024);
     const uint64_t kd = umma_smem_desc(smem_u32(ring), S::GROUP_BYTES);
     const uint64_t vd = umma_smem_desc(smem_u32(ring) + S::SLABS * 1024, S::GROUP_BYTES, 1024);
@@ -309,7 +319,6 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     int chunks = 0;               // chunks begun (O buffer)
     uint32_t qphase = 0;
     bool ok = true;
-    bool waited = false;
     // the tile whose PV is still to be issued
     bool pend = false, pend_first = false, pend_last = false;
     int pend_nb = 0, pend_stage = 0, pend_tile = 0, pend_chunk = 0;
@@ -340,7 +349,6 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
       UnitTiles u;
       u.open(p, w / p.Hkv, TK);
       if (!u.live()) continue;
-      if (!waited) { pdl_wait(); waited = true; }
       bool first_of_unit = true;
       for (; u.live() && ok;) {
         // QK of this tile goes ahead of the pending PV when its operands are there; else the PV is issued first
@@ -383,24 +391,19 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     if (ok && pend) issue_pv();
   } else if (warp >= 4 && warp < 8) {
     // ---- softmax: thread = query row 32 * (warp & 3) + lane ----
+    pdl_wait();
     const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    const float scale_log2 = p.scale * 1.4426950408889634f;
-    const bool capped = p.softcap > 0.f;
-    const float cap_arg = capped ? p.scale / p.softcap : 0.f;
+    const float scale_log2 = FOLDED ? p.scale * 1.4426950408889634f : 1.4426950408889634f;
+    const float cap_arg = FOLDED && p.softcap > 0.f ? p.scale / p.softcap : 0.f;
     const float cap_log2 = p.softcap * 1.4426950408889634f;
-    // The scale goes into the multiplier of the exponent, behind mask and maximum: right for a positive one only (a
-    // masked -inf times 0 is NaN, times a negative scale +inf). With any other scale, and with factors that leave the
-    // range of fp32, the scores are scaled and capped where they lie first.
-    const bool folded = p.scale > 0.f && scale_log2 < INFINITY && (!capped || (cap_arg > 0.f && cap_arg < INFINITY && cap_log2 < INFINITY));
     int tile = 0, chunks = 0;
-    bool ok = true, waited = false;
+    bool ok = true;
     for (int r = 0, w; ok && r * (int)gridDim.x < total; ++r) {
       if ((w = unit_index(r, blockIdx.x, gridDim.x, total)) < 0) break;
       UnitTiles u;
       u.open(p, w / p.Hkv, TK);
       if (!u.live()) continue;
-      if (!waited) { pdl_wait(); waited = true; }
       const bool warp_live = quarter * 32 < u.rows;
       const int pos = u.pos0 + min(row / p.gqa, u.ntok - 1);      // dead rows of a live warp compute the last token's row
       const int w_excl = p.window > 0 ? pos - p.window : -1;       // keys <= this are outside the window
@@ -419,7 +422,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
           const int hi = pos - key0, lo = w_excl - key0 + 1;
           // every key of the tile is visible to every row of the unit: the same arithmetic without the predicates
           const bool edge = !(nb * 16 == TK && key0 + TK - 1 <= u.pos0 && (p.window == 0 || key0 > u.pos_max - p.window));
-          if (!folded) {
+          if (!FOLDED) {
 #pragma unroll 1
             for (int c = 0; c < TK / 32; ++c) {
               uint32_t x[32];
@@ -427,7 +430,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
                 float f = __uint_as_float(x[j]) * p.scale;
-                if (capped) f = p.softcap * tanhf(f / p.softcap);
+                if (p.softcap > 0.f) f = p.softcap * tanhf(f / p.softcap);
                 x[j] = __float_as_uint(f);
               }
               tmem_st32(s_addr + c * 32, x);
@@ -453,8 +456,8 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
             t2 = fmaxf(t2, fmaxf(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5])));
             t3 = fmaxf(t3, fmaxf(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7])));
           }
-          float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)), mul = folded ? scale_log2 : 1.4426950408889634f;
-          if (capped && folded) {
+          float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)), mul = scale_log2;
+          if (FOLDED && p.softcap > 0.f) {
             mul = cap_log2;
             // A tile with no score past 2.2 caps takes the fraction alone, two elements at a time; an element's value is the
             // same on both sides.
@@ -697,17 +700,23 @@ __global__ void attn_combine_kernel(const AttnParams p, int n_rows) {
   store_row(out, q, row_aligned(p.out, PER * 2));
 }
 
-template <int D, bool WHOLE>
-cudaError_t launch_attn(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, bool in_order, int sm_count,
+template <int D, bool WHOLE, bool FOLDED>
+cudaError_t launch_attn_as(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, bool in_order, int sm_count,
                         cudaStream_t s) {
   using S = AttnShape<D>;
   static DeviceOnce configured;   // the attribute belongs to the device's copy of the kernel
   if (configured.first_on_current_device()) {
-    cudaError_t e = cudaFuncSetAttribute(attn_kernel<D, WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(attn_kernel<D, WHOLE, FOLDED>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
     if (e != cudaSuccess) { configured.forget_current_device(); return e; }
   }
   const int grid = std::min(p.n_units * p.Hkv, sm_count);
-  return launch_k_opt(!in_order, attn_kernel<D, WHOLE>, dim3(grid), dim3(ATT_THREADS), S::SMEM, s, map, q, q_small, p);
+  return launch_k_opt(!in_order, attn_kernel<D, WHOLE, FOLDED>, dim3(grid), dim3(ATT_THREADS), S::SMEM, s, map, q, q_small, p);
+}
+template <int D, bool WHOLE>
+cudaError_t launch_attn(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, bool in_order, int sm_count,
+                        cudaStream_t s) {
+  return scale_folds(p.scale, p.softcap) ? launch_attn_as<D, WHOLE, true>(map, q, q_small, p, in_order, sm_count, s)
+                                         : launch_attn_as<D, WHOLE, false>(map, q, q_small, p, in_order, sm_count, s);
 }
 
 template <int D>
