@@ -1669,14 +1669,24 @@ extern "C" int kc_paged_attention(kc_ctx_t c, kc_kv_t kv, int32_t layer, const v
   if (!rc) rc = upload_meta(m, kv, ids.data(), seqs, p);
   if (!rc) rc = ensure_attn_ws(m, p);
   if (!rc) rc = ensure_q_maps(m, (const bf16*)q_dev, n, num_heads, num_heads / kv->kv_heads, p);
+  // The kernels store 16 bytes at a time: an output that starts elsewhere gets a copy of an aligned one.
+  const size_t out_bytes = (size_t)std::max(n, 1) * num_heads * kv->head_dim * sizeof(bf16);
+  bf16* out = (bf16*)out_dev;
+  if (!rc && (uintptr_t)out_dev % 16) {
+    cudaError_t e = cudaMalloc(&out, out_bytes);
+    if (e != cudaSuccess) { out = (bf16*)out_dev; rc = fail(KC_ERR_OOM, "kc_paged_attention: %zu bytes: %s", out_bytes, cudaGetErrorString(e)); }
+  }
   if (!rc) {
-    AttnParams a = attn_params(m, kv, p, layer, (const bf16*)q_dev, (bf16*)out_dev, scale, softcap, window, num_heads);
+    AttnParams a = attn_params(m, kv, p, layer, (const bf16*)q_dev, out, scale, softcap, window, num_heads);
     rc = [&]() -> int {
       LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, true, kv->head_dim, n, c->sm_count, c->stream));
+      if (out != out_dev) CK(cudaMemcpyAsync(out_dev, out, out_bytes, cudaMemcpyDeviceToDevice, c->stream));
       return KC_OK;
     }();
   }
-  return op_shell_done(c, rc, "kc_paged_attention");
+  rc = op_shell_done(c, rc, "kc_paged_attention");
+  if (out != out_dev) cudaFree(out);
+  return rc;
 }
 
 extern "C" int kc_rope_kv_write(kc_ctx_t c, kc_kv_t kv, int32_t layer, const void* qkv_dev, const void* qkv_bias_dev,

@@ -136,25 +136,6 @@ __device__ __forceinline__ uint32_t finish2(float a, float b, const RowSum& s) {
   return pack_bf162(v.x, v.y);
 }
 
-// Eight (two, four) bf16 of an output row in one store, or one by one where the caller's output starts off that boundary.
-__device__ __forceinline__ bool row_aligned(const void* p, int bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
-template <int N>
-__device__ __forceinline__ void store_row(bf16* out, const uint32_t (&v)[N], bool aligned) {
-  if (!aligned) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      reinterpret_cast<uint16_t*>(out)[2 * i] = (uint16_t)v[i];
-      reinterpret_cast<uint16_t*>(out)[2 * i + 1] = (uint16_t)(v[i] >> 16);
-    }
-  } else if constexpr (N == 4) {
-    *reinterpret_cast<uint4*>(out) = make_uint4(v[0], v[1], v[2], v[3]);
-  } else if constexpr (N == 2) {
-    *reinterpret_cast<uint2*>(out) = make_uint2(v[0], v[1]);
-  } else {
-    *reinterpret_cast<uint32_t*>(out) = v[0];
-  }
-}
-
 // The tiles of one unit in order, as every role walks them.
 struct UnitTiles {
   int seq, tok0, ntok, pos0, small, rows, pos_max, wlo;
@@ -547,7 +528,6 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
     pdl_wait();   // the stores below may overwrite what an earlier kernel still reads
     const int quarter = warp & 3, row = quarter * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
-    const bool aligned = row_aligned(p.out, 16);
     int chunks = 0;
     bool ok = true;
     constexpr int ACC = WHOLE ? D : 1;
@@ -605,7 +585,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
 #pragma unroll
                   for (int k = 0; k < 4; ++k)
                     q[k] = finish2(0.f + __uint_as_float(o[j + 2 * k]), 0.f + __uint_as_float(o[j + 2 * k + 1]), l);
-                  store_row(out + j, q, aligned);
+                  *reinterpret_cast<uint4*>(out + j) = make_uint4(q[0], q[1], q[2], q[3]);
                 }
               } else if (row_live) {
 #pragma unroll
@@ -627,7 +607,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
           uint32_t q[4];
 #pragma unroll
           for (int k = 0; k < 4; ++k) q[k] = finish2(acc[(j + 2 * k) % ACC], acc[(j + 2 * k + 1) % ACC], l);
-          store_row(out + j, q, aligned);
+          *reinterpret_cast<uint4*>(out + j) = make_uint4(q[0], q[1], q[2], q[3]);
         }
       }
       __syncwarp();
@@ -697,7 +677,9 @@ __global__ void attn_combine_kernel(const AttnParams p, int n_rows) {
   uint32_t q[PER / 2];
 #pragma unroll
   for (int i = 0; i < PER / 2; ++i) q[i] = finish2(acc[2 * i], acc[2 * i + 1], l);
-  store_row(out, q, row_aligned(p.out, PER * 2));
+  if constexpr (PER == 8) *reinterpret_cast<uint4*>(out) = make_uint4(q[0], q[1], q[2], q[3]);
+  else if constexpr (PER == 4) *reinterpret_cast<uint2*>(out) = make_uint2(q[0], q[1]);
+  else *reinterpret_cast<uint32_t*>(out) = q[0];
 }
 
 template <int D, bool WHOLE, bool FOLDED>
