@@ -123,20 +123,19 @@ __device__ __forceinline__ MergeW merge_weights(float m_acc, float m_chunk) {
   return w;
 }
 __device__ __forceinline__ float merge_value(float acc, float v, const MergeW& w) { return __fmaf_rn(v, w.b, __fmul_rn(acc, w.a)); }
-// Two values of a finished row divided by its sum (a row without one keeps its zeros): the product with the rounded
-// reciprocal, then one step that adds what it leaves over, which makes the quotient the correctly rounded one (Markstein,
-// IBM J. Res. Dev. 34, 1990). The division operator gives the same and took 5 us a unit of 128 values a thread more. An
-// infinite value leaves NaN over: the minimum drops it.
-struct RowSum { float2 minus_l, r; };
+__device__ __forceinline__ float2 merge_values(float2 acc, float2 v, const MergeW& w) { return fma2(v, make_float2(w.b, w.b), mul2(acc, make_float2(w.a, w.a))); }
+// Two values of a finished row divided by its sum (a row without one keeps its zeros): times the reciprocal in two parts,
+// one rounded down and what it leaves, so that the fp32 result is the rounded quotient but for quotients within 2^-48 of a
+// rounding boundary. (The division operator took 5 us a unit of 128 values a thread more.) The second part is positive: an
+// infinite value stays what it is. A -0 becomes +0.
+struct RowSum { float2 r, rest; };
 __device__ __forceinline__ RowSum row_sum(float l) {
   if (l == 0.f) l = 1.f;
-  const float r = __frcp_rn(l);
-  return {make_float2(-l, -l), make_float2(r, r)};
+  const float r = __frcp_rd(l), rest = fmaxf(__fmaf_rn(-l, r, 1.f) * r, 1e-35f);
+  return {make_float2(r, r), make_float2(rest, rest)};
 }
 __device__ __forceinline__ uint32_t finish2(float a, float b, const RowSum& s) {
-  const float2 x = make_float2(a, b), q = mul2(x, s.r);
-  const float2 over = fma2(q, s.minus_l, x);
-  const float2 v = fma2(make_float2(fminf(over.x, 3.402823466e38f), fminf(over.y, 3.402823466e38f)), s.r, q);
+  const float2 x = make_float2(a, b), v = fma2(x, s.r, fma2(x, s.rest, make_float2(0.f, 0.f)));
   return pack_bf162(v.x, v.y);
 }
 
@@ -581,7 +580,11 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
               uint32_t o[32];
               tmem_ld32(o_addr + c * 32, o);
 #pragma unroll
-              for (int j = 0; j < 32; ++j) acc[(c * 32 + j) % ACC] = merge_value(acc[(c * 32 + j) % ACC], __uint_as_float(o[j]), mw);
+              for (int j = 0; j < 32; j += 2) {
+                const float2 v = merge_values(make_float2(acc[(c * 32 + j) % ACC], acc[(c * 32 + j + 1) % ACC]),
+                                              make_float2(__uint_as_float(o[j]), __uint_as_float(o[j + 1])), mw);
+                acc[(c * 32 + j) % ACC] = v.x; acc[(c * 32 + j + 1) % ACC] = v.y;
+              }
             }
           } else {
             const size_t prow = orow * p.max_chunks + u.c;
@@ -601,7 +604,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
                   uint32_t q[4];
 #pragma unroll
                   for (int k = 0; k < 4; ++k)
-                    q[k] = finish2(0.f + __uint_as_float(o[j + 2 * k]), 0.f + __uint_as_float(o[j + 2 * k + 1]), l);
+                    q[k] = finish2(__uint_as_float(o[j + 2 * k]), __uint_as_float(o[j + 2 * k + 1]), l);
                   *reinterpret_cast<uint4*>(out + j) = make_uint4(q[0], q[1], q[2], q[3]);
                 }
               } else if (row_live) {
