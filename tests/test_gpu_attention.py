@@ -316,3 +316,31 @@ def test_error_is_that_of_the_output(ctx, hd, keys, gain):
         norm += float(want.square().sum())
     assert (err / norm) ** 0.5 < 1.71e-3
     assert ctx.device_status() == 0
+
+
+def test_softcap_is_exact_to_a_rounding(ctx):
+    """The cap's relative error, brought out by a cap of 2^20: two keys whose scores differ by a few units before the cap,
+    weights read off one-hot values. Bound of a pair's log ratio: 1.1e-7 of either capped score below 0.75 caps, 1.7e-7
+    above, and the two outputs' rounding to bf16 (2^-8 together)."""
+    hd, kvh, bs, n, cap = 64, 8, 16, 400, 2.0 ** 20
+    g = torch.Generator().manual_seed(99)
+    y = torch.empty(n, kvh).uniform_(0.05, 2.5, generator=g)
+    s = (y * cap).to(torch.bfloat16).double()
+    y = s / cap
+    d = torch.ceil(torch.empty(n, kvh).uniform_(0.2, 1.5, generator=g).double() / (1 - torch.tanh(y) ** 2)).to(torch.bfloat16).double()
+    k = torch.zeros(n, kvh, bs, hd)
+    k[:, :, 0, 0], k[:, :, 1, 0], k[:, :, 1, 1] = s.float(), s.float(), d.float()
+    v = torch.zeros(n, kvh, bs, hd)
+    v[:, :, 0, 0] = v[:, :, 1, 1] = 1
+    kv = api.PagedKv(ctx, api.KvSpec(1, kvh, hd, n, bs))
+    for b in range(n):
+        kv.write_block_bytes(b, torch.cat([k[b].reshape(-1), v[b].reshape(-1)]).to(torch.bfloat16).view(torch.uint8).numpy().tobytes())
+    q = torch.zeros(n, kvh, hd, dtype=torch.bfloat16)
+    q[:, :, :2] = 1
+    got = api.paged_attention(ctx, kv, 0, q.cuda(), [api.SeqStep(1, 1, 1, [b]) for b in range(n)], 1.0, cap).cpu().double().view(n, kvh, hd)
+    ratio = torch.log(got[:, :, 1] / got[:, :, 0])
+    want = cap * (torch.tanh((s + d) / cap) - torch.tanh(y))
+    bound = torch.where(y < 0.75, 1.1e-7, 1.7e-7) * 2 * cap * torch.tanh(y) + 2 ** -8
+    over = (ratio - want).abs() / bound
+    assert float(over.max()) < 1, f"{float(over.max()):.2f} of the bound at {float(y.view(-1)[int(over.argmax())]):.3f} caps"
+    assert ctx.device_status() == 0
