@@ -340,10 +340,17 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
       if (!u.live()) continue;
       bool first_of_unit = true;
       for (; u.live() && ok;) {
-        // QK of this tile goes ahead of the pending PV when its operands are there; else the PV is issued first
-        bool ready = mbar_test_wait(&kv_full[kv.stage], kv.phase) && (!first_of_unit || mbar_test_wait(q_full, qphase));
-        ready = __all_sync(0xffffffffu, ready);
-        if (!ready && pend) { issue_pv(); if (!ok) break; }
+        // QK of this tile goes ahead of the pending PV when its operands are there before the probabilities are; a PV that
+        // is waited for first leaves the softmax warps without scores for the time of both products. The looks are limited:
+        // whatever is missing after them is waited for in the bounded waits below.
+        if (pend) {
+          for (int looks = 0; looks < 256; ++looks) {
+            const bool scores = mbar_test_wait(&kv_full[kv.stage], kv.phase) && (!first_of_unit || mbar_test_wait(q_full, qphase));
+            if (__all_sync(0xffffffffu, scores)) break;
+            if (looks == 255 || __all_sync(0xffffffffu, mbar_test_wait(&p_ready[pend_tile & 1], (pend_tile >> 1) & 1))) { issue_pv(); break; }
+          }
+          if (!ok) break;
+        }
         if (first_of_unit) {
           ok = warp_wait(q_full, qphase, p.status, KC_DEV_ATTN | 5);
           if (!ok) break;
@@ -426,52 +433,40 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
             }
             tmem_wait_st();
           }
-          uint32_t v[TK];
+          // Two passes over the tile's scores, 64 columns a turn: unrolled over the tile they were 25 KB of instructions, which
+          // a launch fetches anew, most of the time of a short context.
+          uint32_t va[32], vb[32];
+          auto mask = [&](uint32_t (&v)[32], int c) {
+            if (edge) {
 #pragma unroll
-          for (int c = 0; c < TK / 32; ++c) tmem_ld32_issue(s_addr + c * 32, v + c * 32);
-          tmem_wait_ld();
-          auto mask = [&]() {
-#pragma unroll
-            for (int j = 0; j < TK; ++j)
-              if (j > hi || j < lo) v[j] = 0xff800000u;   // -inf
+              for (int j = 0; j < 32; ++j)
+                if (c + j > hi || c + j < lo) v[j] = 0xff800000u;   // -inf
+            }
           };
-          if (edge) mask();
           // three operands an instruction
           float t0 = -INFINITY, t1 = -INFINITY, t2 = -INFINITY, t3 = -INFINITY;
+#pragma unroll 1
+          for (int c = 0; c < TK; c += 64) {
+            tmem_ld32_issue(s_addr + c, va);
+            tmem_ld32_issue(s_addr + c + 32, vb);
+            tmem_wait_ld();
+            tmem_pin32(va);
+            tmem_pin32(vb);
+            mask(va, c);
+            mask(vb, c + 32);
 #pragma unroll
-          for (int j = 0; j < TK; j += 8) {
-            t0 = fmaxf(t0, fmaxf(__uint_as_float(v[j]), __uint_as_float(v[j + 1])));
-            t1 = fmaxf(t1, fmaxf(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])));
-            t2 = fmaxf(t2, fmaxf(__uint_as_float(v[j + 4]), __uint_as_float(v[j + 5])));
-            t3 = fmaxf(t3, fmaxf(__uint_as_float(v[j + 6]), __uint_as_float(v[j + 7])));
-          }
-          float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)), mul = scale_log2;
-          if (FOLDED && p.softcap > 0.f) {
-            mul = cap_log2;
-            // A tile with no score past 0.75 caps takes the polynomial alone, two elements at a time; an element's value is
-            // the same on both sides.
-            float b0 = INFINITY, b1 = INFINITY;
-#pragma unroll
-            for (int j = 0; j < TK; j += 2) { b0 = fminf(b0, __uint_as_float(v[j])); b1 = fminf(b1, __uint_as_float(v[j + 1])); }
-            const float reach = fmaxf(tmax, -fminf(b0, b1)) * cap_arg;
-            // false where a mask has left -inf; rows past the unit's hold whatever shared memory held and have no say
-            const bool all_near = __all_sync(0xffffffffu, reach < SOFTCAP_NEAR || row >= u.rows);
-            const float2 arg = make_float2(cap_arg, cap_arg);
-            if (all_near) {
-#pragma unroll
-              for (int j = 0; j < TK; j += 2) {
-                const float2 r = softcap_near(mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg));
-                v[j] = __float_as_uint(r.x); v[j + 1] = __float_as_uint(r.y);
-              }
-            } else {
-#pragma unroll
-              for (int j = 0; j < TK; j += 2) {
-                const float2 y = mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg);
-                const float2 r = softcap_near(y);
-                v[j] = __float_as_uint(softcap_any(y.x, r.x)); v[j + 1] = __float_as_uint(softcap_any(y.y, r.y));
-              }
-              if (edge) mask();   // -inf has become -1
+            for (int j = 0; j < 32; j += 4) {
+              t0 = fmaxf(t0, fmaxf(__uint_as_float(va[j]), __uint_as_float(va[j + 1])));
+              t1 = fmaxf(t1, fmaxf(__uint_as_float(va[j + 2]), __uint_as_float(va[j + 3])));
+              t2 = fmaxf(t2, fmaxf(__uint_as_float(vb[j]), __uint_as_float(vb[j + 1])));
+              t3 = fmaxf(t3, fmaxf(__uint_as_float(vb[j + 2]), __uint_as_float(vb[j + 3])));
             }
+          }
+          tmem_ld32_issue(s_addr, va);   // arrives under what follows
+          float tmax = fmaxf(fmaxf(t0, t1), fmaxf(t2, t3)), mul = scale_log2;
+          const bool capped = FOLDED && p.softcap > 0.f;
+          if (capped) {
+            mul = cap_log2;
             const bool seen = !edge || (hi >= 0 && lo < TK && lo <= hi);   // any key: a score of -inf is a key of weight e^-cap
             if (seen) { tmax *= cap_arg; tmax = softcap_any(tmax, softcap_near(make_float2(tmax, tmax)).x); }   // grows with the score
           }
@@ -481,28 +476,67 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
           // precision: l, O and the two parts of a probability are floating-point numbers.
           if (tmax > m + 8.f) { alpha = ex2(m - tmax); m = tmax; }   // from -inf: alpha = 0
           const float ref = m == -INFINITY ? 0.f : m;
-          const float2 muls = make_float2(mul, mul), refs = make_float2(-ref, -ref);
-          const float2 minus1 = make_float2(-1.f, -1.f);
+          const float2 muls = make_float2(mul, mul), refs = make_float2(-ref, -ref), minus1 = make_float2(-1.f, -1.f);
           float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-          uint32_t w[32];
+          // 32 scores of the row -> 32 columns of probabilities, as two bf16 numbers each: the columns of a 16-key block get
+          // its eight pairs' upper parts, then what those leave over
+          auto group = [&](uint32_t (&v)[32], int c) {
+            if (capped) {
+              // A group with no score past 0.75 caps takes the polynomial alone, two elements at a time; an element's value
+              // is the same on both sides.
+              float b0 = 0.f, b1 = 0.f;
 #pragma unroll
-          for (int j = 0; j < TK; j += 4) {
-            float2 e = fma2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), muls, refs);
-            float2 f = fma2(make_float2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), muls, refs);
-            e.x = ex2(e.x); e.y = ex2(e.y); f.x = ex2(f.x); f.y = ex2(f.y);
-            s0 = add2(s0, e); s1 = add2(s1, f);
-            // probabilities as two bf16 numbers each: the columns of a 16-key block get its eight pairs' upper parts, then
-            // what those leave over
-            const uint32_t eh[2] = {__float_as_uint(e.x) & 0xffff0000u, __float_as_uint(e.y) & 0xffff0000u};
-            const uint32_t fh[2] = {__float_as_uint(f.x) & 0xffff0000u, __float_as_uint(f.y) & 0xffff0000u};
-            const int at = (j & 16) + (j & 15) / 2;
-            w[at] = __byte_perm(eh[0], eh[1], 0x7632);
-            w[at + 1] = __byte_perm(fh[0], fh[1], 0x7632);
-            const float2 el = fma2(make_float2(__uint_as_float(eh[0]), __uint_as_float(eh[1])), minus1, e);
-            const float2 fl = fma2(make_float2(__uint_as_float(fh[0]), __uint_as_float(fh[1])), minus1, f);
-            w[at + 8] = pack_bf162(el.x, el.y);
-            w[at + 9] = pack_bf162(fl.x, fl.y);
-            if ((j & 31) == 28) tmem_st32(s_addr + (j & ~31), w);
+              for (int j = 0; j < 32; j += 2) { b0 = fmaxf(b0, fabsf(__uint_as_float(v[j]))); b1 = fmaxf(b1, fabsf(__uint_as_float(v[j + 1]))); }
+              // columns that hold an older tile's scores and rows past the unit's have no say but in the time it takes
+              const bool all_near = __all_sync(0xffffffffu, fmaxf(b0, b1) * cap_arg < SOFTCAP_NEAR || row >= u.rows);
+              const float2 arg = make_float2(cap_arg, cap_arg);
+              if (all_near) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                  const float2 r = softcap_near(mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg));
+                  v[j] = __float_as_uint(r.x); v[j + 1] = __float_as_uint(r.y);
+                }
+              } else {
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                  const float2 y = mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg);
+                  const float2 r = softcap_near(y);
+                  v[j] = __float_as_uint(softcap_any(y.x, r.x)); v[j + 1] = __float_as_uint(softcap_any(y.y, r.y));
+                }
+              }
+            }
+            mask(v, c);
+            uint32_t w[32];
+#pragma unroll
+            for (int j = 0; j < 32; j += 4) {
+              float2 e = fma2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), muls, refs);
+              float2 f = fma2(make_float2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), muls, refs);
+              e.x = ex2(e.x); e.y = ex2(e.y); f.x = ex2(f.x); f.y = ex2(f.y);
+              s0 = add2(s0, e); s1 = add2(s1, f);
+              const uint32_t eh[2] = {__float_as_uint(e.x) & 0xffff0000u, __float_as_uint(e.y) & 0xffff0000u};
+              const uint32_t fh[2] = {__float_as_uint(f.x) & 0xffff0000u, __float_as_uint(f.y) & 0xffff0000u};
+              const int at = (j & 16) + (j & 15) / 2;
+              w[at] = __byte_perm(eh[0], eh[1], 0x7632);
+              w[at + 1] = __byte_perm(fh[0], fh[1], 0x7632);
+              const float2 el = fma2(make_float2(__uint_as_float(eh[0]), __uint_as_float(eh[1])), minus1, e);
+              const float2 fl = fma2(make_float2(__uint_as_float(fh[0]), __uint_as_float(fh[1])), minus1, f);
+              w[at + 8] = pack_bf162(el.x, el.y);
+              w[at + 9] = pack_bf162(fl.x, fl.y);
+            }
+            tmem_st32(s_addr + c, w);
+          };
+          tmem_wait_ld();
+          tmem_pin32(va);
+#pragma unroll 1
+          for (int c = 0; c < TK; c += 64) {
+            tmem_ld32_issue(s_addr + c + 32, vb);
+            group(va, c);
+            tmem_wait_ld();
+            tmem_pin32(vb);
+            if (c + 64 < TK) tmem_ld32_issue(s_addr + c + 64, va);
+            group(vb, c + 32);
+            tmem_wait_ld();
+            tmem_pin32(va);
           }
           l = __fmaf_rn(l, alpha, (s0.x + s0.y) + (s1.x + s1.y));
           if (!first && !__all_sync(0xffffffffu, alpha == 1.f || row >= u.rows)) {
