@@ -307,7 +307,6 @@ struct QlKernelParams {
   int row0;              // first activation row
   int splits;
   int a_stages, r_stages, b_stages;   // ring depths: stages in TMEM, k-blocks of records and stages of activations in shared memory
-  int wide;              // a scale of the weight is past ql_scale_limit
   int glu;               // 0, or 1 (silu) / 2 (gelu_approx): the epilogue writes act = activation(gate tile) * up tile
   bf16* act; int ld_act;
   uint32_t tmem_cols;    // columns allocated: a power of two
@@ -423,7 +422,7 @@ __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* sm
 //
 // TMEM columns: [2 accumulators of round32(m_pad)] [a_stages x 2 units x 32 columns of bf16 pairs].
 // ---------------------------------------------------------------------------
-template <int BITS, int GPK, int NT, int P>
+template <int BITS, int GPK, int NT, int P, bool WIDE>
 __global__ void __launch_bounds__(QL_THREADS, 1)
 qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKernelParams p) {
   constexpr int KC = NT == 1 ? 2 : 1;                   // slots of records and activations in a stage (see below)
@@ -600,7 +599,7 @@ qlinear_umma_ta_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKer
           const uint2 s = *reinterpret_cast<const uint2*>(row_sb + at);
           sb[0] = bf2_bits(s.x); sb[GPK - 1] = bf2_bits(s.y);
         }
-        if (!p.wide) dequant_row<BITS, GPK>(row_raw + at, sb, v);
+        if (!WIDE) dequant_row<BITS, GPK>(row_raw + at, sb, v);
         else dequant_row_wide<BITS, GPK>(row_raw + at, sb, v);
         if (q == 0) {
           if (!__all_sync(0xffffffffu, a_free)) ok = warp_wait(&a_empty[2 * as + unit], aphase ^ 1, p.status, KC_DEV_QLINEAR | 6);
@@ -665,7 +664,7 @@ static TaPlan plan_ta(int nt, int per, int m_pad, uint32_t record_bytes) {
   return t;
 }
 
-template <int BITS, int GPK, int NT, int P>
+template <int BITS, int GPK, int NT, int P, bool WIDE>
 static cudaError_t launch_umma_ta(const QLinearLaunch& l, QlKernelParams& p, cudaStream_t s) {
   const QWeight& w = *l.w;
   const TaPlan t = plan_ta(NT, P, p.m_pad, p.record_bytes);
@@ -674,20 +673,22 @@ static cudaError_t launch_umma_ta(const QLinearLaunch& l, QlKernelParams& p, cud
   p.a_stages = t.sa; p.b_stages = t.sb; p.r_stages = t.rs;
   static DeviceOnce configured;   // the attribute belongs to the device's copy of the kernel
   if (configured.first_on_current_device()) {
-    cudaError_t e = cudaFuncSetAttribute(qlinear_umma_ta_kernel<BITS, GPK, NT, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(qlinear_umma_ta_kernel<BITS, GPK, NT, P, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) { configured.forget_current_device(); return e; }
   }
   const CUtensorMap* rows = act_operand_rows_map(l.x, p.m_pad);
   if (!rows) return cudaErrorInvalidValue;
   dim3 grid((w.n_tiles + NT - 1) / NT, w.splits, (p.M + p.m_pad - 1) / p.m_pad);
-  return launch_k(qlinear_umma_ta_kernel<BITS, GPK, NT, P>, grid, dim3(QL_THREADS), t.smem, s, *rows, p);
+  return launch_k(qlinear_umma_ta_kernel<BITS, GPK, NT, P, WIDE>, grid, dim3(QL_THREADS), t.smem, s, *rows, p);
 }
 
 template <int BITS, int GPK>
 static cudaError_t launch_umma_nt(const QLinearLaunch& l, QlKernelParams& p, int nt, cudaStream_t s) {
+  // a scale of the weight is past ql_scale_limit: kernels of its own, so that the others don't carry the conversion
+  if (l.w->wide_scale) return nt == 2 ? launch_umma_ta<BITS, GPK, 2, 1, true>(l, p, s) : launch_umma_ta<BITS, GPK, 1, 1, true>(l, p, s);
   if (plan_ta(nt, 2, p.m_pad, p.record_bytes).ok)
-    return nt == 2 ? launch_umma_ta<BITS, GPK, 2, 2>(l, p, s) : launch_umma_ta<BITS, GPK, 1, 2>(l, p, s);
-  return nt == 2 ? launch_umma_ta<BITS, GPK, 2, 1>(l, p, s) : launch_umma_ta<BITS, GPK, 1, 1>(l, p, s);
+    return nt == 2 ? launch_umma_ta<BITS, GPK, 2, 2, false>(l, p, s) : launch_umma_ta<BITS, GPK, 1, 2, false>(l, p, s);
+  return nt == 2 ? launch_umma_ta<BITS, GPK, 2, 1, false>(l, p, s) : launch_umma_ta<BITS, GPK, 1, 1, false>(l, p, s);
 }
 
 // Weight tiles per CTA: two when the grid then still has about 0.7 CTAs per SM (measured: 112 CTAs of two tiles beat
@@ -740,7 +741,6 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   p.N = w.N; p.n_tiles = w.n_tiles; p.kblocks = w.kblocks;
   p.M = l.M; p.m_pad = plan_chunk_rows(w, nt, cap, l.M); p.row0 = l.row0;
   p.splits = w.splits;
-  p.wide = w.wide_scale;
   p.y = l.y; p.ldy = l.ldy; p.partial = l.partial; p.status = l.status;
   p.glu = glu ? l.glu : 0; p.act = l.act; p.ld_act = l.ld_act;
   if (w.bits == 4) return w.gpk == 2 ? launch_umma_nt<4, 2>(l, p, nt, s) : launch_umma_nt<4, 1>(l, p, nt, s);
