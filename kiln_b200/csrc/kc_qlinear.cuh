@@ -93,10 +93,15 @@ void qweight_free(QWeight* w);
 // *err) if the driver entry point is unavailable or rejects the geometry.
 bool act_operand_init(ActOperand* op, const bf16* ptr, int rows, int K, const char** err);
 
-// The GEMM (tcgen05 + TMEM + TMA). Returns a CUDA error. One launch, whatever the number of rows.
+// The GEMM (tcgen05 + TMEM + TMA). Returns a CUDA error. One launch of at most qlinear_slab_rows rows.
 cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s);
-// Rows that one call takes out of M: the workspace of a weight that is split along K holds QL_MAX_M.
-inline int qlinear_slab_rows(const QWeight& w, int M) { return w.splits > 1 && M > QL_MAX_M ? QL_MAX_M : M; }
+// Rows that one call takes out of M: the workspace of a weight that is split along K holds QL_MAX_M; a grid has 65535
+// chunks of 96 rows or more, and looking for the best number of them is host time that a launch of a million rows hides.
+constexpr int QL_LAUNCH_ROWS = 1 << 20;
+inline int qlinear_slab_rows(const QWeight& w, int M) {
+  const int most = w.splits > 1 ? QL_MAX_M : QL_LAUNCH_ROWS;
+  return M < most ? M : most;
+}
 
 // The weight-streaming lane for at most QL_STREAM_MAX_M rows: x bf16 [M, ldx] against dequant(W)^T, left as fp32
 // partials [qlinear_stream_pieces(w)][M][N] that the caller's consumer kernel (or qlinear_reduce_splits) sums in index

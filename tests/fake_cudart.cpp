@@ -79,5 +79,5 @@ EXPORT cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*,
   for (unsigned i = 0; i < c->numAttrs; ++i)
     early |= c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization && c->attrs[i].val.programmaticStreamSerializationAllowed;
   note(early ? "launch early" : "launch in order");
-  return cudaSuccess;
+  return c->gridDim.y > 65535 || c->gridDim.z > 65535 ? cudaErrorInvalidConfiguration : cudaSuccess;
 }

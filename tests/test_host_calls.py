@@ -89,3 +89,17 @@ fake.fake_reset()
 ok(attention([(3, 40)]))
 assert calls().count("copy") == 1
 """)
+
+
+@pytest.mark.parametrize("out_features", [384, 26700])
+def test_rows_beyond_the_chunks_of_one_launch(fake, out_features):
+    """Row chunks are the third dimension of a launch's grid, of which there are 65535 at most: more rows are more launches."""
+    run(fake, f"""
+w = C.c_void_p()
+words = C.create_string_buffer({out_features} * 64 // 2 + 256)
+ok(lib.kc_qweight_create(ctx, C.cast(words, C.POINTER(C.c_uint32)), words, words, {out_features}, 64, 4, 64, 0, C.byref(w)))
+for rows in (1, 700, 40000, 7000000, 17000000):
+    fake.fake_reset()
+    ok(lib.kc_quantized_matmul(ctx, w, at, rows, at))
+    assert calls().count("launch early") >= (1 if rows < 65535 * 192 else 2)
+""")
