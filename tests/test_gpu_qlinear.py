@@ -186,7 +186,8 @@ def test_stream_lane_rows_do_not_depend_on_row_count(ctx):
 @pytest.mark.parametrize("n,k,bits,group,m,gain", [
     (26700, 192, 4, 64, 33, 1.0),     # 209 tiles, two per CTA: the last CTA owns one; three k-blocks
     (26700, 64, 8, 64, 192, 1.0),     # one k-block: the second issuer has nothing to do
-    (384, 1088, 4, 32, 256, 1.0),     # one tile per CTA, 256 rows, splits of 8 and 9 k-blocks: stages with one k-block
+    (384, 1088, 4, 32, 192, 1.0),     # one tile per CTA, the most rows of one chunk, splits of 8 and 9 k-blocks: stages with one k-block
+    (384, 1088, 4, 32, 256, 1.0),     # the same in two chunks
     (384, 1088, 8, 32, 177, 1.0),     # 8-bit, rows past the activations' end inside the last group of 16
     (300, 512, 4, 64, 20, 200.0),     # scales of 0.5 and more: integers converted before the multiply-add
     (300, 512, 8, 64, 20, 300.0),     # the same for 8 bits (scales of 1/32 and more)
