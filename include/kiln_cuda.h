@@ -360,8 +360,11 @@ KC_API int kc_rms_norm(kc_ctx_t ctx, const void* x_dev, const void* weight_dev, 
  * bf16 [n, num_heads, head_dim] post-RoPE, this step's K/V already written.
  * Replaces PagedKv::gather + fast::scaled_dot_product_attention
  * (paged.rs:191-225, nn.rs:800-817) and the Metal kernels of
- * crates/kiln-engine/src/paged_attn.rs:59-303. softcap = 0 disables capping;
- * window = 0 is global. out: bf16 [n, num_heads*head_dim]. Synchronous (like kc_rope_kv_write below): the context keeps
+ * crates/kiln-engine/src/paged_attn.rs:59-303. scale: any number (0 weighs all
+ * keys alike, a negative one turns their order round). softcap = 0 disables
+ * capping; window = 0 is global. q: 16-byte aligned. out: bf16
+ * [n, num_heads*head_dim], best 16-byte aligned too (elsewhere the rows are
+ * copied there from a buffer of the call). Synchronous (like kc_rope_kv_write below): the context keeps
  * the call's metadata buffers and workspace for the next one, up to 64 MB. */
 KC_API int kc_paged_attention(kc_ctx_t ctx, kc_kv_t kv, int32_t layer, const void* q_dev,
                               int32_t n, int32_t num_heads, const kc_seq_step* seqs,

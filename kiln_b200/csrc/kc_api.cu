@@ -1192,11 +1192,11 @@ int ensure_attn_ws(kc_model* m, const StepPlan& p) {
   return KC_OK;
 }
 
-AttnParams attn_params(kc_model* m, kc_kv* kv, const StepPlan& p, int layer, const bf16* q, bf16* out, float scale,
-                       float softcap, int window, int Hq) {
+AttnParams attn_params(kc_model* m, kc_kv* kv, const StepPlan& p, int layer, bf16* out, float scale, float softcap, int window,
+                       int Hq) {
   AttnParams a{};
   const size_t rows = (size_t)p.n * Hq * p.max_chunks;
-  a.q = q; a.out = out;
+  a.out = out;
   a.part_o = m->attn_ws;
   a.part_ml = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(m->attn_ws) + align_up(rows * m->d.head_dim * 4, 256));
   a.block_tables = reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.tables);
@@ -1313,7 +1313,7 @@ int run_forward(kc_model* m, kc_kv* kv, const uint32_t* tokens_dev, const StepPl
     LAUNCH(c, KC_PROF_ROWWISE, 1, launch_rope_kv_write(so, L.qkv_bias, m->inv_freq, token_pos, kv_slot, n, m->Hq, m->Hkv, D, d.rope_traditional, l,
                             kv->num_blocks, kv->block_size, kv->pool, m->q_rot, c->stream));
     const int window = (d.sliding_window > 0 && (l % 2 == 0)) ? d.sliding_window : 0;
-    AttnParams a = attn_params(m, kv, p, l, m->q_rot, m->attn, m->attn_scale, gemma ? d.attn_logit_softcapping : 0.f, window, m->Hq);
+    AttnParams a = attn_params(m, kv, p, l, m->attn, m->attn_scale, gemma ? d.attn_logit_softcapping : 0.f, window, m->Hq);
     LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, false, D, n, c->sm_count, c->stream));
     if (streams(L.o)) RC(run_stream(c, L.o, m->attn, n, m->proj, H, m->partial, &so));
     else if (small(L.o)) RC(run_gemv(c, L.o, m->attn, n, m->proj, H, m->partial, &so));
@@ -1490,7 +1490,7 @@ extern "C" int kc_verify_step(kc_model_t m, kc_kv_t kv, const uint32_t* token_id
                             reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.v_draft_off),
                             reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.v_draft_len), n_seqs, 0, m->committed,
                             (int32_t*)(hb + o1), (int32_t*)(hb + o2), c->stream));
-      CK(cudaEventRecord(c->step_b, c->stream));
+    CK(cudaEventRecord(c->step_b, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     cudaEventElapsedTime(&c->last_step_ms, c->step_a, c->step_b);
     RC(status_verdict(c, "kc_verify_step"));
@@ -1498,7 +1498,7 @@ extern "C" int kc_verify_step(kc_model_t m, kc_kv_t kv, const uint32_t* token_id
     if (n_committed_out) memcpy(n_committed_out, hb + o1, (size_t)n_seqs * 4);
     if (n_accepted_out) memcpy(n_accepted_out, hb + o2, (size_t)n_seqs * 4);
   } else {
-      CK(cudaEventRecord(c->step_b, c->stream));
+    CK(cudaEventRecord(c->step_b, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     cudaEventElapsedTime(&c->last_step_ms, c->step_a, c->step_b);
     RC(status_verdict(c, "kc_verify_step"));
@@ -1677,7 +1677,7 @@ extern "C" int kc_paged_attention(kc_ctx_t c, kc_kv_t kv, int32_t layer, const v
     if (e != cudaSuccess) { out = (bf16*)out_dev; rc = fail(KC_ERR_OOM, "kc_paged_attention: %zu bytes: %s", out_bytes, cudaGetErrorString(e)); }
   }
   if (!rc) {
-    AttnParams a = attn_params(m, kv, p, layer, (const bf16*)q_dev, out, scale, softcap, window, num_heads);
+    AttnParams a = attn_params(m, kv, p, layer, out, scale, softcap, window, num_heads);
     rc = [&]() -> int {
       LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, true, kv->head_dim, n, c->sm_count, c->stream));
       if (out != out_dev) CK(cudaMemcpyAsync(out_dev, out, out_bytes, cudaMemcpyDeviceToDevice, c->stream));

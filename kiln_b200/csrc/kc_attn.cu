@@ -16,7 +16,7 @@
 //
 // What a row sees is a function of its own position only, so its bits do not depend on how many other rows share the
 // launch: keys are cut into chunks of ATT_CHUNK at absolute positions and a chunk into tiles; a chunk's sums start from
-// nothing, and the chunks of a row are merged one after the other in index order (merge_chunk) — by the kernel itself
+// nothing, and the chunks of a row are merged one after the other in index order (merge_values) — by the kernel itself
 // where a unit holds all chunks of its rows, by the combine kernel where the chunks of an item are units of their own.
 //
 // A probability goes to the tensor core as two bf16 numbers, its upper 16 bits and what they leave: with one, rounded, the
@@ -56,7 +56,6 @@ struct AttnShape {
   static constexpr int O_BUFS = D == 256 ? 1 : 2;
   static constexpr int TMEM_O = 256;                   // columns: S0 at 0, S1 at TK, O from 256
   static constexpr int TMEM_COLS = 512;
-  static constexpr int TILES_PER_CHUNK = ATT_CHUNK / TK;
   static constexpr int SMEM = RING * TILE_BYTES + Q_BYTES + 2 * ATT_ROWS * 8 + 32 * 8;
   static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
 };

@@ -19,7 +19,6 @@ struct AttnUnit {
 constexpr int ATT_SMALL_TOKENS = 8;
 
 struct AttnParams {
-  const bf16* q;               // [n_tokens, Hq, D] post-RoPE
   bf16* out;                   // [n_tokens, Hq * D], 16-byte aligned
   float* part_o;               // [n_tokens * Hq][max_chunks][D]  un-normalised partial outputs
   float2* part_ml;             // [n_tokens * Hq][max_chunks]     (running max in log2 units, sum)

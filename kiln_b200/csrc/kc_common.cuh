@@ -89,21 +89,6 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded busy-poll (no hardware suspend): lowest wake-up latency, costs issue slots.
-__device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, uint32_t* status, uint32_t code) {
-  if (mbar_test_wait(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
-  uint32_t spins = 0;
-  while (!mbar_test_wait(bar, parity)) {
-    if ((++spins & 0xfff) == 0) {
-      if (globaltimer_ns() - t0 > KC_SPIN_LIMIT_NS) {
-        if (status) atomicOr(status, code);
-        return false;
-      }
-    }
-  }
-  return true;
-}
 // Bounded wait. On timeout: ORs `code` into *status (if non-null) and returns
 // false; the caller must then leave its pipeline loop.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* status,

@@ -71,10 +71,10 @@ extern "C" int kc_quantized_matmul_static(kc_ctx_t c, kc_qweight_t q, const void
   }
 
   // Tensor maps of the activation buffer live on this stack frame; the launch copies them into the kernel's
-  // parameters. x must be readable for round_up(m, 16) rows, like kc_quantized_matmul.
+  // parameters. They end at row m, like kc_quantized_matmul's.
   ActOperand op;
   const char* terr = "";
-  if (!act_operand_init(&op, (const bf16*)x_dev, (m + 15) & ~15, w.K, &terr)) {
+  if (!act_operand_init(&op, (const bf16*)x_dev, m, w.K, &terr)) {
     snprintf(msg, sizeof msg, "kc_quantized_matmul_static: %s", terr);
     return api_fail(KC_ERR_CUDA, msg);
   }

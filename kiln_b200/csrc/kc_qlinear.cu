@@ -4,8 +4,7 @@
 //   warp 0      bulk-copies the weight records (cp.async.bulk, mbarrier tx)
 //   warp 1      TMA-loads the activation k-blocks (cp.async.bulk.tensor, 128B swizzle)
 //   warps 2-3   allocate TMEM, issue tcgen05.mma (weights = A/M side from TENSOR MEMORY, activations = B/N side
-//               from shared memory); the two issuing threads take alternate pipeline stages and pass the issue order
-//               to each other through an mbarrier
+//               from shared memory), each into an accumulator of its own: nothing orders them to each other
 //   warps 4-19  unpack the 4/8-bit words, apply scale/bias in registers and write the bf16 A operand into tensor
 //               memory with tcgen05.st; afterwards drain the accumulators (tcgen05.ld) into y, the split-K
 //               partials or the gated activation.
@@ -28,7 +27,7 @@ namespace kc {
 // Re-tiling
 // ---------------------------------------------------------------------------
 
-// Scales below this limit can be multiplied by 2^129 (4-bit) or 2^133 (8-bit) within bf16: see dequant_pairs.
+// Scales below this limit can be multiplied by 2^129 (4-bit) or 2^133 (8-bit) within bf16: see dequant_row.
 __host__ __device__ constexpr float ql_scale_limit(int bits) { return bits == 4 ? 0.5f : 0.03125f; }
 
 __global__ void qweight_retile_kernel(uint8_t* __restrict__ records, const uint32_t* __restrict__ w,
@@ -416,7 +415,7 @@ __device__ __forceinline__ void ql_epilogue(const QlKernelParams& p, uint8_t* sm
 // own — the CTA's two tiles, or the even and the odd k-blocks of its one tile, summed in the epilogue. A stage is one
 // unit of each. An issuing warp runs its loop converged with one elected lane around the MMAs: with `if (lane == 0)`
 // around the loop the operands of each MMA went through vector registers and eight MMAs took 700 cycles to issue.
-// 28672 x 4096 in 4 bits, 112 CTAs, every launch from HBM: 35.7 us -> 24 us at 1 row, 40.7 -> 37 us at 192 rows.
+// 28672 x 4096 in 4 bits, 112 CTAs, every launch from HBM: 35.7 us -> 21 us at 1 row, 40.7 -> 37 us at 192 rows.
 //
 // The order in which an element's k-blocks are accumulated is a function of the weight's shape only.
 //
@@ -697,10 +696,13 @@ static int plan_tiles_per_cta(const QWeight& w, int sm_count) {
   return ((w.n_tiles + 1) / 2) * w.splits * 10 >= sm_count * 7 ? 2 : 1;
 }
 
-// The most rows one CTA takes: what the accumulators (two tiles: 192 columns each, one tile: 256) and the rings of the
-// weight's record size leave room for.
+// The most rows one CTA takes: what the two accumulators (192 columns each) and the rings of the weight's record size
+// leave room for. With one tile per CTA and one accumulator it was 256 rows; the two accumulators of that form (even and
+// odd k-blocks) take 10 to 30 % off launches of up to 192 rows and of more than 256, and the second chunk that 193 to 256
+// rows need costs up to 25 % (4096 x 4096, L2 flushed: 23.6 -> 27.6 us at 193 rows, 25.6 -> 29.7 at 256; 21.5 at 192,
+// 33.8 -> 31.7 at 257). One accumulator for these rows alone would give them other bits than fewer rows have.
 static int plan_row_cap(int nt, uint32_t record_bytes) {
-  static const int caps[] = {256, 192, 128, 64, 32, 16};
+  static const int caps[] = {192, 128, 64, 32, 16};
   for (int c : caps)
     if (plan_ta(nt, 1, c, record_bytes).ok) return c;
   return 0;
@@ -708,7 +710,9 @@ static int plan_row_cap(int nt, uint32_t record_bytes) {
 
 // Rows of a chunk (one CTA's share of the rows) for M rows. All chunks are one launch, CTAs of the next filling the SMs
 // that the last wave of one leaves idle; the chunk size is the one whose waves take the least time, counted in MMA
-// cycles: a unit of 128 x 64 weights takes 2 cycles per row, not less than 184, and a CTA about 6000 around them.
+// cycles: a unit of 128 x 64 weights takes 2 cycles per row, not less than 184, and a CTA about 6000 around them. Chunks of
+// fewer than 96 rows are not looked at: a unit takes its 184 cycles then, whatever the rows, so more chunks are only more
+// waves.
 // 28672 x 4096, 2048 rows: 13 chunks of 160 rows are 10 waves, 368 us; 11 chunks of 192, a launch each, took 450.
 static int plan_chunk_rows(const QWeight& w, int nt, int cap, int M) {
   const int ctas = ((w.n_tiles + nt - 1) / nt) * w.splits;
