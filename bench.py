@@ -192,12 +192,12 @@ def algorithmic(cfg, batch, k, mean_ctx):
             "attn_flops": attn_flops, "M": M}
 
 
-# DRAM traffic of the dominant kernel (the quantised GEMM) relative to its algorithmic weight bytes, from one ncu
-# capture of a single launch larger than L2 (out 128256 x in 4096, 192 rows; summary committed under profiles/):
-# dram__bytes_read.sum + dram__bytes_write.sum = 299.9 MB + 33.6 MB for 295.5 MB of weight records. The traffic of a
-# launch grows in proportion to its weight bytes, so the per-launch figure reported is this ratio times the mean
-# algorithmic weight bytes per GEMM launch of the step.
-GEMM_DRAM_TRAFFIC_PER_WEIGHT_BYTE = (299.9 + 33.6) / 295.5
+# DRAM traffic of the dominant kernel (the quantised GEMM) relative to its algorithmic weight bytes, from ncu captures of
+# single launches at 192 rows (summary committed under profiles/): dram__bytes_read.sum + dram__bytes_write.sum = 67.7 MB +
+# 1.7 MB for the 66.1 MB of records of a layer's gate_up, whose rows are one chunk, and 594.6 MB + 41.8 MB for the 295.5 MB
+# of the head, whose rows are two. Weighted by the step's bytes (the head is 0.07 of them); the per-launch figure reported
+# is this ratio times the mean algorithmic weight bytes per GEMM launch of the step.
+GEMM_DRAM_TRAFFIC_PER_WEIGHT_BYTE = 0.93 * (67.7 + 1.7) / 66.1 + 0.07 * (594.6 + 41.8) / 295.5
 
 # --------------------------------------------------------------------------------------
 # GPU arm

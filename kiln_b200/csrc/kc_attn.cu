@@ -21,7 +21,8 @@
 //
 // A probability goes to the tensor core as two bf16 numbers, its upper 16 bits and what they leave: with one, rounded, the
 // result was 0.3 to 5 % further from fp64 than with the kernel before this one, whose smaller tiles had more of their
-// largest weights at exactly 1; with two the error is that of rounding the output (1.65e-3 of its norm; one: 2.1 to 2.2e-3).
+// largest weights at exactly 1; with two the error is that of rounding the output (1.65e-3 of its norm; one: up to 2.2e-3).
+// Whether a row is computed alone or among others, its probabilities, their order and so its bits are the same.
 //
 // Roles (12 warps, one CTA per SM, units taken grid-stride so that K/V tiles of the next unit arrive under the last one):
 //   warp 0      TMA: queries of a unit, K/V tiles through a ring
@@ -29,10 +30,12 @@
 //   warps 4-7   softmax, one row per thread: S -> P, rescaling O when a row's maximum moved
 //   warps 8-11  a finished chunk's O: store the partial, or merge it into the row and store the row
 //
-// What bounds it: per 128-key tile of head size 128, HBM takes 2800 cycles of an SM's share, a softmax warp about 2400
-// (scores and maximum 430, 128 exponentials 1300, of which 1024 the special-function unit's, stores 280, next tile 375),
-// the MMAs 1024. Against one mma.sync warp per 16 query rows with a combine launch: 32 sequences of 1438 keys and 6 rows
-// 69.1 -> 55.8 us; prefill of 2048 tokens after 2048 on the 8B model 64.9 -> 43.2 ms, its attention now 140 us a layer.
+// What bounds it: per 128-key tile of head size 128, HBM takes 2800 cycles of an SM's share, a softmax warp about 2900
+// (scores and maximum 590, exponentials and both parts of the probabilities 2000, of which 1024 the special-function
+// unit's, next tile 200) and 800 to 1300 in which it waits for scores, the MMAs 1500. Against one mma.sync warp per 16
+// query rows with a combine launch: 32 sequences of 1438 keys and 6 rows 69.1 -> 54.9 us; 1024 rows after 2048 keys 397 ->
+// 83 us; slower with a soft cap at head sizes 64 and 128 (16 sequences of 6000 keys, 4 rows: 121 -> 133 us at 128) and for
+// many short contexts (48 of 40 keys: 16 -> 23 us).
 #include "kc_attn.cuh"
 
 #include "kc_umma.cuh"
