@@ -125,6 +125,10 @@ struct kc_kv {
   size_t bytes = 0;
   CUtensorMap map;             // all pool rows x head_dim, box {64, 8}, 128-byte swizzle; or, with map5d, the 5-D
   bool map5d = false;          // map whose box is 16 keys of K and V of a layer (make_tmap_kv_5d)
+  CUtensorMap map_one;         // the same for 16 keys of K or of V; without map5d a copy of `map`
+  struct Written { uint32_t step = 0; int32_t seq = 0; };
+  std::vector<Written> written;   // the last step that wrote a block, and for which sequence (-1: several)
+  uint32_t step = 0;
 };
 
 struct kc_qweight {
@@ -404,12 +408,14 @@ extern "C" int kc_kv_create(kc_ctx_t c, int32_t layers, int32_t kv_heads, int32_
   const char* terr = "";
   if (e == cudaSuccess && !getenv("KILN_KV_MAP_2D")) {   // KILN_KV_MAP_2D=1 keeps the 2-D map
     const char* e4 = "";
-    kv->map5d = make_tmap_kv_5d(&kv->map, kv->pool, head_dim, (uint64_t)num_blocks * kv_heads * block_size, (uint64_t)layers * 2, &e4);
+    const uint64_t plane_rows = (uint64_t)num_blocks * kv_heads * block_size, planes = (uint64_t)layers * 2;
+    kv->map5d = make_tmap_kv_5d(&kv->map, kv->pool, head_dim, plane_rows, planes, 2, &e4) && make_tmap_kv_5d(&kv->map_one, kv->pool, head_dim, plane_rows, planes, 1, &e4);
   }
   if (e != cudaSuccess || (!kv->map5d && !make_tmap_kv_2d(&kv->map, kv->pool, head_dim, rows, &terr))) {
     cudaFree(kv->pool); delete kv;
     return fail(KC_ERR_CUDA, "kc_kv_create: %s", e != cudaSuccess ? cudaGetErrorString(e) : terr);
   }
+  if (!kv->map5d) kv->map_one = kv->map;
   g_live++;
   *out = kv;
   return KC_OK;
@@ -1034,8 +1040,8 @@ struct StepPlan {
 };
 
 // The step's attention units: items of up to tokens_per_item tokens of a sequence, each as one unit over all its chunks,
-// longest first, or as one unit per chunk, whole chunks first.
-void plan_attention(StepPlan* p, const kc_seq_step* seqs, int head_dim, int kv_heads, int sm_count) {
+// longest first, or as one unit per chunk, whole chunks first. old: per sequence, see AttnUnit.
+void plan_attention(StepPlan* p, const kc_seq_step* seqs, const std::vector<int>& old, int head_dim, int gqa, int kv_heads, int sm_count) {
   std::vector<AttnUnit>& items = p->units;
   items.clear();
   int row = 0;
@@ -1046,6 +1052,7 @@ void plan_attention(StepPlan* p, const kc_seq_step* seqs, int head_dim, int kv_h
       u.seq = i; u.tok0 = row + t; u.ntok = std::min(p->tokens_per_item, s.len - t); u.pos0 = s.offset + t;
       u.chunk0 = 0; u.chunk1 = (u.pos0 + u.ntok - 1) / ATT_CHUNK + 1;
       u.small = p->tokens_per_item > ATT_SMALL_TOKENS && u.ntok <= ATT_SMALL_TOKENS ? 1 : 0;
+      u.old = old[i];
       items.push_back(u);
     }
     row += s.len;
@@ -1053,7 +1060,7 @@ void plan_attention(StepPlan* p, const kc_seq_step* seqs, int head_dim, int kv_h
   std::stable_sort(items.begin(), items.end(), [](const AttnUnit& a, const AttnUnit& b) { return a.pos0 + a.ntok > b.pos0 + b.ntok; });
   std::vector<int> tiles(items.size());
   for (size_t i = 0; i < items.size(); ++i) tiles[i] = (items[i].pos0 + items[i].ntok + 127) / 128;
-  p->whole = attn_whole(head_dim, tiles.data(), (int)items.size(), kv_heads, sm_count);
+  p->whole = attn_whole(head_dim, p->tokens_per_item * gqa, tiles.data(), (int)items.size(), kv_heads, sm_count);
   if (p->whole) return;
   std::vector<AttnUnit> full, rest;
   for (const AttnUnit& u : items)
@@ -1065,6 +1072,28 @@ void plan_attention(StepPlan* p, const kc_seq_step* seqs, int head_dim, int kv_h
   std::stable_sort(rest.begin(), rest.end(), [](const AttnUnit& a, const AttnUnit& b) { return (a.pos0 + a.ntok - 1) % ATT_CHUNK > (b.pos0 + b.ntok - 1) % ATT_CHUNK; });
   full.insert(full.end(), rest.begin(), rest.end());
   items.swap(full);
+}
+
+// Per sequence, the keys from its start that nothing in this step writes: those before its new tokens, as far as no other
+// sequence of the step writes into one of their blocks (a caller may hand in pieces of one sequence as several).
+std::vector<int> old_keys(kc_kv* kv, const kc_seq_step* seqs, int n_seqs) {
+  if (kv->written.empty()) kv->written.resize(kv->num_blocks);
+  if (++kv->step == 0) { std::fill(kv->written.begin(), kv->written.end(), kc_kv::Written{}); kv->step = 1; }
+  for (int i = 0; i < n_seqs; ++i)
+    for (int b = seqs[i].offset / kv->block_size; b <= (seqs[i].offset + seqs[i].len - 1) / kv->block_size; ++b) {
+      kc_kv::Written& w = kv->written[seqs[i].blocks[b]];
+      w.seq = w.step == kv->step && w.seq != i ? -1 : i;
+      w.step = kv->step;
+    }
+  std::vector<int> old(n_seqs);
+  for (int i = 0; i < n_seqs; ++i) {
+    old[i] = seqs[i].offset;
+    for (int b = 0; b * kv->block_size < seqs[i].offset; ++b) {
+      const kc_kv::Written& w = kv->written[seqs[i].blocks[b]];
+      if (w.step == kv->step && w.seq != i) { old[i] = b * kv->block_size; break; }
+    }
+  }
+  return old;
 }
 
 int validate_step(kc_model* m, kc_kv* kv, const uint32_t* token_ids, int32_t n, const kc_seq_step* seqs, int32_t n_seqs,
@@ -1105,7 +1134,7 @@ int validate_step(kc_model* m, kc_kv* kv, const uint32_t* token_ids, int32_t n, 
   const int gqa = m->d.num_heads / m->d.num_kv_heads;
   p.tokens_per_item = attn_tokens_per_item(gqa, p.max_len);
   p.max_chunks = (max_ctx + ATT_CHUNK - 1) / ATT_CHUNK;
-  plan_attention(&p, seqs, m->d.head_dim, m->Hkv, m->ctx->sm_count);
+  plan_attention(&p, seqs, old_keys(kv, seqs, n_seqs), m->d.head_dim, gqa, m->Hkv, m->ctx->sm_count);
   MetaLayout& L = p.lay;
   size_t at = 0;
   auto put = [&](size_t bytes) { size_t o = at; at = align_up(at + bytes, 16); return o; };
@@ -1314,7 +1343,7 @@ int run_forward(kc_model* m, kc_kv* kv, const uint32_t* tokens_dev, const StepPl
                             kv->num_blocks, kv->block_size, kv->pool, m->q_rot, c->stream));
     const int window = (d.sliding_window > 0 && (l % 2 == 0)) ? d.sliding_window : 0;
     AttnParams a = attn_params(m, kv, p, l, m->attn, m->attn_scale, gemma ? d.attn_logit_softcapping : 0.f, window, m->Hq);
-    LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, false, D, n, c->sm_count, c->stream));
+    LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, kv->map_one, m->q_map, m->q_map_small, a, false, D, n, c->sm_count, c->stream));
     if (streams(L.o)) RC(run_stream(c, L.o, m->attn, n, m->proj, H, m->partial, &so));
     else if (small(L.o)) RC(run_gemv(c, L.o, m->attn, n, m->proj, H, m->partial, &so));
     else RC(run_qlinear(c, L.o, m->op_attn, n, d.tp_world > 1 ? tp_out_buffer(m) : m->proj, H, m->partial, d.tp_world > 1 ? nullptr : &so));
@@ -1679,7 +1708,7 @@ extern "C" int kc_paged_attention(kc_ctx_t c, kc_kv_t kv, int32_t layer, const v
   if (!rc) {
     AttnParams a = attn_params(m, kv, p, layer, out, scale, softcap, window, num_heads);
     rc = [&]() -> int {
-      LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, m->q_map, m->q_map_small, a, true, kv->head_dim, n, c->sm_count, c->stream));
+      LAUNCH(c, KC_PROF_ATTN, attn_launches(p), paged_attention(kv->map, kv->map_one, m->q_map, m->q_map_small, a, true, kv->head_dim, n, c->sm_count, c->stream));
       if (out != out_dev) CK(cudaMemcpyAsync(out_dev, out, out_bytes, cudaMemcpyDeviceToDevice, c->stream));
       return KC_OK;
     }();

@@ -30,15 +30,15 @@
 //   warps 4-7   softmax, one row per thread: S -> P, rescaling O when a row's maximum moved
 //   warps 8-11  a finished chunk's O: store the partial, or merge it into the row and store the row
 //
+// Units of at most KEY_ROWS rows go to kc_attn_keys.cu: this kernel takes prompts and steps that hold a piece of one.
+//
 // What bounds it: per 128-key tile of head size 128, HBM takes 2800 cycles of an SM's share, a softmax warp about 2900
 // (scores and maximum 590, exponentials and both parts of the probabilities 2000, of which 1024 the special-function
-// unit's, next tile 200) and 800 to 1300 in which it waits for scores, the MMAs 1500. Against one mma.sync warp per 16
-// query rows with a combine launch: 32 sequences of 1438 keys and 6 rows 69.1 -> 54.9 us; 1024 rows after 2048 keys 397 ->
-// 83 us; slower with a soft cap at head sizes 64 and 128 (16 sequences of 6000 keys, 4 rows: 121 -> 133 us at 128) and for
-// many short contexts (48 of 40 keys: 16 -> 23 us).
+// unit's, next tile 200) and 800 to 1300 in which it waits for scores, the MMAs 1500. 1024 rows after 2048 keys 83 us (397 by
+// one mma.sync warp per 16 query rows with a combine launch).
 #include "kc_attn.cuh"
 
-#include "kc_umma.cuh"
+#include "kc_attn_dev.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -62,124 +62,6 @@ struct AttnShape {
   static constexpr int SMEM = RING * TILE_BYTES + Q_BYTES + 2 * ATT_ROWS * 8 + 32 * 8;
   static_assert(SMEM <= 227 * 1024, "shared memory of one CTA");
 };
-
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Two fp32 operations an instruction.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
-      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return r;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-
-// tanh(y) for |y| < SOFTCAP_NEAR: y + y^3 p(y^2), p fitted for the smallest largest relative error; 1.0e-7 at most, 3.5e-8
-// root mean square. No special-function operation.
-constexpr float SOFTCAP_NEAR = 0.75f;
-__device__ __forceinline__ float2 softcap_near(float2 y) {
-  auto both = [](float x) { return make_float2(x, x); };
-  const float2 z = mul2(y, y);
-  float2 p = fma2(z, both(-0.0047694784589f), both(0.0196648966521f));
-  p = fma2(p, z, both(-0.0533902496099f));
-  p = fma2(p, z, both(0.1332652121782f));
-  p = fma2(p, z, both(-0.3333306908607f));
-  return fma2(mul2(y, z), p, y);
-}
-// tanh(y) anywhere: further out (1 - u) / (1 + u) with u = e^(-2 |y|), 1.7e-7 at most; 1 and -1 at the infinities, NaN stays
-// NaN. Nowhere less exact than tanhf, which is up to 2.0e-7 off.
-__device__ __forceinline__ float softcap_any(float y, float near) {
-  const float u = ex2(fabsf(y) * -2.8853900817779268f), d = u + 1.f;
-  float r = rcp_approx(d);
-  r = __fmaf_rn(r, __fmaf_rn(-d, r, 1.f), r);
-  const float far = copysignf(__fmaf_rn(-2.f * u, r, 1.f), y);
-  return fabsf(y) < SOFTCAP_NEAR ? near : far;
-}
-
-// Adds a chunk (o scaled by 2^-m, sum l) to what a row has accumulated: the weights of one merge.
-struct MergeW { float a, b, m; };
-__device__ __forceinline__ MergeW merge_weights(float m_acc, float m_chunk) {
-  MergeW w;
-  w.m = fmaxf(m_acc, m_chunk);
-  w.a = m_acc == -INFINITY ? 0.f : ex2(m_acc - w.m);
-  w.b = m_chunk == -INFINITY ? 0.f : ex2(m_chunk - w.m);
-  return w;
-}
-__device__ __forceinline__ float merge_value(float acc, float v, const MergeW& w) { return __fmaf_rn(v, w.b, __fmul_rn(acc, w.a)); }
-__device__ __forceinline__ float2 merge_values(float2 acc, float2 v, const MergeW& w) { return fma2(v, make_float2(w.b, w.b), mul2(acc, make_float2(w.a, w.a))); }
-// Two values of a finished row divided by its sum (a row without one keeps its zeros): times the reciprocal in two parts,
-// one rounded down and what it leaves, so that the fp32 result is the rounded quotient but for quotients within 2^-48 of a
-// rounding boundary. (The division operator took 5 us a unit of 128 values a thread more.) The second part is positive: an
-// infinite value stays what it is. A -0 becomes +0.
-struct RowSum { float2 r, rest; };
-__device__ __forceinline__ RowSum row_sum(float l) {
-  if (l == 0.f) l = 1.f;
-  const float r = __frcp_rd(l), rest = fmaxf(__fmaf_rn(-l, r, 1.f) * r, 1e-35f);
-  return {make_float2(r, r), make_float2(rest, rest)};
-}
-__device__ __forceinline__ uint32_t finish2(float a, float b, const RowSum& s) {
-  const float2 x = make_float2(a, b), v = fma2(x, s.r, fma2(x, s.rest, make_float2(0.f, 0.f)));
-  return pack_bf162(v.x, v.y);
-}
-
-// The tiles of one unit in order, as every role walks them.
-struct UnitTiles {
-  int seq, tok0, ntok, pos0, small, rows, pos_max, wlo;
-  int c, c1, t, t1, keys;       // chunk, end of chunks, tile, end of tiles of the chunk, keys of the chunk
-  __device__ __forceinline__ void open(const AttnParams& p, int unit, int tk) {
-    const int4 a = *reinterpret_cast<const int4*>(&p.units[unit]);
-    const int4 b = *(reinterpret_cast<const int4*>(&p.units[unit]) + 1);
-    seq = a.x; tok0 = a.y; ntok = a.z; pos0 = a.w;
-    c = b.x; c1 = b.y; small = b.z;
-    rows = ntok * p.gqa;
-    pos_max = pos0 + ntok - 1;
-    wlo = p.window > 0 ? max(0, pos0 - p.window + 1) : 0;    // first key that any row of the unit sees
-    c = max(c, wlo / ATT_CHUNK);
-    chunk(tk);
-  }
-  __device__ __forceinline__ void chunk(int tk) {
-    keys = min(ATT_CHUNK, pos_max + 1 - c * ATT_CHUNK);
-    t = max(0, wlo - c * ATT_CHUNK) / tk;
-    t1 = (keys + tk - 1) / tk;
-  }
-  __device__ __forceinline__ bool live() const { return c < c1; }
-  __device__ __forceinline__ bool last() const { return t == t1 - 1; }
-  __device__ __forceinline__ int first_tile(int tk) const { return max(0, wlo - c * ATT_CHUNK) / tk; }
-  __device__ __forceinline__ int key0(int tk) const { return c * ATT_CHUNK + t * tk; }
-  // 16-key blocks of the tile that hold a key of the sequence
-  __device__ __forceinline__ int blocks(int tk) const { return (min(tk, keys - t * tk) + 15) >> 4; }
-  __device__ __forceinline__ void next(int tk) {
-    if (++t == t1) { if (++c < c1) chunk(tk); }
-  }
-};
-
-// The r-th unit of a CTA: forth and back over the CTAs, so that with units in falling order of length every CTA gets about
-// the same number of tiles (attn_whole counts them the same way). -1: no more.
-__host__ __device__ __forceinline__ int unit_index(int r, int cta, int ctas, int total) {
-  const int i = r * ctas + ((r & 1) ? ctas - 1 - cta : cta);
-  return i < total ? i : -1;
-}
 
 // Whether the scale can go into the multiplier of the exponent, behind mask and maximum (FOLDED): right for a positive one
 // only (a masked -inf times 0 is NaN, times a negative scale +inf) whose factors stay in the range of fp32. With any other
@@ -479,7 +361,8 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
           if (tmax > m + 8.f) { alpha = ex2(m - tmax); m = tmax; }   // from -inf: alpha = 0
           const float ref = m == -INFINITY ? 0.f : m;
           const float2 muls = make_float2(mul, mul), refs = make_float2(-ref, -ref), minus1 = make_float2(-1.f, -1.f);
-          float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+          // Sums: 32 keys pairwise, keys 16, 8, 4, 2 and 1 apart, then the tile's (kc_attn_keys.cu adds across lanes in this order).
+          float part = 0.f, tile_sum = 0.f;
           // 32 scores of the row -> 32 columns of probabilities, as two bf16 numbers each: the columns of a 16-key block get
           // its eight pairs' upper parts, then what those leave over
           auto group = [&](uint32_t (&v)[32], int c) {
@@ -509,38 +392,44 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
             }
             mask(v, c);
             uint32_t w[32];
+            float2 sums[8];
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
+            for (int j = 0; j < 16; j += 2) {
               float2 e = fma2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), muls, refs);
-              float2 f = fma2(make_float2(__uint_as_float(v[j + 2]), __uint_as_float(v[j + 3])), muls, refs);
+              float2 f = fma2(make_float2(__uint_as_float(v[j + 16]), __uint_as_float(v[j + 17])), muls, refs);
               e.x = ex2(e.x); e.y = ex2(e.y); f.x = ex2(f.x); f.y = ex2(f.y);
-              s0 = add2(s0, e); s1 = add2(s1, f);
+              sums[j / 2] = add2(e, f);
               const uint32_t eh[2] = {__float_as_uint(e.x) & 0xffff0000u, __float_as_uint(e.y) & 0xffff0000u};
               const uint32_t fh[2] = {__float_as_uint(f.x) & 0xffff0000u, __float_as_uint(f.y) & 0xffff0000u};
-              const int at = (j & 16) + (j & 15) / 2;
-              w[at] = __byte_perm(eh[0], eh[1], 0x7632);
-              w[at + 1] = __byte_perm(fh[0], fh[1], 0x7632);
+              w[j / 2] = __byte_perm(eh[0], eh[1], 0x7632);
+              w[j / 2 + 16] = __byte_perm(fh[0], fh[1], 0x7632);
               const float2 el = fma2(make_float2(__uint_as_float(eh[0]), __uint_as_float(eh[1])), minus1, e);
               const float2 fl = fma2(make_float2(__uint_as_float(fh[0]), __uint_as_float(fh[1])), minus1, f);
-              w[at + 8] = pack_bf162(el.x, el.y);
-              w[at + 9] = pack_bf162(fl.x, fl.y);
+              w[j / 2 + 8] = pack_bf162(el.x, el.y);
+              w[j / 2 + 24] = pack_bf162(fl.x, fl.y);
             }
             tmem_st32(s_addr + c, w);
+#pragma unroll
+            for (int d = 4; d > 0; d /= 2)
+#pragma unroll
+              for (int j = 0; j < d; ++j) sums[j] = add2(sums[j], sums[j + d]);
+            return sums[0].x + sums[0].y;
           };
           tmem_wait_ld();
           tmem_pin32(va);
 #pragma unroll 1
           for (int c = 0; c < TK; c += 64) {
             tmem_ld32_issue(s_addr + c + 32, vb);
-            group(va, c);
+            part = group(va, c);
             tmem_wait_ld();
             tmem_pin32(vb);
             if (c + 64 < TK) tmem_ld32_issue(s_addr + c + 64, va);
-            group(vb, c + 32);
+            part += group(vb, c + 32);
+            tile_sum = c == 0 ? part : tile_sum + part;
             tmem_wait_ld();
             tmem_pin32(va);
           }
-          l = __fmaf_rn(l, alpha, (s0.x + s0.y) + (s1.x + s1.y));
+          l = __fmaf_rn(l, alpha, tile_sum);
           if (!first && !__all_sync(0xffffffffu, alpha == 1.f || row >= u.rows)) {
             // a row's maximum moved: what O holds of it is rescaled once the previous tile's product is in
             const int pt = tile - 1;
@@ -760,13 +649,19 @@ cudaError_t launch_attn(const CUtensorMap& map, const CUtensorMap& q, const CUte
 }
 
 template <int D>
-cudaError_t launch_d(const CUtensorMap& map, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p, bool in_order,
-                     int n_tokens, int sm_count, cudaStream_t s) {
-  if (p.whole) {
-    if constexpr (D <= 128) return launch_attn<D, true>(map, q, q_small, p, in_order, sm_count, s);
-    else return cudaErrorInvalidValue;
+cudaError_t launch_d(const CUtensorMap& map, const CUtensorMap& kmap, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p,
+                     bool in_order, int n_tokens, int sm_count, cudaStream_t s) {
+  cudaError_t e;
+  if (p.gqa * p.q_tokens <= KEY_ROWS) {
+    e = attn_keys(kmap, q, q_small, p, in_order, scale_folds(p.scale, p.softcap), D, sm_count, s);
+    if (p.whole) return e;
+  } else {
+    if (p.whole) {
+      if constexpr (D <= 128) return launch_attn<D, true>(map, q, q_small, p, in_order, sm_count, s);
+      else return cudaErrorInvalidValue;
+    }
+    e = launch_attn<D, false>(map, q, q_small, p, in_order, sm_count, s);
   }
-  cudaError_t e = launch_attn<D, false>(map, q, q_small, p, in_order, sm_count, s);
   if (e != cudaSuccess || p.single) return e;
   const int n_rows = n_tokens * p.Hq;
   return launch_k(attn_combine_kernel<D>, dim3((n_rows + 7) / 8), dim3(256), 0, s, p, n_rows);
@@ -778,8 +673,8 @@ int attn_tokens_per_item(int gqa, int max_len) {
   return std::min(std::max(1, ATT_ROWS / gqa), std::max(1, max_len));
 }
 
-bool attn_whole(int head_dim, const int* item_tiles, int n_items, int kv_heads, int sm_count) {
-  if (head_dim > 128) return false;   // a thread of the last role holds a row of the output in registers
+bool attn_whole(int head_dim, int rows, const int* item_tiles, int n_items, int kv_heads, int sm_count) {
+  if (head_dim > 128 && rows > KEY_ROWS) return false;   // a thread of attn_kernel's last role holds a row of the output in registers
   const int total = n_items * kv_heads, ctas = std::min(total, sm_count);
   long long sum = 0, most = 0;
   for (int i = 0; i < n_items; ++i) sum += (long long)item_tiles[i] * kv_heads;
@@ -805,15 +700,15 @@ bool make_tmap_q(CUtensorMap* map, const bf16* q, int n_tokens, int Hq, int gqa,
   return encode_tmap_bf16(map, 5, q, dims, strides, box, err);
 }
 
-// K/V pools as a 5-D tensor {64 features, 8 rows, head_dim / 64 slabs, planes, plane_rows / 8} with box {64, 8, slabs, 2, 2}:
-// ONE operation brings 16 keys of K and V of a layer (plane 2 * layer and the next) as two groups of 8 keys, each with
-// its K slabs and then its V slabs of [8][128 B], 128-byte swizzle. Groups of 8 rows at one constant stride are what a
+// K/V pools as a 5-D tensor {64 features, 8 rows, head_dim / 64 slabs, planes, plane_rows / 8} with box {64, 8, slabs, 1 or 2, 2}:
+// ONE operation brings 16 keys of K or V, or of both, of a layer (plane 2 * layer and the next) as two groups of 8 keys, each
+// with its K slabs and then its V slabs of [8][128 B], 128-byte swizzle. Groups of 8 rows at one constant stride are what a
 // tensor-core operand of many 16-key blocks needs, wherever the block table scatters them. The slab stride (128 B) is
 // smaller than the row stride, which the encoder may refuse: the caller then keeps the 2-D map (8 rows x 64 features).
-bool make_tmap_kv_5d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t plane_rows, uint64_t planes, const char** err) {
+bool make_tmap_kv_5d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t plane_rows, uint64_t planes, uint32_t box_planes, const char** err) {
   const uint64_t D = head_dim, dims[5] = {64, 8, D / 64, planes, plane_rows / 8};
   const uint64_t strides[4] = {D * 2, 128, plane_rows * D * 2, 8 * D * 2};
-  const uint32_t box[5] = {64, 8, head_dim / 64, 2, 2};
+  const uint32_t box[5] = {64, 8, head_dim / 64, box_planes, 2};
   return encode_tmap_bf16(map, 5, pool, dims, strides, box, err);
 }
 bool make_tmap_kv_2d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t rows, const char** err) {
@@ -822,13 +717,13 @@ bool make_tmap_kv_2d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint
   return encode_tmap_bf16(map, 2, pool, dims, strides, box, err);
 }
 
-cudaError_t paged_attention(const CUtensorMap& kvmap, const CUtensorMap& qmap, const CUtensorMap& qmap_small, const AttnParams& p,
-                            bool in_order, int head_dim, int n_tokens, int sm_count, cudaStream_t s) {
+cudaError_t paged_attention(const CUtensorMap& kvmap, const CUtensorMap& kmap, const CUtensorMap& qmap, const CUtensorMap& qmap_small,
+                            const AttnParams& p, bool in_order, int head_dim, int n_tokens, int sm_count, cudaStream_t s) {
   if (p.gqa < 1 || p.gqa * p.q_tokens > ATT_ROWS || p.n_units < 1) return cudaErrorInvalidValue;
   switch (head_dim) {
-    case 64: return launch_d<64>(kvmap, qmap, qmap_small, p, in_order, n_tokens, sm_count, s);
-    case 128: return launch_d<128>(kvmap, qmap, qmap_small, p, in_order, n_tokens, sm_count, s);
-    case 256: return launch_d<256>(kvmap, qmap, qmap_small, p, in_order, n_tokens, sm_count, s);
+    case 64: return launch_d<64>(kvmap, kmap, qmap, qmap_small, p, in_order, n_tokens, sm_count, s);
+    case 128: return launch_d<128>(kvmap, kmap, qmap, qmap_small, p, in_order, n_tokens, sm_count, s);
+    case 256: return launch_d<256>(kvmap, kmap, qmap, qmap_small, p, in_order, n_tokens, sm_count, s);
     default: return cudaErrorInvalidValue;
   }
 }

@@ -14,9 +14,11 @@ constexpr int ATT_ROWS = 128;   // query rows (token x head of the group) of one
 struct AttnUnit {
   int seq, tok0, ntok, pos0;    // sequence, first token row in the step, tokens, absolute position of the first
   int chunk0, chunk1;
-  int small, pad;               // 1: at most ATT_SMALL_TOKENS tokens (the query map with the small box)
+  int small;                    // 1: at most ATT_SMALL_TOKENS tokens (the query map with the small box)
+  int old;                      // keys from the sequence's start that nothing in this step writes
 };
 constexpr int ATT_SMALL_TOKENS = 8;
+constexpr int KEY_ROWS = 64;    // a step whose units have no more rows takes the kernel with a key per thread (kc_attn_keys.cu)
 
 struct AttnParams {
   bf16* out;                   // [n_tokens, Hq * D], 16-byte aligned
@@ -37,24 +39,28 @@ struct AttnParams {
   float softcap;               // 0 = off
   int window;                  // 0 = global
   int q_tokens;                // tokens in the box of the large query map
-  int kv5d;                    // kvmap is the 5-D map (one operation per 16 keys of K and V) instead of the 2-D one
+  int kv5d;                    // the maps of the pools are 5-D (one operation per 16 keys) instead of 2-D
 };
 
 // Tokens of one sequence that share a CTA (their rows x gqa must fit ATT_ROWS).
 int attn_tokens_per_item(int gqa, int max_len);
 // Whether units of whole rows (all chunks of an item in one unit) keep the SMs about as busy as units of single chunks:
-// item_tiles = tiles of 128 keys of each item, in the order of the units.
-bool attn_whole(int head_dim, const int* item_tiles, int n_items, int kv_heads, int sm_count);
+// item_tiles = tiles of 128 keys of each item, in the order of the units. rows: the most query rows of an item.
+bool attn_whole(int head_dim, int rows, const int* item_tiles, int n_items, int kv_heads, int sm_count);
 
 // Query maps over [n_tokens, Hq, D] (5-D: 64 features, heads of a group, slabs, groups, tokens).
 bool make_tmap_q(CUtensorMap* map, const bf16* q, int n_tokens, int Hq, int gqa, int head_dim, int box_tokens, const char** err);
 // K/V pools [planes = layers * 2][plane_rows = NB * Hkv * BS][head_dim]: see kc_attn.cu.
-bool make_tmap_kv_5d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t plane_rows, uint64_t planes, const char** err);
+// box_planes: 2 for K and V in one operation, 1 for either.
+bool make_tmap_kv_5d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t plane_rows, uint64_t planes, uint32_t box_planes, const char** err);
 bool make_tmap_kv_2d(CUtensorMap* map, const void* pool, uint32_t head_dim, uint64_t rows, const char** err);
 
 // in_order: the work before this call in the stream is not one of a step's kernels (the copy of units and block tables, a
-// caller's own work): the first kernel is then launched behind it in plain stream order.
-cudaError_t paged_attention(const CUtensorMap& kvmap, const CUtensorMap& qmap, const CUtensorMap& qmap_small, const AttnParams& p,
-                            bool in_order, int head_dim, int n_tokens, int sm_count, cudaStream_t s);
+// caller's own work): the first kernel is then launched behind it in plain stream order. kvmap: K and V of 16 keys; kmap: either.
+cudaError_t paged_attention(const CUtensorMap& kvmap, const CUtensorMap& kmap, const CUtensorMap& qmap, const CUtensorMap& qmap_small,
+                            const AttnParams& p, bool in_order, int head_dim, int n_tokens, int sm_count, cudaStream_t s);
+// Its kernel for units of at most KEY_ROWS rows (kc_attn_keys.cu).
+cudaError_t attn_keys(const CUtensorMap& kmap, const CUtensorMap& qmap, const CUtensorMap& qmap_small, const AttnParams& p, bool in_order, bool folded,
+                      int head_dim, int sm_count, cudaStream_t s);
 
 }  // namespace kc

@@ -19,13 +19,14 @@ __device__ __forceinline__ uint64_t umma_smem_desc(uint32_t smem_addr, uint32_t 
 }
 
 // kind::f16, bf16 x bf16 -> fp32. kind::f16 takes A and B of the SAME 16-bit type: an f16 A against a bf16 B is an
-// illegal instruction. b_mn: B is MN-major.
-__device__ __forceinline__ uint32_t umma_idesc_bf16(int m, int n, bool b_mn = false) {
+// illegal instruction. b_mn, a_mn: B, A is MN-major.
+__device__ __forceinline__ uint32_t umma_idesc_bf16(int m, int n, bool b_mn = false, bool a_mn = false) {
   uint32_t d = 0;
   d |= 1u << 4;                    // D format f32
   d |= 1u << 7;                    // A format bf16
   d |= 1u << 10;                   // B format bf16
-  d |= (b_mn ? 1u : 0u) << 16;     // bit 15: A, bit 16: B is MN-major
+  d |= (a_mn ? 1u : 0u) << 15;     // A is MN-major
+  d |= (b_mn ? 1u : 0u) << 16;     // B is MN-major
   d |= (uint32_t)(n >> 3) << 17;   // N
   d |= (uint32_t)(m >> 4) << 24;   // M
   return d;
@@ -76,6 +77,19 @@ __device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t* r) {
         "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
         "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld8_issue(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // Keeps the uses of r behind the wait before this: to the compiler the load's results are there at once.

@@ -114,6 +114,27 @@ def test_verify_rows_carry_decode_bits(ctx, hd, heads, kvh, bs):
             row += 1
 
 
+@pytest.mark.parametrize("hd,heads,kvh,softcap,window", [
+    (64, 8, 2, 0.0, 0), (128, 8, 2, 0.0, 0), (128, 8, 2, 20.0, 300), (256, 4, 2, 50.0, 0), (256, 4, 2, 0.0, 90),
+    (128, 7, 1, 0.0, 0), (64, 33, 1, 0.0, 0), (128, 64, 1, 0.0, 0), (256, 40, 1, 30.0, 700), (64, 1, 1, 0.0, 0), (128, 64, 1, 7.0, 513)])
+@pytest.mark.parametrize("scale", [1.0, -0.5])
+def test_prompt_rows_carry_decode_bits(ctx, hd, heads, kvh, softcap, window, scale):
+    """The rows of a prompt's piece (more than 64 rows a unit: a thread holds a row) against the same rows a few at a time (a
+    thread holds a key): the same bits, on both sides of tile and chunk edges, with 1 to 64 rows a unit."""
+    gqa, bs = heads // kvh, 16
+    start, length = 480, 80
+    nb = (start + length + bs - 1) // bs
+    kv, _ = fill_pools(ctx, api.KvSpec(1, kvh, hd, nb, bs), 41)
+    blocks = build_seqs([(length, start)], bs, nb, 42)[0].blocks
+    q = outlier_values((length, heads, hd), 43).cuda()
+    scale *= hd ** -0.5
+    whole = api.paged_attention(ctx, kv, 0, q, [api.SeqStep(length, start, length, blocks)], scale, softcap, window).cpu()
+    for at, rows in [(0, 1), (27, min(53, 64 // gqa)), (31, 1), (32, 1), (length - 64 // gqa, 64 // gqa), (30, max(1, 32 // gqa)), (29, max(1, 17 // gqa))]:
+        few = api.paged_attention(ctx, kv, 0, q[at: at + rows].contiguous(), [api.SeqStep(rows, start + at, rows, blocks)], scale, softcap, window).cpu()
+        assert torch.equal(few.view(torch.int16), whole[at: at + rows].view(torch.int16)), f"rows {at} .. {at + rows}"
+    assert ctx.device_status() == 0
+
+
 @pytest.mark.parametrize("hd,heads,kvh,bs,layers", [(128, 8, 2, 16, 3), (64, 8, 2, 32, 2), (256, 4, 2, 16, 2)])
 def test_one_operation_per_tile_pair_matches_the_slab_loads(ctx, monkeypatch, hd, heads, kvh, bs, layers):
     """A pool created with KILN_KV_MAP_2D=1 is read with one TMA operation per 64-feature slab of a K or V tile, the

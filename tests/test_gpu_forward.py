@@ -257,6 +257,29 @@ def test_pipelined_decode_equals_stepwise(ctx):
         model.decode_launch(api.StepBatch([0, 0], [api.SeqStep(2, 40, 1, tables[0])]), kv2, [-1])
 
 
+@pytest.mark.parametrize("name", ["tiny-llama-d128", "tiny-gemma2"])
+def test_pieces_of_a_sequence_in_one_step(ctx, name):
+    """A step may hold consecutive pieces of one sequence: the later one's attention reads keys that the same step writes, a
+    whole tile of them below its own rows. Against the pieces in steps of their own, bit for bit."""
+    cfg, model, _, _, _ = load(ctx, name)
+    ids = prompts(cfg, [400], 3)[0]
+    blocks = list(range(2, 30))
+    cuts = [(0, 120), (120, 128), (128, 136), (136, 250), (250, 256), (256, 260)]
+
+    def run(steps):
+        kv, rows = api.PagedKv(ctx, model.kv_spec(64, BS)), []
+        for step in steps:
+            logits = model.forward_step(api.StepBatch(ids[step[0][0]: step[-1][1]], [api.SeqStep(b - a, a, b - a, blocks) for a, b in step]), kv)
+            ctx.sync()
+            rows.append(logits.cpu())
+        return torch.cat(rows).view(torch.int16)
+
+    want = run([[c] for c in cuts])
+    for steps in ([cuts[:1], cuts[1:3], cuts[3:4], cuts[4:]], [cuts[:1], cuts[1:]]):
+        assert torch.equal(run(steps), want)
+    assert ctx.device_status() == 0
+
+
 def test_engine_pipelines_plain_decode_on_the_device(ctx):
     """The host engine over the CUDA model: plain decode takes the pipelined path and emits what the synchronous
     engine emits (prefix cache on, three requests of different lengths, one with a stop token)."""
