@@ -1736,7 +1736,7 @@ extern "C" int kc_rope_kv_write(kc_ctx_t c, kc_kv_t kv, int32_t layer, const voi
                                          reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.token_pos),
                                          reinterpret_cast<const int32_t*>(m->meta_dev + p.lay.kv_slot), n, num_heads,
                                          kv->kv_heads, kv->head_dim, traditional, layer, kv->num_blocks, kv->block_size,
-                                         kv->pool, (bf16*)q_out_dev, c->stream);
+                                         kv->pool, (bf16*)q_out_dev, c->stream, true);
     if (e != cudaSuccess) rc = fail(KC_ERR_CUDA, "kc_rope_kv_write: %s", cudaGetErrorString(e));
   }
   return op_shell_done(c, rc, "kc_rope_kv_write");

@@ -247,36 +247,46 @@ add_rmsnorm_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __restri
   }
 }
 
-// The same operation for the common case (no sandwich norm, H = 2048 * CPT): the row stays in registers and all
+// The same operation for rows of up to 2048 * CPT features (FULL: of exactly that many): the row stays in registers and all
 // loads of a thread are issued before the first use, so a row costs one round trip to L2 instead of one per chunk.
-// Element for element the arithmetic (and its order) is that of add_rmsnorm_kernel.
-template <int CPT>
+// Element for element the arithmetic (and its order) is that of add_rmsnorm_kernel. PRE: with the sandwich norm.
+// H = 3584, time that it adds to a step, add_rmsnorm_kernel -> this: 320 rows of five partials 8.4 -> 7.0 us, 64 rows with
+// the sandwich norm 8.0 -> 6.2; what is left is launch latency and two or three round trips.
+template <int CPT, bool FULL, bool PRE>
 __global__ void __launch_bounds__(256)
-add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __restrict__ w_out,
-                       const int32_t* __restrict__ row_map, float eps, bf16* __restrict__ h_out,
+add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __restrict__ w_pre, const bf16* __restrict__ w_out,
+                       const int32_t* __restrict__ row_map, int h, float eps, bf16* __restrict__ h_out,
                        bf16* __restrict__ normed) {
   if (!y.peers) pdl_launch_dependents();
-  constexpr int H = 2048 * CPT;
+  const int H = FULL ? 2048 * CPT : h;
   __shared__ float red[32];
-  uint4 wraw[CPT];   // a model's weight depends on no kernel: it arrives under the tail of the one before this
+  const uint4 none = make_uint4(0, 0, 0, 0);
+  int at[CPT];
+  bool on[CPT];
 #pragma unroll
-  for (int c = 0; c < CPT; ++c) wraw[c] = w_out ? *reinterpret_cast<const uint4*>(w_out + (c * 256 + threadIdx.x) * 8) : make_uint4(0, 0, 0, 0);
+  for (int c = 0; c < CPT; ++c) { at[c] = (c * 256 + threadIdx.x) * 8; on[c] = FULL || at[c] < H; }
+  uint4 wraw[CPT], praw[PRE ? CPT : 1];   // a model's weights depend on no kernel: they arrive under the tail of the one before this
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) {
+    wraw[c] = w_out && on[c] ? *reinterpret_cast<const uint4*>(w_out + at[c]) : none;
+    if (PRE) praw[c % (PRE ? CPT : 1)] = on[c] ? *reinterpret_cast<const uint4*>(w_pre + at[c]) : none;
+  }
   pdl_wait();
   if (y.peers) { tp_wait(y); pdl_launch_dependents(); }
   const int row = blockIdx.x;
   const size_t src = row_map ? row_map[row] : row;
   const bf16* xr = x + src * H;
-  const bool has_y = y.y || y.part || y.rank_y || y.peers;
+  const bool has_y = PRE || y.y || y.part || y.rank_y || y.peers;
   float v[CPT][8];
   uint4 xraw[CPT];
 #pragma unroll
-  for (int c = 0; c < CPT; ++c) xraw[c] = *reinterpret_cast<const uint4*>(xr + (c * 256 + threadIdx.x) * 8);
+  for (int c = 0; c < CPT; ++c) xraw[c] = on[c] ? *reinterpret_cast<const uint4*>(xr + at[c]) : none;
   if (has_y) {
     if (y.part) {
       float4 a[CPT], b[CPT];
 #pragma unroll
       for (int c = 0; c < CPT; ++c) {
-        const float* p0 = y.part + src * y.ld + (c * 256 + threadIdx.x) * 8;
+        const float* p0 = y.part + src * y.ld + (on[c] ? at[c] : 0);
         a[c] = *reinterpret_cast<const float4*>(p0);
         b[c] = *reinterpret_cast<const float4*>(p0 + 4);
       }
@@ -284,7 +294,7 @@ add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __re
       for (int k = 1; k < y.splits; ++k) {
 #pragma unroll
         for (int c = 0; c < CPT; ++c) {
-          const float* p0 = y.part + k * y.split_stride + src * y.ld + (c * 256 + threadIdx.x) * 8;
+          const float* p0 = y.part + k * y.split_stride + src * y.ld + (on[c] ? at[c] : 0);
           const float4 e = *reinterpret_cast<const float4*>(p0), f = *reinterpret_cast<const float4*>(p0 + 4);
           a[c].x += e.x; a[c].y += e.y; a[c].z += e.z; a[c].w += e.w;
           b[c].x += f.x; b[c].y += f.y; b[c].z += f.z; b[c].w += f.w;
@@ -297,8 +307,28 @@ add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __re
       }
     } else {
 #pragma unroll
-      for (int c = 0; c < CPT; ++c) load8(y, src, (c * 256 + threadIdx.x) * 8, v[c]);
+      for (int c = 0; c < CPT; ++c) load8(y, src, on[c] ? at[c] : 0, v[c]);
     }
+  }
+  if (PRE) {
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c)
+      if (on[c]) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) ss += v[c][k] * v[c][k];
+      }
+    ss = block_sum(ss, red);
+    const float inv = rsqrtf(ss / (float)H + eps);
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) {
+      const uint4 w = praw[c % (PRE ? CPT : 1)];
+      const float2 w0 = unpack_bf162(w.x), w1 = unpack_bf162(w.y), w2 = unpack_bf162(w.z), w3 = unpack_bf162(w.w);
+      const float wv[8] = {w0.x, w0.y, w1.x, w1.y, w2.x, w2.y, w3.x, w3.y};
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[c][k] = bf16_round(wv[k] * (v[c][k] * inv));
+    }
+    __syncthreads();   // `red` is written again below
   }
   float ss = 0.f;
 #pragma unroll
@@ -308,14 +338,15 @@ add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __re
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
       v[c][k] = has_y ? bf16_round(xv[k] + v[c][k]) : xv[k];
-      ss += v[c][k] * v[c][k];
+      if (on[c]) ss += v[c][k] * v[c][k];
     }
   }
   ss = block_sum(ss, red);
   const float inv = rsqrtf(ss / (float)H + eps);
 #pragma unroll
   for (int c = 0; c < CPT; ++c) {
-    const int i = (c * 256 + threadIdx.x) * 8;
+    if (!on[c]) continue;
+    const int i = at[c];
     if (h_out) store8_bf16(h_out + (size_t)row * H + i, v[c]);
     if (w_out) {
       const float2 w0 = unpack_bf162(wraw[c].x), w1 = unpack_bf162(wraw[c].y), w2 = unpack_bf162(wraw[c].z), w3 = unpack_bf162(wraw[c].w);
@@ -333,15 +364,19 @@ add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __re
 // fast::rope, crates/kiln-mlx/src/fast.rs:45-104). One CTA per token; K is
 // rotated, V copied, both land in the pool rows of the token's slot.
 // ---------------------------------------------------------------------------
-// sin/cos of the token's angles are computed once per CTA and shared by all heads; every thread then moves
-// 8 consecutive features of each half with 16-byte loads and stores.
-__global__ void __launch_bounds__(256)
+// sin/cos of the token's angles are computed once per CTA and shared by its heads, before the wait for the kernel ahead (the
+// step's metadata is older than its first kernel; a single call's is not, see launch_rope_kv_write); every thread then moves
+// 8 consecutive features of each half with 16-byte loads and stores. A token's work items lie over CTAs of 128 threads, one
+// a thread: what bounds it is one item's chain of loads. Time that it adds to a step, all of a token's items in one CTA of
+// 256 threads and sin/cos behind the wait -> this: one token 6.2 -> 3.5 us, 192 tokens of three partials 5.8 -> 4.8, 320 of
+// four 12.7 -> 5.9.
+constexpr int ROPE_THREADS = 128;
+__global__ void __launch_bounds__(ROPE_THREADS)
 rope_kv_write_kernel(RowSource qkv, const bf16* __restrict__ bias, const float* __restrict__ inv_freq,
                      const int32_t* __restrict__ token_pos, const int32_t* __restrict__ kv_slot, int Hq, int Hkv,
                      int D, int traditional, int layer, int NB, int BS, bf16* __restrict__ pool,
                      bf16* __restrict__ q_out) {
   pdl_launch_dependents();
-  pdl_wait();
   __shared__ float s_cs[128], s_sn[128];   // head_dim <= 256
   const int tok = blockIdx.x;
   const int heads = Hq + 2 * Hkv;
@@ -351,8 +386,10 @@ rope_kv_write_kernel(RowSource qkv, const bf16* __restrict__ bias, const float* 
   const int blk = slot / BS, r = slot % BS;
   for (int j = threadIdx.x; j < half; j += blockDim.x) sincosf(pos * inv_freq[j], &s_sn[j], &s_cs[j]);
   __syncthreads();
+  pdl_wait();
   const int per_head = D / 16;             // work items per head: 8 features of each half, or 16 interleaved ones
-  for (int it = threadIdx.x; it < heads * per_head; it += blockDim.x) {
+  const int it = blockIdx.y * ROPE_THREADS + threadIdx.x;
+  if (it < heads * per_head) {
     const int h = it / per_head, c = it - h * per_head;
     // features [e0, e0 + 8) and [e1, e1 + 8) of head h; the rotation pairs are (e0 + k, e1 + k) for split
     // halves and (e0 + 2k, e0 + 2k + 1), (e1 + 2k, e1 + 2k + 1) for the interleaved convention
@@ -524,19 +561,25 @@ cudaError_t launch_add_rmsnorm(const bf16* x, const SublayerOut& y, const bf16* 
   if (H % 8) return cudaErrorInvalidValue;
   const bool aligned = !y.part || ((reinterpret_cast<uintptr_t>(y.part) & 15) == 0 && (y.ld & 3) == 0 && (y.split_stride & 3) == 0);
   const bool early = y.rank_y == nullptr && !in_order;   // per-rank inputs arrive from a collective: see launch_k_opt
-  if (!w_pre && aligned) {
-    if (H == 2048) return launch_k_opt(early, add_rmsnorm_reg_kernel<1>, dim3(rows), dim3(256), 0, s, x, row_source(y), w_out, row_map, eps, h_out, normed);
-    if (H == 4096) return launch_k_opt(early, add_rmsnorm_reg_kernel<2>, dim3(rows), dim3(256), 0, s, x, row_source(y), w_out, row_map, eps, h_out, normed);
-    if (H == 8192) return launch_k_opt(early, add_rmsnorm_reg_kernel<4>, dim3(rows), dim3(256), 0, s, x, row_source(y), w_out, row_map, eps, h_out, normed);
+  const bool has_y = y.y || y.part || y.rank_y || y.peers;
+  // Past 4096 features the sandwich norm's kernel would take 254 registers.
+  if (aligned && H <= (w_pre ? 4096 : 8192) && (!w_pre || has_y)) {
+    auto launch = [&](auto kernel) { return launch_k_opt(early, kernel, dim3(rows), dim3(256), 0, s, x, row_source(y), w_pre, w_out, row_map, H, eps, h_out, normed); };
+    if (w_pre) return H <= 2048 ? launch(add_rmsnorm_reg_kernel<1, false, true>) : launch(add_rmsnorm_reg_kernel<2, false, true>);
+    if (H == 2048) return launch(add_rmsnorm_reg_kernel<1, true, false>);
+    if (H == 4096) return launch(add_rmsnorm_reg_kernel<2, true, false>);
+    if (H == 8192) return launch(add_rmsnorm_reg_kernel<4, true, false>);
+    return H <= 2048 ? launch(add_rmsnorm_reg_kernel<1, false, false>) : H <= 4096 ? launch(add_rmsnorm_reg_kernel<2, false, false>) : launch(add_rmsnorm_reg_kernel<4, false, false>);
   }
   return launch_k_opt(early, add_rmsnorm_kernel, dim3(rows), dim3(256), H * sizeof(float), s, x, row_source(y), w_pre, w_out, row_map, H, eps, h_out, normed);
 }
 
 cudaError_t launch_rope_kv_write(const SublayerOut& qkv, const bf16* bias, const float* inv_freq, const int32_t* token_pos,
                                  const int32_t* kv_slot, int n, int Hq, int Hkv, int D, int traditional, int layer,
-                                 int NB, int BS, bf16* pool, bf16* q_out, cudaStream_t s) {
+                                 int NB, int BS, bf16* pool, bf16* q_out, cudaStream_t s, bool in_order) {
   if (D % 16 || D > 256) return cudaErrorInvalidValue;
-  return launch_k(rope_kv_write_kernel, dim3(n), dim3(256), 0, s, row_source(qkv), bias, inv_freq, token_pos, kv_slot, Hq, Hkv, D,
+  const int items = (Hq + 2 * Hkv) * (D / 16);
+  return launch_k_opt(!in_order, rope_kv_write_kernel, dim3(n, (items + ROPE_THREADS - 1) / ROPE_THREADS), dim3(ROPE_THREADS), 0, s, row_source(qkv), bias, inv_freq, token_pos, kv_slot, Hq, Hkv, D,
                   traditional, layer, NB, BS, pool, q_out);
 }
 

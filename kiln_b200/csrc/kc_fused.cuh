@@ -61,9 +61,11 @@ cudaError_t launch_add_rmsnorm(const bf16* x, const SublayerOut& y, const bf16* 
                                const int32_t* row_map, int rows, int H, float eps, bf16* h_out, bf16* normed,
                                cudaStream_t s, bool in_order = false);
 
+// Positions, slots and frequencies are read before the kernel ahead has finished; in_order: it may write them (or is the copy
+// that brings them), so this kernel is launched behind it in plain stream order.
 cudaError_t launch_rope_kv_write(const SublayerOut& qkv, const bf16* bias, const float* inv_freq, const int32_t* token_pos,
                                  const int32_t* kv_slot, int n, int Hq, int Hkv, int D, int traditional, int layer,
-                                 int NB, int BS, bf16* pool, bf16* q_out, cudaStream_t s);
+                                 int NB, int BS, bf16* pool, bf16* q_out, cudaStream_t s, bool in_order = false);
 
 // After the kernels before it on the stream have finished, stores `epoch` into slot `rank` of every rank's flag array
 // (peer_flags[r] = rank r's array as mapped into this process): "this rank's output of exchange `epoch` is complete".

@@ -65,6 +65,18 @@ assert seen[2:] == ["launch early"], seen
 """)
 
 
+def test_rope_waits_for_its_metadata(fake):
+    """Positions, slots and a caller's frequencies are read before the wait for the kernel ahead: a single call's launch is
+    ordered behind the copy that brings them, and behind the caller's own work."""
+    run(fake, """
+fake.fake_reset()
+seqs = (L.KcSeqStep * 1)(L.KcSeqStep(3, 40, 3, 3, table))
+ok(lib.kc_rope_kv_write(ctx, kv, 0, at, None, C.cast(at, C.POINTER(C.c_float)), 3, 4, 0, seqs, 1, at))
+seen = [c for c in calls() if c.startswith(("copy", "launch"))]
+assert seen == ["copy", "launch in order"], seen
+""")
+
+
 @pytest.mark.parametrize("dim", [1024, 2048, 4096, 8192])
 def test_rms_norm_waits_for_its_weight(fake, dim):
     """The weight is read before the kernel ahead has finished, and a caller's weight may be what that kernel writes."""
