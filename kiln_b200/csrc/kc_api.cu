@@ -482,14 +482,14 @@ extern "C" int kc_kv_write_block(kc_kv_t kv, uint32_t block, const void* src, si
 // through memory less). Rows beyond one 512-row slab always go through the reduction kernel.
 static int run_qlinear(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, bf16* y, int ldy, float* partial,
                        SublayerOut* fused = nullptr) {
-  const bool defer = fused && w.splits > 1 && M <= QL_MAX_M;
+  const bool defer = fused && w.splits > 1 && M <= QL_MAX_M && !qlinear_in_turn(w, M);
   const int slab = qlinear_slab_rows(w, M);
   for (int row0 = 0; row0 < M; row0 += slab) {
     QLinearLaunch l;
     l.w = &w; l.x = &x; l.row0 = row0; l.M = std::min(slab, M - row0);
     l.y = y; l.ldy = ldy; l.partial = partial; l.status = c->status;
     LAUNCH(c, KC_PROF_GEMM, 1, qlinear_umma(l, c->stream));
-    if (w.splits > 1 && !defer)
+    if (w.splits > 1 && !defer && !qlinear_in_turn(w, l.M))
       LAUNCH(c, KC_PROF_GEMM_REDUCE, 1, qlinear_reduce_splits(partial, w.splits, l.M, w.N, y + (size_t)row0 * ldy, ldy, c->stream));
   }
   if (fused) *fused = defer ? SublayerOut::partials(partial, w.splits, (size_t)M, w.N) : SublayerOut::dense(y, ldy);
@@ -511,7 +511,7 @@ static int run_gated(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, bf
     if (interleaved) { l.glu = gelu ? 2 : 1; l.act = act; l.ld_act = F; l.glu_done = &done; }
     LAUNCH(c, KC_PROF_GEMM, 1, qlinear_umma(l, c->stream));
     if (done) continue;
-    if (w.splits > 1)
+    if (w.splits > 1 && !qlinear_in_turn(w, rows))
       LAUNCH(c, KC_PROF_GEMM_REDUCE, 1, qlinear_reduce_splits(partial, w.splits, rows, w.N, gu + (size_t)row0 * 2 * F, 2 * F, c->stream));
     LAUNCH(c, KC_PROF_ROWWISE, 1, launch_glu(gu + (size_t)row0 * 2 * F, rows, F, gelu, interleaved ? 1 : 0, act + (size_t)row0 * F, c->stream));
   }

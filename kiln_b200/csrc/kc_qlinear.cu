@@ -305,6 +305,7 @@ struct QlKernelParams {
   uint32_t tmem_cols;    // columns allocated: a power of two
   bf16* y; int ldy;
   float* partial;        // [splits][M][N]
+  int chunks;            // of rows (qlinear_umma_rows_kernel)
   uint32_t* status;
 };
 
@@ -657,6 +658,299 @@ static TaPlan plan_ta(int nt, int per, int m_pad, uint32_t record_bytes) {
   return t;
 }
 
+// ---------------------------------------------------------------------------
+// Many rows against a weight that is split along K: qlinear_umma_rows_kernel. The splits are there to fill the SMs at few rows;
+// with many, chunks of rows do, and a CTA takes all splits of its tile and rows one after the other, so that no partial goes
+// through memory and nothing is left to reduce. Persistent: a CTA walks over (tile, chunk) items, weights and activations of
+// the next split or item arriving under the last one.
+//
+// The sums are those of the launches with a split a CTA: the even and the odd k-blocks of a split in an accumulator each, the
+// split's sum of the two, and the splits' sums added in order, which lie in shared memory meanwhile.
+//
+// Roles as in qlinear_umma_ta_kernel. A segment is one split of one item. A stage is two k-blocks, one for each accumulator;
+// where a segment ends on an odd one the stage's second unit passes through the rings empty. At a segment's end the
+// dequantisers, who have the next segment's first stages in tensor memory by then, read the accumulators.
+//
+// What bounds it: the hand-over of the dequantised weights as in qlinear_umma_ta_kernel (about 500 cycles a k-block up to 112
+// rows), then the activations: every CTA reads its own, 24 KB a k-block of 192 rows, 45 bytes a cycle and SM of L2. A form with
+// two tiles a CTA sharing them, four accumulators of 96 rows, took 980 cycles a pair of k-blocks, 349 us where this takes 231.
+// TMEM columns: [even, odd: round32(m_pad) each] [a_stages x 2 units x 32 columns].
+// ---------------------------------------------------------------------------
+template <int BITS, int GPK, bool WIDE>
+__global__ void __launch_bounds__(QL_THREADS, 1)
+qlinear_umma_rows_kernel(const __grid_constant__ CUtensorMap map_rows, const QlKernelParams p) {
+  constexpr uint32_t PACKED = QL_TILE_N * (QL_KB * BITS / 8);
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int SA = p.a_stages, SB = p.b_stages, RS = p.r_stages;   // SB, RS: k-blocks
+  const uint32_t b_bytes = (uint32_t)p.m_pad * 128u;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int items = p.n_tiles * p.chunks;
+  const uint32_t cs = (uint32_t)(p.m_pad + 31) & ~31u, a_col0 = 2 * cs;
+  auto first_kb = [&](int split) { return (int)((long long)p.kblocks * split / p.splits); };
+
+  uint8_t* sB = smem;
+  uint8_t* sR = sB + (size_t)SB * b_bytes;
+  float* sums = reinterpret_cast<float*>(sR + (size_t)RS * p.record_bytes);   // [row][128] of the splits so far
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sums + p.m_pad * QL_TILE_N);
+  uint64_t* raw_full = bars;
+  uint64_t* raw_empty = raw_full + RS;
+  uint64_t* b_full = raw_empty + RS;
+  uint64_t* b_empty = b_full + SB;
+  uint64_t* a_ready = b_empty + SB;       // [stage][unit]
+  uint64_t* a_empty = a_ready + 2 * SA;
+  uint64_t* acc_full = a_empty + 2 * SA;  // a segment's products are in
+  uint64_t* acc_free = acc_full + 1;      // .. and read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
+
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < RS; ++i) { mbar_init(&raw_full[i], 1); mbar_init(&raw_empty[i], 4); }
+    for (int i = 0; i < SB; ++i) { mbar_init(&b_full[i], 1); mbar_init(&b_empty[i], 1); }
+    for (int i = 0; i < 2 * SA; ++i) { mbar_init(&a_ready[i], 4); mbar_init(&a_empty[i], 1); }
+    mbar_init(acc_full, 2); mbar_init(acc_free, QL_DQ_WARPS);
+    mbar_fence_init();
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(p.tmem_cols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (warp == 1 && lane == 0) tma_prefetch_desc(&map_rows);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp < 2) {
+    // ---- producers: warp 0 the weight records, warp 1 the activations, the first access of this kernel to memory written by
+    // earlier kernels. Both walk the same k-blocks; an empty unit's barrier is completed without a copy. ----
+    if (lane == 0) {
+      if (warp == 1) pdl_wait();
+      RingPos rp;
+      const int depth = warp == 0 ? RS : SB;
+      uint64_t *full = warp == 0 ? raw_full : b_full, *empty = warp == 0 ? raw_empty : b_empty;
+      bool ok = true;
+      for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
+        const int tile = item % p.n_tiles, row = p.row0 + item / p.n_tiles * p.m_pad;
+        const uint8_t* src = p.records + ((size_t)(tile / QL_TILE_GROUP) * p.kblocks * QL_TILE_GROUP + tile % QL_TILE_GROUP) * p.record_bytes;
+        for (int split = 0; ok && split < p.splits; ++split) {
+          const int kb1 = first_kb(split + 1);
+          int kb = first_kb(split);
+          for (int left = (kb1 - kb + 1) & ~1; left > 0; --left, ++kb, rp.advance(depth)) {
+            ok = mbar_wait(&empty[rp.stage], rp.phase ^ 1, p.status, KC_DEV_QLINEAR | (1 + warp));
+            if (!ok) break;
+            if (kb >= kb1) {
+              mbar_arrive(&full[rp.stage]);
+            } else if (warp == 0) {
+              mbar_arrive_expect_tx(&full[rp.stage], p.record_bytes);
+              bulk_g2s(sR + (size_t)rp.stage * p.record_bytes, src + (size_t)kb * QL_TILE_GROUP * p.record_bytes, p.record_bytes, &full[rp.stage]);
+            } else {
+              mbar_arrive_expect_tx(&full[rp.stage], b_bytes);
+              tma_load_2d(sB + (size_t)rp.stage * b_bytes, &map_rows, kb * QL_KB, row, &full[rp.stage]);
+            }
+          }
+        }
+      }
+    }
+  } else if (warp < QL_DQ_WARP0) {
+    // ---- MMA issuers: warp 2 + u has accumulator u, the k-blocks u, u + 2, .. of a segment ----
+    pdl_wait();
+    const int u = warp - 2;
+    const uint32_t idesc = umma_idesc_bf16(QL_TILE_N, p.m_pad);
+    const uint64_t proto = umma_smem_desc(0, 1024);
+    const uint32_t d_hi = (uint32_t)(proto >> 32), b_lo0 = (uint32_t)proto | ((smem_u32(sB) >> 4) & 0x3FFF);
+    const uint32_t d = tmem_base + u * cs, a_t0 = tmem_base + a_col0 + u * 32;
+    int as = 0, bs = u, seg = 0;
+    uint32_t aphase = 0, bphase = 0;
+    bool ok = true, ready = false;
+    for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
+      for (int split = 0; ok && split < p.splits; ++split, ++seg) {
+        const int nkb = first_kb(split + 1) - first_kb(split), stages = (nkb + 1) >> 1;
+        if (seg > 0) ok = warp_wait(acc_free, (seg - 1) & 1, p.status, KC_DEV_QLINEAR | 8);
+        for (int j = 0; ok && j < stages; ++j) {
+          if (!__all_sync(0xffffffffu, ready)) {
+            ok = warp_wait(&b_full[bs], bphase, p.status, KC_DEV_QLINEAR | 4) &&
+                 warp_wait(&a_ready[2 * as + u], aphase, p.status, KC_DEV_QLINEAR | 3);
+            if (!ok) break;
+          }
+          tc_fence_after();
+          const uint32_t b_lo = b_lo0 + bs * (b_bytes >> 4), a_t = a_t0 + as * 64;
+          uint64_t *a_done = &a_empty[2 * as + u], *b_done = &b_empty[bs];
+          if (++as == SA) { as = 0; aphase ^= 1u; }
+          bs += 2;
+          if (bs >= SB) { bs -= SB; bphase ^= 1u; }
+          ready = j + 1 < stages && (mbar_test_wait(&b_full[bs], bphase) & mbar_test_wait(&a_ready[2 * as + u], aphase));
+          if (elect_one()) {
+            if (2 * j + u < nkb) {
+#pragma unroll
+              for (int ks = 0; ks < QL_KB / 16; ++ks)
+                umma_bf16_ts(d, a_t + 8 * ks, b_lo + 2 * ks, d_hi, idesc, j == 0 && ks == 0 ? 0u : 1u);
+            }
+            umma_commit(a_done);
+            umma_commit(b_done);
+          }
+          __syncwarp();
+        }
+        if (ok && elect_one()) umma_commit(acc_full);
+        __syncwarp();
+      }
+    }
+  } else {
+    // ---- dequantisers: group g converts unit g & 1 of the stages g >> 1, (g >> 1) + 2, .. over all segments ----
+    const int grp = (warp - QL_DQ_WARP0) >> 2, unit = grp & 1, q = warp & 3;
+    const int n_in = q * 32 + lane;
+    const uint32_t lanes = (uint32_t)(q * 32) << 16;
+    const uint32_t a_addr = tmem_base + lanes + a_col0 + unit * 32;
+    const uint8_t *row_raw = sR + n_in * 16, *row_sb = sR + PACKED + n_in * (GPK * 4);
+    int rs = (grp >> 1) * 2 + unit, as = grp >> 1, seg = 0, stage0 = 0;   // stage0: parity of the segment's first stage
+    uint32_t rphase = 0, aphase = 0;
+    int done = 0;
+    bool ok = true, released = false, raw_ready = false;
+    int waiting_item = -1, waiting_split = 0;   // the segment whose accumulators are still to be read
+    // eight columns (rows of the step) at a time: the split's sum, added to those before it or written out
+    auto drain = [&]() {
+      if (!released) { pdl_wait(); released = true; }   // the stores may overwrite what an earlier kernel still reads
+      ok = warp_wait(acc_full, (seg - 1) & 1, p.status, KC_DEV_QLINEAR | 7);
+      if (!ok) return;
+      tc_fence_after();
+      const bool odd = first_kb(waiting_split + 1) - first_kb(waiting_split) > 1, last = waiting_split == p.splits - 1;
+      const int n = waiting_item % p.n_tiles * QL_TILE_N + n_in, row0 = waiting_item / p.n_tiles * p.m_pad;
+#pragma unroll 1
+      for (int c = grp * 8; c < p.m_pad; c += QL_DQ_GROUPS * 8) {
+        const uint32_t at = tmem_base + lanes + c;
+        uint32_t e[8], o[8];
+        tmem_ld8_issue(at, e);
+        tmem_ld8_issue(odd ? at + cs : at, o);
+        float* sum = sums + c * QL_TILE_N + n_in;
+        float before[8];
+        if (waiting_split > 0) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) before[j] = sum[j * QL_TILE_N];
+        }
+        tmem_wait_ld();
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          asm volatile("" : "+r"(e[j]), "+r"(o[j]));   // no use before the wait
+          v[j] = odd ? __uint_as_float(e[j]) + __uint_as_float(o[j]) : __uint_as_float(e[j]);
+          if (waiting_split > 0) v[j] = before[j] + v[j];
+        }
+        if (!last) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) sum[j * QL_TILE_N] = v[j];
+        } else if (n < p.N) {
+          const int m = row0 + c;
+          bf16* dst = p.y + (size_t)(p.row0 + m) * p.ldy + n;
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            if (m + j < p.M) dst[(size_t)j * p.ldy] = __float2bfloat16_rn(v[j]);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_free);
+      waiting_item = -1;
+    };
+    for (int item = blockIdx.x; ok && item < items; item += gridDim.x) {
+      for (int split = 0; ok && split < p.splits; ++split) {
+        const int nkb = first_kb(split + 1) - first_kb(split), stages = (nkb + 1) >> 1;
+        for (int j = (grp >> 1) ^ stage0; ok && j < stages; j += 2) {
+          // the first stages are dequantised under the tail of the previous kernel: see qlinear_umma_ta_kernel
+          if (!released && 2 * done >= SA) { pdl_wait(); released = true; }
+          ++done;
+          if (!__all_sync(0xffffffffu, raw_ready)) {
+            ok = warp_wait(&raw_full[rs], rphase, p.status, KC_DEV_QLINEAR | 5);
+            if (!ok) break;
+          }
+          const bool a_free = mbar_test_wait(&a_empty[2 * as + unit], aphase ^ 1);
+          const size_t at = (size_t)rs * p.record_bytes;
+          uint32_t v[32];   // of an empty unit: whatever its slot holds, which no product takes
+          bf162 sb[GPK];
+          if (GPK == 1) {
+            sb[0] = *reinterpret_cast<const bf162*>(row_sb + at);
+          } else {
+            const uint2 s = *reinterpret_cast<const uint2*>(row_sb + at);
+            sb[0] = bf2_bits(s.x); sb[GPK - 1] = bf2_bits(s.y);
+          }
+          if (!WIDE) dequant_row<BITS, GPK>(row_raw + at, sb, v);
+          else dequant_row_wide<BITS, GPK>(row_raw + at, sb, v);
+          if (!__all_sync(0xffffffffu, a_free)) ok = warp_wait(&a_empty[2 * as + unit], aphase ^ 1, p.status, KC_DEV_QLINEAR | 6);
+          if (!ok) break;
+          tc_fence_after();
+          tmem_st32(a_addr + as * 64, v);
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&raw_empty[rs]);
+          rs += 4;
+          if (rs >= RS) { rs -= RS; rphase ^= 1u; }
+          raw_ready = mbar_test_wait(&raw_full[rs], rphase);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&a_ready[2 * as + unit]);
+          as += 2;
+          if (as >= SA) { as -= SA; aphase ^= 1u; }
+          if (waiting_item >= 0) drain();
+        }
+        if (ok && waiting_item >= 0) drain();   // a segment without a stage of this group
+        waiting_item = item; waiting_split = split;
+        ++seg;
+        stage0 ^= stages & 1;
+      }
+    }
+    if (ok && waiting_item >= 0) drain();
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 2) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(p.tmem_cols) : "memory");
+  }
+}
+
+// Ring depths and shared memory of qlinear_umma_rows_kernel.
+static TaPlan plan_rows(const QWeight& w, int m_pad) {
+  TaPlan t{};
+  const int acc_cols = 2 * ((m_pad + 31) & ~31);
+  t.sa = std::min(6, (512 - acc_cols) / 64) & ~1;
+  t.tmem_cols = 512;
+  const size_t sums = (size_t)m_pad * QL_TILE_N * 4, budget = (size_t)224 * 1024 - sums;
+  const size_t b_stage = (size_t)m_pad * 128, r_stage = w.record_bytes;
+  t.rs = 4; t.sb = 4;
+  if (t.sb * b_stage + t.rs * r_stage > budget) return t;
+  // Deeper as far as there is room, activations by stages of two k-blocks, records by two stages (see the kernel). Three stages
+  // of activations come first: with two a k-block of 160 rows took 690 cycles, with three one of 144 took 517.
+  for (bool more = true; more;) {
+    more = false;
+    if (t.sb < 12 && (t.sb + 2) * b_stage + t.rs * r_stage <= budget) { t.sb += 2; more = true; }
+    if (t.rs < 16 && t.sb * b_stage + (t.rs + 4) * r_stage <= budget) { t.rs += 4; more = true; }
+  }
+  t.smem = 1024 + t.sb * b_stage + t.rs * r_stage + sums + (2 * t.rs + 2 * t.sb + 4 * t.sa + 2) * 8 + 16;
+  t.ok = t.sa >= 2 && t.smem <= 227 * 1024;
+  return t;
+}
+
+template <int BITS, int GPK, bool WIDE>
+static cudaError_t launch_umma_rows_as(const QLinearLaunch& l, QlKernelParams& p, cudaStream_t s) {
+  const QWeight& w = *l.w;
+  const TaPlan t = plan_rows(w, p.m_pad);
+  if (!t.ok) return cudaErrorInvalidValue;
+  p.tmem_cols = t.tmem_cols;
+  p.a_stages = t.sa; p.b_stages = t.sb; p.r_stages = t.rs;
+  static DeviceOnce configured;   // the attribute belongs to the device's copy of the kernel
+  if (configured.first_on_current_device()) {
+    cudaError_t e = cudaFuncSetAttribute(qlinear_umma_rows_kernel<BITS, GPK, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) { configured.forget_current_device(); return e; }
+  }
+  const CUtensorMap* rows = act_operand_rows_map(l.x, p.m_pad);
+  if (!rows) return cudaErrorInvalidValue;
+  return launch_k(qlinear_umma_rows_kernel<BITS, GPK, WIDE>, dim3(std::min(w.n_tiles * p.chunks, w.sm_count)), dim3(QL_THREADS), t.smem, s, *rows, p);
+}
+template <int BITS, int GPK>
+static cudaError_t launch_umma_rows(const QLinearLaunch& l, QlKernelParams& p, cudaStream_t s) {
+  return l.w->wide_scale ? launch_umma_rows_as<BITS, GPK, true>(l, p, s) : launch_umma_rows_as<BITS, GPK, false>(l, p, s);
+}
+
 template <int BITS, int GPK, int NT, int P, bool WIDE>
 static cudaError_t launch_umma_ta(const QLinearLaunch& l, QlKernelParams& p, cudaStream_t s) {
   const QWeight& w = *l.w;
@@ -723,6 +1017,39 @@ static int plan_chunk_rows(const QWeight& w, int nt, int cap, int M) {
   return best;
 }
 
+constexpr int QL_ROWS_MIN = 257;   // below, a chunk or two of rows never fill the SMs
+// Whether a weight's rows are taken by qlinear_umma_rows_kernel, and how many a chunk: 0 where a split a CTA takes about as long
+// or less. In cycles, fitted to launches of 264 to 2048 rows against eight weights of 16 to 64 tiles and 56 to 448 k-blocks, the
+// fit within a tenth of them: a k-block there takes 330 and 1.55 a row, a CTA's start and end 9500; here 330 and 1.9 a row, 2.3
+// where two stages of activations only have room, a segment's end 600. Partials cost their consumer 6500 bytes a cycle over all
+// SMs, a reduction of their own, which more than QL_MAX_M rows have, 2150.
+// At 2048 rows, split a CTA -> this: 4096 x 4096 156 -> 96 us, 4096 x 14336 281 -> 231, 6144 x 4096 185 -> 131, 8192 x 8192
+// 310 -> 262, 3584 x 18944 of 8 bits 319 -> 307. At 366: 24 -> 27 (and 2 us less in the consumer), 46 -> 67, 28 -> 29: not taken.
+static int plan_rows_chunk(const QWeight& w, int M) {
+  if (w.splits == 1 || plan_tiles_per_cta(w, w.sm_count) != 1 || M < QL_ROWS_MIN) return 0;
+  const int cap = plan_row_cap(1, w.record_bytes);
+  if (cap == 0) return 0;
+  auto apart_cost = [&](int rows) -> long long {
+    if (rows == 0) return 0;
+    const int per = plan_chunk_rows(w, 1, cap, rows);
+    const long long ctas = (long long)w.n_tiles * w.splits * ((rows + per - 1) / per), waves = (ctas + w.sm_count - 1) / w.sm_count;
+    const long long values = (long long)rows * w.N;
+    return waves * (w.kblocks * (330 + per * 31 / 20) / w.splits + 9500) + (M > QL_MAX_M ? values * (4 * w.splits + 2) / 2150 : values * 4 * w.splits / 6500);
+  };
+  const long long apart = M / QL_MAX_M * apart_cost(QL_MAX_M) + apart_cost(M % QL_MAX_M);
+  int best = 0;
+  long long best_cost = apart / 100 * 92;
+  for (int per = 192; per >= 96; per -= 16) {
+    const TaPlan t = plan_rows(w, per);
+    if (!t.ok) continue;
+    const long long items = (long long)w.n_tiles * ((M + per - 1) / per), waves = (items + w.sm_count - 1) / w.sm_count;
+    const long long cost = waves * (w.kblocks * (330 + per * (t.sb >= 6 ? 19 : 23) / 10) + w.splits * 600) + 8000;
+    if (cost < best_cost) { best = per; best_cost = cost; }
+  }
+  return best;
+}
+bool qlinear_in_turn(const QWeight& w, int M) { return plan_rows_chunk(w, M) > 0; }
+
 cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   const QWeight& w = *l.w;
   if (l.M < 1 || l.M > qlinear_slab_rows(w, l.M)) return cudaErrorInvalidValue;
@@ -738,9 +1065,14 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   p.records = w.records; p.record_bytes = w.record_bytes;
   p.N = w.N; p.n_tiles = w.n_tiles; p.kblocks = w.kblocks;
   p.M = l.M; p.m_pad = plan_chunk_rows(w, nt, cap, l.M); p.row0 = l.row0;
-  p.splits = w.splits;
+  p.splits = w.splits; p.chunks = 0;
   p.y = l.y; p.ldy = l.ldy; p.partial = l.partial; p.status = l.status;
   p.glu = glu ? l.glu : 0; p.act = l.act; p.ld_act = l.ld_act;
+  if (const int rows = plan_rows_chunk(w, l.M)) {
+    p.m_pad = rows; p.chunks = (l.M + rows - 1) / rows;
+    if (w.bits == 4) return w.gpk == 2 ? launch_umma_rows<4, 2>(l, p, s) : launch_umma_rows<4, 1>(l, p, s);
+    return w.gpk == 2 ? launch_umma_rows<8, 2>(l, p, s) : launch_umma_rows<8, 1>(l, p, s);
+  }
   if (w.bits == 4) return w.gpk == 2 ? launch_umma_nt<4, 2>(l, p, nt, s) : launch_umma_nt<4, 1>(l, p, nt, s);
   return w.gpk == 2 ? launch_umma_nt<8, 2>(l, p, nt, s) : launch_umma_nt<8, 1>(l, p, nt, s);
 }

@@ -64,7 +64,7 @@ struct QLinearLaunch {
   const ActOperand* x;
   int row0;         // first activation row of this launch (x, y and partial are indexed from it)
   int M;            // live activation rows, at most qlinear_slab_rows
-  bf16* y;          // [M, ldy] bf16 when the weight has splits == 1 (else unused)
+  bf16* y;          // [M, ldy] bf16 when the weight has splits == 1 or qlinear_in_turn(w, M) (else unused)
   int ldy;
   float* partial;   // [splits][M][N] fp32 workspace when splits > 1 (rows relative to row0)
   uint32_t* status; // device status word
@@ -98,8 +98,10 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s);
 // Rows that one call takes out of M: the workspace of a weight that is split along K holds QL_MAX_M; a grid has 65535
 // chunks of 96 rows or more, and looking for the best number of them is host time that a launch of a million rows hides.
 constexpr int QL_LAUNCH_ROWS = 1 << 20;
+// Whether a launch of M rows takes the splits of its weight one after the other and writes y, no partials.
+bool qlinear_in_turn(const QWeight& w, int M);
 inline int qlinear_slab_rows(const QWeight& w, int M) {
-  const int most = w.splits > 1 ? QL_MAX_M : QL_LAUNCH_ROWS;
+  const int most = w.splits > 1 && !qlinear_in_turn(w, M) ? QL_MAX_M : QL_LAUNCH_ROWS;
   return M < most ? M : most;
 }
 

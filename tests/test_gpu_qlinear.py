@@ -238,6 +238,28 @@ def test_row_chunks_carry_the_bits_of_few_rows(ctx, n, k, bits, group, m):
     assert ctx.device_status() == 0
 
 
+@pytest.mark.parametrize("n,k,bits,group,m,gain", [
+    (384, 1088, 4, 32, 1201, 1.0),    # three tiles, splits of 8 and 9 k-blocks, a last chunk of few rows
+    (4100, 2176, 4, 128, 1300, 1.0),  # several items a CTA, splits of 8 and 9 k-blocks, a ragged last tile
+    (300, 1024, 4, 64, 1000, 200.0),  # integers converted before the multiply-add
+    (4608, 3584, 8, 32, 1111, 1.0),
+    (6144, 4096, 4, 64, 700, 1.0),    # three splits
+    (1000, 1024, 8, 64, 5003, 1.0),
+])
+def test_many_rows_carry_the_bits_of_few(ctx, n, k, bits, group, m, gain):
+    """Many rows: persistent CTAs, which take all splits of their tile and rows one after the other instead of leaving
+    partials. A row's bits are those it has in a launch of few rows, where a split is a CTA of its own."""
+    g = torch.Generator().manual_seed(43)
+    p, s, b = quantize_affine(torch.empty(n, k).normal_(0, 0.02 * gain, generator=g), bits, group)
+    qw = api.QuantizedWeight(ctx, p.cuda(), s.cuda(), b.cuda(), bits, group)
+    x = acts(m, k, 44).cuda()
+    full = qw.matmul(x).cpu()
+    for r0, r1 in ((0, 1), (90, 131), (m // 2, m // 2 + 170), (m - 70, m), (m - 1, m)):
+        part = qw.matmul(x[r0:r1].contiguous()).cpu()
+        assert torch.equal(part.view(torch.int16), full[r0:r1].view(torch.int16)), f"rows {r0}..{r1}"
+    assert ctx.device_status() == 0
+
+
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("scale", [129 / 2 ** 10, 129 / 2 ** 8])     # below and above the line where the integers are converted first
 def test_weights_are_rounded_once(ctx, bits, scale):
