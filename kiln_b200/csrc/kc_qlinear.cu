@@ -1039,6 +1039,7 @@ static int plan_rows_chunk(const QWeight& w, int M) {
   const long long apart = M / QL_MAX_M * apart_cost(QL_MAX_M) + apart_cost(M % QL_MAX_M);
   int best = 0;
   long long best_cost = apart / 100 * 92;
+  if (w.kblocks * (330 + 96 * 19 / 10) + w.splits * 600 + 8000 >= best_cost) return 0;   // one wave of the smallest chunks
   for (int per = 192; per >= 96; per -= 16) {
     const TaPlan t = plan_rows(w, per);
     if (!t.ok) continue;
