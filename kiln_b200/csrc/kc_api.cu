@@ -479,14 +479,14 @@ extern "C" int kc_kv_write_block(kc_kv_t kv, uint32_t block, const void* src, si
 
 // y = x . dequant(W)^T for M rows. When `fused` is given and the weight is split along K, the reduction is left
 // to the consumer kernel: *fused then describes the fp32 partials instead of y (one launch and one round trip
-// through memory less). Rows beyond one 512-row slab always go through the reduction kernel.
+// through memory less). More rows than one 512-row slab go through the reduction kernel, or take the splits in turn.
 static int run_qlinear(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, bf16* y, int ldy, float* partial,
                        SublayerOut* fused = nullptr) {
   const bool defer = fused && w.splits > 1 && M <= QL_MAX_M && !qlinear_in_turn(w, M);
-  const int slab = qlinear_slab_rows(w, M);
-  for (int row0 = 0; row0 < M; row0 += slab) {
+  for (int row0 = 0, rows; row0 < M; row0 += rows) {
+    rows = qlinear_slab_rows(w, M - row0);
     QLinearLaunch l;
-    l.w = &w; l.x = &x; l.row0 = row0; l.M = std::min(slab, M - row0);
+    l.w = &w; l.x = &x; l.row0 = row0; l.M = rows;
     l.y = y; l.ldy = ldy; l.partial = partial; l.status = c->status;
     LAUNCH(c, KC_PROF_GEMM, 1, qlinear_umma(l, c->stream));
     if (w.splits > 1 && !defer && !qlinear_in_turn(w, l.M))
@@ -501,9 +501,8 @@ static int run_qlinear(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, 
 // interleaved [M, 2F] product and run the element-wise kernel on it. Both ways round at the same points.
 static int run_gated(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, bf16* gu, int F, int gelu, bool interleaved,
                      bf16* act, float* partial) {
-  const int slab = qlinear_slab_rows(w, M);
-  for (int row0 = 0; row0 < M; row0 += slab) {
-    const int rows = std::min(slab, M - row0);
+  for (int row0 = 0, rows; row0 < M; row0 += rows) {
+    rows = qlinear_slab_rows(w, M - row0);
     int done = 0;
     QLinearLaunch l;
     l.w = &w; l.x = &x; l.row0 = row0; l.M = rows;

@@ -79,10 +79,10 @@ extern "C" int kc_quantized_matmul_static(kc_ctx_t c, kc_qweight_t q, const void
     return api_fail(KC_ERR_CUDA, msg);
   }
   bf16* y = (bf16*)y_dev;
-  const int rows = qlinear_slab_rows(w, m);
-  for (int row0 = 0; row0 < m; row0 += rows) {
+  for (int row0 = 0, rows; row0 < m; row0 += rows) {
+    rows = qlinear_slab_rows(w, m - row0);
     QLinearLaunch l;
-    l.w = &w; l.x = &op; l.row0 = row0; l.M = (m - row0) < rows ? (m - row0) : rows;
+    l.w = &w; l.x = &op; l.row0 = row0; l.M = rows;
     l.y = y; l.ldy = w.N; l.partial = scratch; l.status = cv.status;
     // launches are counted once they are queued; this entry point takes no part in kc_profile_* timing
     e = qlinear_umma(l, cv.stream);

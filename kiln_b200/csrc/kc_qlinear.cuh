@@ -95,14 +95,15 @@ bool act_operand_init(ActOperand* op, const bf16* ptr, int rows, int K, const ch
 
 // The GEMM (tcgen05 + TMEM + TMA). Returns a CUDA error. One launch of at most qlinear_slab_rows rows.
 cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s);
-// Rows that one call takes out of M: the workspace of a weight that is split along K holds QL_MAX_M; a grid has 65535
-// chunks of 96 rows or more, and looking for the best number of them is host time that a launch of a million rows hides.
+// Rows that one call takes of the M that are left: the workspace of a weight that is split along K holds QL_MAX_M; a grid
+// has 65535 chunks of 96 rows or more, and looking for the best number of them is host time that a launch of a million rows
+// hides. Asked again for each launch, since what a large one leaves may go the other way.
 constexpr int QL_LAUNCH_ROWS = 1 << 20;
 // Whether a launch of M rows takes the splits of its weight one after the other and writes y, no partials.
 bool qlinear_in_turn(const QWeight& w, int M);
 inline int qlinear_slab_rows(const QWeight& w, int M) {
-  const int most = w.splits > 1 && !qlinear_in_turn(w, M) ? QL_MAX_M : QL_LAUNCH_ROWS;
-  return M < most ? M : most;
+  const int all = M < QL_LAUNCH_ROWS ? M : QL_LAUNCH_ROWS;
+  return all <= QL_MAX_M || w.splits == 1 || qlinear_in_turn(w, all) ? all : QL_MAX_M;
 }
 
 // The weight-streaming lane for at most QL_STREAM_MAX_M rows: x bf16 [M, ldx] against dequant(W)^T, left as fp32

@@ -115,3 +115,24 @@ for rows in (1, 700, 40000, 7000000, 17000000):
     ok(lib.kc_quantized_matmul(ctx, w, at, rows, at))
     assert calls().count("launch early") >= (1 if rows < 65535 * 192 else 2)
 """)
+
+
+@pytest.mark.parametrize("out_features,in_features,bits,group", [(4096, 14336, 4, 64), (8192, 8192, 4, 64), (3584, 18944, 8, 32), (3584, 14336, 4, 128), (6144, 4096, 4, 64)])
+def test_rows_left_over_by_a_large_launch(fake, out_features, in_features, bits, group):
+    """Weights that are split along K: a launch of many rows takes the splits in turn and has no limit of 512 rows, the rows
+    that the last launch is left with may be too few for that and are launches of 512. All counts are taken, by all calls."""
+    run(fake, f"""
+w = C.c_void_p()
+words = C.create_string_buffer({out_features} * {in_features} * {bits} // 8 + 256)
+ok(lib.kc_qweight_create(ctx, C.cast(words, C.POINTER(C.c_uint32)), words, words, {out_features}, {in_features}, {bits}, {group}, 0, C.byref(w)))
+in_turn = apart = 0
+for rows in [2 ** 20 * k + left for k in (0, 1, 2) for left in (1, 257, 512, 513, 600, 641, 774, 896, 961, 1296, 2000)]:
+    fake.fake_reset()
+    ok(lib.kc_quantized_matmul(ctx, w, at, rows, at))
+    seen = calls().count("launch early")
+    in_turn += rows > 512 and seen <= rows // 2 ** 20 + 1
+    apart += rows > 2 ** 20 and seen > rows // 2 ** 20 + 1
+    rc = lib.kc_quantized_matmul_static(ctx, w, at, rows, at)
+    assert rc == L.KC_OK or rc == L.KC_ERR_UNSUPPORTED and rows > 256, (rows, rc, lib.kc_last_error())
+assert in_turn and apart, (in_turn, apart)     # both ways, the second one in what a large launch leaves
+""")
