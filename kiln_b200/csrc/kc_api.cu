@@ -127,7 +127,7 @@ struct kc_kv {
   bool map5d = false;          // map whose box is 16 keys of K and V of a layer (make_tmap_kv_5d)
   CUtensorMap map_one;         // the same for 16 keys of K or of V; without map5d a copy of `map`
   struct Written { uint32_t step = 0; int32_t seq = 0; };
-  std::vector<Written> written;   // the last step that wrote a block, and for which sequence (-1: several)
+  std::vector<Written> written;   // the last step that wrote a block, and the sequence whose table named it for that (-1: named several times)
   uint32_t step = 0;
 };
 
@@ -1073,23 +1073,26 @@ void plan_attention(StepPlan* p, const kc_seq_step* seqs, const std::vector<int>
   items.swap(full);
 }
 
-// Per sequence, the keys from its start that nothing in this step writes: those before its new tokens, as far as no other
-// sequence of the step writes into one of their blocks (a caller may hand in pieces of one sequence as several).
+// Per sequence, the keys from its start that nothing in this step writes: those before its new tokens, as far as the step
+// does not write into one of their blocks. The block that the new tokens begin in is both theirs and the old keys'; any other
+// write there or below counts, another sequence's (a caller may hand in pieces of one sequence as several) as well as the
+// sequence's own to a block that its table names twice.
 std::vector<int> old_keys(kc_kv* kv, const kc_seq_step* seqs, int n_seqs) {
   if (kv->written.empty()) kv->written.resize(kv->num_blocks);
   if (++kv->step == 0) { std::fill(kv->written.begin(), kv->written.end(), kc_kv::Written{}); kv->step = 1; }
   for (int i = 0; i < n_seqs; ++i)
     for (int b = seqs[i].offset / kv->block_size; b <= (seqs[i].offset + seqs[i].len - 1) / kv->block_size; ++b) {
       kc_kv::Written& w = kv->written[seqs[i].blocks[b]];
-      w.seq = w.step == kv->step && w.seq != i ? -1 : i;
+      w.seq = w.step == kv->step ? -1 : i;
       w.step = kv->step;
     }
   std::vector<int> old(n_seqs);
   for (int i = 0; i < n_seqs; ++i) {
+    const int first = seqs[i].offset / kv->block_size;   // block of the first new token
     old[i] = seqs[i].offset;
     for (int b = 0; b * kv->block_size < seqs[i].offset; ++b) {
       const kc_kv::Written& w = kv->written[seqs[i].blocks[b]];
-      if (w.step == kv->step && w.seq != i) { old[i] = b * kv->block_size; break; }
+      if (w.step == kv->step && (w.seq != i || b != first)) { old[i] = b * kv->block_size; break; }
     }
   }
   return old;

@@ -15,6 +15,7 @@ std::mutex mu;
 std::string calls;
 size_t fail_above = ~size_t(0);
 bool fail_host_only = false;
+std::string copied;
 
 void note(const char* what) {
   std::lock_guard<std::mutex> lk(mu);
@@ -34,6 +35,7 @@ CUresult encode(CUtensorMap*, ...) { return CUDA_SUCCESS; }
 
 // what the tests call
 EXPORT const char* fake_calls() { return calls.c_str(); }
+EXPORT const char* fake_copied(size_t* n) { *n = copied.size(); return copied.data(); }   // the bytes of the last copy
 EXPORT void fake_reset() { std::lock_guard<std::mutex> lk(mu); calls.clear(); }
 EXPORT void fake_fail_above(size_t bytes) { fail_above = bytes; }         // allocations larger than this fail
 EXPORT void fake_fail_host_only(int on) { fail_host_only = on != 0; }     // ... of pinned memory only
@@ -45,7 +47,12 @@ EXPORT cudaError_t cudaFree(void* p) { note("free"); free(p); return cudaSuccess
 EXPORT cudaError_t cudaFreeHost(void* p) { note("free"); free(p); return cudaSuccess; }
 EXPORT cudaError_t cudaHostGetDevicePointer(void** d, void* h, unsigned) { *d = h; return cudaSuccess; }
 EXPORT cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind) { memcpy(d, s, n); return cudaSuccess; }
-EXPORT cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) { note("copy"); memcpy(d, s, n); return cudaSuccess; }
+EXPORT cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind, cudaStream_t) {
+  note("copy");
+  memcpy(d, s, n);
+  copied.assign(static_cast<const char*>(s), n);
+  return cudaSuccess;
+}
 EXPORT cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { note("fill"); memset(d, v, n); return cudaSuccess; }
 EXPORT cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) { *s = reinterpret_cast<cudaStream_t>(malloc(1)); return cudaSuccess; }
 EXPORT cudaError_t cudaStreamDestroy(cudaStream_t s) { free(s); return cudaSuccess; }

@@ -136,3 +136,37 @@ for rows in [2 ** 20 * k + left for k in (0, 1, 2) for left in (1, 257, 512, 513
     assert rc == L.KC_OK or rc == L.KC_ERR_UNSUPPORTED and rows > 256, (rows, rc, lib.kc_last_error())
 assert in_turn and apart, (in_turn, apart)     # both ways, the second one in what a large launch leaves
 """)
+
+
+@pytest.mark.parametrize("segments,old", [
+    ([(4, 60, list(range(4)))], [60]),                                  # its own last block holds old and new keys
+    ([(4, 64, list(range(5)))], [64]),
+    ([(1, 40, [0, 1, 2]), (1, 40, [0, 1, 3])], [40, 40]),               # a shared prefix that neither writes
+    ([(16, 0, [7]), (1, 40, [0, 7, 2])], [0, 16]),                      # another sequence writes its second block
+    ([(20, 40, [0, 1, 2, 3]), (4, 60, [0, 1, 2, 3])], [40, 32]),        # pieces of one sequence
+    ([(10, 40, [5, 1, 2, 5])], [0]),                                    # its own writes come to its first block again
+    ([(10, 40, [1, 5, 2, 5])], [16]),
+    ([(20, 40, [0, 1, 2, 2])], [32]),                                   # .. and to the one that they begin in
+    ([(1, 40, [0, 3, 3])], [16]),
+    ([(1, 40, [3, 3, 0])], [40]),                                       # named twice, not written
+])
+def test_keys_that_a_step_writes_are_not_old(fake, segments, old):
+    """Attention loads a sequence's old keys before it waits for the kernel ahead, which writes the new ones: none of them may
+    lie in a block that the step writes at another position or for another sequence. Read off the units that are copied."""
+    run(fake, f"""
+import struct
+segments, old = {segments}, {old}
+tables = [(C.c_uint32 * len(b))(*b) for _, _, b in segments]
+seqs = (L.KcSeqStep * len(segments))(*[L.KcSeqStep(n, off, n, len(b), t) for (n, off, b), t in zip(segments, tables)])
+rows = sum(n for n, _, _ in segments)
+ok(lib.kc_paged_attention(ctx, kv, 0, at, rows, 4, seqs, len(segments), 0.125, 0.0, 0, at))
+fake.fake_copied.restype, size = C.c_void_p, C.c_size_t()
+data = C.string_at(fake.fake_copied(C.byref(size)), size.value)
+found, row = [], 0
+for i, (n, off, _) in enumerate(segments):
+    units = [j for j in range(0, len(data) - 31, 16) if data[j: j + 24] == struct.pack("6i", i, row, n, off, 0, 1)]   # sequence, rows, position, chunk 0 alone
+    assert len(units) == 1, (i, units)
+    found.append(struct.unpack_from("i", data, units[0] + 28)[0])
+    row += n
+assert found == old, (found, old)
+""")
