@@ -1018,15 +1018,23 @@ static int plan_chunk_rows(const QWeight& w, int nt, int cap, int M) {
 }
 
 constexpr int QL_ROWS_MIN = 257;   // below, a chunk or two of rows never fill the SMs
+// With more k-blocks all splits in turn are the slower way at most row counts: 7000 x 28672 (448) 499 -> 564 us at 1200 rows, 805
+// -> 885 at 2048; 8192 x 28672 316 -> 334 at 640, 757 -> 780 at 1500, though 265 -> 251 at 513. 3584 x 18944 (296): the same
+// within a fiftieth up to 2048 rows, a tenth faster from there.
+constexpr int QL_ROWS_MAX_KBLOCKS = 300;
 // Whether a weight's rows are taken by qlinear_umma_rows_kernel, and how many a chunk: 0 where a split a CTA takes about as long
 // or less. In cycles, fitted to launches of 264 to 2048 rows against eight weights of 16 to 64 tiles and 56 to 448 k-blocks, the
 // fit within a tenth of them: a k-block there takes 330 and 1.55 a row, a CTA's start and end 9500; here 330 and 1.9 a row, 2.3
 // where two stages of activations only have room, a segment's end 600. Partials cost their consumer 6500 bytes a cycle over all
-// SMs, a reduction of their own, which more than QL_MAX_M rows have, 2150.
+// SMs, a reduction of their own, which more than QL_MAX_M rows have, 2150. More than eight splits are short ones, whose ends
+// lie less under the next one's start, 900: at 600 a call of 1024 x 8192 (16 splits) and 768 rows went from 48.5 to 56.1 us.
+// The choice against both ways at 23 row counts from 257 to 4096 and 26 weights: 22 % ahead of a split a CTA on average and
+// within 1 % of the best choice of way and chunk; behind a split a CTA by more than 2 % at two of the 598, 6000 x 12288 of 8
+// bits and 768 rows (3 %) and 3584 x 18944 of 8 bits and 2048 rows (1 % in three runs, 9 % in one).
 // At 2048 rows, split a CTA -> this: 4096 x 4096 156 -> 96 us, 4096 x 14336 281 -> 231, 6144 x 4096 185 -> 131, 8192 x 8192
-// 310 -> 262, 3584 x 18944 of 8 bits 319 -> 307. At 366: 24 -> 27 (and 2 us less in the consumer), 46 -> 67, 28 -> 29: not taken.
+// 310 -> 262. At 366: 24 -> 27 (and 2 us less in the consumer), 46 -> 67, 28 -> 29: not taken.
 static int plan_rows_chunk(const QWeight& w, int M) {
-  if (w.splits == 1 || plan_tiles_per_cta(w, w.sm_count) != 1 || M < QL_ROWS_MIN) return 0;
+  if (w.splits == 1 || plan_tiles_per_cta(w, w.sm_count) != 1 || M < QL_ROWS_MIN || w.kblocks > QL_ROWS_MAX_KBLOCKS) return 0;
   const int cap = plan_row_cap(1, w.record_bytes);
   if (cap == 0) return 0;
   auto apart_cost = [&](int rows) -> long long {
@@ -1039,12 +1047,13 @@ static int plan_rows_chunk(const QWeight& w, int M) {
   const long long apart = M / QL_MAX_M * apart_cost(QL_MAX_M) + apart_cost(M % QL_MAX_M);
   int best = 0;
   long long best_cost = apart / 100 * 92;
-  if (w.kblocks * (330 + 96 * 19 / 10) + w.splits * 600 + 8000 >= best_cost) return 0;   // one wave of the smallest chunks
+  const int ends = w.splits * (w.splits > 8 ? 900 : 600);
+  if (w.kblocks * (330 + 96 * 19 / 10) + ends + 8000 >= best_cost) return 0;   // one wave of the smallest chunks
   for (int per = 192; per >= 96; per -= 16) {
     const TaPlan t = plan_rows(w, per);
     if (!t.ok) continue;
     const long long items = (long long)w.n_tiles * ((M + per - 1) / per), waves = (items + w.sm_count - 1) / w.sm_count;
-    const long long cost = waves * (w.kblocks * (330 + per * (t.sb >= 6 ? 19 : 23) / 10) + w.splits * 600) + 8000;
+    const long long cost = waves * (w.kblocks * (330 + per * (t.sb >= 6 ? 19 : 23) / 10) + ends) + 8000;
     if (cost < best_cost) { best = per; best_cost = cost; }
   }
   return best;

@@ -170,3 +170,20 @@ for i, (n, off, _) in enumerate(segments):
     row += n
 assert found == old, (found, old)
 """)
+
+
+@pytest.mark.parametrize("out_features,in_features,bits,rows,in_turn", [
+    (4096, 4096, 4, 384, False), (4096, 4096, 4, 512, True), (4096, 4096, 4, 2048, True), (4096, 14336, 4, 2048, True), (6144, 4096, 4, 2048, True),
+    (7000, 28672, 4, 1200, False), (8192, 28672, 4, 1500, False), (1024, 8192, 4, 768, False), (1024, 8192, 4, 2048, True), (2048, 8192, 4, 513, False),
+    (2048, 8192, 4, 1024, True)])
+def test_many_rows_take_the_faster_way(fake, out_features, in_features, bits, rows, in_turn):
+    """One launch with the splits in turn, or launches of 512 rows with a reduction each: on both sides of the rule, where each
+    way was measured to be the faster one by a twentieth or more."""
+    run(fake, f"""
+w = C.c_void_p()
+words = C.create_string_buffer({out_features} * {in_features} * {bits} // 8 + 256)
+ok(lib.kc_qweight_create(ctx, C.cast(words, C.POINTER(C.c_uint32)), words, words, {out_features}, {in_features}, {bits}, 64, 0, C.byref(w)))
+fake.fake_reset()
+ok(lib.kc_quantized_matmul(ctx, w, at, {rows}, at))
+assert calls().count("launch early") == ({1 if in_turn else 2 * -(-rows // 512)})
+""")
