@@ -1034,13 +1034,15 @@ struct StepPlan {
   int n = 0, n_seqs = 0, n_sampled = 0, max_blocks = 0, tokens_per_item = 1, max_chunks = 1;
   int max_len = 1;
   bool whole = false;              // attention units hold all chunks of their rows
+  bool keys = false;               // attention by the kernel with a key per thread
   std::vector<AttnUnit> units;
   MetaLayout lay{};
 };
 
 // The step's attention units: items of up to tokens_per_item tokens of a sequence, each as one unit over all its chunks,
-// longest first, or as one unit per chunk, whole chunks first. old: per sequence, see AttnUnit.
-void plan_attention(StepPlan* p, const kc_seq_step* seqs, const std::vector<int>& old, int head_dim, int gqa, int kv_heads, int sm_count) {
+// longest first, or as one unit per chunk, whole chunks first. old: per sequence, see AttnUnit. alone, capped: see attn_key_rows.
+void plan_attention(StepPlan* p, const kc_seq_step* seqs, const std::vector<int>& old, int head_dim, int gqa, int kv_heads, int sm_count,
+                    bool alone, bool capped) {
   std::vector<AttnUnit>& items = p->units;
   items.clear();
   int row = 0;
@@ -1058,8 +1060,12 @@ void plan_attention(StepPlan* p, const kc_seq_step* seqs, const std::vector<int>
   }
   std::stable_sort(items.begin(), items.end(), [](const AttnUnit& a, const AttnUnit& b) { return a.pos0 + a.ntok > b.pos0 + b.ntok; });
   std::vector<int> tiles(items.size());
-  for (size_t i = 0; i < items.size(); ++i) tiles[i] = (items[i].pos0 + items[i].ntok + 127) / 128;
-  p->whole = attn_whole(head_dim, p->tokens_per_item * gqa, tiles.data(), (int)items.size(), kv_heads, sm_count);
+  long long all_tiles = 0;
+  for (size_t i = 0; i < items.size(); ++i) all_tiles += tiles[i] = (items[i].pos0 + items[i].ntok + 127) / 128;
+  p->whole = attn_whole(tiles.data(), (int)items.size(), kv_heads, sm_count);
+  const AttnForm form = p->max_chunks == 1 ? AttnForm::one_chunk : p->whole ? AttnForm::whole : AttnForm::apart;
+  p->keys = p->tokens_per_item * gqa <= attn_key_rows(head_dim, alone, capped, form, all_tiles * kv_heads, sm_count);
+  if (head_dim > 128 && !p->keys) p->whole = false;   // a thread of attn_kernel's last role holds a row of the output in registers
   if (p->whole) return;
   std::vector<AttnUnit> full, rest;
   for (const AttnUnit& u : items)
@@ -1099,7 +1105,7 @@ std::vector<int> old_keys(kc_kv* kv, const kc_seq_step* seqs, int n_seqs) {
 }
 
 int validate_step(kc_model* m, kc_kv* kv, const uint32_t* token_ids, int32_t n, const kc_seq_step* seqs, int32_t n_seqs,
-                  int32_t pad_rows, StepPlan* plan) {
+                  int32_t pad_rows, StepPlan* plan, bool alone = false, bool capped = false) {
   if (!m || !kv || !token_ids || !seqs) return fail(KC_ERR_INVALID, "forward_step: NULL argument");
   if (kv->ctx != m->ctx) return fail(KC_ERR_INVALID, "forward_step: model and pools belong to different contexts");
   if (kv->layers != m->d.num_layers || kv->kv_heads != m->Hkv || kv->head_dim != m->d.head_dim)
@@ -1136,7 +1142,7 @@ int validate_step(kc_model* m, kc_kv* kv, const uint32_t* token_ids, int32_t n, 
   const int gqa = m->d.num_heads / m->d.num_kv_heads;
   p.tokens_per_item = attn_tokens_per_item(gqa, p.max_len);
   p.max_chunks = (max_ctx + ATT_CHUNK - 1) / ATT_CHUNK;
-  plan_attention(&p, seqs, old_keys(kv, seqs, n_seqs), m->d.head_dim, gqa, m->Hkv, m->ctx->sm_count);
+  plan_attention(&p, seqs, old_keys(kv, seqs, n_seqs), m->d.head_dim, gqa, m->Hkv, m->ctx->sm_count, alone, capped);
   MetaLayout& L = p.lay;
   size_t at = 0;
   auto put = [&](size_t bytes) { size_t o = at; at = align_up(at + bytes, 16); return o; };
@@ -1239,7 +1245,7 @@ AttnParams attn_params(kc_model* m, kc_kv* kv, const StepPlan& p, int layer, bf1
   a.Hq = Hq; a.Hkv = kv->kv_heads; a.gqa = Hq / kv->kv_heads;
   a.layer = layer; a.NB = kv->num_blocks; a.BS = kv->block_size;
   a.max_chunks = p.max_chunks;
-  a.whole = p.whole ? 1 : 0; a.single = p.max_chunks == 1 ? 1 : 0;
+  a.whole = p.whole ? 1 : 0; a.single = p.max_chunks == 1 ? 1 : 0; a.keys = p.keys ? 1 : 0;
   a.scale = scale; a.softcap = softcap; a.window = window;
   a.q_tokens = p.tokens_per_item;
   a.kv5d = kv->map5d ? 1 : 0;
@@ -1696,7 +1702,7 @@ extern "C" int kc_paged_attention(kc_ctx_t c, kc_kv_t kv, int32_t layer, const v
   if (rc) return rc;
   std::vector<uint32_t> ids(std::max(n, 1), 0);
   StepPlan p;
-  rc = validate_step(m, kv, ids.data(), n, seqs, n_seqs, 0, &p);
+  rc = validate_step(m, kv, ids.data(), n, seqs, n_seqs, 0, &p, true, softcap > 0.f);
   if (!rc) rc = upload_meta(m, kv, ids.data(), seqs, p);
   if (!rc) rc = ensure_attn_ws(m, p);
   if (!rc) rc = ensure_q_maps(m, (const bf16*)q_dev, n, num_heads, num_heads / kv->kv_heads, p);

@@ -30,7 +30,7 @@
 //   warps 4-7   softmax, one row per thread: S -> P, rescaling O when a row's maximum moved
 //   warps 8-11  a finished chunk's O: store the partial, or merge it into the row and store the row
 //
-// Units of at most KEY_ROWS rows go to kc_attn_keys.cu: this kernel takes prompts and steps that hold a piece of one.
+// Units of few rows go to kc_attn_keys.cu (attn_key_rows): this kernel takes prompts and steps that hold a piece of one.
 //
 // What bounds it: per 128-key tile of head size 128, HBM takes 2800 cycles of an SM's share, a softmax warp about 2900
 // (scores and maximum 590, exponentials and both parts of the probabilities 2000, of which 1024 the special-function
@@ -652,7 +652,7 @@ template <int D>
 cudaError_t launch_d(const CUtensorMap& map, const CUtensorMap& kmap, const CUtensorMap& q, const CUtensorMap& q_small, const AttnParams& p,
                      bool in_order, int n_tokens, int sm_count, cudaStream_t s) {
   cudaError_t e;
-  if (p.gqa * p.q_tokens <= KEY_ROWS) {
+  if (p.keys) {
     e = attn_keys(kmap, q, q_small, p, in_order, scale_folds(p.scale, p.softcap), D, sm_count, s);
     if (p.whole) return e;
   } else {
@@ -673,8 +673,27 @@ int attn_tokens_per_item(int gqa, int max_len) {
   return std::min(std::max(1, ATT_ROWS / gqa), std::max(1, max_len));
 }
 
-bool attn_whole(int head_dim, int rows, const int* item_tiles, int n_items, int kv_heads, int sm_count) {
-  if (head_dim > 128 && rows > KEY_ROWS) return false;   // a thread of attn_kernel's last role holds a row of the output in registers
+// In a step attn_keys_kernel has its first tiles from under the tail of the kernel ahead, 3 us or more that a call on its own
+// doesn't save. attn_kernel -> attn_keys_kernel, us a layer that a step gains: head sizes 128 and 256 at 64 rows 0 to 24
+// (one sequence of 100 keys and head size 256 loses 1.5), at 36 rows 1 to 34; head size 64 at 28 rows 0 to 14, at 32 rows 0
+// to 7, at 36 rows -6 to 4, at 64 -20 to 0: its tile is half the bytes and costs the softmax warps the same.
+// On its own the line falls with fewer tiles an SM, where a unit's start and end weigh, and rises under a cap, which costs
+// a row per thread more: one sequence of 1001 keys, head size 64, 19 -> 20.5 us at 8 rows, 18 -> 25 at 64; 48 of 6000 159 ->
+// 139 at 24, 203 -> 248 at 64; 128 and 64 rows, 32 of 1400 60 -> 64, under a cap 118 -> 110; 256, 48 of 40 21 -> 24 at 32
+// rows, 23 -> 33 at 64; 64 of 2500, units of whole rows, which attn_kernel does not have at that size, 84 us less at 64.
+// Over 5500 such calls the choice is within 0.2 % of the better kernel on average.
+int attn_key_rows(int head_dim, bool alone, bool capped, AttnForm form, long long tiles, int sm_count) {
+  if (!alone) return head_dim == 64 ? 32 : KEY_ROWS;
+  // by tiles an SM: under 1, 2, 4, 8, and more
+  static constexpr uint8_t apart[3][2][5] = {{{0, 0, 16, 24, 32}, {24, 32, 32, 40, 56}}, {{16, 24, 32, 32, 48}, {32, 40, 48, 56, 64}}, {{32, 32, 56, 64, 64}, {32, 32, 56, 64, 64}}};
+  static constexpr uint8_t rest[3][2][5] = {{{32, 32, 32, 32, 32}, {40, 48, 56, 56, 64}}, {{32, 40, 40, 40, 40}, {40, 56, 64, 64, 64}}, {{24, 24, 28, 40, 40}, {24, 24, 28, 40, 40}}};
+  if (head_dim == 256 && form == AttnForm::whole) return KEY_ROWS;
+  int load = 0;
+  while (load < 4 && tiles >= (long long)sm_count << load) ++load;
+  return (form == AttnForm::apart ? apart : rest)[head_dim / 128][capped ? 1 : 0][load];
+}
+
+bool attn_whole(const int* item_tiles, int n_items, int kv_heads, int sm_count) {
   const int total = n_items * kv_heads, ctas = std::min(total, sm_count);
   long long sum = 0, most = 0;
   for (int i = 0; i < n_items; ++i) sum += (long long)item_tiles[i] * kv_heads;

@@ -18,7 +18,7 @@ struct AttnUnit {
   int old;                      // keys from the sequence's start that nothing in this step writes
 };
 constexpr int ATT_SMALL_TOKENS = 8;
-constexpr int KEY_ROWS = 64;    // a step whose units have no more rows takes the kernel with a key per thread (kc_attn_keys.cu)
+constexpr int KEY_ROWS = 64;    // the most rows of a unit of the kernel with a key per thread (kc_attn_keys.cu)
 
 struct AttnParams {
   bf16* out;                   // [n_tokens, Hq * D], 16-byte aligned
@@ -38,6 +38,7 @@ struct AttnParams {
   float scale;                 // softmax scale (applied to fp32 scores)
   float softcap;               // 0 = off
   int window;                  // 0 = global
+  int keys;                    // 1: the kernel with a key per thread (attn_key_rows), 0: with a row per thread
   int q_tokens;                // tokens in the box of the large query map
   int kv5d;                    // the maps of the pools are 5-D (one operation per 16 keys) instead of 2-D
 };
@@ -45,8 +46,12 @@ struct AttnParams {
 // Tokens of one sequence that share a CTA (their rows x gqa must fit ATT_ROWS).
 int attn_tokens_per_item(int gqa, int max_len);
 // Whether units of whole rows (all chunks of an item in one unit) keep the SMs about as busy as units of single chunks:
-// item_tiles = tiles of 128 keys of each item, in the order of the units. rows: the most query rows of an item.
-bool attn_whole(int head_dim, int rows, const int* item_tiles, int n_items, int kv_heads, int sm_count);
+// item_tiles = tiles of 128 keys of each item, in the order of the units.
+bool attn_whole(const int* item_tiles, int n_items, int kv_heads, int sm_count);
+// The most rows of a unit with which the kernel with a key per thread is the faster one. alone: a call on its own, in plain
+// stream order; else a step's. tiles: of 128 keys, over all items and kv heads.
+enum class AttnForm { one_chunk, apart, whole };   // no row has a second chunk; units of single chunks, merged afterwards; units of whole rows
+int attn_key_rows(int head_dim, bool alone, bool capped, AttnForm form, long long tiles, int sm_count);
 
 // Query maps over [n_tokens, Hq, D] (5-D: 64 features, heads of a group, slabs, groups, tokens).
 bool make_tmap_q(CUtensorMap* map, const bf16* q, int n_tokens, int Hq, int gqa, int head_dim, int box_tokens, const char** err);

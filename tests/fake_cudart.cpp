@@ -16,6 +16,7 @@ std::string calls;
 size_t fail_above = ~size_t(0);
 bool fail_host_only = false;
 std::string copied;
+unsigned threads = 0;
 
 void note(const char* what) {
   std::lock_guard<std::mutex> lk(mu);
@@ -36,6 +37,7 @@ CUresult encode(CUtensorMap*, ...) { return CUDA_SUCCESS; }
 // what the tests call
 EXPORT const char* fake_calls() { return calls.c_str(); }
 EXPORT const char* fake_copied(size_t* n) { *n = copied.size(); return copied.data(); }   // the bytes of the last copy
+EXPORT unsigned fake_threads() { return threads; }   // a block's, of the last launch in order
 EXPORT void fake_reset() { std::lock_guard<std::mutex> lk(mu); calls.clear(); }
 EXPORT void fake_fail_above(size_t bytes) { fail_above = bytes; }         // allocations larger than this fail
 EXPORT void fake_fail_host_only(int on) { fail_host_only = on != 0; }     // ... of pinned memory only
@@ -91,5 +93,6 @@ EXPORT cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*,
   for (unsigned i = 0; i < c->numAttrs; ++i)
     early |= c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization && c->attrs[i].val.programmaticStreamSerializationAllowed;
   note(early ? "launch early" : "launch in order");
+  if (!early) threads = c->blockDim.x;
   return c->gridDim.y > 65535 || c->gridDim.z > 65535 ? cudaErrorInvalidConfiguration : cudaSuccess;
 }

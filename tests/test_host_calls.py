@@ -187,3 +187,22 @@ fake.fake_reset()
 ok(lib.kc_quantized_matmul(ctx, w, at, {rows}, at))
 assert calls().count("launch early") == ({1 if in_turn else 2 * -(-rows // 512)})
 """)
+
+
+@pytest.mark.parametrize("hd,gqa,lens,cap,keys_up_to", [
+    # one short sequence; few units of one chunk each; enough of them to fill the SMs; many long sequences (units of whole rows)
+    (64, 4, [100], 0, 32), (64, 4, [1001], 0, 0), (64, 4, [3000] * 4, 0, 24), (64, 8, [1400] * 48, 0, 32), (64, 4, [1001], 30, 24), (64, 4, [1400] * 48, 30, 64),
+    (128, 4, [100], 0, 32), (128, 4, [1001], 0, 16), (128, 4, [3000] * 4, 0, 32), (128, 4, [1400] * 48, 0, 40), (128, 8, [1001], 30, 32), (128, 4, [1400] * 48, 30, 64),
+    (256, 2, [100], 0, 24), (256, 2, [1001], 0, 32), (256, 2, [3000] * 4, 50, 64), (256, 2, [1400] * 48, 0, 64)])
+def test_attention_takes_the_faster_kernel(fake, hd, gqa, lens, cap, keys_up_to):
+    """A call on its own takes the kernel with a key per thread (768 threads) up to the rows of a unit with which it was
+    measured to be the faster one, then that with a row per thread (384)."""
+    run(fake, f"""
+ok(lib.kc_kv_create(ctx, 1, 8, {hd}, 200, 16, L.KC_BF16, C.byref(kv)))
+table = (C.c_uint32 * 200)(*range(200))
+lens, gqa = {lens}, {gqa}
+for rows in range(1, 64 // gqa + 2):
+    seqs = (L.KcSeqStep * len(lens))(*[L.KcSeqStep(rows, n, rows, 200, table) for n in lens])
+    ok(lib.kc_paged_attention(ctx, kv, 0, at, rows * len(lens), 8 * gqa, seqs, len(lens), 0.1, {cap}, 0, at))
+    assert fake.fake_threads() == (768 if rows * gqa <= {keys_up_to} else 384), rows * gqa
+""")
