@@ -160,11 +160,27 @@ def test_one_operation_per_tile_pair_matches_the_slab_loads(ctx, monkeypatch, hd
 def test_units_of_whole_rows_carry_the_bits_of_single_chunks(ctx, hd, heads, kvh, softcap, window):
     """Many long sequences in one step: a unit holds all chunks of its rows and merges them itself. One sequence alone: a
     unit per chunk, merged by the combine kernel. Same bits, with lengths on both sides of tile and chunk edges."""
+    check_whole_rows(ctx, hd, heads, kvh, 3, softcap, window)
+
+
+@pytest.mark.parametrize("hd,heads,kvh,rows,softcap,window", [
+    # a key per thread: two halves of the features, 32 rows and less, then 33 to 64
+    (256, 8, 4, 3, 0.0, 0), (256, 8, 4, 3, 50.0, 700), (256, 8, 4, 16, 0.0, 0), (256, 8, 4, 17, 0.0, 700), (256, 16, 4, 16, 30.0, 0),
+    (128, 16, 4, 9, 30.0, 0), (128, 16, 4, 16, 30.0, 600), (64, 16, 4, 11, 20.0, 0), (64, 16, 4, 16, 20.0, 0),
+    # a row per thread
+    (128, 8, 4, 40, 0.0, 0), (128, 8, 4, 40, 30.0, 700), (64, 8, 4, 40, 0.0, 700), (64, 16, 4, 11, 0.0, 0)])
+def test_units_of_whole_rows_of_many_rows(ctx, hd, heads, kvh, rows, softcap, window):
+    """The same with up to 64 rows a unit and more, and at head size 256, which the kernel with a key per thread alone has
+    units of whole rows of."""
+    check_whole_rows(ctx, hd, heads, kvh, rows, softcap, window)
+
+
+def check_whole_rows(ctx, hd, heads, kvh, rows, softcap, window):
     rng = np.random.default_rng(3)
     # 74 sequences fill whole rounds of 148 CTAs: the most loaded one has 0.82 of what whole rows are allowed. With the
     # window, key 511 is seen by the first row of 1210 and not by its second: a chunk that is masked for some rows.
     lens = [511, 512, 513, 1023, 1024, 1151, 1210, 1537] + [int(v) for v in rng.integers(600, 1600, 66)]
-    bs, rows = 16, 3
+    bs = 16
     nb = sum((n + rows + bs - 1) // bs for n in lens)
     kv = api.PagedKv(ctx, api.KvSpec(1, kvh, hd, nb, bs))
     data = outlier_values((64, kv.bytes_per_block() // 2), 51)
@@ -370,4 +386,48 @@ def test_softcap_is_exact_to_a_rounding(ctx):
     bound = torch.where(y < 0.75, 1.1e-7, 1.7e-7) * 2 * cap * torch.tanh(y) + 2 ** -8
     over = (ratio - want).abs() / bound
     assert float(over.max()) < 1, f"{float(over.max()):.2f} of the bound at {float(y.view(-1)[int(over.argmax())]):.3f} caps"
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("hd,heads,kvh,bs", [(128, 8, 2, 16), (64, 8, 2, 32), (256, 4, 2, 16)])
+def test_slab_loads_of_prompt_rows(ctx, monkeypatch, hd, heads, kvh, bs):
+    """The kernel with a row per thread over a pool of KILN_KV_MAP_2D=1: a slab of 8 keys an operation against 16 keys of K
+    and V, the same bits."""
+    segs = [(70, 500), (40, 0), (6, 1020)]
+    nb = sum((off + ln + bs - 1) // bs for ln, off in segs) + 2
+    spec = api.KvSpec(2, kvh, hd, nb, bs)
+    kv5, _ = fill_pools(ctx, spec, 33)
+    monkeypatch.setenv("KILN_KV_MAP_2D", "1")
+    kv2, _ = fill_pools(ctx, spec, 33)
+    monkeypatch.delenv("KILN_KV_MAP_2D")
+    seqs = build_seqs(segs, bs, nb, 6)
+    q = outlier_values((sum(s.len for s in seqs), heads, hd), 13).cuda()
+    for layer in range(2):
+        a, b = (api.paged_attention(ctx, kv, layer, q, seqs, hd ** -0.5).cpu() for kv in (kv5, kv2))
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16)), f"layer {layer}"
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("hd", [64, 128, 256])
+@pytest.mark.parametrize("cap", [0.0, 4.0])
+def test_prompt_rows_with_scores_that_are_not_finite(ctx, hd, cap):
+    """Infinite and NaN scores in the kernel with a row per thread (80 rows a unit) against the rows one at a time (a key per
+    thread): the same rows are NaN, the others have the same bits."""
+    heads, kvh, bs, n, rows = 2, 1, 16, 140, 40
+    g = torch.Generator().manual_seed(83)
+    k = torch.empty(12 * bs, hd).normal_(generator=g) * 6
+    v = torch.empty(12 * bs, hd).normal_(generator=g).to(torch.bfloat16)
+    k[40], k[140:144] = -3e38, -3e38
+    k[160] = 3e38
+    k[172] = float("nan")
+    k = k.to(torch.bfloat16)
+    kv = api.PagedKv(ctx, api.KvSpec(1, kvh, hd, 12, bs))
+    for b in range(12):
+        kv.write_block_bytes(b, torch.cat([k[b * bs: (b + 1) * bs].reshape(-1), v[b * bs: (b + 1) * bs].reshape(-1)]).view(torch.uint8).numpy().tobytes())
+    q = (torch.empty(rows, heads, hd).uniform_(0.5, 1.5, generator=g)).to(torch.bfloat16).cuda()
+    many = api.paged_attention(ctx, kv, 0, q, [api.SeqStep(rows, n, rows, list(range(12)))], hd ** -0.5, cap).cpu()
+    one = torch.cat([api.paged_attention(ctx, kv, 0, q[t: t + 1].contiguous(), [api.SeqStep(1, n + t, 1, list(range(12)))], hd ** -0.5, cap).cpu() for t in range(rows)])
+    assert torch.equal(torch.isnan(many), torch.isnan(one))
+    assert not bool(torch.isnan(many[: 160 - n]).any()) and bool(torch.isnan(many[172 - n:]).all())
+    assert torch.equal(torch.nan_to_num(many, nan=0.0).view(torch.int16), torch.nan_to_num(one, nan=0.0).view(torch.int16))
     assert ctx.device_status() == 0

@@ -10,6 +10,8 @@ here is of the tile class (weights dequantised to bf16 first), so the 2e-2 bar i
 that class; against the row-vector class — two of MLX's own kernels apart — the distance is reported and
 bounded at 4e-2 (the oracle's two classes are themselves up to 1.8e-2 apart on these models).
 """
+import dataclasses
+
 import numpy as np
 import pytest
 import torch
@@ -26,10 +28,10 @@ MODELS = ["tiny-llama", "tiny-llama-d128", "tiny-qwen2", "tiny-gemma2", "tiny-ll
 BS = 16
 
 
-def load(ctx, name, num_blocks=64):
-    cfg = PRESETS[name]
+def load(ctx, name, num_blocks=64, max_step_tokens=256, **changed):
+    cfg = dataclasses.replace(PRESETS[name], **changed)
     ck = synth_checkpoint(cfg, seed=0)
-    model = api.CudaModel(ctx, cfg, ck, max_step_tokens=256, max_step_seqs=16)
+    model = api.CudaModel(ctx, cfg, ck, max_step_tokens=max_step_tokens, max_step_seqs=16)
     kv = api.PagedKv(ctx, model.kv_spec(num_blocks, BS))
     omodel = O.OracleModel(cfg, ck)
     okv = O.OracleKv(cfg.num_hidden_layers, cfg.num_key_value_heads, cfg.head_dim, num_blocks, BS)
@@ -277,6 +279,71 @@ def test_pieces_of_a_sequence_in_one_step(ctx, name):
     want = run([[c] for c in cuts])
     for steps in ([cuts[:1], cuts[1:3], cuts[3:4], cuts[4:]], [cuts[:1], cuts[1:]]):
         assert torch.equal(run(steps), want)
+    assert ctx.device_status() == 0
+
+
+def rows_of(ctx, model, ids, blocks, steps):
+    """The logits of every row of a sequence that runs in these steps, each a list of pieces (first, end)."""
+    kv, rows = api.PagedKv(ctx, model.kv_spec(64, BS)), []
+    for step in steps:
+        batch = api.StepBatch(ids[step[0][0]: step[-1][1]], [api.SeqStep(b - a, a, b - a, blocks) for a, b in step])
+        logits = model.forward_step(batch, kv)
+        ctx.sync()
+        rows.append(logits.cpu())
+    return torch.cat(rows).view(torch.int16)
+
+
+@pytest.mark.parametrize("name", ["tiny-llama", "tiny-llama-d128", "tiny-gemma2"])
+def test_pieces_of_up_to_64_rows_a_unit(ctx, name):
+    """Pieces whose units have 32 to 64 rows, each in a step of its own (at head sizes 128 and 256 the kernel with a key per
+    thread, its first keys loaded under the kernel ahead), against steps that hold a larger piece (a row per thread)."""
+    cfg, model, _, _, _ = load(ctx, name)
+    sizes = [250, 240, 16, 12, 9, 8, 32, 24, 18, 60, 30]
+    at = np.concatenate([[0], np.cumsum(sizes)]).tolist()
+    cuts = list(zip(at, at[1:]))
+    ids, blocks = prompts(cfg, [at[-1]], 5)[0], list(range(1, 1 + -(-at[-1] // BS)))
+    want = rows_of(ctx, model, ids, blocks, [[c] for c in cuts])
+    assert torch.equal(rows_of(ctx, model, ids, blocks, [cuts[:1], cuts[1:3], cuts[3:7], cuts[7:10], cuts[10:]]), want)
+    assert torch.equal(rows_of(ctx, model, ids, blocks, [cuts[:1], [(250, 490)], [(490, 599), (599, at[-1])]]), want)
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("name,changed", [("tiny-llama-h2048", {}), ("tiny-gemma2", dict(hidden_size=2304)), ("tiny-qwen2", dict(hidden_size=1792))])
+def test_steps_of_many_rows_carry_the_bits_of_small_ones(ctx, name, changed):
+    """Steps of more rows than one grid's splits are for: the linears take a weight's splits in turn and hand their consumers
+    finished rows instead of partials. The same logits as in steps of 100 rows, bit for bit."""
+    cfg, model, _, _, _ = load(ctx, name, max_step_tokens=768, **changed)
+    n = 700
+    ids, blocks = prompts(cfg, [n], 7)[0], list(range(3, 3 + -(-n // BS)))
+    want = rows_of(ctx, model, ids, blocks, [[(a, a + 100)] for a in range(0, n, 100)])
+    for ends in ([700], [450, 700], [300, 620, 700]):
+        kv, first = api.PagedKv(ctx, model.kv_spec(64, BS)), 0
+        for end in ends:
+            sampled = min(end - first, 500)     # a step has at most 512 rows of logits
+            got = model.forward_step(api.StepBatch(ids[first:end], [api.SeqStep(end - first, first, sampled, blocks)]), kv)
+            ctx.sync()
+            assert torch.equal(got.cpu().view(torch.int16), want[end - sampled: end]), (first, end)
+            first = end
+    assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("hidden", [2176, 3584, 4096])
+def test_sandwich_norm_of_wide_rows(ctx, hidden):
+    """Gemma-2's norms on both sides of a sublayer, at widths of more than one register chunk a thread, against the oracle."""
+    cfg, model, kv, omodel, okv = load(ctx, "tiny-gemma2", hidden_size=hidden)
+    ids = prompts(cfg, [40], 9)[0]
+    batch = api.StepBatch(ids, [api.SeqStep(40, 0, 40, [2, 5, 1])])
+    O.set_weight_class(0)
+    rowvec = omodel.forward_step(batch, O.OracleKv(cfg.num_hidden_layers, cfg.num_key_value_heads, cfg.head_dim, 64, BS)).double()
+    O.set_weight_class(1)
+    want = omodel.forward_step(batch, okv).double()
+    got = model.forward_step(batch, kv)
+    ctx.sync()
+    # Rounding noise grows with the width and the size of the logits (27 at 4096). The oracle's own two arithmetic classes show
+    # how much there is, about 1e-2 of the norm; another implementation is as far from either, half as much again at most.
+    noise, err = float((rowvec - want).norm()), float((got.cpu().double() - want).norm())
+    print(f"tiny-gemma2 hidden {hidden}: {err / float(want.norm()):.5f} from the oracle, its classes {noise / float(want.norm()):.5f} apart")
+    assert err < 1.5 * noise
     assert ctx.device_status() == 0
 
 

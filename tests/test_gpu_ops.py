@@ -9,7 +9,7 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows,dim", [(1, 256), (7, 2048), (192, 4096), (3, 3584)])
+@pytest.mark.parametrize("rows,dim", [(1, 256), (7, 2048), (192, 4096), (3, 3584), (5, 8), (4, 2056), (9, 4104), (130, 6144), (3, 8184), (2, 8192), (6, 8200)])
 def test_rms_norm(ctx, rows, dim):
     g = torch.Generator().manual_seed(rows * 1000 + dim)
     x = torch.empty(rows, dim).normal_(0, 1.5, generator=g).to(torch.bfloat16)
