@@ -116,7 +116,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
   const uint32_t tmem = *tmem_slot;
   // Units and block tables reach the device before a step's first kernel and no kernel writes them, so in a step the
   // producer reads them under the tail of the kernel before this one; where this kernel is the first one behind their copy
-  // it is launched in plain stream order (paged_attention). q, K and V are loaded after pdl_wait, and every role is past it
+  // it is launched in plain stream order (paged_attention). This kernel loads q, K and V after pdl_wait, and every role is past it
   // before its first bounded wait: the time that the kernel before this one takes does not count against the limit.
 
   const int total = p.n_units * p.Hkv;

@@ -11,13 +11,16 @@
 // K and V are separate slots of the ring: scores are taken from half a tile's bytes, and a slot of K is free again one
 // product earlier.
 //
-// What bounds it: up to 32 rows HBM, 5.5 TB/s of the 6.5 that a copy makes, and about 4 us until the first tile is there, 3
-// of which lie under the kernel ahead in a step; at 40 rows and more the softmax warps, whose time is instruction fetch and
-// latencies as much as issue: four sets of warps with eight rows each in a loop take a third less than one set with all of
-// them unrolled. L2 flushed, attn_kernel -> this: 32 sequences of 512 to 2048 keys 48.8 -> 41.3 us at 4 rows of a unit, 49.2
-// -> 43.4 at 24 (25.7 at the copy's rate); 64 of 1024 to 4096 and 40 rows 149.6 -> 143.7 (102.9); 16 of 6144 under a soft
-// cap, head size 256, 212 + 36 for the combine kernel -> 150 (123), with a window of 4096 202 + 14 -> 107 (82); one of 1001
-// 13.0 -> 10.9; 48 of 40 18.6 -> 10.5. In a decode step of 32 sequences a layer's attention adds 48.2 -> 31.1 us.
+// What bounds it: over long contexts and up to 32 rows HBM, 5.6 TB/s of the 6.5 that a copy makes (18 sequences of 8191 keys).
+// Over 32 sequences of 512 to 2048 keys HBM is at 0.6 of that: 41 to 43 us where the copy's rate would take 26. Of the
+// difference 4 us are the start until the first tile is there (3 lie under the kernel ahead in a step), the rest is 256
+// units of 4 to 16 tiles that fall on 148 SMs unevenly and begin and end one after the other. At 40 rows and more the softmax
+// warps bound it, whose time is instruction fetch and latencies as much as issue: four sets of warps with eight rows each in
+// a loop take a third less than one set with all of them unrolled. A call on its own, L2 flushed, attn_kernel -> this: 32
+// sequences of 512 to 2048 keys 48.8 -> 41.3 us at 4 rows of a unit, 49.2 -> 43.4 at 24; 64 of 1024 to 4096 and 40 rows 149.6 ->
+// 143.7 (102.9 at the copy's rate); 16 of 6144 under a soft cap, head size 256, 212 + 36 for the combine kernel -> 150 (123),
+// with a window of 4096 202 + 14 -> 107 (82); one of 1001 13.0 -> 10.9; 48 of 40 18.6 -> 10.5. In a decode step of 32
+// sequences a layer's attention adds 48.2 -> 31.1 us. Where it is the slower one: attn_key_rows.
 #include "kc_attn_dev.cuh"
 
 #include <algorithm>
@@ -135,7 +138,11 @@ attn_keys_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  // What is read before pdl_wait and why that is sound: see attn_kernel.
+  // Before pdl_wait only the producer reads memory: units and block tables, and K and V of keys below AttnUnit::old. All of
+  // it was written ahead of the step's first kernel, which starts when all that is complete (see pdl_wait), and
+  // nothing in the step writes it: old_keys ends a sequence's old keys at the first block that the step writes, but the one
+  // in which its new tokens begin, and a tile is loaded early only where all of it lies below. Q is loaded after the wait.
+  // The other roles are past it before their first bounded wait: see attn_kernel.
 
   const int total = p.n_units * p.Hkv;
   if (warp == 0) {

@@ -173,10 +173,15 @@ __device__ __forceinline__ float warp_max(float v) {
 }
 
 // ---- programmatic dependent launch ---------------------------------------
-// Every kernel of the step is launched with programmatic stream serialization: it may become resident while
-// its predecessor in the stream is still running, executes whatever touches no step data (barrier set-up,
-// TMEM allocation, descriptor prefetch, loads of WEIGHTS, which no kernel writes), and calls pdl_wait() before
-// its first access to memory that an earlier kernel of the stream writes or reads. pdl_wait() returns once the
+// Every kernel of the step but the first is launched with programmatic stream serialization: it may become resident while
+// its predecessor in the stream is still running, executes whatever touches no data that a kernel of the step writes (barrier
+// set-up, TMEM allocation, descriptor prefetch, loads of WEIGHTS), and calls pdl_wait() before its first access to memory
+// that an earlier kernel of the step writes or reads. The step's first kernel (launch_embed) is launched in plain stream
+// order: it starts when everything ahead of it is complete, and the others start after it has, so the copy of the step's
+// metadata and all that earlier steps, block copies and resets wrote to the K/V pools is there for each of them. What only
+// those wrote may therefore be read before pdl_wait() too: RoPE reads positions and slots, attention units, block tables and
+// K/V of keys that the step does not write (AttnUnit::old). Where such a kernel may come first behind such a write it is
+// launched in plain stream order itself (in_order). pdl_wait() returns once the
 // predecessor grid has completed and its writes are visible; since every kernel calls it before it ends, a
 // kernel's completion implies the completion of everything queued before it. pdl_launch_dependents() lets the
 // successor start being scheduled; it is issued first thing, so the successor fills SMs as they drain.

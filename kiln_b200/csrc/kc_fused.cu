@@ -251,7 +251,8 @@ add_rmsnorm_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __restri
 // loads of a thread are issued before the first use, so a row costs one round trip to L2 instead of one per chunk.
 // Element for element the arithmetic (and its order) is that of add_rmsnorm_kernel. PRE: with the sandwich norm.
 // H = 3584, time that it adds to a step, add_rmsnorm_kernel -> this: 320 rows of five partials 8.4 -> 7.0 us, 64 rows with
-// the sandwich norm 8.0 -> 6.2; what is left is launch latency and two or three round trips.
+// the sandwich norm 8.0 -> 6.2; what is left is launch latency and two or three round trips. <4, true, false> spills one
+// register (128 a thread).
 template <int CPT, bool FULL, bool PRE>
 __global__ void __launch_bounds__(256)
 add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __restrict__ w_pre, const bf16* __restrict__ w_out,
@@ -539,8 +540,9 @@ __global__ void copy_block_kernel(bf16* __restrict__ pool, int planes, int NB, s
 
 cudaError_t launch_embed(const uint32_t* w, const bf16* scales, const bf16* biases, const uint32_t* ids, int n, int H,
                          int bits, int group, float embed_scale, int vocab, bf16* out, cudaStream_t s) {
-  // The first kernel of a step follows the copy of the step's metadata: it is launched with plain stream order so
-  // that its dependency on that copy is the ordinary one; the kernels after it chain from it.
+  // The first kernel of a step: in plain stream order behind the copy of the step's metadata and behind all that earlier
+  // steps and copies wrote to the K/V pools. The kernels after it chain from it and read both before their waits (see
+  // pdl_wait): launched early, or left out, it would leave them racing with those writes.
   embed_kernel<<<n, 256, 0, s>>>(w, scales, biases, ids, H, bits, group, embed_scale, vocab, out);
   return cudaGetLastError();
 }

@@ -11,8 +11,10 @@
 //
 // Limits and behaviour a caller must know:
 //   * the partials of one launch (splits x min(m, 512) x out_features fp32) must fit KC_STATIC_SCRATCH_BYTES
-//     (16 MiB); a larger request is rejected with KC_ERR_UNSUPPORTED before anything is launched. Weights that are
-//     not split along K use no scratch and are never rejected for size;
+//     (16 MiB); a larger request is rejected with KC_ERR_UNSUPPORTED before anything is launched. Counted by the sizes
+//     alone, also where the launch takes a weight's splits in turn and leaves no partials, so that what is accepted does
+//     not hang on which way is the faster one. Weights that are not split along K use no scratch and are never rejected
+//     for size;
 //   * the first call on a device resolves the array's address (cudaGetSymbolAddress, which loads the module on
 //     that device if it is not loaded yet) and creates the kernel's attributes; make that first call before any
 //     stream capture begins;

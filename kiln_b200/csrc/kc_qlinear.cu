@@ -674,6 +674,8 @@ static TaPlan plan_ta(int nt, int per, int m_pad, uint32_t record_bytes) {
 // What bounds it: the hand-over of the dequantised weights as in qlinear_umma_ta_kernel (about 500 cycles a k-block up to 112
 // rows), then the activations: every CTA reads its own, 24 KB a k-block of 192 rows, 45 bytes a cycle and SM of L2. A form with
 // two tiles a CTA sharing them, four accumulators of 96 rows, took 980 cycles a pair of k-blocks, 349 us where this takes 231.
+// 4096 x 14336 at 2048 rows: tensor pipe 51 % active, HBM at 6 % of its rate. The 8-bit instantiations for large scales spill
+// (40 and 48 bytes at 96 registers, the most that 640 threads leave).
 // TMEM columns: [even, odd: round32(m_pad) each] [a_stages x 2 units x 32 columns].
 // ---------------------------------------------------------------------------
 template <int BITS, int GPK, bool WIDE>

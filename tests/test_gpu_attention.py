@@ -137,8 +137,8 @@ def test_prompt_rows_carry_decode_bits(ctx, hd, heads, kvh, softcap, window, sca
 
 @pytest.mark.parametrize("hd,heads,kvh,bs,layers", [(128, 8, 2, 16, 3), (64, 8, 2, 32, 2), (256, 4, 2, 16, 2)])
 def test_one_operation_per_tile_pair_matches_the_slab_loads(ctx, monkeypatch, hd, heads, kvh, bs, layers):
-    """A pool created with KILN_KV_MAP_2D=1 is read with one TMA operation per 64-feature slab of a K or V tile, the
-    default with one 4-D operation per K+V tile pair: the same shared-memory image, so the same bits, in every layer."""
+    """A pool created with KILN_KV_MAP_2D=1 is read with one TMA operation per 64-feature slab of 8 keys, the default with one
+    5-D operation per 16 keys of K or of V: the same shared-memory image, so the same bits, in every layer."""
     segs = [(6, 40), (1, 511), (6, 1020), (5, 7)]
     nb = sum((off + ln + bs - 1) // bs for ln, off in segs) + 2
     spec = api.KvSpec(layers, kvh, hd, nb, bs)
