@@ -1027,15 +1027,18 @@ constexpr int QL_ROWS_MAX_KBLOCKS = 300;
 // Whether a weight's rows are taken by qlinear_umma_rows_kernel, and how many a chunk: 0 where a split a CTA takes about as long
 // or less. In cycles, fitted to launches of 264 to 2048 rows against eight weights of 16 to 64 tiles and 56 to 448 k-blocks, the
 // fit within a tenth of them: a k-block there takes 330 and 1.55 a row, a CTA's start and end 9500; here 330 and 1.9 a row, 2.3
-// where two stages of activations only have room, a segment's end 600. Partials cost their consumer 6500 bytes a cycle over all
-// SMs, a reduction of their own, which more than QL_MAX_M rows have, 2150. More than eight splits are short ones, whose ends
+// where two stages of activations only have room, a segment's end 600. A reduction of their own costs partials 2150 bytes a
+// cycle over all SMs where there are more than QL_MAX_M rows, else 6500. Summed by the kernel that reads the result anyway
+// they cost that next to nothing, and of the two ways the one with a launch of its own size has to be faster by a seventh:
+// a layer of a step, splits apart -> in turn, us: 1B (2048 features) 96 -> 100 at 257 rows, 142 -> 147 at 448; 9B (3584) 201 -> 206 at
+// 333; 8B (4096) 289 -> 284 at 448, 300 -> 293 at 512; 7B (3584, 8 bits) 335 -> 330 at 448. More than eight splits are short ones, whose ends
 // lie less under the next one's start, 900: at 600 a call of 1024 x 8192 (16 splits) and 768 rows went from 48.5 to 56.1 us.
 // The choice against both ways at 23 row counts from 257 to 4096 and 26 weights: 22 % ahead of a split a CTA on average and
 // within 1 % of the best choice of way and chunk; behind a split a CTA by more than 2 % at two of the 598, 6000 x 12288 of 8
 // bits and 768 rows (3 %) and 3584 x 18944 of 8 bits and 2048 rows (1 % in three runs, 9 % in one).
 // At 2048 rows, split a CTA -> this: 4096 x 4096 156 -> 96 us, 4096 x 14336 281 -> 231, 6144 x 4096 185 -> 131, 8192 x 8192
 // 310 -> 262. At 366: 24 -> 27 (and 2 us less in the consumer), 46 -> 67, 28 -> 29: not taken.
-static int plan_rows_chunk(const QWeight& w, int M) {
+static int plan_rows_chunk(const QWeight& w, int M, bool summed) {
   if (w.splits == 1 || plan_tiles_per_cta(w, w.sm_count) != 1 || M < QL_ROWS_MIN || w.kblocks > QL_ROWS_MAX_KBLOCKS) return 0;
   const int cap = plan_row_cap(1, w.record_bytes);
   if (cap == 0) return 0;
@@ -1044,11 +1047,12 @@ static int plan_rows_chunk(const QWeight& w, int M) {
     const int per = plan_chunk_rows(w, 1, cap, rows);
     const long long ctas = (long long)w.n_tiles * w.splits * ((rows + per - 1) / per), waves = (ctas + w.sm_count - 1) / w.sm_count;
     const long long values = (long long)rows * w.N;
-    return waves * (w.kblocks * (330 + per * 31 / 20) / w.splits + 9500) + (M > QL_MAX_M ? values * (4 * w.splits + 2) / 2150 : values * 4 * w.splits / 6500);
+    return waves * (w.kblocks * (330 + per * 31 / 20) / w.splits + 9500) +
+           (summed ? 0 : M > QL_MAX_M ? values * (4 * w.splits + 2) / 2150 : values * 4 * w.splits / 6500);
   };
   const long long apart = M / QL_MAX_M * apart_cost(QL_MAX_M) + apart_cost(M % QL_MAX_M);
   int best = 0;
-  long long best_cost = apart / 100 * 92;
+  long long best_cost = apart / 100 * (summed ? 86 : 92);
   const int ends = w.splits * (w.splits > 8 ? 900 : 600);
   if (w.kblocks * (330 + 96 * 19 / 10) + ends + 8000 >= best_cost) return 0;   // one wave of the smallest chunks
   for (int per = 192; per >= 96; per -= 16) {
@@ -1060,7 +1064,7 @@ static int plan_rows_chunk(const QWeight& w, int M) {
   }
   return best;
 }
-bool qlinear_in_turn(const QWeight& w, int M) { return plan_rows_chunk(w, M) > 0; }
+bool qlinear_in_turn(const QWeight& w, int M, bool summed) { return plan_rows_chunk(w, M, summed) > 0; }
 
 cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   const QWeight& w = *l.w;
@@ -1080,7 +1084,7 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   p.splits = w.splits; p.chunks = 0;
   p.y = l.y; p.ldy = l.ldy; p.partial = l.partial; p.status = l.status;
   p.glu = glu ? l.glu : 0; p.act = l.act; p.ld_act = l.ld_act;
-  if (const int rows = plan_rows_chunk(w, l.M)) {
+  if (const int rows = plan_rows_chunk(w, l.M, l.summed)) {
     p.m_pad = rows; p.chunks = (l.M + rows - 1) / rows;
     if (w.bits == 4) return w.gpk == 2 ? launch_umma_rows<4, 2>(l, p, s) : launch_umma_rows<4, 1>(l, p, s);
     return w.gpk == 2 ? launch_umma_rows<8, 2>(l, p, s) : launch_umma_rows<8, 1>(l, p, s);

@@ -17,6 +17,7 @@ size_t fail_above = ~size_t(0);
 bool fail_host_only = false;
 std::string copied;
 unsigned threads = 0;
+std::string shapes;
 
 void note(const char* what) {
   std::lock_guard<std::mutex> lk(mu);
@@ -38,7 +39,8 @@ CUresult encode(CUtensorMap*, ...) { return CUDA_SUCCESS; }
 EXPORT const char* fake_calls() { return calls.c_str(); }
 EXPORT const char* fake_copied(size_t* n) { *n = copied.size(); return copied.data(); }   // the bytes of the last copy
 EXPORT unsigned fake_threads() { return threads; }   // a block's, of the last launch in order
-EXPORT void fake_reset() { std::lock_guard<std::mutex> lk(mu); calls.clear(); }
+EXPORT const char* fake_shapes() { return shapes.c_str(); }   // threads:grid of the launches with attributes
+EXPORT void fake_reset() { std::lock_guard<std::mutex> lk(mu); calls.clear(); shapes.clear(); }
 EXPORT void fake_fail_above(size_t bytes) { fail_above = bytes; }         // allocations larger than this fail
 EXPORT void fake_fail_host_only(int on) { fail_host_only = on != 0; }     // ... of pinned memory only
 
@@ -53,6 +55,10 @@ EXPORT cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyK
   note("copy");
   memcpy(d, s, n);
   copied.assign(static_cast<const char*>(s), n);
+  return cudaSuccess;
+}
+EXPORT cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind, cudaStream_t) {
+  for (size_t i = 0; i < h; ++i) memcpy(static_cast<char*>(d) + i * dp, static_cast<const char*>(s) + i * sp, w);
   return cudaSuccess;
 }
 EXPORT cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { note("fill"); memset(d, v, n); return cudaSuccess; }
@@ -94,5 +100,6 @@ EXPORT cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* c, const void*,
     early |= c->attrs[i].id == cudaLaunchAttributeProgrammaticStreamSerialization && c->attrs[i].val.programmaticStreamSerializationAllowed;
   note(early ? "launch early" : "launch in order");
   if (!early) threads = c->blockDim.x;
+  shapes += std::to_string(c->blockDim.x) + ':' + std::to_string(c->gridDim.x) + 'x' + std::to_string(c->gridDim.y) + 'x' + std::to_string(c->gridDim.z) + '\n';
   return c->gridDim.y > 65535 || c->gridDim.z > 65535 ? cudaErrorInvalidConfiguration : cudaSuccess;
 }

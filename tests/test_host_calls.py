@@ -45,8 +45,8 @@ def fake(tmp_path_factory):
     return so
 
 
-def run(fake, code):
-    r = subprocess.run([sys.executable, "-c", PRELUDE + code], cwd=ROOT, env={**os.environ, "LD_PRELOAD": str(fake), "PYTHONPATH": str(ROOT)},
+def run(fake, code, first=""):
+    r = subprocess.run([sys.executable, "-c", first + PRELUDE + code], cwd=ROOT, env={**os.environ, "LD_PRELOAD": str(fake), "PYTHONPATH": str(ROOT)},
                        capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
 
@@ -206,3 +206,30 @@ for rows in range(1, 64 // gqa + 2):
     ok(lib.kc_paged_attention(ctx, kv, 0, at, rows * len(lens), 8 * gqa, seqs, len(lens), 0.1, {cap}, 0, at))
     assert fake.fake_threads() == (768 if rows * gqa <= {keys_up_to} else 384), rows * gqa
 """)
+
+
+@pytest.mark.parametrize("hidden,heads,kv_heads,hd,rows,qkv,o", [
+    (2048, 32, 8, 64, 257, "640:24x4x2", "640:16x4x2"), (2048, 32, 8, 64, 500, "640:24x4x3", "640:16x4x4"),      # splits apart
+    (4096, 32, 8, 128, 384, "640:48x3x2", "640:32x4x2"), (4096, 32, 8, 128, 448, "640:144x1x1", "640:128x1x1"),  # .. and in turn
+    (3584, 16, 8, 256, 333, "640:64x2x2", "640:28x5x2")])
+def test_partials_that_a_consumer_sums(fake, hidden, heads, kv_heads, hd, rows, qkv, o):
+    """In a step the kernel behind a linear sums its partials at next to no cost: the linear takes its splits in turn only where
+    that is faster by itself. Read off the grids of a layer's first two linears (tiles x splits x chunks of rows, or CTAs)."""
+    run(fake, f"""
+import dataclasses
+import numpy as np
+from kiln_b200 import api
+from kiln_b200.synth import PRESETS, synth_checkpoint
+fake.fake_shapes.restype = C.c_char_p
+cfg = dataclasses.replace(PRESETS["tiny-llama"], hidden_size={hidden}, num_attention_heads={heads}, num_key_value_heads={kv_heads}, head_dim={hd},
+                          num_hidden_layers=1)
+c = api.Context(0)
+model = api.CudaModel(c, cfg, synth_checkpoint(cfg, seed=0), max_step_tokens=512, max_step_seqs=1)
+pool = api.PagedKv(c, model.kv_spec(32, 16))
+p = api._PackedStep(api.StepBatch(np.zeros({rows}, dtype=np.uint32), [api.SeqStep({rows}, 0, 0, list(range(32)))]))
+logits, n = C.c_void_p(), C.c_int32()
+fake.fake_reset()
+ok(L.lib().kc_forward_step(model._h, pool._h, p.ids_p, p.n, p.seq_arr, p.n_seqs, 0, C.byref(logits), C.byref(n)))
+grids = [s for s in fake.fake_shapes().decode().split() if s.startswith("640:")]
+assert grids[:2] == ["{qkv}", "{o}"], grids
+""", first="import torch")   # before the library, whose NCCL is another one
