@@ -368,11 +368,13 @@ add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __re
 // sin/cos of the token's angles are computed once per CTA and shared by its heads, before the wait for the kernel ahead (the
 // step's metadata is older than its first kernel; a single call's is not, see launch_rope_kv_write); every thread then moves
 // 8 consecutive features of each half with 16-byte loads and stores. A token's work items lie over CTAs of 128 threads, one
-// a thread: what bounds it is one item's chain of loads. Time that it adds to a step, all of a token's items in one CTA of
-// 256 threads and sin/cos behind the wait -> this: one token 6.2 -> 3.5 us, 192 tokens of three partials 5.8 -> 4.8, 320 of
-// four 12.7 -> 5.9.
-constexpr int ROPE_THREADS = 128;
-__global__ void __launch_bounds__(ROPE_THREADS)
+// a thread: what bounds it is one item's chain of loads. Up to 256 items are one CTA's: two would compute sin/cos twice and
+// gain no round. Time that it adds to a step, all of a token's items in one CTA of 256 threads and sin/cos behind the wait ->
+// this: one token 6.2 -> 3.5 us, 192 tokens of three partials 5.8 -> 4.8, 320 of four 12.7 -> 5.9. A layer of the 1B model (192
+// items), CTAs of 128 -> one of 192: 385 tokens 133.5 -> 131.0 us, 500 135.5 -> 136.4, one 39.3 -> 39.1; with 384 to 640 items
+// CTAs of up to 256 threads made no difference beyond 1 % either way.
+constexpr int ROPE_THREADS = 128, ROPE_ONE_CTA = 256;
+__global__ void __launch_bounds__(ROPE_ONE_CTA)
 rope_kv_write_kernel(RowSource qkv, const bf16* __restrict__ bias, const float* __restrict__ inv_freq,
                      const int32_t* __restrict__ token_pos, const int32_t* __restrict__ kv_slot, int Hq, int Hkv,
                      int D, int traditional, int layer, int NB, int BS, bf16* __restrict__ pool,
@@ -389,7 +391,7 @@ rope_kv_write_kernel(RowSource qkv, const bf16* __restrict__ bias, const float* 
   __syncthreads();
   pdl_wait();
   const int per_head = D / 16;             // work items per head: 8 features of each half, or 16 interleaved ones
-  const int it = blockIdx.y * ROPE_THREADS + threadIdx.x;
+  const int it = blockIdx.y * blockDim.x + threadIdx.x;
   if (it < heads * per_head) {
     const int h = it / per_head, c = it - h * per_head;
     // features [e0, e0 + 8) and [e1, e1 + 8) of head h; the rotation pairs are (e0 + k, e1 + k) for split
@@ -581,7 +583,8 @@ cudaError_t launch_rope_kv_write(const SublayerOut& qkv, const bf16* bias, const
                                  int NB, int BS, bf16* pool, bf16* q_out, cudaStream_t s, bool in_order) {
   if (D % 16 || D > 256) return cudaErrorInvalidValue;
   const int items = (Hq + 2 * Hkv) * (D / 16);
-  return launch_k_opt(!in_order, rope_kv_write_kernel, dim3(n, (items + ROPE_THREADS - 1) / ROPE_THREADS), dim3(ROPE_THREADS), 0, s, row_source(qkv), bias, inv_freq, token_pos, kv_slot, Hq, Hkv, D,
+  const int threads = items <= ROPE_ONE_CTA ? (std::max(items, D / 2) + 31) & ~31 : ROPE_THREADS;   // D / 2 pairs of sin and cos
+  return launch_k_opt(!in_order, rope_kv_write_kernel, dim3(n, (items + threads - 1) / threads), dim3(threads), 0, s, row_source(qkv), bias, inv_freq, token_pos, kv_slot, Hq, Hkv, D,
                   traditional, layer, NB, BS, pool, q_out);
 }
 

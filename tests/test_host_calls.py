@@ -233,3 +233,17 @@ ok(L.lib().kc_forward_step(model._h, pool._h, p.ids_p, p.n, p.seq_arr, p.n_seqs,
 grids = [s for s in fake.fake_shapes().decode().split() if s.startswith("640:")]
 assert grids[:2] == ["{qkv}", "{o}"], grids
 """, first="import torch")   # before the library, whose NCCL is another one
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd,shape", [(4, 2, 64, "32:3x1x1"), (32, 8, 64, "192:3x1x1"), (16, 8, 64, "128:3x1x1"), (32, 8, 128, "128:3x3x1"), (16, 8, 256, "128:3x4x1"), (64, 8, 64, "128:3x3x1")])
+def test_rope_items_of_a_token(fake, heads, kv_heads, hd, shape):
+    """Up to 256 work items of a token are one block's, more are blocks of 128."""
+    run(fake, f"""
+fake.fake_shapes.restype = C.c_char_p
+pool = C.c_void_p()
+ok(lib.kc_kv_create(ctx, 1, {kv_heads}, {hd}, 80, 16, L.KC_BF16, C.byref(pool)))
+fake.fake_reset()
+seqs = (L.KcSeqStep * 1)(L.KcSeqStep(3, 40, 3, 3, table))
+ok(lib.kc_rope_kv_write(ctx, pool, 0, at, None, C.cast(at, C.POINTER(C.c_float)), 3, {heads}, 0, seqs, 1, at))
+assert fake.fake_shapes().decode().split() == ["{shape}"], fake.fake_shapes()
+""")
