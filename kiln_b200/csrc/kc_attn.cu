@@ -676,14 +676,16 @@ int attn_tokens_per_item(int gqa, int max_len) {
 // In a step attn_keys_kernel has its first tiles from under the tail of the kernel ahead, 3 us or more that a call on its own
 // doesn't save. attn_kernel -> attn_keys_kernel, us a layer that a step gains: head sizes 128 and 256 at 64 rows 0 to 24
 // (one sequence of 100 keys and head size 256 loses 1.5), at 36 rows 1 to 34; head size 64 at 28 rows 0 to 14, at 32 rows 0
-// to 7, at 36 rows -6 to 4, at 64 -20 to 0: its tile is half the bytes and costs the softmax warps the same.
+// to 7, at 36 rows -6 to 4, at 64 -20 to 0: its tile is half the bytes and costs the softmax warps the same. Where no row has
+// a second chunk there is little but the start: one sequence of 100 keys 2.1 at 36 rows, 0.4 at 64; 32 of 100 1.8 at 48, -1.1
+// at 64.
 // On its own the line falls with fewer tiles an SM, where a unit's start and end weigh, and rises under a cap, which costs
 // a row per thread more: one sequence of 1001 keys, head size 64, 19 -> 20.5 us at 8 rows, 18 -> 25 at 64; 48 of 6000 159 ->
 // 139 at 24, 203 -> 248 at 64; 128 and 64 rows, 32 of 1400 60 -> 64, under a cap 118 -> 110; 256, 48 of 40 21 -> 24 at 32
 // rows, 23 -> 33 at 64; 64 of 2500, units of whole rows, which attn_kernel does not have at that size, 84 us less at 64.
 // Over 7500 such calls the choice is 0.13 % behind the better kernel on average, 12 % at most.
 int attn_key_rows(int head_dim, bool alone, bool capped, AttnForm form, long long tiles, int sm_count) {
-  if (!alone) return head_dim == 64 ? 32 : KEY_ROWS;
+  if (!alone) return head_dim > 64 ? KEY_ROWS : form != AttnForm::one_chunk ? 32 : tiles < sm_count ? KEY_ROWS : 48;
   // by tiles an SM: under 1, 2, 4, 8, and more
   static constexpr uint8_t apart[3][2][5] = {{{0, 0, 16, 24, 32}, {24, 32, 32, 40, 56}}, {{16, 24, 32, 32, 48}, {32, 40, 48, 56, 64}}, {{32, 32, 56, 64, 64}, {32, 32, 56, 64, 64}}};
   static constexpr uint8_t rest[3][2][5] = {{{32, 32, 32, 32, 32}, {40, 48, 56, 56, 64}}, {{32, 40, 40, 40, 40}, {40, 56, 64, 64, 64}}, {{24, 24, 28, 40, 40}, {24, 24, 28, 40, 40}}};

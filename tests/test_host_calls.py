@@ -247,3 +247,28 @@ seqs = (L.KcSeqStep * 1)(L.KcSeqStep(3, 40, 3, 3, table))
 ok(lib.kc_rope_kv_write(ctx, pool, 0, at, None, C.cast(at, C.POINTER(C.c_float)), 3, {heads}, 0, seqs, 1, at))
 assert fake.fake_shapes().decode().split() == ["{shape}"], fake.fake_shapes()
 """)
+
+
+@pytest.mark.parametrize("heads,kv_heads,hd,offset,rows,threads", [
+    (32, 8, 64, 600, 8, 768), (32, 8, 64, 600, 9, 384), (32, 8, 64, 70, 16, 768), (32, 8, 64, 70, 17, 384), (32, 8, 128, 600, 16, 768), (32, 8, 128, 600, 17, 384),
+    (16, 8, 256, 600, 32, 768), (16, 8, 256, 600, 33, 384)])
+def test_attention_in_a_step_takes_the_faster_kernel(fake, heads, kv_heads, hd, offset, rows, threads):
+    """A step's units of up to 64 rows take the kernel with a key per thread (768 threads), 32 at head size 64 and more than
+    one chunk."""
+    run(fake, f"""
+import dataclasses
+import numpy as np
+from kiln_b200 import api
+from kiln_b200.synth import PRESETS, synth_checkpoint
+fake.fake_shapes.restype = C.c_char_p
+cfg = dataclasses.replace(PRESETS["tiny-llama"], num_attention_heads={heads}, num_key_value_heads={kv_heads}, head_dim={hd}, num_hidden_layers=1)
+c = api.Context(0)
+model = api.CudaModel(c, cfg, synth_checkpoint(cfg, seed=0), max_step_tokens=64, max_step_seqs=1)
+pool = api.PagedKv(c, model.kv_spec(64, 16))
+p = api._PackedStep(api.StepBatch(np.zeros({rows}, dtype=np.uint32), [api.SeqStep({rows}, {offset}, 0, list(range(64)))]))
+logits, n = C.c_void_p(), C.c_int32()
+fake.fake_reset()
+ok(L.lib().kc_forward_step(model._h, pool._h, p.ids_p, p.n, p.seq_arr, p.n_seqs, 0, C.byref(logits), C.byref(n)))
+threads = [s.split(":")[0] for s in fake.fake_shapes().decode().split()]
+assert [t for t in threads if t in ("384", "768")] == ["{threads}"], threads
+""", first="import torch")
