@@ -368,11 +368,12 @@ add_rmsnorm_reg_kernel(const bf16* __restrict__ x, RowSource y, const bf16* __re
 // sin/cos of the token's angles are computed once per CTA and shared by its heads, before the wait for the kernel ahead (the
 // step's metadata is older than its first kernel; a single call's is not, see launch_rope_kv_write); every thread then moves
 // 8 consecutive features of each half with 16-byte loads and stores. A token's work items lie over CTAs of 128 threads, one
-// a thread: what bounds it is one item's chain of loads. Up to 256 items are one CTA's: two would compute sin/cos twice and
-// gain no round. Time that it adds to a step, all of a token's items in one CTA of 256 threads and sin/cos behind the wait ->
+// a thread: what bounds it is one item's chain of loads. Up to 256 items are one CTA's of 256 threads: two of 128 would compute
+// sin/cos twice and gain no round, and smaller ones let the kernels around it in at worse times. Time that it adds to a step, all of a token's items in one CTA of 256 threads and sin/cos behind the wait ->
 // this: one token 6.2 -> 3.5 us, 192 tokens of three partials 5.8 -> 4.8, 320 of four 12.7 -> 5.9. A layer of the 1B model (192
-// items), CTAs of 128 -> one of 192: 385 tokens 133.5 -> 131.0 us, 500 135.5 -> 136.4, one 39.3 -> 39.1; with 384 to 640 items
-// CTAs of up to 256 threads made no difference beyond 1 % either way.
+// items), CTAs of 128, one of 192, one of 256 threads: 385 tokens 133.5, 130.9, 129.5 us, 500 135.5, 136.8, 135.2, 120 61.6,
+// 62.0, 61.1, 16 sequences of 12 tokens after 2000 106, 108, 105. With 384 to 640 items CTAs of up to 256 threads made no
+// difference beyond 1 % either way.
 constexpr int ROPE_THREADS = 128, ROPE_ONE_CTA = 256;
 __global__ void __launch_bounds__(ROPE_ONE_CTA)
 rope_kv_write_kernel(RowSource qkv, const bf16* __restrict__ bias, const float* __restrict__ inv_freq,
@@ -583,7 +584,7 @@ cudaError_t launch_rope_kv_write(const SublayerOut& qkv, const bf16* bias, const
                                  int NB, int BS, bf16* pool, bf16* q_out, cudaStream_t s, bool in_order) {
   if (D % 16 || D > 256) return cudaErrorInvalidValue;
   const int items = (Hq + 2 * Hkv) * (D / 16);
-  const int threads = items <= ROPE_ONE_CTA ? (std::max(items, D / 2) + 31) & ~31 : ROPE_THREADS;   // D / 2 pairs of sin and cos
+  const int threads = items <= ROPE_ONE_CTA ? ROPE_ONE_CTA : ROPE_THREADS;
   return launch_k_opt(!in_order, rope_kv_write_kernel, dim3(n, (items + threads - 1) / threads), dim3(threads), 0, s, row_source(qkv), bias, inv_freq, token_pos, kv_slot, Hq, Hkv, D,
                   traditional, layer, NB, BS, pool, q_out);
 }

@@ -235,9 +235,9 @@ assert grids[:2] == ["{qkv}", "{o}"], grids
 """, first="import torch")   # before the library, whose NCCL is another one
 
 
-@pytest.mark.parametrize("heads,kv_heads,hd,shape", [(4, 2, 64, "32:3x1x1"), (32, 8, 64, "192:3x1x1"), (16, 8, 64, "128:3x1x1"), (32, 8, 128, "128:3x3x1"), (16, 8, 256, "128:3x4x1"), (64, 8, 64, "128:3x3x1")])
+@pytest.mark.parametrize("heads,kv_heads,hd,shape", [(4, 2, 64, "256:3x1x1"), (32, 8, 64, "256:3x1x1"), (48, 8, 64, "256:3x1x1"), (4, 4, 128, "256:3x1x1"), (32, 8, 128, "128:3x3x1"), (16, 8, 256, "128:3x4x1"), (64, 8, 64, "128:3x3x1")])
 def test_rope_items_of_a_token(fake, heads, kv_heads, hd, shape):
-    """Up to 256 work items of a token are one block's, more are blocks of 128."""
+    """Up to 256 work items of a token are one block's of 256 threads, more are blocks of 128."""
     run(fake, f"""
 fake.fake_shapes.restype = C.c_char_p
 pool = C.c_void_p()
