@@ -76,6 +76,9 @@ struct kc_ctx {
   uint32_t* status = nullptr;             // the device's address of it
   volatile uint32_t* status_host = nullptr;
   kc_model* op = nullptr;                 // metadata and workspace of the single-op entry points (op_shell)
+  // What the teams of a GEMM leave for one another (QLinearLaunch::fix): made with the first weight that needs it, shared by the
+  // context's launches, which run one after the other on its stream, and given back with the context.
+  float* gemm_fix = nullptr;
   ncclComm_t comm = nullptr;
   int tp_rank = 0, tp_world = 1;
   // launch accounting and optional per-class timing (kc_profile_*)
@@ -168,7 +171,7 @@ struct kc_model {
   int F = 0;                           // local intermediate size
   bool stream_lane = false;            // forwards of at most QL_STREAM_MAX_M rows take the weight-streaming kernels
   size_t stream_min_bytes = QL_STREAM_MIN_BYTES;   // ... for weights of at least this many bytes of records
-  bool glu_interleaved = false;        // gate_up rows alternate gate / up in blocks of 128 (so the GEMM can fuse the activation)
+  bool glu_interleaved = false;        // gate_up's rows are 16 gate and 16 up rows in turn (so that the GEMM can fuse the activation)
   int n_qkv = 0;
   std::vector<Layer> layers;
   // embedding table in mlx layout (gather) and the head as GEMM records
@@ -294,11 +297,26 @@ extern "C" void kc_ctx_destroy(kc_ctx_t c) {
   cudaEventDestroy(c->step_a);
   cudaEventDestroy(c->step_b);
   if (c->comm) ncclCommDestroy(c->comm);
+  cudaFree(c->gemm_fix);
   free_op_shell(c);
   cudaFreeHost((void*)c->status_host);
   cudaStreamDestroy(c->stream);
   delete c;
   g_live--;
+}
+
+// A launch that gave up may have left in it what the next one would take for its own.
+static void clear_gemm_fix(kc_ctx* c) {
+  if (c->gemm_fix) cudaMemsetAsync(c->gemm_fix, 0xFF, qlinear_fix_bytes(c->sm_count), c->stream);
+}
+// The workspace, with the first weight that has a use for it: a team's share is a pair of tiles at least.
+static int ensure_gemm_fix(kc_ctx* c, const QWeight& w) {
+  if (w.n_tiles < c->sm_count || c->gemm_fix) return KC_OK;
+  const size_t bytes = qlinear_fix_bytes(c->sm_count);
+  cudaError_t e = cudaMalloc(&c->gemm_fix, bytes);
+  if (e != cudaSuccess) { c->gemm_fix = nullptr; return fail(KC_ERR_OOM, "GEMM workspace of %zu bytes: %s", bytes, cudaGetErrorString(e)); }
+  clear_gemm_fix(c);
+  return KC_OK;
 }
 
 // Read after a synchronisation. A bounded wait that gave up never passes as success: every entry point that
@@ -307,6 +325,7 @@ static int status_verdict(kc_ctx* c, const char* where) {
   const uint32_t st = *c->status_host;
   if (!st) return KC_OK;
   *c->status_host = 0;
+  clear_gemm_fix(c);
   return fail(KC_ERR_TIMEOUT, "%s: device status 0x%x: a bounded wait gave up (kernel 0x%x, wait %u); the results of the "
               "calls since the last synchronisation are not valid", where, st, st & 0xff00u, st & 0xffu);
 }
@@ -488,6 +507,7 @@ static int run_qlinear(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, 
     QLinearLaunch l;
     l.w = &w; l.x = &x; l.row0 = row0; l.M = rows;
     l.y = y; l.ldy = ldy; l.partial = partial; l.summed = summed; l.status = c->status;
+    l.fix = c->gemm_fix;
     LAUNCH(c, KC_PROF_GEMM, 1, qlinear_umma(l, c->stream));
     if (w.splits > 1 && !defer && !qlinear_in_turn(w, l.M, summed))
       LAUNCH(c, KC_PROF_GEMM_REDUCE, 1, qlinear_reduce_splits(partial, w.splits, l.M, w.N, y + (size_t)row0 * ldy, ldy, c->stream));
@@ -496,9 +516,9 @@ static int run_qlinear(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, 
   return KC_OK;
 }
 
-// act[M, F] = activation(x . Wgate^T) * (x . Wup^T) for a gate_up weight whose tiles alternate gate / up. Row slabs
-// whose GEMM launch owns whole tile pairs get the activation in the GEMM's epilogue; the others write the
-// interleaved [M, 2F] product and run the element-wise kernel on it. Both ways round at the same points.
+// act[M, F] = activation(x . Wgate^T) * (x . Wup^T) for a gate_up weight whose rows are 16 gate and 16 up rows in turn. A weight
+// that is not split along K gets the activation in the GEMM's epilogue; the others write the interleaved [M, 2F] product and
+// run the element-wise kernel on it. Both ways round at the same points.
 static int run_gated(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, bf16* gu, int F, int gelu, bool interleaved,
                      bf16* act, float* partial) {
   for (int row0 = 0, rows; row0 < M; row0 += rows) {
@@ -507,6 +527,7 @@ static int run_gated(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, bf
     QLinearLaunch l;
     l.w = &w; l.x = &x; l.row0 = row0; l.M = rows;
     l.y = gu; l.ldy = 2 * F; l.partial = partial; l.status = c->status;
+    l.fix = c->gemm_fix;
     if (interleaved) { l.glu = gelu ? 2 : 1; l.act = act; l.ld_act = F; l.glu_done = &done; }
     LAUNCH(c, KC_PROF_GEMM, 1, qlinear_umma(l, c->stream));
     if (done) continue;
@@ -583,6 +604,7 @@ extern "C" int kc_qweight_create(kc_ctx_t c, const uint32_t* w, const void* scal
   cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = qweight_finish(&q->w);
   cudaFree(dw); cudaFree(ds); cudaFree(db);
+  if (e == cudaSuccess && (rc = ensure_gemm_fix(c, q->w))) { cudaFree(q->partial); qweight_free(&q->w); delete q; return rc; }
   if (e != cudaSuccess) { qweight_free(&q->w); delete q; return fail(KC_ERR_CUDA, "kc_qweight_create: %s", cudaGetErrorString(e)); }
   g_live++;
   *out = q;
@@ -677,9 +699,9 @@ int copy_slice(kc_ctx* c, const kc_tensor_view* t, size_t row_bytes, int64_t r0,
 
 struct Part { std::string prefix; int64_t r0, r1; };  // one source linear and the output rows taken from it
 
-// Builds one QWeight from the row-concatenation of `parts`, taking input columns [k0, k1).
+// Builds one QWeight from the row-concatenation of `parts`, taking input columns [k0, k1); alternate: see qweight_build.
 int build_linear(kc_model* m, TensorIndex& idx, const std::vector<Part>& parts, int K_full, int k0, int k1, QWeight* out,
-                 bf16** bias_out) {
+                 bf16** bias_out, bool alternate = false) {
   kc_ctx* c = m->ctx;
   const int bits = m->d.bits, group = m->d.group_size;
   const int K = k1 - k0;
@@ -729,13 +751,13 @@ int build_linear(kc_model* m, TensorIndex& idx, const std::vector<Part>& parts, 
     *bias_out = dbias;
   }
   cudaError_t e = qweight_build(out, (const uint32_t*)dw, (const bf16*)ds, (const bf16*)db, (int)N, K, bits, group,
-                                c->sm_count, c->stream);
+                                c->sm_count, c->stream, alternate);
   cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = qweight_finish(out);
   cudaFree(dw); cudaFree(ds); cudaFree(db);
   if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? KC_ERR_OOM : KC_ERR_CUDA, "re-tiling %s: %s", parts[0].prefix.c_str(), cudaGetErrorString(e));
   m->weight_bytes += (int64_t)out->mlx_bytes();
-  return KC_OK;
+  return ensure_gemm_fix(c, *out);
 }
 
 // Norm weight [H] bf16; Gemma's 1 + w is folded in at load (NormStyle::OnePlus, nn.rs:241-257).
@@ -897,17 +919,9 @@ extern "C" int kc_model_load(kc_ctx_t c, const kc_model_desc* desc, const kc_ten
     {
       // gate and up rows alternate in blocks of one GEMM tile (128 rows) when the width allows it, so a CTA that owns
       // two neighbouring tiles holds gate and up of the same features
-      std::vector<Part> gu_parts;
-      m->glu_interleaved = m->F % 128 == 0;
-      if (m->glu_interleaved) {
-        for (int64_t r = f0; r < f1; r += 128) {
-          gu_parts.push_back({p + ".mlp.gate_proj", r, r + 128});
-          gu_parts.push_back({p + ".mlp.up_proj", r, r + 128});
-        }
-      } else {
-        gu_parts = {{p + ".mlp.gate_proj", f0, f1}, {p + ".mlp.up_proj", f0, f1}};
-      }
-      LOAD_FAIL(build_linear(m, idx, gu_parts, H, 0, H, &L.gate_up, nullptr));
+      m->glu_interleaved = m->F % 64 == 0;
+      const std::vector<Part> gu_parts = {{p + ".mlp.gate_proj", f0, f1}, {p + ".mlp.up_proj", f0, f1}};
+      LOAD_FAIL(build_linear(m, idx, gu_parts, H, 0, H, &L.gate_up, nullptr, m->glu_interleaved));
     }
     LOAD_FAIL(build_linear(m, idx, {{p + ".mlp.down_proj", 0, H}}, d.intermediate_size, (int)f0, (int)f1, &L.down, nullptr));
     LOAD_FAIL(load_norm(m, idx, p + ".input_layernorm.weight", gemma, &L.input_ln));
@@ -1638,6 +1652,7 @@ extern "C" int kc_decode_collect(kc_model_t m, uint64_t ticket, uint32_t* row_to
   const uint32_t st = m->pipe_host[slot][m->max_seqs];
   if (st) {
     CK(cudaMemsetAsync(c->status, 0, sizeof(uint32_t), c->stream));
+    clear_gemm_fix(c);
     return fail(KC_ERR_TIMEOUT, "kc_decode_collect: device status 0x%x: a bounded wait gave up (kernel 0x%x, wait %u); the tokens of "
                 "this launch and of any launch fed from it are not valid", st, st & 0xff00u, st & 0xffu);
   }

@@ -352,7 +352,7 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
           if (capped) {
             mul = cap_log2;
             const bool seen = !edge || (hi >= 0 && lo < TK && lo <= hi);   // any key: a score of -inf is a key of weight e^-cap
-            if (seen) { tmax *= cap_arg; tmax = softcap_any(tmax, softcap_near(make_float2(tmax, tmax)).x); }   // grows with the score
+            if (seen) { tmax *= cap_arg; tmax = tanh_any(tmax, tanh_near(make_float2(tmax, tmax)).x); }   // grows with the score
           }
           tmax *= mul;
           float alpha = 1.f;
@@ -373,20 +373,20 @@ attn_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constant__ C
 #pragma unroll
               for (int j = 0; j < 32; j += 2) { b0 = fmaxf(b0, fabsf(__uint_as_float(v[j]))); b1 = fmaxf(b1, fabsf(__uint_as_float(v[j + 1]))); }
               // columns that hold an older tile's scores and rows past the unit's have no say but in the time it takes
-              const bool all_near = __all_sync(0xffffffffu, fmaxf(b0, b1) * cap_arg < SOFTCAP_NEAR || row >= u.rows);
+              const bool all_near = __all_sync(0xffffffffu, fmaxf(b0, b1) * cap_arg < TANH_NEAR || row >= u.rows);
               const float2 arg = make_float2(cap_arg, cap_arg);
               if (all_near) {
 #pragma unroll
                 for (int j = 0; j < 32; j += 2) {
-                  const float2 r = softcap_near(mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg));
+                  const float2 r = tanh_near(mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg));
                   v[j] = __float_as_uint(r.x); v[j + 1] = __float_as_uint(r.y);
                 }
               } else {
 #pragma unroll
                 for (int j = 0; j < 32; j += 2) {
                   const float2 y = mul2(make_float2(__uint_as_float(v[j]), __uint_as_float(v[j + 1])), arg);
-                  const float2 r = softcap_near(y);
-                  v[j] = __float_as_uint(softcap_any(y.x, r.x)); v[j + 1] = __float_as_uint(softcap_any(y.y, r.y));
+                  const float2 r = tanh_near(y);
+                  v[j] = __float_as_uint(tanh_any(y.x, r.x)); v[j + 1] = __float_as_uint(tanh_any(y.y, r.y));
                 }
               }
             }

@@ -7,60 +7,6 @@
 
 namespace kc {
 
-__device__ __forceinline__ float ex2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Two fp32 operations an instruction.
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
-      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return r;
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 r;
-  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
-      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return r;
-}
-
-// tanh(y) for |y| < SOFTCAP_NEAR: y + y^3 p(y^2), p fitted for the smallest largest relative error; 1.0e-7 at most, 3.5e-8
-// root mean square. No special-function operation.
-constexpr float SOFTCAP_NEAR = 0.75f;
-__device__ __forceinline__ float2 softcap_near(float2 y) {
-  auto both = [](float x) { return make_float2(x, x); };
-  const float2 z = mul2(y, y);
-  float2 p = fma2(z, both(-0.0047694784589f), both(0.0196648966521f));
-  p = fma2(p, z, both(-0.0533902496099f));
-  p = fma2(p, z, both(0.1332652121782f));
-  p = fma2(p, z, both(-0.3333306908607f));
-  return fma2(mul2(y, z), p, y);
-}
-// tanh(y) anywhere: further out (1 - u) / (1 + u) with u = e^(-2 |y|), 1.7e-7 at most; 1 and -1 at the infinities, NaN stays
-// NaN. Nowhere less exact than tanhf, which is up to 2.0e-7 off.
-__device__ __forceinline__ float softcap_any(float y, float near) {
-  const float u = ex2(fabsf(y) * -2.8853900817779268f), d = u + 1.f;
-  float r = rcp_approx(d);
-  r = __fmaf_rn(r, __fmaf_rn(-d, r, 1.f), r);
-  const float far = copysignf(__fmaf_rn(-2.f * u, r, 1.f), y);
-  return fabsf(y) < SOFTCAP_NEAR ? near : far;
-}
-
 // Adds a chunk (o scaled by 2^-m, sum l) to what a row has accumulated: the weights of one merge.
 struct MergeW { float a, b, m; };
 __device__ __forceinline__ MergeW merge_weights(float m_acc, float m_chunk) {

@@ -394,7 +394,7 @@ attn_keys_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constan
         if (MODE == CAPPED) {
           const int hi = pos - key0, lo = p.window > 0 ? pos - p.window - key0 + 1 : -key0;
           const bool seen = !edge || (hi >= 0 && lo < TK && lo <= hi);   // any key: a score of -inf is a key of weight e^-cap
-          if (seen) { tmax *= cap_arg; tmax = softcap_any(tmax, softcap_near(make_float2(tmax, tmax)).x); }   // grows with the score
+          if (seen) { tmax *= cap_arg; tmax = tanh_any(tmax, tanh_near(make_float2(tmax, tmax)).x); }   // grows with the score
         }
         tmax *= mul;
         alpha = 1.f;
@@ -443,19 +443,19 @@ attn_keys_kernel(const __grid_constant__ CUtensorMap kvmap, const __grid_constan
               for (int j = 0; j < 8; j += 2) { b0 = fmaxf(b0, fabsf(v[j])); b1 = fmaxf(b1, fabsf(v[j + 1])); }
               // no score past 0.75 caps: the polynomial alone (an element's value is the same on both sides). Keys past the
               // sequence have no say.
-              const bool all_near = __all_sync(0xffffffffu, fmaxf(b0, b1) * cap_arg < SOFTCAP_NEAR || key > u.pos_max);
+              const bool all_near = __all_sync(0xffffffffu, fmaxf(b0, b1) * cap_arg < TANH_NEAR || key > u.pos_max);
               const float2 arg = make_float2(cap_arg, cap_arg);
               if (all_near) {
 #pragma unroll
                 for (int j = 0; j < 8; j += 2) {
-                  const float2 t = softcap_near(mul2(make_float2(v[j], v[j + 1]), arg));
+                  const float2 t = tanh_near(mul2(make_float2(v[j], v[j + 1]), arg));
                   v[j] = t.x; v[j + 1] = t.y;
                 }
               } else {
 #pragma unroll
                 for (int j = 0; j < 8; j += 2) {
-                  const float2 y = mul2(make_float2(v[j], v[j + 1]), arg), t = softcap_near(y);
-                  v[j] = softcap_any(y.x, t.x); v[j + 1] = softcap_any(y.y, t.y);
+                  const float2 y = mul2(make_float2(v[j], v[j + 1]), arg), t = tanh_near(y);
+                  v[j] = tanh_any(y.x, t.x); v[j + 1] = tanh_any(y.y, t.y);
                 }
               }
             }

@@ -50,48 +50,52 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 
-// ---- mbarrier ----------------------------------------------------------
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
+// ---- mbarrier: by shared address, or by pointer --------------------------
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) { mbar_init(smem_u32(bar), count); }
 __device__ __forceinline__ void mbar_fence_init() {
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) { mbar_arrive(smem_u32(bar)); }
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
                "r"(bytes)
                : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) { mbar_arrive_expect_tx(smem_u32(bar), bytes); }
 // One try_wait: the thread may be suspended by the hardware until the phase completes or the hinted time
 // (nanoseconds) has passed, so a waiting warp does not burn issue slots spinning.
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity), "r"(20000u)
+      : "r"(bar), "r"(parity), "r"(20000u)
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
+      : "r"(bar), "r"(parity)
       : "memory");
   return ok != 0;
 }
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) { return mbar_test_wait(smem_u32(bar), parity); }
 // Bounded wait. On timeout: ORs `code` into *status (if non-null) and returns
 // false; the caller must then leave its pipeline loop.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* status,
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t* status,
                                           uint32_t code) {
   if (mbar_try_wait(bar, parity)) return true;
   const unsigned long long t0 = globaltimer_ns();
@@ -106,6 +110,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   }
   return true;
 }
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t* status, uint32_t code) {
+  return mbar_wait(smem_u32(bar), parity, status, code);
+}
 
 // ---- async-proxy fences, bulk copies (TMA) --------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {
@@ -114,13 +121,15 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 
 // 1-D bulk copy global -> shared, completion counted on an mbarrier.
 // Both addresses 16-byte aligned, bytes a multiple of 16.
-__device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gsrc, uint32_t bytes,
-                                         uint64_t* bar) {
+__device__ __forceinline__ void bulk_g2s(uint32_t smem_dst, const void* gsrc, uint32_t bytes, uint32_t bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-          "r"(smem_u32(smem_dst)),
-      "l"(gsrc), "r"(bytes), "r"(smem_u32(bar))
+          "r"(smem_dst),
+      "l"(gsrc), "r"(bytes), "r"(bar)
       : "memory");
+}
+__device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gsrc, uint32_t bytes, uint64_t* bar) {
+  bulk_g2s(smem_u32(smem_dst), gsrc, bytes, smem_u32(bar));
 }
 
 // 2-D tiled TMA load (no multicast): coordinates {x = innermost, y}.
@@ -224,20 +233,111 @@ inline cudaError_t launch_k(void (*kernel)(KArgs...), dim3 grid, dim3 block, siz
   return launch_k_opt(true, kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
+// In clusters of `cluster` CTAs along x.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_k_cluster(int cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// Two fp32 operations an instruction.
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\t"
+      "fma.rn.f32x2 x, x, y, z;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 r;
+  asm("{\n\t.reg .b64 x, y;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 x, x, y;\n\tmov.b64 {%0, %1}, x;\n\t}"
+      : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return r;
+}
+
+// tanh(y) for |y| < TANH_NEAR: y + y^3 p(y^2), p fitted for the smallest largest relative error; 1.0e-7 at most, 3.5e-8
+// root mean square. No special-function operation.
+constexpr float TANH_NEAR = 0.75f;
+__device__ __forceinline__ float2 tanh_near(float2 y) {
+  auto both = [](float x) { return make_float2(x, x); };
+  const float2 z = mul2(y, y);
+  float2 p = fma2(z, both(-0.0047694784589f), both(0.0196648966521f));
+  p = fma2(p, z, both(-0.0533902496099f));
+  p = fma2(p, z, both(0.1332652121782f));
+  p = fma2(p, z, both(-0.3333306908607f));
+  return fma2(mul2(y, z), p, y);
+}
+// tanh(y) anywhere: further out (1 - u) / (1 + u) with u = e^(-2 |y|), 1.7e-7 at most; 1 and -1 at the infinities, NaN stays
+// NaN. Nowhere less exact than tanhf, which is up to 2.0e-7 off.
+__device__ __forceinline__ float tanh_any(float y, float near) {
+  const float u = ex2(fabsf(y) * -2.8853900817779268f), d = u + 1.f;
+  float r = rcp_approx(d);
+  r = __fmaf_rn(r, __fmaf_rn(-d, r, 1.f), r);
+  const float far = copysignf(__fmaf_rn(-2.f * u, r, 1.f), y);
+  return fabsf(y) < TANH_NEAR ? near : far;
+}
+
 // Mlp::forward activation (nn.rs:284-294): silu(gate) * up with the three bf16 roundings of the composed ops, or
 // gelu_approx(gate) * up op for op (nn.rs:221-235). g and u are bf16 values held in fp32; so is the result.
+// 1 / (1 + e^-g), the reciprocal by the hardware's estimate and one step of Newton's iteration, r + r (1 - d r): within 0.501 units
+// of fp32's last place of the quotient, which is what a division gives, and without a division's branches, which cost a warp 100
+// cycles each where others compute. An infinite denominator is a zero.
+__device__ __forceinline__ float act_sigmoid(float g) {
+  const float d = 1.f + __expf(-g), r = rcp_approx(d), n = fmaf(r, fmaf(-d, r, 1.f), r);
+  return d > 1e37f ? r : n;
+}
 __device__ __forceinline__ float act_silu_mul(float g, float u) {
-  const float s = bf16_round(1.f / (1.f + __expf(-g)));
+  const float s = bf16_round(act_sigmoid(g));
   const float t = bf16_round(g * s);
   return bf16_round(t * u);
 }
-__device__ __forceinline__ float act_gelu_mul(float g, float u) {
+__device__ __forceinline__ float gelu_scaled(float g) {
   const float cube = bf16_round(g * g * g);  // power(x, 3) in fp32, rounded once
   const float inner = bf16_round(g + bf16_round(bf16_round(0.044715f) * cube));
-  const float scaled = bf16_round(bf16_round(0.7978845608028654f) * inner);
-  const float gate = bf16_round(1.f + bf16_round(tanhf(scaled)));
-  const float act = bf16_round(bf16_round(0.5f * g) * gate);
-  return bf16_round(act * u);
+  return bf16_round(bf16_round(0.7978845608028654f) * inner);
+}
+__device__ __forceinline__ float2 act_gelu_mul(float2 g, float2 u) {
+  const float2 y = make_float2(gelu_scaled(g.x), gelu_scaled(g.y)), near = tanh_near(y);   // no branch, as in act_sigmoid
+  const float gx = bf16_round(1.f + bf16_round(tanh_any(y.x, near.x))), gy = bf16_round(1.f + bf16_round(tanh_any(y.y, near.y)));
+  return make_float2(bf16_round(bf16_round(bf16_round(0.5f * g.x) * gx) * u.x), bf16_round(bf16_round(bf16_round(0.5f * g.y) * gy) * u.y));
+}
+__device__ __forceinline__ float act_gelu_mul(float g, float u) { return act_gelu_mul(make_float2(g, g), make_float2(u, u)).x; }
+
+// Two of them at once, bf16 pairs in and out: a product of two bf16 numbers rounded to bf16 is what a multiplication of bf16 gives.
+__device__ __forceinline__ uint32_t act_pair(uint32_t gate, uint32_t up, bool gelu) {
+  const float2 g = unpack_bf162(gate);
+  if (gelu) {
+    const float2 a = act_gelu_mul(g, unpack_bf162(up));
+    return pack_bf162(a.x, a.y);
+  }
+  const uint32_t s = pack_bf162(act_sigmoid(g.x), act_sigmoid(g.y));
+  const bf162 t = __hmul2(*reinterpret_cast<const bf162*>(&gate), *reinterpret_cast<const bf162*>(&s));
+  const bf162 r = __hmul2(t, *reinterpret_cast<const bf162*>(&up));
+  return *reinterpret_cast<const uint32_t*>(&r);
 }
 
 // A ring position: stage index and phase bit, advanced without division.

@@ -446,8 +446,8 @@ rope_kv_write_kernel(RowSource qkv, const bf16* __restrict__ bias, const float* 
 // roundings of the composed ops, or gelu_approx(gate) * up op for op (nn.rs:221-235).
 // gu: [n, 2F] (gate | up)
 // ---------------------------------------------------------------------------
-// interleaved: gate and up features alternate in blocks of 128 columns (gate block j at columns 256 j, up block j at
-// 256 j + 128) instead of all gate columns followed by all up columns.
+// interleaved: gate and up features alternate in blocks of 16 columns (gate block j at columns 32 j, up block j at
+// 32 j + 16) instead of all gate columns followed by all up columns.
 __global__ void __launch_bounds__(256) glu_kernel(const bf16* __restrict__ gu, int n, int F, int gelu, int interleaved, bf16* __restrict__ out) {
   pdl_launch_dependents();
   pdl_wait();
@@ -455,8 +455,8 @@ __global__ void __launch_bounds__(256) glu_kernel(const bf16* __restrict__ gu, i
   const int total = n * per_row;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const int row = i / per_row, col = (i - row * per_row) * 8;
-    const int gcol = interleaved ? (col >> 7) * 256 + (col & 127) : col;
-    const int ucol = interleaved ? gcol + 128 : F + col;
+    const int gcol = interleaved ? (col >> 4) * 32 + (col & 15) : col;
+    const int ucol = interleaved ? gcol + 16 : F + col;
     float g[8], u[8];
     load8_bf16(gu + (size_t)row * 2 * F + gcol, g);
     load8_bf16(gu + (size_t)row * 2 * F + ucol, u);
@@ -474,8 +474,8 @@ __global__ void __launch_bounds__(256) glu_from_kernel(const RowSource gu, int n
   const int total = n * per_row;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     const int row = i / per_row, col = (i - row * per_row) * 8;
-    const int gcol = interleaved ? (col >> 7) * 256 + (col & 127) : col;
-    const int ucol = interleaved ? gcol + 128 : F + col;
+    const int gcol = interleaved ? (col >> 4) * 32 + (col & 15) : col;
+    const int ucol = interleaved ? gcol + 16 : F + col;
     float g[8], u[8];
     load8(gu, (size_t)row, gcol, g);
     load8(gu, (size_t)row, ucol, u);
@@ -590,7 +590,7 @@ cudaError_t launch_rope_kv_write(const SublayerOut& qkv, const bf16* bias, const
 }
 
 cudaError_t launch_glu(const bf16* gu, int n, int F, int gelu, int interleaved, bf16* out, cudaStream_t s) {
-  if (F % 8 || (interleaved && F % 128)) return cudaErrorInvalidValue;
+  if (F % 8 || (interleaved && F % 16)) return cudaErrorInvalidValue;
   const long long total = (long long)n * (F / 8);
   const int blocks = (int)std::min<long long>((total + 255) / 256, 148LL * 8);
   return launch_k(glu_kernel, dim3(blocks), dim3(256), 0, s, gu, n, F, gelu, interleaved, out);
@@ -613,7 +613,7 @@ cudaError_t launch_tp_reduce_slice(const bf16* const* peer_y, int world, int ran
 
 cudaError_t launch_glu_from(const SublayerOut& gu, int n, int F, int gelu, int interleaved, bf16* out, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  if (F % 8 || (interleaved && F % 128) || gu.ld != 2 * F) return cudaErrorInvalidValue;
+  if (F % 8 || (interleaved && F % 16) || gu.ld != 2 * F) return cudaErrorInvalidValue;
   const int total = n * (F / 8);
   const int blocks = std::max(1, std::min((total + 255) / 256, 148 * 8));
   return launch_k(glu_from_kernel, dim3(blocks), dim3(256), 0, s, row_source(gu), n, F, gelu, interleaved, out);

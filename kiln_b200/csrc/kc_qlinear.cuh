@@ -41,8 +41,8 @@ struct QWeight {
   uint32_t record_bytes = 0;
   int splits = 1;              // fixed function of (N, K): never of M
   int sm_count = 148;
-  int* wide = nullptr;         // device flag of the re-tiling (inside the records' allocation)
-  int wide_scale = 0;          // its value, read once at load: a scale is too large for the conversion-free dequantisation
+  int* top = nullptr;          // the re-tiling's largest exponent of a scale (inside the records' allocation)
+  int shift = 0;               // from it, read once at load: the GEMM takes the weights times 2^-shift
   size_t bytes() const { return (size_t)((n_tiles + QL_TILE_GROUP - 1) / QL_TILE_GROUP) * QL_TILE_GROUP * kblocks * record_bytes; }
   // Algorithmic bytes of the mlx tensors this weight was built from.
   size_t mlx_bytes() const { return (size_t)N * K * bits / 8 + (size_t)2 * N * (K / group) * 2; }
@@ -68,31 +68,42 @@ struct QLinearLaunch {
   int ldy;
   float* partial;   // [splits][M][N] fp32 workspace when splits > 1 (rows relative to row0)
   bool summed = false;   // partials, if there are any, are summed by the kernel that reads the result, not by one of their own
+  // Workspace of qlinear_fix_bytes for what teams that share a weight's k-blocks leave for one another, all its bits set between
+  // launches; without it they share whole pairs of tiles. Launches that have the same one run one after the other.
+  float* fix = nullptr;
   uint32_t* status; // device status word
-  // Optional fused gated activation for a weight whose 128-row tiles alternate gate / up (tile 2j = gate features
-  // 128 j.., tile 2j + 1 = the matching up features): glu = 1 (silu) or 2 (gelu_approx) asks the epilogue to write
-  // act[M, N / 2] = activation(gate) * up instead of y. Honoured only when one CTA owns whole gate/up tile pairs and
-  // K is not split; *glu_done then is set to 1, otherwise y is written as usual and *glu_done is 0.
+  // Optional fused gated activation for a weight whose rows are 16 gate and 16 up rows in turn: glu = 1 (silu) or 2 (gelu_approx)
+  // asks the kernel to write act[M, N / 2] = activation(gate) * up instead of y. Honoured only when K is not split
+  // (QWeight::splits) and the last tile is whole; *glu_done then is set to 1, otherwise y is written as usual and *glu_done is 0.
   int glu = 0;
   bf16* act = nullptr;
   int ld_act = 0;
   int* glu_done = nullptr;
 };
 
+constexpr int QL_CHUNK_ROWS = 192;   // rows of a chunk, at most: two accumulators of them and four slots of dequantised weights are tensor memory's 512 columns
+constexpr int QL_SOLO_ROWS = 64;     // up to these rows the CTAs of a team read the activations each for itself
+constexpr int QL_FIX_CHUNKS = 3;     // chunks of rows that a launch of cut pairs keeps parts' sums for
+size_t qlinear_fix_bytes(int sm_count);
+
 // Fixed split-K plan: a function of the weight's shape only, so a row's
 // accumulation order never depends on how many rows ride the step.
 int qlinear_plan_splits(int n_tiles, int kblocks, int sm_count);
 
 // Re-tile on the device. w/scales/biases are device pointers in mlx layout.
-// The caller reads the weight's flag with qweight_finish once the stream has run.
+// alternate: the first N / 2 rows are the gate's, the others the up projection's, and the weight's rows are 16 of each in turn.
+// The caller completes the weight with qweight_finish once the stream has run.
 cudaError_t qweight_build(QWeight* out, const uint32_t* w, const bf16* scales, const bf16* biases,
-                          int N, int K, int bits, int group, int sm_count, cudaStream_t s);
+                          int N, int K, int bits, int group, int sm_count, cudaStream_t s, bool alternate = false);
 cudaError_t qweight_finish(QWeight* w);
 void qweight_free(QWeight* w);
 
 // Creates the tensor maps of an activation buffer. Returns false (and sets
 // *err) if the driver entry point is unavailable or rejects the geometry.
 bool act_operand_init(ActOperand* op, const bf16* ptr, int rows, int K, const char** err);
+
+// The map whose box covers `rows` rows (<= 256); null if the driver refuses it.
+const CUtensorMap* act_operand_rows_map(const ActOperand* op, int rows);
 
 // The GEMM (tcgen05 + TMEM + TMA). Returns a CUDA error. One launch of at most qlinear_slab_rows rows.
 cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s);

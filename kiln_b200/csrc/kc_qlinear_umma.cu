@@ -1,0 +1,822 @@
+// The affine-dequant GEMM on the tensor cores. See kc_qlinear.cuh for the data layout.
+//
+// qlinear_umma_kernel — teams of two CTAs. A team has a PAIR of neighbouring 128-row weight tiles at a time, one tile a CTA,
+// and the same k-blocks of both. Up to 64 activation rows its CTAs know nothing of each other; with more they are a cluster
+// whose two SMs work on one M = 256 product (tcgen05 cta_group::2), each holding half of the activations. 20 warps:
+//   warp 0        bulk-copies the weight records (cp.async.bulk, mbarrier tx)
+//   warp 1        TMA-loads the activation k-blocks (cp.async.bulk.tensor, 128B swizzle), of a cluster its CTA's half of the rows
+//   warp 2        allocates TMEM; issues tcgen05.mma (weights = A/M side from TENSOR MEMORY, activations = B/N side from shared
+//                 memory), of a cluster the first CTA's for both
+//   warps 4-19    four groups of four warps. Dequantisers unpack the 4/8-bit words, apply scale and bias in registers and write
+//                 the bf16 A operand into tensor memory (tcgen05.st); of a cluster the first group drains accumulators
+//                 (tcgen05.ld) under the next task's products instead.
+// The accumulator D[n, m] lives in TMEM: lane = weight row n, column = activation row m.
+//
+// Every output element depends only on its own activation row and on an order of sums fixed by (N, K) and the SM count: a
+// pair's k-blocks are cut into parts at fixed places, a part is one chain of products, and the parts are added in order. That
+// is what lets verify rows share a step with other rows and still reproduce the bits of a one-row decode. More rows than one
+// accumulator holds are chunks of rows: rows are independent, so no bit changes.
+#include "kc_qlinear.cuh"
+#include "kc_umma.cuh"
+
+#include <algorithm>
+#include <cmath>
+
+namespace kc {
+
+// ---------------------------------------------------------------------------
+// Dequantisation of one weight row of one k-block: 64 values -> 32 bf16 pairs, w = bf16(q * scale + bias), one rounding.
+//
+// The integers become bf16 operands of the multiply-add without a conversion: the bf16 with bit pattern N < 256 is N * 2^-133
+// (subnormals and the first binade have the same spacing), so a nibble masked into bits 0..3 or a byte in bits 0..7 of a
+// half-word IS q * 2^-133, a nibble in bits 4..7 q * 2^-129. One fused multiply-add with the scale times 2^133 (2^129: exact,
+// powers of two) gives q * scale + bias rounded once — the value that converting q first gives. 9 instructions for 8 weights
+// of 4 bits (two nibbles of a half-word in place, two behind one shift), 4 for 4 of 8 bits. The scaled scale must stay below
+// 2^128: a weight with larger scales (2^-5 and more) is taken at 2^-shift of its size, QWeight::shift, and its sums are
+// multiplied back, both exact.
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ bf162 bf2_bits(uint32_t u) { return *reinterpret_cast<const bf162*>(&u); }
+__device__ __forceinline__ uint32_t bf2_fma(uint32_t a, bf162 s, bf162 b) {
+  const bf162 r = __hfma2(*reinterpret_cast<const bf162*>(&a), s, b);
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
+__device__ __forceinline__ uint4 lds128(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+
+// The factors of a weight's scales and biases: scale * s0 * s1 = scale * 2^(133 - shift), bias * b = bias * 2^-shift.
+struct QlFactors { uint32_t s0, s1, b; };
+
+// Packed words of a row (16-byte chunk c at row + c * QL_TILE_N * 16), its scale and bias pairs at sb -> v[32].
+template <int BITS, int GPK>
+__device__ __forceinline__ void dequant_row(uint32_t row, uint32_t sb, const QlFactors& f, uint32_t (&v)[32]) {
+  constexpr int CHUNKS = BITS / 2;
+  bf162 s_lo[GPK], s_hi[GPK], bias[GPK];
+  uint32_t raw[GPK];
+  if (GPK == 1) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(raw[0]) : "r"(sb));
+  else asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(raw[0]), "=r"(raw[GPK - 1]) : "r"(sb));
+  uint4 w[CHUNKS];
+#pragma unroll
+  for (int h = 0; h < CHUNKS; ++h) w[h] = lds128(row + h * (QL_TILE_N * 16));
+#pragma unroll
+  for (int g = 0; g < GPK; ++g) {
+    const bf162 pair = bf2_bits(raw[g]);
+    s_lo[g] = __hmul2(__hmul2(__bfloat162bfloat162(pair.x), bf2_bits(f.s0)), bf2_bits(f.s1));
+    if (BITS == 4) s_hi[g] = __hmul2(s_lo[g], bf2_bits(0x3D803D80u));   // 2^-4
+    bias[g] = __hmul2(__bfloat162bfloat162(pair.y), bf2_bits(f.b));
+  }
+#pragma unroll
+  for (int h = 0; h < CHUNKS; ++h) {
+    const uint32_t word[4] = {w[h].x, w[h].y, w[h].z, w[h].w};
+    const int g = GPK == 2 ? h * 2 / CHUNKS : 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      if (BITS == 4) {
+        // the record's nibble order: element 2j at bits 4j, element 2j + 1 at bits 16 + 4j
+        uint32_t* o = v + (h * 4 + c) * 4;
+        const uint32_t up = word[c] >> 8;
+        o[0] = bf2_fma(word[c] & 0x000F000Fu, s_lo[g], bias[g]);
+        o[1] = bf2_fma(word[c] & 0x00F000F0u, s_hi[g], bias[g]);
+        o[2] = bf2_fma(up & 0x000F000Fu, s_lo[g], bias[g]);
+        o[3] = bf2_fma(up & 0x00F000F0u, s_hi[g], bias[g]);
+      } else {
+        uint32_t* o = v + (h * 4 + c) * 2;
+        o[0] = bf2_fma(__byte_perm(word[c], 0u, 0x4140u), s_lo[g], bias[g]);
+        o[1] = bf2_fma(__byte_perm(word[c], 0u, 0x4342u), s_lo[g], bias[g]);
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Tasks
+// ---------------------------------------------------------------------------
+
+constexpr int QL_GROUP0 = 4;                                   // first warp of the four groups
+constexpr int QL_GROUPS = 4;
+constexpr int QL_THREADS = (QL_GROUP0 + 4 * QL_GROUPS) * 32;   // 20 warps
+constexpr int QL_REG_BOUND = 896;                              // as if for so many threads: 72 registers, so that a row-wise kernel's block has room beside the CTA
+constexpr int QL_SUM_ROWS = 160;                               // rows of a chunk whose parts' sums lie in shared memory, at most
+// k-blocks of a unit: two where a unit's products take few cycles a k-block, one where two accumulators of many rows leave tensor
+// memory for four k-blocks only.
+__host__ __device__ constexpr int ql_unit(int cg) { return cg == 1 ? 2 : 1; }
+
+// How a launch's teams share the work:
+//   APART    a team a (pair, split, chunk of rows); the splits are left to the kernel that reads the result, or there is one
+//   RUNS     the k-blocks of all pairs, one after the other, in as many equal runs as the SMs have teams, each at least a pair's:
+//            where a run ends inside a pair, its sums so far go through global memory to the team with the pair's end, which goes
+//            on from them: the same chain of products as one team's
+//   IN_TURN  a team takes a (pair, chunk) at a time, its splits one after the other, their sums in shared memory
+constexpr int QL_MAX_SPLITS = 16;
+constexpr uint32_t QL_NOTHING = 0xFFFFFFFFu;
+enum : int { QL_APART = 0, QL_RUNS = 1, QL_IN_TURN = 2 };
+
+struct QlKernelParams {
+  const uint8_t* records;
+  uint32_t record_bytes;
+  int N, kblocks, n_pairs;
+  int splits;            // parts of a pair with a chain each (split s has k-blocks [K s / S, K (s + 1) / S)), added in order
+  int teams;             // of the grid
+  int M, m_pad, chunks;  // live rows of the launch; rows of a chunk, a multiple of 16, of 32 in a cluster
+  int row0;              // first activation row
+  int way;
+  int a_slots, b_slots, r_slots, accs;   // ring depths, in units: dequantised weights, activations, records; accumulators
+  uint32_t tmem_cols;    // columns allocated: a power of two
+  QlFactors factors;
+  float back0, back1;    // the products' sums times back0 * back1 = 2^shift
+  int glu;               // 0, or 1 (silu) / 2 (gelu_approx): act = activation(gate) * up, see ql_drain
+  bf16* act; int ld_act;
+  bf16* y; int ldy;
+  float* partial;        // APART with several splits: [splits][M][N]
+  uint4* fix;            // RUNS: [chunk][team][CTA][m_pad / 4][128], see ql_fix_slot
+  uint32_t* status;
+};
+
+// first, last: whether it has its pair's first split or k-block, its last; acc: the accumulator, its wait's parity above
+struct QlTask { int pair, chunk, split, kb0, nkb; bool first, last; uint32_t acc; };
+
+// Where the work of a CTA is cut, in shared memory: a division takes one of the single-thread roles a microsecond between the
+// arithmetic of the dequantisers, so one idle warp does them all before the roles start.
+struct QlCuts {
+  int r0, r1, p0, segments;            // RUNS: the run (in a pair it starts at an even k-block: only a pair's end makes half a unit), its first pair, its pairs
+  int pair, chunk;                     // IN_TURN: the team's first item
+  int units;                           // of all tasks
+  int split[QL_MAX_SPLITS + 1];        // k-blocks where the splits of a pair start
+};
+template <int UNIT>
+__device__ __forceinline__ void ql_cut(const QlKernelParams& p, QlCuts* c, int lane) {
+  const unsigned team = blockIdx.x >> 1, K = p.kblocks;
+  auto of = [](int k) { return (k + UNIT - 1) / UNIT; };
+  if (lane <= p.splits) c->split[lane] = K * lane / p.splits;
+  __syncwarp();
+  if (lane) return;
+  int n = 0;
+  if (p.way == QL_RUNS) {
+    auto start = [&](unsigned t) {
+      const int at = (int)((unsigned long long)p.n_pairs * K * t / p.teams);
+      return at - (at % (int)K & 1);
+    };
+    c->r0 = start(team); c->r1 = start(team + 1);
+    c->p0 = c->r0 / (int)K;
+    int pairs = 0;
+    for (int a = c->r0, e = (c->p0 + 1) * K; a < c->r1; a = e, e += K, ++pairs) n += of(min(c->r1, e) - a);
+    c->segments = pairs;
+    n *= p.chunks;
+  } else if (p.way == QL_APART) {
+    n = of(c->split[blockIdx.y + 1] - c->split[blockIdx.y]);
+  } else {
+    for (int i = 0; i < p.splits; ++i) n += of(c->split[i + 1] - c->split[i]);
+    n *= (p.n_pairs * p.chunks - team + p.teams - 1) / p.teams;
+    c->pair = team % p.n_pairs; c->chunk = team / p.n_pairs;
+  }
+  c->units = n;
+}
+
+// The tasks of a team, in order.
+struct QlTasks {
+  const QlKernelParams& p;
+  const QlCuts& c;
+  int at = 0, chunk = 0;      // APART: done; RUNS: segment of the run, chunk; IN_TURN: the item's pair, chunk
+  int split = 0;              // IN_TURN: of the item, the next one
+  __device__ QlTasks(const QlKernelParams& params, const QlCuts& cuts) : p(params), c(cuts) {
+    if (p.way == QL_IN_TURN) { at = c.pair; chunk = c.chunk; }
+  }
+  // Segments of a run: what another team waits for comes first, what waits for another team last: the run's last pair, of which
+  // it may hold a part without the end; the whole pairs; its first pair, whose start may be another's.
+  __device__ bool next(QlTask& t) {
+    const int K = p.kblocks;
+    if (p.way == QL_RUNS) {
+      if (chunk >= p.chunks) return false;
+      const int n = c.segments, pair = c.p0 + (at == 0 ? n - 1 : at == n - 1 ? 0 : at);
+      const int a = max(c.r0, pair * K), b = min(c.r1, (pair + 1) * K);
+      t = QlTask{pair, chunk, 0, a - pair * K, b - a, a == pair * K, b == (pair + 1) * K, 0};
+      if (++at == n) { at = 0; ++chunk; }
+      return true;
+    }
+    if (p.way == QL_APART) {
+      if (at++) return false;
+      const int s = blockIdx.y;
+      t = QlTask{(int)(blockIdx.x >> 1), (int)blockIdx.z, s, c.split[s], c.split[s + 1] - c.split[s], s == 0, s == p.splits - 1, 0};
+      return true;
+    }
+    if (chunk >= p.chunks) return false;
+    t = QlTask{at, chunk, split, c.split[split], c.split[split + 1] - c.split[split], split == 0, split == p.splits - 1, 0};
+    if (++split == p.splits) {
+      split = 0; at += p.teams;
+      while (at >= p.n_pairs) { at -= p.n_pairs; ++chunk; }
+    }
+    return true;
+  }
+  // A task that goes on from another team's sums.
+  __device__ bool goes_on(const QlTask& t) const { return p.way == QL_RUNS && !t.first; }
+};
+
+// The sums that a run leaves of a pair whose end it does not hold: [row / 4][128][4], of a CTA. Between launches every word is
+// QL_NOTHING, and a word that is something else is there: the reader polls the sums themselves and puts QL_NOTHING back. A word
+// that says so needs a fence before it, which took 4 us beside the copies that are under way.
+__device__ __forceinline__ uint4* ql_fix_slot(const QlKernelParams& p, int chunk, int team, int row) {
+  return p.fix + (((size_t)chunk * p.teams + team) * 2 + (blockIdx.x & 1)) * (p.m_pad / 4) * QL_TILE_N + row;
+}
+__device__ __forceinline__ bool ql_fix_load(const uint4* src, uint4& v) {
+  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src) : "memory");
+  return v.x != QL_NOTHING && v.y != QL_NOTHING && v.z != QL_NOTHING && v.w != QL_NOTHING;
+}
+
+// Puts another team's sums into a task's accumulator: one group's warps, a lane quarter each.
+__device__ __forceinline__ bool ql_go_on(const QlKernelParams& p, const QlTask& t, uint32_t acc, int q, int lane) {
+  uint4* src = ql_fix_slot(p, t.chunk, (blockIdx.x >> 1) - 1, q * 32 + lane);
+  const uint4 nothing = make_uint4(QL_NOTHING, QL_NOTHING, QL_NOTHING, QL_NOTHING);
+  const int last = p.m_pad / 4 - 1;
+  for (int s = 0; s < p.m_pad; s += 32) {   // a round trip to L2 each; the last 16 rows may be past the chunk's, in columns that nothing else has
+    uint4 f[8];
+    unsigned long long t0 = 0;
+    while (true) {
+      bool there = true;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) there &= ql_fix_load(src + min(s / 4 + j, last) * QL_TILE_N, f[j]);
+      if (__all_sync(0xffffffffu, there)) break;
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (__any_sync(0xffffffffu, now - t0 > KC_SPIN_LIMIT_NS)) {
+        if (p.status) atomicOr(p.status, KC_DEV_QLINEAR | 9u);
+        return false;
+      }
+    }
+    uint32_t v[32];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[4 * j] = f[j].x; v[4 * j + 1] = f[j].y; v[4 * j + 2] = f[j].z; v[4 * j + 3] = f[j].w;
+      if (s / 4 + j <= last) src[(s / 4 + j) * QL_TILE_N] = nothing;
+    }
+    tmem_st32(acc + s, v);
+  }
+  tmem_wait_st();
+  return true;
+}
+
+// Leaves a run's sums of a pair for the team that has its end: one group's warps, a lane quarter each.
+__device__ __forceinline__ void ql_leave(const QlKernelParams& p, const QlTask& t, uint32_t acc, int q, int lane) {
+  uint4* dst = ql_fix_slot(p, t.chunk, blockIdx.x >> 1, q * 32 + lane);
+  for (int s = 0; s < p.m_pad; s += 16, dst += 4 * QL_TILE_N) {
+    uint32_t e[16];
+    tmem_ld16_issue(acc + s, e);
+    tmem_wait_ld();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      asm volatile("" : "+r"(e[j]));   // no use before the wait
+      e[j] = e[j] == QL_NOTHING ? 0x7FFFFFFFu : e[j];   // both are NaN
+    }
+#pragma unroll
+    for (int j = 0; j < 16; j += 4) dst[j / 4 * QL_TILE_N] = make_uint4(e[j], e[j + 1], e[j + 2], e[j + 3]);
+  }
+}
+
+// A group's share of a task's accumulator: slices of 16 columns (rows of the step), every ng-th from gi. A thread has one
+// weight row (TMEM lane). What is not a pair's last task leaves its sums (in shared memory, or as partials for the next kernel); the
+// last one writes y, or the gated activation: in such a weight 16 gate rows and the 16 up rows of the same features take turns, so
+// the two meet in a warp, each lane taking eight of the slice's rows. Instructions count here: the warps of the first group get
+// one in about ten cycles between those of the dequantisers.
+__device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& t, uint32_t acc, int gi, int ng, float* sums, int q, int lane) {
+  const int tile = 2 * t.pair + (blockIdx.x & 1), n_in = q * 32 + lane, n = tile * QL_TILE_N + n_in;
+  const bool live = n < p.N, in_turn = p.way == QL_IN_TURN, apart = p.way == QL_APART && p.splits > 1;
+  for (int s = gi; s < p.m_pad >> 4; s += ng) {
+    const int m0 = t.chunk * p.m_pad + s * 16, rows = min(16, p.M - m0);
+    float v[16];
+    {
+      uint32_t e[16];
+      tmem_ld16_issue(acc + s * 16, e);
+      tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        asm volatile("" : "+r"(e[j]));   // no use before the wait
+        v[j] = __uint_as_float(e[j]);
+      }
+    }
+    if (p.back0 != 1.f) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = v[j] * p.back0 * p.back1;
+    }
+    float* before = sums + s * 16 * QL_TILE_N + n_in;
+    if (in_turn && !t.first) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) v[j] = before[j * QL_TILE_N] + v[j];
+    }
+    if (in_turn && !t.last) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) before[j * QL_TILE_N] = v[j];
+    } else if (apart) {
+      if (!live) continue;
+      float* dst = p.partial + ((size_t)t.split * p.M + m0) * p.N + n;
+      if (rows >= 16) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j, dst += p.N) *dst = v[j];
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j, dst += p.N)
+          if (j < rows) *dst = v[j];
+      }
+    } else if (p.glu) {
+      uint32_t pair[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) pair[j] = pack_bf162(v[2 * j], v[2 * j + 1]);
+      const bool up = lane & 16;      // this lane has up values; it takes rows 8 .. 15, its gate lane 0 .. 7
+      if (tile * QL_TILE_N < p.N) {   // whole tiles only
+        bf16* dst = p.act + (size_t)(p.row0 + m0 + (up ? 8 : 0)) * p.ld_act + tile * 64 + q * 16 + (lane & 15);
+        const int mine = rows - (up ? 8 : 0);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? pair[j] : pair[4 + j], 16);
+          const uint32_t g = up ? got : pair[j], u = up ? pair[4 + j] : got;
+          const uint32_t o = act_pair(g, u, p.glu == 2);
+          if (2 * j < mine) dst[0] = __ushort_as_bfloat16((unsigned short)(o & 0xFFFFu));
+          if (2 * j + 1 < mine) dst[p.ld_act] = __ushort_as_bfloat16((unsigned short)(o >> 16));
+          dst += 2 * p.ld_act;
+        }
+      }
+    } else if (live) {
+      bf16* dst = p.y + (size_t)(p.row0 + m0) * p.ldy + n;
+      if (rows >= 16) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j, dst += p.ldy) *dst = __float2bfloat16_rn(v[j]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j, dst += p.ldy)
+          if (j < rows) *dst = __float2bfloat16_rn(v[j]);
+      }
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The kernel. The dequantised weights reach the tensor core through TENSOR MEMORY (tcgen05.mma with the A operand in TMEM),
+// not through shared memory. A dequantiser thread owns one weight row (= one TMEM lane) of a UNIT, one or two 64-feature
+// k-blocks of a 128-row tile, expands the 64 weights of a k-block in registers and writes them with one tcgen05.st (column c =
+// weights 2c and 2c + 1), so the MMAs read only the activation k-block from shared memory.
+//
+// TMEM columns: [accs accumulators of round32(m_pad)] [a_slots x unit x 32 columns of bf16 pairs].
+// ---------------------------------------------------------------------------
+
+// A wait whose loop holds one instruction: a try_wait comes back after 4 us at the latest, so many of them are 1.6 s.
+__device__ __forceinline__ bool mbar_wait_count(uint32_t bar, uint32_t parity) {
+  int tries = 0;
+  while (!mbar_try_wait(bar, parity))
+    if (++tries > 400000) return false;
+  return true;
+}
+// What was asked for still lands in shared memory; it takes microseconds.
+__device__ __noinline__ void ql_gave_up(uint32_t* status, uint32_t wait) {
+  if (status) atomicOr(status, KC_DEV_QLINEAR | wait);
+  const unsigned long long t0 = globaltimer_ns();
+  while (globaltimer_ns() - t0 < 2000000ull) {}
+}
+
+template <int CG>
+__device__ __forceinline__ void ql_mma(uint32_t d, uint32_t a, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+  if (CG == 1) umma_bf16_ts(d, a, b_lo, b_hi, idesc, accumulate);
+  else umma_bf16_ts_pair(d, a, b_lo, b_hi, idesc, accumulate);
+}
+template <int CG>
+__device__ __forceinline__ void ql_commit(uint32_t bar) {
+  if (CG == 1) umma_commit(bar);
+  else umma_commit_pair(bar);
+}
+
+template <int BITS, int GPK, int CG>
+__global__ void __launch_bounds__(QL_REG_BOUND)
+qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ QlKernelParams p) {
+  constexpr uint32_t PACKED = QL_TILE_N * (QL_KB * BITS / 8);
+  constexpr int UNIT = ql_unit(CG), DQ = QL_GROUPS - 1;   // the first group drains
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const uint32_t kb_bytes = (uint32_t)p.m_pad / CG * 128u, b_bytes = UNIT * kb_bytes;   // this CTA's rows of a k-block, of a unit
+  const uint32_t r_bytes = UNIT * p.record_bytes;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const int side = blockIdx.x & 1;             // in a cluster: the CTA's rank
+  const uint32_t cs = (uint32_t)(p.m_pad + 31) & ~31u, a_col0 = p.accs * cs;
+
+  uint8_t* sB = smem;
+  uint8_t* sR = sB + (size_t)p.b_slots * b_bytes;
+  float* sums = reinterpret_cast<float*>(sR + (size_t)p.r_slots * r_bytes);
+  const bool has_sums = p.way == QL_IN_TURN && p.splits > 1;
+  // Barriers, by shared address: 8 bytes each. The n-th unit has record slot n % r_slots, A slot n % a_slots and activation slot
+  // n % b_slots.
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sums + (has_sums ? p.m_pad * QL_TILE_N : 0));
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars);
+  QlTask* last_task = reinterpret_cast<QlTask*>(bars + 2);   // with its accumulator, for the groups that join at the end
+  const uint32_t r_end = 8 * p.r_slots, b_end = 8 * p.b_slots;
+  QlCuts* cuts = reinterpret_cast<QlCuts*>(bars + 8);
+  const uint32_t raw_full = smem_u32(bars + 8 + (sizeof(QlCuts) + 7) / 8);   // by record slot: the records are in ..
+  const uint32_t raw_empty = raw_full + r_end;    // .. and read
+  const uint32_t done = raw_empty + r_end;        // by activation slot: the unit's products are; its other slots are free
+  const uint32_t ready = done + b_end;            // .. its activations are in, of both CTAs, and its weights dequantised
+  const uint32_t acc_full = ready + b_end;        // a task's products are in
+  const uint32_t acc_free = acc_full + 16;        // .. its accumulator has been read, and holds what the next one goes on from
+
+  pdl_launch_dependents();
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < p.r_slots; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, 4); }
+    for (int i = 0; i < p.b_slots; ++i) { mbar_init(ready + 8 * i, 4 * CG + 1); mbar_init(done + 8 * i, 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_free + 8 * i, 4 * CG); }
+    mbar_fence_init();
+  }
+  if (warp == 2) tmem_alloc<CG>(tmem_slot, p.tmem_cols);
+  if (warp == 1 && lane == 0) tma_prefetch_desc(&map_rows);
+  if (warp == 3) ql_cut<UNIT>(p, cuts, lane);
+  tc_fence_before();
+  __syncthreads();
+  if (CG == 2) cluster_sync();   // the other CTA's barriers are there
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp < QL_GROUP0) {
+    // ---- The roles of one thread each. In a turn of their loops a taken branch costs about 100 cycles, beside the arithmetic of
+    // the dequantiser warps on the same scheduler, and the turn has to keep up with a unit's products: so tasks are loops of their
+    // own with running addresses, a wait is one loop around one instruction, and one barrier stands for all that a unit waits for. ----
+    if (warp == 0 && elect_one()) {
+      // the weight records, which depend on no kernel before this one
+      const uint32_t r0 = smem_u32(sR);
+      const size_t pitch = (size_t)QL_TILE_GROUP * p.record_bytes;
+      uint32_t dst = r0, slot = 0, phase = 1;
+      bool ok = true;
+      QlTasks tasks(p, *cuts);
+      QlTask t;
+      while (ok && tasks.next(t)) {
+        const int tile = 2 * t.pair + side;
+        const uint8_t* src = p.records + ((size_t)(tile / QL_TILE_GROUP) * p.kblocks + t.kb0) * pitch + (size_t)(tile % QL_TILE_GROUP) * p.record_bytes;
+        auto copy = [&](int kbs) {
+          const uint32_t full = raw_full + slot;
+          ok = mbar_wait_count(raw_empty + slot, phase);
+          if (!ok) return;
+          mbar_arrive_expect_tx(full, kbs * p.record_bytes);
+          bulk_g2s(dst, src, p.record_bytes, full);
+          if (kbs > 1) bulk_g2s(dst + p.record_bytes, src + pitch, p.record_bytes, full);
+          src += UNIT * pitch; dst += r_bytes; slot += 8;
+          if (slot == r_end) { slot = 0; dst = r0; phase ^= 1u; }
+        };
+        for (int n = t.nkb / UNIT; ok && n > 0; --n) copy(UNIT);
+        if (UNIT == 2 && ok && (t.nkb & 1)) copy(1);
+      }
+      if (!ok) ql_gave_up(p.status, 1);
+    } else if (warp == 1 && elect_one()) {
+      // the activations, the first access of this kernel to memory written by earlier kernels
+      pdl_wait();
+      const uint32_t b0 = smem_u32(sB), lead = CG == 2 ? cluster_addr(ready, 0) : ready;
+      uint32_t dst = b0, slot = 0, phase = 1;
+      bool ok = true;
+      QlTasks tasks(p, *cuts);
+      QlTask t;
+      while (ok && tasks.next(t)) {
+        const int row = p.row0 + t.chunk * p.m_pad + (CG == 2 ? side * (p.m_pad / 2) : 0);
+        int x = t.kb0 * QL_KB;
+        auto copy = [&](int kbs) {
+          ok = mbar_wait_count(done + slot, phase);
+          if (!ok) return;
+          if (CG == 1 || side == 0) mbar_arrive_expect_tx(ready + slot, kbs * kb_bytes * CG);
+          tma_load_2d_pair<CG>(dst, &map_rows, x, row, lead + slot);
+          if (kbs > 1) tma_load_2d_pair<CG>(dst + kb_bytes, &map_rows, x + QL_KB, row, lead + slot);
+          x += UNIT * QL_KB; dst += b_bytes; slot += 8;
+          if (slot == b_end) { slot = 0; dst = b0; phase ^= 1u; }
+        };
+        for (int n = t.nkb / UNIT; ok && n > 0; --n) copy(UNIT);
+        if (UNIT == 2 && ok && (t.nkb & 1)) copy(1);
+      }
+      if (!ok) ql_gave_up(p.status, 2);
+    } else if (warp == 2 && (CG == 1 || side == 0) && elect_one()) {
+      // the MMAs. With the loop around the election four of them and two commits took the warp 160 cycles to issue alone, this way 65.
+      pdl_wait();
+      const uint32_t idesc = umma_idesc_bf16(QL_TILE_N * CG, p.m_pad);
+      const uint64_t proto = umma_smem_desc(0, 1024);
+      const uint32_t d_hi = (uint32_t)(proto >> 32), b_lo0 = (uint32_t)proto | ((smem_u32(sB) >> 4) & 0x3FFF), b_step = b_bytes >> 4, kb_step = kb_bytes >> 4;
+      const uint32_t a_first = tmem_base + a_col0, a_last = a_first + p.a_slots * UNIT * 32;
+      uint32_t a_t = a_first, b_lo = b_lo0, slot = 0, phase = 0;
+      uint32_t buf = 0, fphase = 0;                   // the task's accumulator
+      bool ok = true;
+      QlTasks tasks(p, *cuts);
+      QlTask t;
+      while (ok && tasks.next(t)) {
+        ok = mbar_wait_count(acc_free + 8 * buf, fphase);
+        const uint32_t d = tmem_base + buf * cs;
+        uint32_t acc = tasks.goes_on(t) ? 1u : 0u;
+        auto issue = [&](int kbs) {
+          ok = mbar_wait_count(ready + slot, phase);
+          if (!ok) return;
+          tc_fence_after();   // the A operand was written with tcgen05.st by other threads
+#pragma unroll
+          for (int ks = 0; ks < QL_KB / 16; ++ks) ql_mma<CG>(d, a_t + 8 * ks, b_lo + 2 * ks, d_hi, idesc, ks == 0 ? acc : 1u);
+          if (kbs > 1) {
+#pragma unroll
+            for (int ks = 0; ks < QL_KB / 16; ++ks) ql_mma<CG>(d, a_t + 32 + 8 * ks, b_lo + kb_step + 2 * ks, d_hi, idesc, 1u);
+          }
+          acc = 1;
+          ql_commit<CG>(done + slot);
+          a_t += UNIT * 32; b_lo += b_step; slot += 8;
+          if (a_t == a_last) a_t = a_first;
+          if (slot == b_end) { slot = 0; b_lo = b_lo0; phase ^= 1u; }
+        };
+        for (int n = t.nkb / UNIT; ok && n > 0; --n) issue(UNIT);
+        if (UNIT == 2 && ok && (t.nkb & 1)) issue(1);
+        if (ok) ql_commit<CG>(acc_full + 8 * buf);
+        if (++buf == (uint32_t)p.accs) { buf = 0; fphase ^= 1u; }
+      }
+      if (!ok) ql_gave_up(p.status, 4);
+    }
+    __syncwarp();
+  } else {
+    const int group = (warp - QL_GROUP0) >> 2, q = warp & 3;
+    const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16);
+    bool ok = true;
+    QlTasks tasks(p, *cuts);
+    if (group > 0) {
+      // ---- dequantisers: thread = one weight row (TMEM lane 32 q + lane) of every third unit. The first slots are filled under the
+      // tail of the previous kernel. A wait names a slot's use by its parity: r_slots is a multiple of three, so that a group meets
+      // every use of its record slots, and units are done in order. ----
+      const uint32_t d = group - 1;
+      const uint32_t row0 = smem_u32(sR) + (q * 32 + lane) * 16, sb0 = smem_u32(sR) + PACKED + (q * 32 + lane) * (GPK * 4);
+      const uint32_t lead = CG == 2 ? cluster_addr(ready, 0) : ready;
+      const uint32_t a0 = lanes + a_col0, a_end = a0 + p.a_slots * UNIT * 32;
+      uint32_t rec = d * r_bytes, raw = 8 * d, a_t = a0 + UNIT * 32 * d, bar = raw, phase = 0;
+      uint32_t old = 8 * (p.b_slots - p.a_slots + d), freed = 1;   // barrier of the unit that had the A slot before; none at first
+      for (int left = cuts->units - (int)d; left > 0; left -= DQ) {
+        ok = __all_sync(0xffffffffu, mbar_wait_count(raw_full + raw, phase));
+        if (!ok) break;
+#pragma unroll
+        for (int k = 0; k < UNIT; ++k) {   // of half a unit at a task's end, the second half is what the slot held before: no MMA reads it
+          uint32_t v[32];
+          dequant_row<BITS, GPK>(row0 + rec + k * p.record_bytes, sb0 + rec + k * p.record_bytes, p.factors, v);
+          if (k == 0) {
+            ok = __all_sync(0xffffffffu, mbar_wait_count(done + old, freed));
+            if (!ok) break;
+            tc_fence_after();
+          }
+          tmem_st32(a_t + 32 * k, v);
+        }
+        if (!ok) break;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(raw_empty + raw);   // the records are in registers
+        raw += 8 * DQ; rec += DQ * r_bytes;
+        if (raw >= r_end) { raw -= r_end; rec -= p.r_slots * r_bytes; phase ^= 1u; }
+        a_t += DQ * UNIT * 32;
+        if (a_t >= a_end) a_t -= p.a_slots * UNIT * 32;
+        old += 8 * DQ;
+        if (old >= b_end) { old -= b_end; freed ^= 1u; }
+        tmem_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) {
+          if (CG == 1) mbar_arrive(ready + bar);
+          else mbar_arrive_cluster(lead + bar);
+        }
+        bar += 8 * DQ;
+        if (bar >= b_end) bar -= b_end;
+      }
+      if (!ok) ql_gave_up(p.status, 5);
+    }
+    // ---- the first group prepares accumulators and drains them, a task under the products of the next one; the last task's is
+    // everybody's ----
+    QlTasks ahead(p, *cuts);
+    QlTask t{}, next{}, fresh{};
+    bool more = group == 0 && tasks.next(next), some = group == 0 && ahead.next(fresh), last = group > 0, released = false;
+    uint32_t acc = 0, facc = 0;
+    int prepared = 0;                              // accumulators that are, of tasks not yet drained
+    auto turn = [&](uint32_t a) { return (a & 1) + 1 == (uint32_t)p.accs ? (a & ~1u) ^ 2u : a + 1; };
+    while (more || last) {
+      if (group == 0) {
+        while (some && prepared < p.accs) {
+          if (ahead.goes_on(fresh)) {
+            // Where the task before it is the one that leaves sums for another team, whichever of the two can go first goes first:
+            // if all teams waited to go on they would wait for one another in a row.
+            if (prepared > 0 && cuts->segments == 2) {
+              const uint4* first = ql_fix_slot(p, fresh.chunk, (blockIdx.x >> 1) - 1, q * 32 + lane);
+              if (!released) { pdl_wait(); released = true; }
+              bool there = false, over = !ok;
+              const unsigned long long t0 = globaltimer_ns();
+              while (!there && !over) {
+                uint4 v;
+                there = __all_sync(0xffffffffu, ql_fix_load(first, v));
+                over = __all_sync(0xffffffffu, mbar_test_wait(acc_full + 8 * (acc & 1), acc >> 1)) || __any_sync(0xffffffffu, globaltimer_ns() - t0 > KC_SPIN_LIMIT_NS);
+              }
+              if (!there) break;
+            }
+            if (!released) { pdl_wait(); released = true; }
+            if (ok) ok = ql_go_on(p, fresh, lanes + (facc & 1) * cs, q, lane);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if (CG == 1) mbar_arrive(acc_free + 8 * (facc & 1));
+            else mbar_arrive_cluster(cluster_addr(acc_free + 8 * (facc & 1), 0));
+          }
+          facc = turn(facc); ++prepared;
+          some = ahead.next(fresh);
+        }
+        t = next; t.acc = acc;
+        acc = turn(acc);
+        more = tasks.next(next); last = !more;
+      }
+      if (last) {   // which one, and the sums so far, are there for all who read them
+        if (group == 0 && q == 0 && lane == 0) *last_task = t;
+        asm volatile("bar.sync 5, %0;" ::"n"(QL_GROUPS * 128) : "memory");
+        t = *last_task;
+      }
+      if (!released) { pdl_wait(); released = true; }   // the stores may overwrite what an earlier kernel still reads
+      if (ok) ok = warp_wait(acc_full + 8 * (t.acc & 1), t.acc >> 1, p.status, KC_DEV_QLINEAR | 7);
+      tc_fence_after();
+      if (p.way == QL_RUNS && !t.last) {
+        if (ok) ql_leave(p, t, lanes + (t.acc & 1) * cs, q, lane);   // never the last task: a run starts with it
+      } else if (ok) ql_drain(p, t, lanes + (t.acc & 1) * cs, group, last ? QL_GROUPS : 1, sums, q, lane);
+      if (last) break;
+      --prepared;
+    }
+  }
+  __syncwarp();
+  tc_fence_before();
+  __syncthreads();
+  if (CG == 2) cluster_sync();   // nothing of the other CTA's is on its way here, or here any more
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_dealloc<CG>(tmem_base, p.tmem_cols);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Plans
+// ---------------------------------------------------------------------------
+
+struct UmmaPlan {
+  int cg, way, m_pad, chunks, teams;             // teams: of the grid
+  int a_slots, b_slots, r_slots, accs;
+  uint32_t tmem_cols;
+  size_t smem;
+};
+
+static int pairs_of(const QWeight& w) { return (w.n_tiles + 1) / 2; }
+
+size_t qlinear_fix_bytes(int sm_count) { return (size_t)QL_FIX_CHUNKS * (sm_count / 2) * 2 * QL_CHUNK_ROWS * QL_TILE_N * sizeof(float); }
+
+// Ring depths, tensor and shared memory. At least three A slots, the step of a dequantiser group; record slots a multiple of it;
+// activation slots, by which a unit's barriers go, as many as A slots at least.
+static bool plan_rings(UmmaPlan* t, const QWeight& w, bool several_tasks, bool sums) {
+  const int cs = (t->m_pad + 31) & ~31, unit = ql_unit(t->cg);
+  t->accs = several_tasks ? 2 : 1;
+  t->a_slots = std::min(8, (512 - t->accs * cs) / (unit * 32));
+  const size_t extra = 1024 + 1024 + (sums ? (size_t)t->m_pad * QL_TILE_N * 4 : 0);
+  const size_t all = (size_t)227 * 1024, b_slot = (size_t)unit * t->m_pad / t->cg * 128, r_slot = (size_t)unit * w.record_bytes;
+  auto bytes = [&](int b, int r) { return extra + b * b_slot + r * r_slot; };   // 1024: barriers, at most 24 * 2 + 12 * 2 + 4, and the words before them
+  while (t->a_slots > 3 && bytes(t->a_slots, 6) > all) --t->a_slots;
+  t->r_slots = 6; t->b_slots = t->a_slots;
+  if (t->a_slots < 3 || bytes(t->b_slots, t->r_slots) > all) return false;
+  for (bool more = true; more;) {   // deeper as far as there is room
+    more = false;
+    if (t->r_slots < 24 / unit && bytes(t->b_slots, t->r_slots + 3) <= all) { t->r_slots += 3; more = true; }
+    if (t->b_slots < 12 && bytes(t->b_slots + 1, t->r_slots) <= all) { ++t->b_slots; more = true; }
+  }
+  t->tmem_cols = 32;
+  while ((int)t->tmem_cols < t->accs * cs + t->a_slots * unit * 32) t->tmem_cols <<= 1;
+  t->smem = bytes(t->b_slots, t->r_slots);
+  return true;
+}
+
+// Rows of a chunk for a weight that is split along K, its parts apart. All chunks are one launch, CTAs of the next filling the
+// SMs that the last wave of one leaves idle; the chunk size is the one whose waves take the least time, counted in MMA
+// cycles: a unit of 128 x 64 weights takes 2 cycles per row, not less than 184, and a CTA about 6000 around them. Chunks of
+// fewer than 96 rows are not looked at: a unit takes its 184 cycles then, whatever the rows, so more chunks are only more
+// waves.
+static int plan_apart_rows(const QWeight& w, int M) {
+  const int ctas = w.n_tiles * w.splits;
+  const long long units = (long long)w.kblocks / w.splits;
+  int best = 0;
+  long long best_cost = 0;
+  for (int chunks = (M + QL_CHUNK_ROWS - 1) / QL_CHUNK_ROWS; best == 0 || chunks * 96 <= M; ++chunks) {
+    const int per = ((M + chunks - 1) / chunks + 15) & ~15;
+    const int n = (M + per - 1) / per;
+    const long long waves = ((long long)ctas * n + w.sm_count - 1) / w.sm_count;
+    const long long cost = waves * (units * std::max(184, 2 * per) + 6000);
+    if (best == 0 || cost < best_cost) { best = per; best_cost = cost; }
+  }
+  return best;
+}
+
+constexpr int QL_ROWS_MIN = 257;   // below, a chunk or two of rows never fill the SMs
+// With more k-blocks all splits in turn are the slower way at most row counts: 7000 x 28672 (448) 499 -> 564 us at 1200 rows, 805
+// -> 885 at 2048; 8192 x 28672 316 -> 334 at 640, 757 -> 780 at 1500, though 265 -> 251 at 513. 3584 x 18944 (296): the same
+// within a fiftieth up to 2048 rows, a tenth faster from there.
+constexpr int QL_ROWS_MAX_KBLOCKS = 300;
+// Whether the rows of a weight that is split along K take its splits in turn, and how many a chunk: 0 where splits apart take about as
+// long or less. In cycles, fitted to launches of 264 to 2048 rows against eight weights of 16 to 64 tiles and 56 to 448 k-blocks, the
+// fit within a tenth of them: a k-block there takes 330 and 1.55 a row, a CTA's start and end 9500; here 330 and 1.9 a row, 2.3
+// where two stages of activations only have room, a segment's end 600. A reduction of their own costs partials 2150 bytes a
+// cycle over all SMs where there are more than QL_MAX_M rows, else 6500. Summed by the kernel that reads the result anyway
+// they cost that next to nothing, and of the two ways the one with a launch of its own size has to be faster by a seventh.
+static int plan_in_turn_rows(const QWeight& w, int M, bool summed) {
+  if (w.splits == 1 || M < QL_ROWS_MIN || w.kblocks > QL_ROWS_MAX_KBLOCKS) return 0;
+  auto apart_cost = [&](int rows) -> long long {
+    if (rows == 0) return 0;
+    const int per = plan_apart_rows(w, rows);
+    const long long ctas = (long long)w.n_tiles * w.splits * ((rows + per - 1) / per), waves = (ctas + w.sm_count - 1) / w.sm_count;
+    const long long values = (long long)rows * w.N;
+    return waves * (w.kblocks * (330 + per * 31 / 20) / w.splits + 9500) +
+           (summed ? 0 : M > QL_MAX_M ? values * (4 * w.splits + 2) / 2150 : values * 4 * w.splits / 6500);
+  };
+  const long long apart = M / QL_MAX_M * apart_cost(QL_MAX_M) + apart_cost(M % QL_MAX_M);
+  int best = 0;
+  long long best_cost = apart / 100 * (summed ? 86 : 92);
+  const int ends = w.splits * (w.splits > 8 ? 900 : 600);
+  if (w.kblocks * (330 + 96 * 19 / 10) + ends + 8000 >= best_cost) return 0;   // one wave of the smallest chunks
+  for (int per = 192; per >= 96; per -= 16) {
+    const int row_cost = w.record_bytes > 5120 && per > 144 ? 23 : per > 160 ? 23 : 19;
+    const long long items = (long long)w.n_tiles * ((M + per - 1) / per), waves = (items + w.sm_count - 1) / w.sm_count;
+    const long long cost = waves * (w.kblocks * (330 + per * row_cost / 10) + ends) + 8000;
+    if (cost < best_cost) { best = per; best_cost = cost; }
+  }
+  return best;
+}
+bool qlinear_in_turn(const QWeight& w, int M, bool summed) { return plan_in_turn_rows(w, M, summed) > 0; }
+
+// Rows of a chunk for a weight that is not split along K, and whether its teams share the work by runs: the choice whose products
+// take the least time, 2 cycles a row and k-block and not less than 256, larger chunks where two are level. Runs leave no team idle and
+// cost a cut pair's way through global memory, counted as 8 k-blocks a chunk; fix: chunks that they may have.
+static int plan_whole_rows(const QWeight& w, int M, int fix, bool* runs) {
+  const int teams = w.sm_count / 2, pairs = pairs_of(w);
+  if (pairs < teams) fix = 0;   // a run holds a whole pair's k-blocks at least
+  int best = 0;
+  double best_cost = 0;
+  for (int per = QL_CHUNK_ROWS; per >= 16; per -= per > QL_SOLO_ROWS ? 32 : 16) {
+    if (per < 96 && M > QL_SOLO_ROWS) break;
+    if (per - 32 >= M && per > QL_SOLO_ROWS) continue;
+    if (per - 16 >= M && per <= QL_SOLO_ROWS) continue;
+    const int chunks = (M + per - 1) / per;
+    if (chunks > 1 && per <= QL_SOLO_ROWS) break;
+    const double whole = (double)((pairs * (long long)chunks + teams - 1) / teams) * w.kblocks, cut = ((double)pairs * w.kblocks / teams + 8) * chunks;
+    const bool r = chunks <= fix && cut < whole;
+    const double cost = (r ? cut : whole) * (std::max(256, 2 * per) + 20);
+    if (best == 0 || cost < best_cost * 0.995) { best = per; best_cost = cost; *runs = r; }
+  }
+  return best;
+}
+
+template <int BITS, int GPK, int CG>
+static cudaError_t launch_umma(const QLinearLaunch& l, const UmmaPlan& t, const QlKernelParams& p, cudaStream_t s) {
+  static DeviceOnce configured;   // the attribute belongs to the device's copy of the kernel
+  if (configured.first_on_current_device()) {
+    cudaError_t e = cudaFuncSetAttribute(qlinear_umma_kernel<BITS, GPK, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) { configured.forget_current_device(); return e; }
+  }
+  const CUtensorMap* rows = act_operand_rows_map(l.x, p.m_pad / CG);
+  if (!rows) return cudaErrorInvalidValue;
+  const dim3 grid = p.way == QL_APART ? dim3(CG == 2 ? 2 * p.n_pairs : l.w->n_tiles, p.splits, p.chunks) : dim3(2 * t.teams);
+  return launch_k_cluster(CG, qlinear_umma_kernel<BITS, GPK, CG>, grid, dim3(QL_THREADS), t.smem, s, *rows, p);
+}
+template <int BITS, int GPK>
+static cudaError_t launch_umma_cg(const QLinearLaunch& l, const UmmaPlan& t, const QlKernelParams& p, cudaStream_t s) {
+  return t.cg == 2 ? launch_umma<BITS, GPK, 2>(l, t, p, s) : launch_umma<BITS, GPK, 1>(l, t, p, s);
+}
+
+static uint32_t bf16_twice(int exponent) {   // 2^exponent as a pair of bf16, subnormals included
+  const uint32_t b = exponent >= -126 ? (uint32_t)(exponent + 127) << 7 : 1u << (exponent + 133);
+  return b << 16 | b;
+}
+
+cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
+  const QWeight& w = *l.w;
+  if (l.M < 1 || l.M > qlinear_slab_rows(w, l.M)) return cudaErrorInvalidValue;
+  if (l.row0 % 16 || l.row0 + l.M > l.x->rows) return cudaErrorInvalidValue;   // rows past the operand's end read as zeros
+  const bool glu = l.glu && w.splits == 1 && w.N % QL_TILE_N == 0 && l.act;
+  if (l.glu_done) *l.glu_done = glu ? 1 : 0;
+  UmmaPlan t{};
+  const int pairs = pairs_of(w), all_teams = std::max(1, w.sm_count / 2);
+  if (w.splits > 1) {
+    const int turn = plan_in_turn_rows(w, l.M, l.summed);
+    t.way = turn ? QL_IN_TURN : QL_APART;
+    t.m_pad = turn ? turn : plan_apart_rows(w, l.M);
+  } else {
+    bool runs = false;
+    t.m_pad = plan_whole_rows(w, l.M, l.fix ? QL_FIX_CHUNKS : 0, &runs);
+    t.way = runs ? QL_RUNS : QL_IN_TURN;
+  }
+  t.cg = t.m_pad > QL_SOLO_ROWS ? 2 : 1;
+  if (t.cg == 2) t.m_pad = (t.m_pad + 31) & ~31;
+  if (t.way == QL_IN_TURN && w.splits > 1) t.m_pad = std::min(t.m_pad, QL_SUM_ROWS);
+  t.chunks = (l.M + t.m_pad - 1) / t.m_pad;
+  t.teams = t.way == QL_IN_TURN ? (int)std::min<long long>((long long)pairs * t.chunks, all_teams) : all_teams;
+  const bool sums = t.way == QL_IN_TURN && w.splits > 1, several = t.way == QL_RUNS || (t.way == QL_IN_TURN && (sums || (long long)pairs * t.chunks > t.teams));
+  if (!plan_rings(&t, w, several, sums)) return cudaErrorInvalidValue;
+  QlKernelParams p;
+  p.records = w.records; p.record_bytes = w.record_bytes;
+  p.N = w.N; p.kblocks = w.kblocks; p.n_pairs = pairs; p.splits = w.splits; p.teams = t.teams;
+  p.M = l.M; p.m_pad = t.m_pad; p.chunks = t.chunks; p.row0 = l.row0;
+  p.way = t.way;
+  p.a_slots = t.a_slots; p.b_slots = t.b_slots; p.r_slots = t.r_slots; p.accs = t.accs; p.tmem_cols = t.tmem_cols;
+  const int up = 133 - w.shift, first = std::min(127, up);
+  p.factors = QlFactors{bf16_twice(first), bf16_twice(up - first), bf16_twice(-w.shift)};
+  p.back0 = ldexpf(1.f, std::min(w.shift, 127)); p.back1 = ldexpf(1.f, w.shift - std::min(w.shift, 127));
+  p.glu = glu ? l.glu : 0; p.act = l.act; p.ld_act = l.ld_act;
+  p.y = l.y; p.ldy = l.ldy; p.partial = l.partial;
+  p.fix = reinterpret_cast<uint4*>(l.fix); p.status = l.status;
+  if (w.bits == 4) return w.gpk == 2 ? launch_umma_cg<4, 2>(l, t, p, s) : launch_umma_cg<4, 1>(l, t, p, s);
+  return w.gpk == 2 ? launch_umma_cg<8, 2>(l, t, p, s) : launch_umma_cg<8, 1>(l, t, p, s);
+}
+
+}  // namespace kc

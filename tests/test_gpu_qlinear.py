@@ -286,3 +286,23 @@ def test_weights_are_rounded_once(ctx, bits, scale):
     got = qw.matmul(torch.eye(k).to(torch.bfloat16).cuda()).cpu().float().T
     assert torch.equal(got, want)
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("n,k,bits,group", [
+    (19000, 1024, 4, 64),         # 75 pairs of tiles (the last tile missing) for 74 teams: runs that end inside a pair
+    (19000, 1088, 4, 32),         # 17 k-blocks: units of one at a pair's end
+    (28672, 448, 8, 32),          # runs of a pair and a half
+])
+def test_teams_that_share_a_pair_carry_its_bits(ctx, n, k, bits, group):
+    """A team that has the end of a pair of weight tiles goes on from the sums of the one that has its start: one chain of products,
+    whoever has it. The entry point without that workspace has whole pairs only; few rows, rows of a cluster, and two to five chunks."""
+    p, s, b = make(n, k, bits, group, 51)
+    qw = api.QuantizedWeight(ctx, p.cuda(), s.cuda(), b.cuda(), bits, group)
+    x = acts(800, k, 52).cuda()
+    want = torch.empty(800, n, dtype=torch.bfloat16, device="cuda")
+    qw.matmul_static(x, 800, want)
+    ctx.sync()
+    for m in (1, 17, 64, 65, 192, 193, 385, 576, 800, 1):
+        y = qw.matmul(x[:m])
+        assert torch.equal(y.view(torch.int16), want[:m].view(torch.int16)), m
+    assert ctx.device_status() == 0
