@@ -98,7 +98,7 @@ __device__ __forceinline__ void dequant_row(uint32_t row, uint32_t sb, const QlF
 constexpr int QL_GROUP0 = 4;                                   // first warp of the four groups
 constexpr int QL_GROUPS = 4;
 constexpr int QL_THREADS = (QL_GROUP0 + 4 * QL_GROUPS) * 32;   // 20 warps
-constexpr int QL_REG_BOUND = 896;                              // as if for so many threads: 72 registers, so that a row-wise kernel's block has room beside the CTA
+constexpr int QL_STAGE_BYTES = 1280;                           // a warp's buffer on the way out: 16 rows of 32 bf16, or 8 of fp32, with padding
 constexpr int QL_SUM_ROWS = 160;                               // rows of a chunk whose parts' sums lie in shared memory, at most
 // k-blocks of a unit: two where a unit's products take few cycles a k-block, one where two accumulators of many rows leave tensor
 // memory for four k-blocks only.
@@ -129,6 +129,7 @@ struct QlKernelParams {
   float back0, back1;    // the products' sums times back0 * back1 = 2^shift
   int glu;               // 0, or 1 (silu) / 2 (gelu_approx): act = activation(gate) * up, see ql_drain
   bf16* act; int ld_act;
+  int vec;               // rows of y, or of the partials, start on 16 bytes, and whole groups of 8 (4) features
   bf16* y; int ldy;
   float* partial;        // APART with several splits: [splits][M][N]
   uint4* fix;            // RUNS: [chunk][team][CTA][m_pad / 4][128], see ql_fix_slot
@@ -274,13 +275,80 @@ __device__ __forceinline__ void ql_leave(const QlKernelParams& p, const QlTask& 
   }
 }
 
-// A group's share of a task's accumulator: slices of 16 columns (rows of the step), every ng-th from gi. A thread has one
-// weight row (TMEM lane). What is not a pair's last task leaves its sums (in shared memory, or as partials for the next kernel); the
-// last one writes y, or the gated activation: in such a weight 16 gate rows and the 16 up rows of the same features take turns, so
-// the two meet in a warp, each lane taking eight of the slice's rows. Instructions count here: the warps of the first group get
-// one in about ten cycles between those of the dequantisers.
-__device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& t, uint32_t acc, int gi, int ng, float* sums, int q, int lane) {
-  const int tile = 2 * t.pair + (blockIdx.x & 1), n_in = q * 32 + lane, n = tile * QL_TILE_N + n_in;
+// A group's share of a task's accumulator: slices of columns (rows of the step), every ng-th from gi. A thread has one weight row (TMEM
+// lane). What is not a pair's last task leaves its sums (in shared memory, or as partials for the next kernel); the last one writes
+// y, or the gated activation: in such a weight 16 gate rows and the 16 up rows of the same features take turns, so the two meet in a
+// warp. Where the output's rows allow it (p.vec) values leave 8 or 16 bytes a lane, through a buffer of the warp.
+//
+// Few rows: slices of 8 in a loop of little code. What bounds it is the fetch of its instructions, which a CTA meets for the first
+// time at its end: 8B decode steps of 32 rows 6113 -> 5972 us against the form below.
+__device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& t, uint32_t acc, int gi, int ng, float* sums, uint8_t* stage, int q, int lane) {
+  const int tile = 2 * t.pair + (blockIdx.x & 1), n0 = tile * QL_TILE_N + q * 32;
+  const bool in_turn = p.way == QL_IN_TURN;
+  float* buf = reinterpret_cast<float*>(stage);   // [8][36]
+  const int r = lane >> 2, f = (lane & 3) * 8, n = n0 + f;   // the lane's row and features on the way out
+#pragma unroll 1
+  for (int s = gi * 8; s < p.m_pad; s += ng * 8) {
+    const int m = t.chunk * p.m_pad + s + r;
+    float v[8];
+    {
+      uint32_t e[8];
+      tmem_ld8_issue(acc + s, e);
+      tmem_wait_ld();
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        asm volatile("" : "+r"(e[j]));   // no use before the wait
+        v[j] = __uint_as_float(e[j]) * p.back0 * p.back1;
+      }
+    }
+    if (in_turn && !(t.first && t.last)) {
+      float* before = sums + s * QL_TILE_N + q * 32 + lane;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        if (!t.first) v[j] = before[j * QL_TILE_N] + v[j];
+        if (!t.last) before[j * QL_TILE_N] = v[j];
+      }
+      if (!t.last) continue;
+    }
+    __syncwarp();                        // the last turn's reads of the buffer are done
+#pragma unroll
+    for (int j = 0; j < 8; ++j) buf[j * 36 + lane] = v[j];
+    __syncwarp();
+    if (m >= p.M) continue;
+    if (p.glu) {                         // four features of a row: gate at 32 of a warp's k .., up 16 further
+      const int c = (lane & 3) * 4;
+      const float4 g = *reinterpret_cast<const float4*>(buf + r * 36 + c), u = *reinterpret_cast<const float4*>(buf + r * 36 + 16 + c);
+      const uint2 o = make_uint2(act_pair(pack_bf162(g.x, g.y), pack_bf162(u.x, u.y), p.glu == 2), act_pair(pack_bf162(g.z, g.w), pack_bf162(u.z, u.w), p.glu == 2));
+      if (tile * QL_TILE_N < p.N) *reinterpret_cast<uint2*>(p.act + (size_t)(p.row0 + m) * p.ld_act + tile * 64 + q * 16 + c) = o;
+      continue;
+    }
+    const float4 a = *reinterpret_cast<const float4*>(buf + r * 36 + f), b = *reinterpret_cast<const float4*>(buf + r * 36 + f + 4);
+    if (p.way == QL_APART && p.splits > 1) {
+      float* dst = p.partial + ((size_t)t.split * p.M + m) * p.N + n;
+      if (p.vec && n < p.N) {
+        *reinterpret_cast<float4*>(dst) = a;
+        if (n + 4 < p.N) *reinterpret_cast<float4*>(dst + 4) = b;
+      } else {
+#pragma unroll 1
+        for (int j = 0; j < 8 && n + j < p.N; ++j) dst[j] = buf[r * 36 + f + j];
+      }
+    } else {
+      bf16* dst = p.y + (size_t)(p.row0 + m) * p.ldy + n;
+      if (p.vec && n < p.N) {
+        *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf162(a.x, a.y), pack_bf162(a.z, a.w), pack_bf162(b.x, b.y), pack_bf162(b.z, b.w));
+      } else {
+#pragma unroll 1
+        for (int j = 0; j < 8 && n + j < p.N; ++j) dst[j] = __float2bfloat16_rn(buf[r * 36 + f + j]);
+      }
+    }
+  }
+}
+
+// Many rows: slices of 16, unrolled, lanes taking eight rows of the activation each. The first group's warps get an instruction in about
+// ten cycles between those of the dequantisers, so their number counts: 4096 x 14336 at 2048 rows 175 -> 163 us against the form
+// above, with stores of 2 bytes a lane 172.
+__device__ __forceinline__ void ql_drain_wide(const QlKernelParams& p, const QlTask& t, uint32_t acc, int gi, int ng, float* sums, uint8_t* stage, int q, int lane) {
+  const int tile = 2 * t.pair + (blockIdx.x & 1), n_in = q * 32 + lane, n0 = tile * QL_TILE_N + q * 32, n = n0 + lane;
   const bool live = n < p.N, in_turn = p.way == QL_IN_TURN, apart = p.way == QL_APART && p.splits > 1;
   for (int s = gi; s < p.m_pad >> 4; s += ng) {
     const int m0 = t.chunk * p.m_pad + s * 16, rows = min(16, p.M - m0);
@@ -308,44 +376,68 @@ __device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& 
 #pragma unroll
       for (int j = 0; j < 16; ++j) before[j * QL_TILE_N] = v[j];
     } else if (apart) {
-      if (!live) continue;
-      float* dst = p.partial + ((size_t)t.split * p.M + m0) * p.N + n;
-      if (rows >= 16) {
+      float* out = p.partial + ((size_t)t.split * p.M + m0) * p.N;
+      if (p.vec) {
+        float* buf = reinterpret_cast<float*>(stage);   // [8][36]
+        const int r = lane >> 3, f = (lane & 7) * 4;
+        float* dst = out + (size_t)r * p.N + n0 + f;
 #pragma unroll
-        for (int j = 0; j < 16; ++j, dst += p.N) *dst = v[j];
-      } else {
+        for (int h = 0; h < 2; ++h) {
+          __syncwarp();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) buf[j * 36 + lane] = v[8 * h + j];
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < 2; ++k, dst += (size_t)4 * p.N) {
+            const float4 x = *reinterpret_cast<const float4*>(buf + (4 * k + r) * 36 + f);
+            if (8 * h + 4 * k + r < rows && n0 + f < p.N) *reinterpret_cast<float4*>(dst) = x;
+          }
+        }
+      } else if (live) {
+        float* dst = out + n;
 #pragma unroll
         for (int j = 0; j < 16; ++j, dst += p.N)
           if (j < rows) *dst = v[j];
       }
     } else if (p.glu) {
-      uint32_t pair[8];
+      if (tile * QL_TILE_N < p.N) {     // whole tiles only
+        uint32_t pair[8];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) pair[j] = pack_bf162(v[2 * j], v[2 * j + 1]);
-      const bool up = lane & 16;      // this lane has up values; it takes rows 8 .. 15, its gate lane 0 .. 7
-      if (tile * QL_TILE_N < p.N) {   // whole tiles only
-        bf16* dst = p.act + (size_t)(p.row0 + m0 + (up ? 8 : 0)) * p.ld_act + tile * 64 + q * 16 + (lane & 15);
-        const int mine = rows - (up ? 8 : 0);
+        for (int j = 0; j < 8; ++j) pair[j] = pack_bf162(v[2 * j], v[2 * j + 1]);
+        const bool up = lane & 16;      // this lane has up values; it takes rows 8 .. 15, its gate lane 0 .. 7
+        uint16_t* buf = reinterpret_cast<uint16_t*>(stage) + (up ? 8 * 24 : 0) + (lane & 15);   // [16][24]
+        __syncwarp();
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? pair[j] : pair[4 + j], 16);
-          const uint32_t g = up ? got : pair[j], u = up ? pair[4 + j] : got;
-          const uint32_t o = act_pair(g, u, p.glu == 2);
-          if (2 * j < mine) dst[0] = __ushort_as_bfloat16((unsigned short)(o & 0xFFFFu));
-          if (2 * j + 1 < mine) dst[p.ld_act] = __ushort_as_bfloat16((unsigned short)(o >> 16));
-          dst += 2 * p.ld_act;
+          const uint32_t o = act_pair(up ? got : pair[j], up ? pair[4 + j] : got, p.glu == 2);
+          buf[2 * j * 24] = (uint16_t)(o & 0xFFFFu);
+          buf[(2 * j + 1) * 24] = (uint16_t)(o >> 16);
         }
+        __syncwarp();
+        const int r = lane >> 1, f = (lane & 1) * 8;
+        if (r < rows)
+          *reinterpret_cast<uint4*>(p.act + (size_t)(p.row0 + m0 + r) * p.ld_act + tile * 64 + q * 16 + f) =
+              *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(stage) + r * 24 + f);
+      }
+    } else if (p.vec) {
+      bf16* buf = reinterpret_cast<bf16*>(stage);       // [16][40]
+      const int r = lane >> 2, f = (lane & 3) * 8;
+      bf16* dst = p.y + (size_t)(p.row0 + m0 + r) * p.ldy + n0 + f;
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) buf[j * 40 + lane] = __float2bfloat16_rn(v[j]);
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < 2; ++k, dst += (size_t)8 * p.ldy) {
+        const uint4 x = *reinterpret_cast<const uint4*>(buf + (8 * k + r) * 40 + f);
+        if (8 * k + r < rows && n0 + f < p.N) *reinterpret_cast<uint4*>(dst) = x;
       }
     } else if (live) {
       bf16* dst = p.y + (size_t)(p.row0 + m0) * p.ldy + n;
-      if (rows >= 16) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j, dst += p.ldy) *dst = __float2bfloat16_rn(v[j]);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j, dst += p.ldy)
-          if (j < rows) *dst = __float2bfloat16_rn(v[j]);
-      }
+      for (int j = 0; j < 16; ++j, dst += p.ldy)
+        if (j < rows) *dst = __float2bfloat16_rn(v[j]);
     }
   }
 }
@@ -385,7 +477,7 @@ __device__ __forceinline__ void ql_commit(uint32_t bar) {
 }
 
 template <int BITS, int GPK, int CG>
-__global__ void __launch_bounds__(QL_REG_BOUND)
+__global__ void __launch_bounds__(QL_THREADS, 1)
 qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ QlKernelParams p) {
   constexpr uint32_t PACKED = QL_TILE_N * (QL_KB * BITS / 8);
   constexpr int UNIT = ql_unit(CG), DQ = QL_GROUPS - 1;   // the first group drains
@@ -399,7 +491,8 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
 
   uint8_t* sB = smem;
   uint8_t* sR = sB + (size_t)p.b_slots * b_bytes;
-  float* sums = reinterpret_cast<float*>(sR + (size_t)p.r_slots * r_bytes);
+  uint8_t* stage = sR + (size_t)p.r_slots * r_bytes;
+  float* sums = reinterpret_cast<float*>(stage + 4 * QL_GROUPS * QL_STAGE_BYTES);
   const bool has_sums = p.way == QL_IN_TURN && p.splits > 1;
   // Barriers, by shared address: 8 bytes each. The n-th unit has record slot n % r_slots, A slot n % a_slots and activation slot
   // n % b_slots.
@@ -527,6 +620,7 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   } else {
     const int group = (warp - QL_GROUP0) >> 2, q = warp & 3;
     const uint32_t lanes = tmem_base + ((uint32_t)(q * 32) << 16);
+    stage += (warp - QL_GROUP0) * QL_STAGE_BYTES;
     bool ok = true;
     QlTasks tasks(p, *cuts);
     if (group > 0) {
@@ -626,7 +720,10 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
       tc_fence_after();
       if (p.way == QL_RUNS && !t.last) {
         if (ok) ql_leave(p, t, lanes + (t.acc & 1) * cs, q, lane);   // never the last task: a run starts with it
-      } else if (ok) ql_drain(p, t, lanes + (t.acc & 1) * cs, group, last ? QL_GROUPS : 1, sums, q, lane);
+      } else if (ok) {
+        if (CG == 1) ql_drain(p, t, lanes + (t.acc & 1) * cs, group, last ? QL_GROUPS : 1, sums, stage, q, lane);
+        else ql_drain_wide(p, t, lanes + (t.acc & 1) * cs, group, last ? QL_GROUPS : 1, sums, stage, q, lane);
+      }
       if (last) break;
       --prepared;
     }
@@ -662,7 +759,7 @@ static bool plan_rings(UmmaPlan* t, const QWeight& w, bool several_tasks, bool s
   const int cs = (t->m_pad + 31) & ~31, unit = ql_unit(t->cg);
   t->accs = several_tasks ? 2 : 1;
   t->a_slots = std::min(8, (512 - t->accs * cs) / (unit * 32));
-  const size_t extra = 1024 + 1024 + (sums ? (size_t)t->m_pad * QL_TILE_N * 4 : 0);
+  const size_t extra = 1024 + 1024 + 4 * QL_GROUPS * QL_STAGE_BYTES + (sums ? (size_t)t->m_pad * QL_TILE_N * 4 : 0);
   const size_t all = (size_t)227 * 1024, b_slot = (size_t)unit * t->m_pad / t->cg * 128, r_slot = (size_t)unit * w.record_bytes;
   auto bytes = [&](int b, int r) { return extra + b * b_slot + r * r_slot; };   // 1024: barriers, at most 24 * 2 + 12 * 2 + 4, and the words before them
   while (t->a_slots > 3 && bytes(t->a_slots, 6) > all) --t->a_slots;
@@ -783,7 +880,7 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   const QWeight& w = *l.w;
   if (l.M < 1 || l.M > qlinear_slab_rows(w, l.M)) return cudaErrorInvalidValue;
   if (l.row0 % 16 || l.row0 + l.M > l.x->rows) return cudaErrorInvalidValue;   // rows past the operand's end read as zeros
-  const bool glu = l.glu && w.splits == 1 && w.N % QL_TILE_N == 0 && l.act;
+  const bool glu = l.glu && w.splits == 1 && w.N % QL_TILE_N == 0 && l.act && (l.ld_act & 7) == 0 && (reinterpret_cast<uintptr_t>(l.act) & 15) == 0;
   if (l.glu_done) *l.glu_done = glu ? 1 : 0;
   UmmaPlan t{};
   const int pairs = pairs_of(w), all_teams = std::max(1, w.sm_count / 2);
@@ -814,6 +911,8 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   p.back0 = ldexpf(1.f, std::min(w.shift, 127)); p.back1 = ldexpf(1.f, w.shift - std::min(w.shift, 127));
   p.glu = glu ? l.glu : 0; p.act = l.act; p.ld_act = l.ld_act;
   p.y = l.y; p.ldy = l.ldy; p.partial = l.partial;
+  p.vec = t.way == QL_APART && w.splits > 1 ? (w.N & 3) == 0 && (reinterpret_cast<uintptr_t>(l.partial) & 15) == 0
+                                            : (w.N & 7) == 0 && (l.ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(l.y) & 15) == 0;
   p.fix = reinterpret_cast<uint4*>(l.fix); p.status = l.status;
   if (w.bits == 4) return w.gpk == 2 ? launch_umma_cg<4, 2>(l, t, p, s) : launch_umma_cg<4, 1>(l, t, p, s);
   return w.gpk == 2 ? launch_umma_cg<8, 2>(l, t, p, s) : launch_umma_cg<8, 1>(l, t, p, s);
