@@ -38,6 +38,26 @@ def test_greedy_rows_match_oracle_and_break_ties_low(ctx):
     assert got_n[1] == 300 and got_r[1] == 300
 
 
+@pytest.mark.parametrize("vocab", [8, 72, 4 * 16384, 4 * 16384 + 8, 8 * 16384, 8 * 16384 + 8, 10 * 16384 + 8, 16 * 16384, 16 * 16384 + 8, 1001])
+def test_greedy_rows_at_the_edges_of_a_share(ctx, vocab):
+    """A row is shared by eight blocks of 256 threads with 4, 8, 10 or 16 vectors of eight each, longer and unaligned rows are one block's:
+    the edges of these, ties, a winner in the last place, values whose differences to the logsumexp round together, and rows with
+    infinities and NaN, against the oracle."""
+    g = torch.Generator().manual_seed(vocab)
+    x = torch.empty(7, vocab).normal_(0, 2.0, generator=g).to(torch.bfloat16)
+    x[1] = 0
+    x[2, -1] = 30
+    x[3] *= 2 ** -10
+    x[4] *= 64
+    x[5] = -x[5].abs()
+    y = x.clone()
+    y[0, 3], y[1], y[2, 5], y[3, 1], y[4], y[5], y[6, 2:] = -torch.inf, -torch.inf, torch.inf, torch.nan, torch.nan, 3.38e38, -torch.inf
+    for rows in (x, y):
+        for normalize in (True, False):
+            got = api.greedy_rows(ctx, rows.cuda(), normalize).cpu().numpy().astype(np.uint32)
+            assert np.array_equal(got, O.greedy_rows(rows, normalize))
+
+
 def test_verify_accept_walk(ctx):
     """engine.rs:2336-2366 on four segments: full agreement (bonus), first-row mismatch, mid mismatch, plain decode."""
     rows = torch.tensor([5, 6, 7, 8,   9, 1, 1,   4, 4, 9, 9,   3], dtype=torch.int32).cuda()
