@@ -193,11 +193,10 @@ def algorithmic(cfg, batch, k, mean_ctx):
 
 
 # DRAM traffic of the dominant kernel (the quantised GEMM) relative to its algorithmic weight bytes, from ncu captures of
-# single launches at 192 rows (summary committed under profiles/): dram__bytes_read.sum + dram__bytes_write.sum = 67.7 MB +
-# 1.7 MB for the 66.1 MB of records of a layer's gate_up, whose rows are one chunk, and 594.6 MB + 41.8 MB for the 295.5 MB
-# of the head, whose rows are two. Weighted by the step's bytes (the head is 0.07 of them); the per-launch figure reported
+# single launches at 192 rows (summary committed under profiles/): dram__bytes_read.sum + dram__bytes_write.sum = 69.0 MB +
+# 3.2 MB for the 66.1 MB of records of a layer's gate_up and 311.3 MB + 47.6 MB for the 295.5 MB of the head. Weighted by the step's bytes (the head is 0.07 of them); the per-launch figure reported
 # is this ratio times the mean algorithmic weight bytes per GEMM launch of the step.
-GEMM_DRAM_TRAFFIC_PER_WEIGHT_BYTE = 0.93 * (67.7 + 1.7) / 66.1 + 0.07 * (594.6 + 41.8) / 295.5
+GEMM_DRAM_TRAFFIC_PER_WEIGHT_BYTE = 0.93 * (69.0 + 3.2) / 66.1 + 0.07 * (311.3 + 47.6) / 295.5
 
 # --------------------------------------------------------------------------------------
 # GPU arm
@@ -484,7 +483,7 @@ def cpu_reference(name: str, tensors, ctxs, steps: int, warmup: int, budget_s: f
                        f"median; a batch round = {batch} such forwards, nothing extrapolated")}
 
 
-GEMM_KERNEL = "qlinear_umma_ta_kernel (affine-dequant GEMM, tcgen05, A operand in TMEM)"
+GEMM_KERNEL = "qlinear_umma_kernel (affine-dequant GEMM, tcgen05, A operand in TMEM)"
 TP_WORKLOAD = "llama-3-70b-8l-w4g64-verify-k4-bs64-tp"
 
 

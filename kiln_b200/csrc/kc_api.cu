@@ -917,8 +917,7 @@ extern "C" int kc_model_load(kc_ctx_t c, const kc_model_desc* desc, const kc_ten
     LOAD_FAIL(build_linear(m, idx, {{p + ".self_attn.o_proj", 0, H}}, d.num_heads * D, (int)q0, (int)q1, &L.o, nullptr));
     const int64_t f0 = (int64_t)d.tp_rank * m->F, f1 = f0 + m->F;
     {
-      // gate and up rows alternate in blocks of one GEMM tile (128 rows) when the width allows it, so a CTA that owns
-      // two neighbouring tiles holds gate and up of the same features
+      // 16 gate and 16 up rows in turn where the width allows it, so that a warp's accumulator lanes hold both of a feature
       m->glu_interleaved = m->F % 64 == 0;
       const std::vector<Part> gu_parts = {{p + ".mlp.gate_proj", f0, f1}, {p + ".mlp.up_proj", f0, f1}};
       LOAD_FAIL(build_linear(m, idx, gu_parts, H, 0, H, &L.gate_up, nullptr, m->glu_interleaved));

@@ -6,7 +6,7 @@
 // warps busy, 2900 cycles a tile of 128 keys and more under a soft cap, which was the bound of every decode step; here a
 // tile's rows x keys lie evenly over the warps. What crosses them is each row's maximum (exact in any order) and its sum
 // (over the 32 keys of a warp pairwise, keys 16, 8, 4, 2 and 1 apart, then the warps pairwise: kc_attn.cu adds in the same
-// tree). A product takes its 46 cycles whether it has 16 columns or 64, so the rows are not padded to 128 either.
+// tree). A product has the unit's columns only: the rows are not padded to 128 either.
 //
 // K and V are separate slots of the ring: scores are taken from half a tile's bytes, and a slot of K is free again one
 // product earlier.

@@ -777,10 +777,9 @@ static bool plan_rings(UmmaPlan* t, const QWeight& w, bool several_tasks, bool s
 }
 
 // Rows of a chunk for a weight that is split along K, its parts apart. All chunks are one launch, CTAs of the next filling the
-// SMs that the last wave of one leaves idle; the chunk size is the one whose waves take the least time, counted in MMA
-// cycles: a unit of 128 x 64 weights takes 2 cycles per row, not less than 184, and a CTA about 6000 around them. Chunks of
-// fewer than 96 rows are not looked at: a unit takes its 184 cycles then, whatever the rows, so more chunks are only more
-// waves.
+// SMs that the last wave of one leaves idle; the chunk size is the one whose waves take the least time, counted in
+// cycles that were fitted to this choice's launches: a unit of 128 x 64 weights 2 per row, not less than 184, and a CTA about 6000
+// around them. Chunks of fewer than 96 rows are not looked at: a unit takes no less time then, so more chunks are only more waves.
 static int plan_apart_rows(const QWeight& w, int M) {
   const int ctas = w.n_tiles * w.splits;
   const long long units = (long long)w.kblocks / w.splits;
@@ -797,13 +796,15 @@ static int plan_apart_rows(const QWeight& w, int M) {
 }
 
 constexpr int QL_ROWS_MIN = 257;   // below, a chunk or two of rows never fill the SMs
-// With more k-blocks all splits in turn are the slower way at most row counts: 7000 x 28672 (448) 499 -> 564 us at 1200 rows, 805
-// -> 885 at 2048; 8192 x 28672 316 -> 334 at 640, 757 -> 780 at 1500, though 265 -> 251 at 513. 3584 x 18944 (296): the same
-// within a fiftieth up to 2048 rows, a tenth faster from there.
+// With more k-blocks all splits in turn were the slower way at most row counts with one CTA a tile: 7000 x 28672 (448) 499 -> 564 us at
+// 1200 rows. 3584 x 18944 (296), apart and in turn: 320 rows 43 and 62 us, 1024 rows 137 and 119.
 constexpr int QL_ROWS_MAX_KBLOCKS = 300;
 // Whether the rows of a weight that is split along K take its splits in turn, and how many a chunk: 0 where splits apart take about as
-// long or less. In cycles, fitted to launches of 264 to 2048 rows against eight weights of 16 to 64 tiles and 56 to 448 k-blocks, the
-// fit within a tenth of them: a k-block there takes 330 and 1.55 a row, a CTA's start and end 9500; here 330 and 1.9 a row, 2.3
+// long or less. Apart (with the reduction behind it) and in turn, us: 4096 x 14336 264 rows 40.5 and 48.0, 320 41.7 and 48.1, 513 80.5
+// and 51.6, 1024 133 and 91, 2048 263 and 160; 4096 x 4096 320 rows 25.7 and 21.6 (the reduction is 5 of the first, which a step does not
+// have), 1024 77 and 38, 2048 153 and 61; 6144 x 4096 1024 rows 91 and 52; 2048 x 8192 513 rows 43.6 and 41.9, 2048 140 and 74. The line
+// is drawn in cycles, fitted to launches of 264 to 2048 rows against eight weights of 16 to 64 tiles and 56 to 448 k-blocks with one CTA a
+// tile; teams gain on both sides, and it still takes the faster one but where both are within a fifth: a k-block there takes 330 and 1.55 a row, a CTA's start and end 9500; here 330 and 1.9 a row, 2.3
 // where two stages of activations only have room, a segment's end 600. A reduction of their own costs partials 2150 bytes a
 // cycle over all SMs where there are more than QL_MAX_M rows, else 6500. Summed by the kernel that reads the result anyway
 // they cost that next to nothing, and of the two ways the one with a launch of its own size has to be faster by a seventh.
@@ -835,6 +836,9 @@ bool qlinear_in_turn(const QWeight& w, int M, bool summed) { return plan_in_turn
 // Rows of a chunk for a weight that is not split along K, and whether its teams share the work by runs: the choice whose products
 // take the least time, 2 cycles a row and k-block and not less than 256, larger chunks where two are level. Runs leave no team idle and
 // cost a cut pair's way through global memory, counted as 8 k-blocks a chunk; fix: chunks that they may have.
+// Whole pairs and runs, us: 28672 x 4096 (112 pairs, 74 teams) 1 row 17.4 and 16.5, 32 rows 18.1 and 17.4, 192 rows 37.2 and 37.0 alone, in a step
+// 44.7 and 42.3; where the difference is smaller the way through memory counts for more than that: 320 rows 57.2 and 60.3, the head's
+// 501 pairs 138 and 142 at 192 rows.
 static int plan_whole_rows(const QWeight& w, int M, int fix, bool* runs) {
   const int teams = w.sm_count / 2, pairs = pairs_of(w);
   if (pairs < teams) fix = 0;   // a run holds a whole pair's k-blocks at least
