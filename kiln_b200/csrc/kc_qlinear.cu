@@ -82,6 +82,8 @@ int qlinear_plan_splits(int n_tiles, int kblocks, int sm_count) {
   return std::max(s, 1);
 }
 
+int qlinear_plan_chains(int n_tiles, int splits, int sm_count) { return (n_tiles + 1) / 2 * splits * 10 >= sm_count * 7 ? 1 : 2; }
+
 cudaError_t qweight_build(QWeight* out, const uint32_t* w, const bf16* scales, const bf16* biases,
                           int N, int K, int bits, int group, int sm_count, cudaStream_t s, bool alternate) {
   QWeight q;
@@ -92,6 +94,7 @@ cudaError_t qweight_build(QWeight* out, const uint32_t* w, const bf16* scales, c
   q.packed_bytes = QL_TILE_N * (QL_KB * bits / 8);
   q.record_bytes = q.packed_bytes + QL_TILE_N * q.gpk * 4;
   q.splits = qlinear_plan_splits(q.n_tiles, q.kblocks, sm_count);
+  q.chains = qlinear_plan_chains(q.n_tiles, q.splits, sm_count);
   q.sm_count = sm_count;
   // one allocation: the records, then the largest exponent of a scale, which the re-tiling finds
   cudaError_t e = cudaMalloc(&q.records, q.bytes() + 16);

@@ -40,6 +40,7 @@ struct QWeight {
   uint32_t packed_bytes = 0;   // per record
   uint32_t record_bytes = 0;
   int splits = 1;              // fixed function of (N, K): never of M
+  int chains = 1;              // .. and chains of products a split has (qlinear_plan_chains)
   int sm_count = 148;
   int* top = nullptr;          // the re-tiling's largest exponent of a scale (inside the records' allocation)
   int shift = 0;               // from it, read once at load: the GEMM takes the weights times 2^-shift
@@ -89,6 +90,8 @@ size_t qlinear_fix_bytes(int sm_count);
 // Fixed split-K plan: a function of the weight's shape only, so a row's
 // accumulation order never depends on how many rows ride the step.
 int qlinear_plan_splits(int n_tiles, int kblocks, int sm_count);
+// Two, a split's even and its odd k-blocks, where pairs of tiles times splits are fewer than seven tenths of the SMs; else one.
+int qlinear_plan_chains(int n_tiles, int splits, int sm_count);
 
 // Re-tile on the device. w/scales/biases are device pointers in mlx layout.
 // alternate: the first N / 2 rows are the gate's, the others the up projection's, and the weight's rows are 16 of each in turn.

@@ -13,9 +13,10 @@
 // The accumulator D[n, m] lives in TMEM: lane = weight row n, column = activation row m.
 //
 // Every output element depends only on its own activation row and on an order of sums fixed by (N, K) and the SM count: a
-// pair's k-blocks are cut into parts at fixed places, a part is one chain of products, and the parts are added in order. That
-// is what lets verify rows share a step with other rows and still reproduce the bits of a one-row decode. More rows than one
-// accumulator holds are chunks of rows: rows are independent, so no bit changes.
+// pair's k-blocks are cut into parts at fixed places, a part is one chain of products or two (its even and its odd k-blocks,
+// QWeight::chains, added at its end), and the parts are added in order. That is what lets verify rows share a step with other
+// rows and still reproduce the bits of a one-row decode. More rows than one accumulator holds are chunks of rows: rows are
+// independent, so no bit changes.
 #include "kc_qlinear.cuh"
 #include "kc_umma.cuh"
 
@@ -118,12 +119,13 @@ struct QlKernelParams {
   const uint8_t* records;
   uint32_t record_bytes;
   int N, kblocks, n_pairs;
-  int splits;            // parts of a pair with a chain each (split s has k-blocks [K s / S, K (s + 1) / S)), added in order
+  int splits;            // parts of a pair (split s has k-blocks [K s / S, K (s + 1) / S)), added in order
+  int chains;            // of a part: one, or its even and its odd k-blocks apart
   int teams;             // of the grid
   int M, m_pad, chunks;  // live rows of the launch; rows of a chunk, a multiple of 16, of 32 in a cluster
   int row0;              // first activation row
   int way;
-  int a_slots, b_slots, r_slots, accs;   // ring depths, in units: dequantised weights, activations, records; accumulators
+  int a_slots, b_slots, r_slots, accs;   // ring depths, in units: dequantised weights, activations, records; accumulators with a barrier
   uint32_t tmem_cols;    // columns allocated: a power of two
   QlFactors factors;
   float back0, back1;    // the products' sums times back0 * back1 = 2^shift
@@ -132,12 +134,13 @@ struct QlKernelParams {
   int vec;               // rows of y, or of the partials, start on 16 bytes, and whole groups of 8 (4) features
   bf16* y; int ldy;
   float* partial;        // APART with several splits: [splits][M][N]
-  uint4* fix;            // RUNS: [chunk][team][CTA][m_pad / 4][128], see ql_fix_slot
+  uint4* fix;            // RUNS: [chunk][chain][team][CTA][m_pad / 4][128], see ql_fix_slot
   uint32_t* status;
 };
 
-// first, last: whether it has its pair's first split or k-block, its last; acc: the accumulator, its wait's parity above
-struct QlTask { int pair, chunk, split, kb0, nkb; bool first, last; uint32_t acc; };
+// first, last: whether it has its pair's first split or k-block, its last; acc: the accumulator, its wait's parity above; of a
+// cluster's second chain: acc1
+struct QlTask { int pair, chunk, split, kb0, nkb; bool first, last; uint32_t acc, acc1; };
 
 // Where the work of a CTA is cut, in shared memory: a division takes one of the single-thread roles a microsecond between the
 // arithmetic of the dequantisers, so one idle warp does them all before the roles start.
@@ -193,18 +196,18 @@ struct QlTasks {
       if (chunk >= p.chunks) return false;
       const int n = c.segments, pair = c.p0 + (at == 0 ? n - 1 : at == n - 1 ? 0 : at);
       const int a = max(c.r0, pair * K), b = min(c.r1, (pair + 1) * K);
-      t = QlTask{pair, chunk, 0, a - pair * K, b - a, a == pair * K, b == (pair + 1) * K, 0};
+      t = QlTask{pair, chunk, 0, a - pair * K, b - a, a == pair * K, b == (pair + 1) * K, 0, 0};
       if (++at == n) { at = 0; ++chunk; }
       return true;
     }
     if (p.way == QL_APART) {
       if (at++) return false;
       const int s = blockIdx.y;
-      t = QlTask{(int)(blockIdx.x >> 1), (int)blockIdx.z, s, c.split[s], c.split[s + 1] - c.split[s], s == 0, s == p.splits - 1, 0};
+      t = QlTask{(int)(blockIdx.x >> 1), (int)blockIdx.z, s, c.split[s], c.split[s + 1] - c.split[s], s == 0, s == p.splits - 1, 0, 0};
       return true;
     }
     if (chunk >= p.chunks) return false;
-    t = QlTask{at, chunk, split, c.split[split], c.split[split + 1] - c.split[split], split == 0, split == p.splits - 1, 0};
+    t = QlTask{at, chunk, split, c.split[split], c.split[split + 1] - c.split[split], split == 0, split == p.splits - 1, 0, 0};
     if (++split == p.splits) {
       split = 0; at += p.teams;
       while (at >= p.n_pairs) { at -= p.n_pairs; ++chunk; }
@@ -213,22 +216,24 @@ struct QlTasks {
   }
   // A task that goes on from another team's sums.
   __device__ bool goes_on(const QlTask& t) const { return p.way == QL_RUNS && !t.first; }
+  // The part has an odd k-block: a second chain that is no chain of nothing.
+  __device__ bool second(const QlTask& t) const { return p.chains == 2 && (p.way == QL_RUNS ? p.kblocks : t.nkb) > 1; }
 };
 
 // The sums that a run leaves of a pair whose end it does not hold: [row / 4][128][4], of a CTA. Between launches every word is
 // QL_NOTHING, and a word that is something else is there: the reader polls the sums themselves and puts QL_NOTHING back. A word
 // that says so needs a fence before it, which took 4 us beside the copies that are under way.
-__device__ __forceinline__ uint4* ql_fix_slot(const QlKernelParams& p, int chunk, int team, int row) {
-  return p.fix + (((size_t)chunk * p.teams + team) * 2 + (blockIdx.x & 1)) * (p.m_pad / 4) * QL_TILE_N + row;
+__device__ __forceinline__ uint4* ql_fix_slot(const QlKernelParams& p, int chunk, int chain, int team, int row) {
+  return p.fix + (((size_t)(chunk * p.chains + chain) * p.teams + team) * 2 + (blockIdx.x & 1)) * (p.m_pad / 4) * QL_TILE_N + row;
 }
 __device__ __forceinline__ bool ql_fix_load(const uint4* src, uint4& v) {
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src) : "memory");
   return v.x != QL_NOTHING && v.y != QL_NOTHING && v.z != QL_NOTHING && v.w != QL_NOTHING;
 }
 
-// Puts another team's sums into a task's accumulator: one group's warps, a lane quarter each.
-__device__ __forceinline__ bool ql_go_on(const QlKernelParams& p, const QlTask& t, uint32_t acc, int q, int lane) {
-  uint4* src = ql_fix_slot(p, t.chunk, (blockIdx.x >> 1) - 1, q * 32 + lane);
+// Puts another team's sums of a chain into a task's accumulator: one group's warps, a lane quarter each.
+__device__ __forceinline__ bool ql_go_on(const QlKernelParams& p, const QlTask& t, int chain, uint32_t acc, int q, int lane) {
+  uint4* src = ql_fix_slot(p, t.chunk, chain, (blockIdx.x >> 1) - 1, q * 32 + lane);
   const uint4 nothing = make_uint4(QL_NOTHING, QL_NOTHING, QL_NOTHING, QL_NOTHING);
   const int last = p.m_pad / 4 - 1;
   for (int s = 0; s < p.m_pad; s += 32) {   // a round trip to L2 each; the last 16 rows may be past the chunk's, in columns that nothing else has
@@ -258,9 +263,9 @@ __device__ __forceinline__ bool ql_go_on(const QlKernelParams& p, const QlTask& 
   return true;
 }
 
-// Leaves a run's sums of a pair for the team that has its end: one group's warps, a lane quarter each.
-__device__ __forceinline__ void ql_leave(const QlKernelParams& p, const QlTask& t, uint32_t acc, int q, int lane) {
-  uint4* dst = ql_fix_slot(p, t.chunk, blockIdx.x >> 1, q * 32 + lane);
+// Leaves a run's sums of a chain of a pair for the team that has its end: one group's warps, a lane quarter each.
+__device__ __forceinline__ void ql_leave(const QlKernelParams& p, const QlTask& t, int chain, uint32_t acc, int q, int lane) {
+  uint4* dst = ql_fix_slot(p, t.chunk, chain, blockIdx.x >> 1, q * 32 + lane);
   for (int s = 0; s < p.m_pad; s += 16, dst += 4 * QL_TILE_N) {
     uint32_t e[16];
     tmem_ld16_issue(acc + s, e);
@@ -275,14 +280,21 @@ __device__ __forceinline__ void ql_leave(const QlKernelParams& p, const QlTask& 
   }
 }
 
-// A group's share of a task's accumulator: slices of columns (rows of the step), every ng-th from gi. A thread has one weight row (TMEM
-// lane). What is not a pair's last task leaves its sums (in shared memory, or as partials for the next kernel); the last one writes
+// The sums of the parts so far, in shared memory: [row / 4][128][4].
+__device__ __forceinline__ float4* ql_sums_of(float* sums, int row, int n_in) { return reinterpret_cast<float4*>(sums) + row / 4 * QL_TILE_N + n_in; }
+__device__ __forceinline__ void ql_add4(float* v, float4 o) {
+  const float2 a = add2(make_float2(o.x, o.y), make_float2(v[0], v[1])), b = add2(make_float2(o.z, o.w), make_float2(v[2], v[3]));
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+}
+
+// A group's share of a task's accumulator, with its second chain's where there is one: slices of columns (rows of the step), every
+// ng-th from gi. A thread has one weight row (TMEM lane). What is not a pair's last task leaves its sums (in shared memory, or as partials for the next kernel); the last one writes
 // y, or the gated activation: in such a weight 16 gate rows and the 16 up rows of the same features take turns, so the two meet in a
 // warp. Where the output's rows allow it (p.vec) values leave 8 or 16 bytes a lane, through a buffer of the warp.
 //
 // Few rows: slices of 8 in a loop of little code. What bounds it is the fetch of its instructions, which a CTA meets for the first
 // time at its end: 8B decode steps of 32 rows 6113 -> 5972 us against the form below.
-__device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& t, uint32_t acc, int gi, int ng, float* sums, uint8_t* stage, int q, int lane) {
+__device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& t, uint32_t acc, bool two, uint32_t acc1, int gi, int ng, float* sums, uint8_t* stage, int q, int lane) {
   const int tile = 2 * t.pair + (blockIdx.x & 1), n0 = tile * QL_TILE_N + q * 32;
   const bool in_turn = p.way == QL_IN_TURN;
   float* buf = reinterpret_cast<float*>(stage);   // [8][36]
@@ -292,21 +304,22 @@ __device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& 
     const int m = t.chunk * p.m_pad + s + r;
     float v[8];
     {
-      uint32_t e[8];
+      uint32_t e[8], o[8];
       tmem_ld8_issue(acc + s, e);
+      if (two) tmem_ld8_issue(acc1 + s, o);
       tmem_wait_ld();
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        asm volatile("" : "+r"(e[j]));   // no use before the wait
-        v[j] = __uint_as_float(e[j]) * p.back0 * p.back1;
+        asm volatile("" : "+r"(e[j]), "+r"(o[j]));   // no use before the wait
+        v[j] = (two ? __uint_as_float(e[j]) + __uint_as_float(o[j]) : __uint_as_float(e[j])) * p.back0 * p.back1;
       }
     }
     if (in_turn && !(t.first && t.last)) {
-      float* before = sums + s * QL_TILE_N + q * 32 + lane;
+      float4* before = ql_sums_of(sums, s, q * 32 + lane);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        if (!t.first) v[j] = before[j * QL_TILE_N] + v[j];
-        if (!t.last) before[j * QL_TILE_N] = v[j];
+      for (int j = 0; j < 8; j += 4) {
+        if (!t.first) ql_add4(v + j, before[j / 4 * QL_TILE_N]);
+        if (!t.last) before[j / 4 * QL_TILE_N] = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
       }
       if (!t.last) continue;
     }
@@ -347,7 +360,7 @@ __device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& 
 // Many rows: slices of 16, unrolled, lanes taking eight rows of the activation each. The first group's warps get an instruction in about
 // ten cycles between those of the dequantisers, so their number counts: 4096 x 14336 at 2048 rows 175 -> 163 us against the form
 // above, with stores of 2 bytes a lane 172.
-__device__ __forceinline__ void ql_drain_wide(const QlKernelParams& p, const QlTask& t, uint32_t acc, int gi, int ng, float* sums, uint8_t* stage, int q, int lane) {
+__device__ __forceinline__ void ql_drain_wide(const QlKernelParams& p, const QlTask& t, uint32_t acc, bool two, uint32_t acc1, int gi, int ng, float* sums, uint8_t* stage, int q, int lane) {
   const int tile = 2 * t.pair + (blockIdx.x & 1), n_in = q * 32 + lane, n0 = tile * QL_TILE_N + q * 32, n = n0 + lane;
   const bool live = n < p.N, in_turn = p.way == QL_IN_TURN, apart = p.way == QL_APART && p.splits > 1;
   for (int s = gi; s < p.m_pad >> 4; s += ng) {
@@ -362,19 +375,28 @@ __device__ __forceinline__ void ql_drain_wide(const QlKernelParams& p, const QlT
         asm volatile("" : "+r"(e[j]));   // no use before the wait
         v[j] = __uint_as_float(e[j]);
       }
+      if (two) {
+        tmem_ld16_issue(acc1 + s * 16, e);
+        tmem_wait_ld();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          asm volatile("" : "+r"(e[j]));
+          v[j] += __uint_as_float(e[j]);
+        }
+      }
     }
     if (p.back0 != 1.f) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) v[j] = v[j] * p.back0 * p.back1;
     }
-    float* before = sums + s * 16 * QL_TILE_N + n_in;
+    float4* before = ql_sums_of(sums, s * 16, n_in);
     if (in_turn && !t.first) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = before[j * QL_TILE_N] + v[j];
+      for (int j = 0; j < 16; j += 4) ql_add4(v + j, before[j / 4 * QL_TILE_N]);
     }
     if (in_turn && !t.last) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) before[j * QL_TILE_N] = v[j];
+      for (int j = 0; j < 16; j += 4) before[j / 4 * QL_TILE_N] = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     } else if (apart) {
       float* out = p.partial + ((size_t)t.split * p.M + m0) * p.N;
       if (p.vec) {
@@ -448,7 +470,10 @@ __device__ __forceinline__ void ql_drain_wide(const QlKernelParams& p, const QlT
 // k-blocks of a 128-row tile, expands the 64 weights of a k-block in registers and writes them with one tcgen05.st (column c =
 // weights 2c and 2c + 1), so the MMAs read only the activation k-block from shared memory.
 //
-// TMEM columns: [accs accumulators of round32(m_pad)] [a_slots x unit x 32 columns of bf16 pairs].
+// TMEM columns: [accs accumulators of round32(m_pad)] [a_slots x unit x 32 columns of bf16 pairs]. With two chains an accumulator is two
+// beside each other up to 64 rows: a unit has a k-block of each. A cluster takes a task's even k-blocks first, then the odd ones, and each
+// chain has an accumulator with a barrier of its own: three of 128 rows are as many as tensor memory holds, and the third is what a task starts
+// with while the one before it is drained.
 // ---------------------------------------------------------------------------
 
 // A wait whose loop holds one instruction: a try_wait comes back after 4 us at the latest, so many of them are 1.6 s.
@@ -487,7 +512,8 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   const uint32_t r_bytes = UNIT * p.record_bytes;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int side = blockIdx.x & 1;             // in a cluster: the CTA's rank
-  const uint32_t cs = (uint32_t)(p.m_pad + 31) & ~31u, a_col0 = p.accs * cs;
+  const uint32_t cs = (uint32_t)(p.m_pad + 31) & ~31u, acc_cols = CG == 1 ? p.chains * cs : cs, a_col0 = p.accs * acc_cols;
+  const int loops = CG == 1 ? 1 : p.chains, halves = loops - 1;   // a task's k-blocks are taken `loops` at a step, as often
 
   uint8_t* sB = smem;
   uint8_t* sR = sB + (size_t)p.b_slots * b_bytes;
@@ -505,14 +531,14 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
   const uint32_t raw_empty = raw_full + r_end;    // .. and read
   const uint32_t done = raw_empty + r_end;        // by activation slot: the unit's products are; its other slots are free
   const uint32_t ready = done + b_end;            // .. its activations are in, of both CTAs, and its weights dequantised
-  const uint32_t acc_full = ready + b_end;        // a task's products are in
-  const uint32_t acc_free = acc_full + 16;        // .. its accumulator has been read, and holds what the next one goes on from
+  const uint32_t acc_full = ready + b_end;        // an accumulator's products are in
+  const uint32_t acc_free = acc_full + 32;        // .. it has been read, and holds what the next ones go on from
 
   pdl_launch_dependents();
   if (threadIdx.x == 0) {
     for (int i = 0; i < p.r_slots; ++i) { mbar_init(raw_full + 8 * i, 1); mbar_init(raw_empty + 8 * i, 4); }
     for (int i = 0; i < p.b_slots; ++i) { mbar_init(ready + 8 * i, 4 * CG + 1); mbar_init(done + 8 * i, 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_free + 8 * i, 4 * CG); }
+    for (int i = 0; i < p.accs; ++i) { mbar_init(acc_full + 8 * i, 1); mbar_init(acc_free + 8 * i, 4 * CG); }
     mbar_fence_init();
   }
   if (warp == 2) tmem_alloc<CG>(tmem_slot, p.tmem_cols);
@@ -531,14 +557,15 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     if (warp == 0 && elect_one()) {
       // the weight records, which depend on no kernel before this one
       const uint32_t r0 = smem_u32(sR);
-      const size_t pitch = (size_t)QL_TILE_GROUP * p.record_bytes;
+      const size_t pitch = (size_t)QL_TILE_GROUP * p.record_bytes, step = pitch * (CG == 1 ? UNIT : loops);
       uint32_t dst = r0, slot = 0, phase = 1;
       bool ok = true;
       QlTasks tasks(p, *cuts);
       QlTask t;
       while (ok && tasks.next(t)) {
         const int tile = 2 * t.pair + side;
-        const uint8_t* src = p.records + ((size_t)(tile / QL_TILE_GROUP) * p.kblocks + t.kb0) * pitch + (size_t)(tile % QL_TILE_GROUP) * p.record_bytes;
+        const uint8_t* first = p.records + ((size_t)(tile / QL_TILE_GROUP) * p.kblocks + t.kb0) * pitch + (size_t)(tile % QL_TILE_GROUP) * p.record_bytes;
+        const uint8_t* src = first;
         auto copy = [&](int kbs) {
           const uint32_t full = raw_full + slot;
           ok = mbar_wait_count(raw_empty + slot, phase);
@@ -546,11 +573,18 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
           mbar_arrive_expect_tx(full, kbs * p.record_bytes);
           bulk_g2s(dst, src, p.record_bytes, full);
           if (kbs > 1) bulk_g2s(dst + p.record_bytes, src + pitch, p.record_bytes, full);
-          src += UNIT * pitch; dst += r_bytes; slot += 8;
+          src += step; dst += r_bytes; slot += 8;
           if (slot == r_end) { slot = 0; dst = r0; phase ^= 1u; }
         };
-        for (int n = t.nkb / UNIT; ok && n > 0; --n) copy(UNIT);
-        if (UNIT == 2 && ok && (t.nkb & 1)) copy(1);
+        if (UNIT == 2) {
+          for (int n = t.nkb / 2; ok && n > 0; --n) copy(2);
+          if (ok && (t.nkb & 1)) copy(1);
+        } else {
+          for (int c = 0; c < loops; ++c) {
+            src = first + c * pitch;
+            for (int n = (t.nkb + halves - c) >> halves; ok && n > 0; --n) copy(1);
+          }
+        }
       }
       if (!ok) ql_gave_up(p.status, 1);
     } else if (warp == 1 && elect_one()) {
@@ -564,17 +598,25 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
       while (ok && tasks.next(t)) {
         const int row = p.row0 + t.chunk * p.m_pad + (CG == 2 ? side * (p.m_pad / 2) : 0);
         int x = t.kb0 * QL_KB;
+        const int step = QL_KB * (CG == 1 ? UNIT : loops);
         auto copy = [&](int kbs) {
           ok = mbar_wait_count(done + slot, phase);
           if (!ok) return;
           if (CG == 1 || side == 0) mbar_arrive_expect_tx(ready + slot, kbs * kb_bytes * CG);
           tma_load_2d_pair<CG>(dst, &map_rows, x, row, lead + slot);
           if (kbs > 1) tma_load_2d_pair<CG>(dst + kb_bytes, &map_rows, x + QL_KB, row, lead + slot);
-          x += UNIT * QL_KB; dst += b_bytes; slot += 8;
+          x += step; dst += b_bytes; slot += 8;
           if (slot == b_end) { slot = 0; dst = b0; phase ^= 1u; }
         };
-        for (int n = t.nkb / UNIT; ok && n > 0; --n) copy(UNIT);
-        if (UNIT == 2 && ok && (t.nkb & 1)) copy(1);
+        if (UNIT == 2) {
+          for (int n = t.nkb / 2; ok && n > 0; --n) copy(2);
+          if (ok && (t.nkb & 1)) copy(1);
+        } else {
+          for (int c = 0; c < loops; ++c) {
+            x = (t.kb0 + c) * QL_KB;
+            for (int n = (t.nkb + halves - c) >> halves; ok && n > 0; --n) copy(1);
+          }
+        }
       }
       if (!ok) ql_gave_up(p.status, 2);
     } else if (warp == 2 && (CG == 1 || side == 0) && elect_one()) {
@@ -585,13 +627,15 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
       const uint32_t d_hi = (uint32_t)(proto >> 32), b_lo0 = (uint32_t)proto | ((smem_u32(sB) >> 4) & 0x3FFF), b_step = b_bytes >> 4, kb_step = kb_bytes >> 4;
       const uint32_t a_first = tmem_base + a_col0, a_last = a_first + p.a_slots * UNIT * 32;
       uint32_t a_t = a_first, b_lo = b_lo0, slot = 0, phase = 0;
-      uint32_t buf = 0, fphase = 0;                   // the task's accumulator
+      uint32_t buf = 0, fphase = 0;                   // the accumulator
+      const uint32_t apart = CG == 1 && p.chains == 2 ? cs : 0u, one = apart ? 0u : 1u;   // a unit's second k-block: to its own chain, or after the first
       bool ok = true;
       QlTasks tasks(p, *cuts);
       QlTask t;
       while (ok && tasks.next(t)) {
+       for (int c = 0; ok && c < loops; ++c) {
         ok = mbar_wait_count(acc_free + 8 * buf, fphase);
-        const uint32_t d = tmem_base + buf * cs;
+        const uint32_t d = tmem_base + buf * acc_cols;
         uint32_t acc = tasks.goes_on(t) ? 1u : 0u;
         auto issue = [&](int kbs) {
           ok = mbar_wait_count(ready + slot, phase);
@@ -601,7 +645,7 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
           for (int ks = 0; ks < QL_KB / 16; ++ks) ql_mma<CG>(d, a_t + 8 * ks, b_lo + 2 * ks, d_hi, idesc, ks == 0 ? acc : 1u);
           if (kbs > 1) {
 #pragma unroll
-            for (int ks = 0; ks < QL_KB / 16; ++ks) ql_mma<CG>(d, a_t + 32 + 8 * ks, b_lo + kb_step + 2 * ks, d_hi, idesc, 1u);
+            for (int ks = 0; ks < QL_KB / 16; ++ks) ql_mma<CG>(d + apart, a_t + 32 + 8 * ks, b_lo + kb_step + 2 * ks, d_hi, idesc, ks == 0 ? acc | one : 1u);
           }
           acc = 1;
           ql_commit<CG>(done + slot);
@@ -609,10 +653,15 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
           if (a_t == a_last) a_t = a_first;
           if (slot == b_end) { slot = 0; b_lo = b_lo0; phase ^= 1u; }
         };
-        for (int n = t.nkb / UNIT; ok && n > 0; --n) issue(UNIT);
-        if (UNIT == 2 && ok && (t.nkb & 1)) issue(1);
+        if (UNIT == 2) {
+          for (int n = t.nkb / 2; ok && n > 0; --n) issue(2);
+          if (ok && (t.nkb & 1)) issue(1);
+        } else {
+          for (int n = (t.nkb + halves - c) >> halves; ok && n > 0; --n) issue(1);
+        }
         if (ok) ql_commit<CG>(acc_full + 8 * buf);
         if (++buf == (uint32_t)p.accs) { buf = 0; fphase ^= 1u; }
+       }
       }
       if (!ok) ql_gave_up(p.status, 4);
     }
@@ -673,41 +722,45 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
     QlTasks ahead(p, *cuts);
     QlTask t{}, next{}, fresh{};
     bool more = group == 0 && tasks.next(next), some = group == 0 && ahead.next(fresh), last = group > 0, released = false;
-    uint32_t acc = 0, facc = 0;
-    int prepared = 0;                              // accumulators that are, of tasks not yet drained
-    auto turn = [&](uint32_t a) { return (a & 1) + 1 == (uint32_t)p.accs ? (a & ~1u) ^ 2u : a + 1; };
+    uint32_t acc = 0, facc = 0;                    // index in bits 0 and 1, parity in bit 2
+    int prepared = 0, chain = 0;                   // accumulators that are, of tasks not yet drained; of `fresh`, the next one
+    auto turn = [&](uint32_t a) { return (a & 3) + 1 == (uint32_t)p.accs ? (a & 4) ^ 4u : a + 1; };
+    auto at = [&](uint32_t a) { return lanes + (a & 3) * acc_cols; };
     while (more || last) {
       if (group == 0) {
         while (some && prepared < p.accs) {
           if (ahead.goes_on(fresh)) {
             // Where the task before it is the one that leaves sums for another team, whichever of the two can go first goes first:
             // if all teams waited to go on they would wait for one another in a row.
-            if (prepared > 0 && cuts->segments == 2) {
-              const uint4* first = ql_fix_slot(p, fresh.chunk, (blockIdx.x >> 1) - 1, q * 32 + lane);
+            if (prepared > chain && cuts->segments == 2) {
+              const uint4* first = ql_fix_slot(p, fresh.chunk, chain, (blockIdx.x >> 1) - 1, q * 32 + lane);
+              const uint32_t before = loops == 2 ? turn(acc) : acc;
               if (!released) { pdl_wait(); released = true; }
               bool there = false, over = !ok;
               const unsigned long long t0 = globaltimer_ns();
               while (!there && !over) {
                 uint4 v;
                 there = __all_sync(0xffffffffu, ql_fix_load(first, v));
-                over = __all_sync(0xffffffffu, mbar_test_wait(acc_full + 8 * (acc & 1), acc >> 1)) || __any_sync(0xffffffffu, globaltimer_ns() - t0 > KC_SPIN_LIMIT_NS);
+                over = __all_sync(0xffffffffu, mbar_test_wait(acc_full + 8 * (before & 3), before >> 2)) || __any_sync(0xffffffffu, globaltimer_ns() - t0 > KC_SPIN_LIMIT_NS);
               }
               if (!there) break;
             }
             if (!released) { pdl_wait(); released = true; }
-            if (ok) ok = ql_go_on(p, fresh, lanes + (facc & 1) * cs, q, lane);
+            if (ok) ok = ql_go_on(p, fresh, chain, at(facc), q, lane);
+            if (CG == 1 && p.chains == 2 && ok) ok = ql_go_on(p, fresh, 1, at(facc) + cs, q, lane);
           }
           tc_fence_before();
           __syncwarp();
           if (lane == 0) {
-            if (CG == 1) mbar_arrive(acc_free + 8 * (facc & 1));
-            else mbar_arrive_cluster(cluster_addr(acc_free + 8 * (facc & 1), 0));
+            if (CG == 1) mbar_arrive(acc_free + 8 * (facc & 3));
+            else mbar_arrive_cluster(cluster_addr(acc_free + 8 * (facc & 3), 0));
           }
           facc = turn(facc); ++prepared;
-          some = ahead.next(fresh);
+          if (++chain == loops) { chain = 0; some = ahead.next(fresh); }
         }
         t = next; t.acc = acc;
         acc = turn(acc);
+        if (loops == 2) { t.acc1 = acc; acc = turn(acc); }
         more = tasks.next(next); last = !more;
       }
       if (last) {   // which one, and the sums so far, are there for all who read them
@@ -716,16 +769,19 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
         t = *last_task;
       }
       if (!released) { pdl_wait(); released = true; }   // the stores may overwrite what an earlier kernel still reads
-      if (ok) ok = warp_wait(acc_full + 8 * (t.acc & 1), t.acc >> 1, p.status, KC_DEV_QLINEAR | 7);
+      if (ok) ok = warp_wait(acc_full + 8 * (t.acc & 3), t.acc >> 2, p.status, KC_DEV_QLINEAR | 7);
+      if (ok && loops == 2) ok = warp_wait(acc_full + 8 * (t.acc1 & 3), t.acc1 >> 2, p.status, KC_DEV_QLINEAR | 7);
       tc_fence_after();
-      if (p.way == QL_RUNS && !t.last) {
-        if (ok) ql_leave(p, t, lanes + (t.acc & 1) * cs, q, lane);   // never the last task: a run starts with it
+      const uint32_t acc0 = at(t.acc), acc1 = CG == 1 ? acc0 + cs : at(t.acc1);
+      if (p.way == QL_RUNS && !t.last) {   // never the last task: a run starts with it
+        if (ok) ql_leave(p, t, 0, acc0, q, lane);
+        if (ok && p.chains == 2) ql_leave(p, t, 1, acc1, q, lane);
       } else if (ok) {
-        if (CG == 1) ql_drain(p, t, lanes + (t.acc & 1) * cs, group, last ? QL_GROUPS : 1, sums, stage, q, lane);
-        else ql_drain_wide(p, t, lanes + (t.acc & 1) * cs, group, last ? QL_GROUPS : 1, sums, stage, q, lane);
+        if (CG == 1) ql_drain(p, t, acc0, tasks.second(t), acc1, group, last ? QL_GROUPS : 1, sums, stage, q, lane);
+        else ql_drain_wide(p, t, acc0, tasks.second(t), acc1, group, last ? QL_GROUPS : 1, sums, stage, q, lane);
       }
       if (last) break;
-      --prepared;
+      prepared -= loops;
     }
   }
   __syncwarp();
@@ -757,11 +813,13 @@ size_t qlinear_fix_bytes(int sm_count) { return (size_t)QL_FIX_CHUNKS * (sm_coun
 // activation slots, by which a unit's barriers go, as many as A slots at least.
 static bool plan_rings(UmmaPlan* t, const QWeight& w, bool several_tasks, bool sums) {
   const int cs = (t->m_pad + 31) & ~31, unit = ql_unit(t->cg);
-  t->accs = several_tasks ? 2 : 1;
-  t->a_slots = std::min(8, (512 - t->accs * cs) / (unit * 32));
+  // of a cluster an accumulator a chain: a task's, and as much of the next one's as leaves three A slots
+  t->accs = t->cg == 1 ? several_tasks + 1 : several_tasks ? std::min(2 * w.chains, std::max(w.chains, (512 - 96) / cs)) : w.chains;
+  const int acc_cols = t->accs * (t->cg == 1 ? w.chains * cs : cs);
+  t->a_slots = std::min(8, (512 - acc_cols) / (unit * 32));
   const size_t extra = 1024 + 1024 + 4 * QL_GROUPS * QL_STAGE_BYTES + (sums ? (size_t)t->m_pad * QL_TILE_N * 4 : 0);
   const size_t all = (size_t)227 * 1024, b_slot = (size_t)unit * t->m_pad / t->cg * 128, r_slot = (size_t)unit * w.record_bytes;
-  auto bytes = [&](int b, int r) { return extra + b * b_slot + r * r_slot; };   // 1024: barriers, at most 24 * 2 + 12 * 2 + 4, and the words before them
+  auto bytes = [&](int b, int r) { return extra + b * b_slot + r * r_slot; };   // 1024: barriers, at most 24 * 2 + 12 * 2 + 8, and the words before them
   while (t->a_slots > 3 && bytes(t->a_slots, 6) > all) --t->a_slots;
   t->r_slots = 6; t->b_slots = t->a_slots;
   if (t->a_slots < 3 || bytes(t->b_slots, t->r_slots) > all) return false;
@@ -771,7 +829,7 @@ static bool plan_rings(UmmaPlan* t, const QWeight& w, bool several_tasks, bool s
     if (t->b_slots < 12 && bytes(t->b_slots + 1, t->r_slots) <= all) { ++t->b_slots; more = true; }
   }
   t->tmem_cols = 32;
-  while ((int)t->tmem_cols < t->accs * cs + t->a_slots * unit * 32) t->tmem_cols <<= 1;
+  while ((int)t->tmem_cols < acc_cols + t->a_slots * unit * 32) t->tmem_cols <<= 1;
   t->smem = bytes(t->b_slots, t->r_slots);
   return true;
 }
@@ -851,7 +909,7 @@ static int plan_whole_rows(const QWeight& w, int M, int fix, bool* runs) {
     const int chunks = (M + per - 1) / per;
     if (chunks > 1 && per <= QL_SOLO_ROWS) break;
     const double whole = (double)((pairs * (long long)chunks + teams - 1) / teams) * w.kblocks, cut = ((double)pairs * w.kblocks / teams + 8) * chunks;
-    const bool r = chunks <= fix && cut < whole;
+    const bool r = chunks * per * w.chains <= fix * QL_CHUNK_ROWS && cut < whole;
     const double cost = (r ? cut : whole) * (std::max(256, 2 * per) + 20);
     if (best == 0 || cost < best_cost * 0.995) { best = per; best_cost = cost; *runs = r; }
   }
@@ -906,7 +964,7 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   if (!plan_rings(&t, w, several, sums)) return cudaErrorInvalidValue;
   QlKernelParams p;
   p.records = w.records; p.record_bytes = w.record_bytes;
-  p.N = w.N; p.kblocks = w.kblocks; p.n_pairs = pairs; p.splits = w.splits; p.teams = t.teams;
+  p.N = w.N; p.kblocks = w.kblocks; p.n_pairs = pairs; p.splits = w.splits; p.chains = w.chains; p.teams = t.teams;
   p.M = l.M; p.m_pad = t.m_pad; p.chunks = t.chunks; p.row0 = l.row0;
   p.way = t.way;
   p.a_slots = t.a_slots; p.b_slots = t.b_slots; p.r_slots = t.r_slots; p.accs = t.accs; p.tmem_cols = t.tmem_cols;

@@ -306,3 +306,29 @@ def test_teams_that_share_a_pair_carry_its_bits(ctx, n, k, bits, group):
         y = qw.matmul(x[:m])
         assert torch.equal(y.view(torch.int16), want[:m].view(torch.int16)), m
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("n,k,bits,group", [
+    (384, 1088, 4, 32),           # splits of 8 and 9 k-blocks
+    (4096, 2048, 8, 32),          # four splits, apart and in turn
+    (11000, 256, 4, 64),          # not split
+    (19000, 1088, 4, 64),         # not split, pairs of tiles cut between teams
+])
+def test_even_and_odd_k_blocks_are_sums_of_their_own(ctx, n, k, bits, group):
+    """Weights of fewer than 207 tiles: a split is two chains of products, its even and its odd k-blocks, half as long as one. Exact:
+    a large value and its negative two k-blocks on cancel, and take what one sum would have had between them with it."""
+    tiles, blocks = -(-n // 128), k // 64
+    splits = 1 if 2 * tiles >= 148 else max(1, min(148 // tiles, 16, blocks // 8))
+    packed = torch.full((n, k * bits // 32), 0x11111111 if bits == 4 else 0x01010101, dtype=torch.int32)
+    one = torch.ones(n, k // group, dtype=torch.bfloat16)
+    qw = api.QuantizedWeight(ctx, packed.cuda(), one.cuda(), (one * 0).cuda(), bits, group)
+    rows = torch.arange(1100)
+    x = torch.zeros(1100, k)
+    for s in range(splits):
+        at = blocks * s // splits * 64
+        x[:, at], x[:, at + 64], x[:, at + 128] = 2.0 ** 30, (rows % 7 + 1).float(), -2.0 ** 30
+    x = x.to(torch.bfloat16).cuda()
+    want = ((rows % 7 + 1) * splits).float().reshape(-1, 1)
+    for m in (1, 17, 64, 65, 130, 192, 320, 1100):
+        assert torch.equal(qw.matmul(x[:m]).cpu().float(), want[:m].expand(m, n)), m
+    assert ctx.device_status() == 0
