@@ -151,6 +151,7 @@ __global__ void __launch_bounds__(GREEDY_THREADS, NV <= 8 ? 4 : NV <= 10 ? 3 : 2
 greedy_cluster_kernel(const bf16* __restrict__ logits, int vocab, int slice, int normalize, uint32_t* __restrict__ tokens,
                       uint32_t* __restrict__ tokens_host, const volatile uint32_t* status, uint32_t* __restrict__ status_copy) {
   pdl_launch_dependents();
+  cluster_arrive();                      // waited for before the first store into another CTA's shared memory: it has started by then
   pdl_wait();
   const bool notes = status_copy && blockIdx.x == 0 && threadIdx.x == 0;
   const uint32_t st = notes ? *status : 0u;   // host memory: on its way under the passes below
@@ -176,6 +177,7 @@ greedy_cluster_kernel(const bf16* __restrict__ logits, int vocab, int slice, int
   float m = warp_max(fmaxf(two.x, two.y));
   if (lane == 0) red_m[warp] = m;
   __syncthreads();
+  cluster_wait();
   if (threadIdx.x < GREEDY_CTAS) {       // this CTA's maximum, to every CTA
     m = red_m[0];
     for (int w = 1; w < nw; ++w) m = fmaxf(m, red_m[w]);

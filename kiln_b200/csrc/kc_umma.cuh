@@ -94,9 +94,11 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t base, uint32_t cols) {
   if (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
   else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(cols) : "memory");
 }
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-}
+// All threads of the cluster's CTAs: what they did before they arrived is seen after the wait. Before the first one a CTA of the cluster
+// may not have started, and its shared memory must not be touched.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_sync() { cluster_arrive(); cluster_wait(); }
 // The shared::cluster address of what `addr` is in this CTA, in the cluster's CTA `rank`.
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
   uint32_t r;

@@ -1,0 +1,38 @@
+"""Rules of the device code that a run on a GPU cannot show to be kept, since what breaks them nearly always works: read from the
+sources. Needs no GPU."""
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parent.parent / "kiln_b200" / "csrc"
+
+
+def functions(qualifier):
+    """(file, name, body) of the functions of that kind."""
+    for path in sorted(CSRC.glob("*.cu*")):
+        text = re.sub(r"//[^\n]*", "", path.read_text())
+        for m in re.finditer(qualifier + r"\s+(?:[\w:*&<>]+\s+)*(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(", text):
+            start = text.index("{", m.end())
+            depth, at = 1, start + 1
+            while depth:
+                depth += {"{": 1, "}": -1}.get(text[at], 0)
+                at += 1
+            yield path.name, m.group(1), text[start:at]
+
+
+KERNELS = {name: (path, body) for path, name, body in functions("__global__")}
+
+
+def test_the_kernels_are_found():
+    assert {"greedy_cluster_kernel", "qlinear_umma_kernel", "attn_kernel", "attn_keys_kernel", "add_rmsnorm_kernel"} <= set(KERNELS)
+
+
+@pytest.mark.parametrize("name", sorted(KERNELS))
+def test_peers_have_started_before_their_shared_memory_is_touched(name):
+    """CTAs of a cluster may start one after the other: a cluster barrier comes before the first access to another one's memory."""
+    body = KERNELS[name][1]
+    remote = [m.start() for m in re.finditer(r"shared::cluster|mbar_arrive_cluster\(|cluster_addr\(", body)]
+    if remote:
+        barrier = [m.start() for m in re.finditer(r"cluster_sync\(\)|cluster_wait\(\)", body)]
+        assert barrier and barrier[0] < remote[0]
