@@ -222,13 +222,18 @@ struct QlTasks {
 
 // The sums that a run leaves of a pair whose end it does not hold: [row / 4][128][4], of a CTA. Between launches every word is
 // QL_NOTHING, and a word that is something else is there: the reader polls the sums themselves and puts QL_NOTHING back. A word
-// that says so needs a fence before it, which took 4 us beside the copies that are under way.
+// that says so needs a fence before it, which took 4 us beside the copies that are under way. Relaxed accesses on both sides: a plain store beside
+// a load of the same word would be a race.
 __device__ __forceinline__ uint4* ql_fix_slot(const QlKernelParams& p, int chunk, int chain, int team, int row) {
   return p.fix + (((size_t)(chunk * p.chains + chain) * p.teams + team) * 2 + (blockIdx.x & 1)) * (p.m_pad / 4) * QL_TILE_N + row;
 }
 __device__ __forceinline__ bool ql_fix_load(const uint4* src, uint4& v) {
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src) : "memory");
   return v.x != QL_NOTHING && v.y != QL_NOTHING && v.z != QL_NOTHING && v.w != QL_NOTHING;
+}
+
+__device__ __forceinline__ void ql_fix_store(uint4* dst, uint4 v) {
+  asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
 // Puts another team's sums of a chain into a task's accumulator: one group's warps, a lane quarter each.
@@ -255,7 +260,7 @@ __device__ __forceinline__ bool ql_go_on(const QlKernelParams& p, const QlTask& 
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       v[4 * j] = f[j].x; v[4 * j + 1] = f[j].y; v[4 * j + 2] = f[j].z; v[4 * j + 3] = f[j].w;
-      if (s / 4 + j <= last) src[(s / 4 + j) * QL_TILE_N] = nothing;
+      if (s / 4 + j <= last) ql_fix_store(src + (s / 4 + j) * QL_TILE_N, nothing);
     }
     tmem_st32(acc + s, v);
   }
@@ -276,7 +281,7 @@ __device__ __forceinline__ void ql_leave(const QlKernelParams& p, const QlTask& 
       e[j] = e[j] == QL_NOTHING ? 0x7FFFFFFFu : e[j];   // both are NaN
     }
 #pragma unroll
-    for (int j = 0; j < 16; j += 4) dst[j / 4 * QL_TILE_N] = make_uint4(e[j], e[j + 1], e[j + 2], e[j + 3]);
+    for (int j = 0; j < 16; j += 4) ql_fix_store(dst + j / 4 * QL_TILE_N, make_uint4(e[j], e[j + 1], e[j + 2], e[j + 3]));
   }
 }
 

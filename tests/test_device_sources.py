@@ -36,3 +36,17 @@ def test_peers_have_started_before_their_shared_memory_is_touched(name):
     if remote:
         barrier = [m.start() for m in re.finditer(r"cluster_sync\(\)|cluster_wait\(\)", body)]
         assert barrier and barrier[0] < remote[0]
+
+
+DEVICE = {name: body for _, name, body in functions("__device__ __forceinline__")}
+
+
+def test_sums_between_teams_are_stored_as_they_are_polled():
+    """What one team leaves in global memory while another one polls it: relaxed stores and loads, never a plain access through the
+    pointer."""
+    assert "ld.relaxed.gpu" in DEVICE["ql_fix_load"] and "st.relaxed.gpu" in DEVICE["ql_fix_store"]
+    for name in ("ql_leave", "ql_go_on"):
+        pointers = re.findall(r"uint4\* (\w+) = ql_fix_slot", DEVICE[name])
+        assert pointers
+        for p in pointers:
+            assert not re.search(rf"\b{p}\[|\*{p}\b", DEVICE[name])
