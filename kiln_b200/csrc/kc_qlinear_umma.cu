@@ -307,6 +307,7 @@ __device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& 
 #pragma unroll 1
   for (int s = gi * 8; s < p.m_pad; s += ng * 8) {
     const int m = t.chunk * p.m_pad + s + r;
+    __syncwarp();                        // lanes left the last turn apart; the loads are the warp's
     float v[8];
     {
       uint32_t e[8], o[8];
@@ -370,6 +371,7 @@ __device__ __forceinline__ void ql_drain_wide(const QlKernelParams& p, const QlT
   const bool live = n < p.N, in_turn = p.way == QL_IN_TURN, apart = p.way == QL_APART && p.splits > 1;
   for (int s = gi; s < p.m_pad >> 4; s += ng) {
     const int m0 = t.chunk * p.m_pad + s * 16, rows = min(16, p.M - m0);
+    __syncwarp();                        // as above
     float v[16];
     {
       uint32_t e[16];

@@ -50,3 +50,11 @@ def test_sums_between_teams_are_stored_as_they_are_polled():
         assert pointers
         for p in pointers:
             assert not re.search(rf"\b{p}\[|\*{p}\b", DEVICE[name])
+
+
+@pytest.mark.parametrize("name", ["ql_drain", "ql_drain_wide"])
+def test_a_warp_is_whole_before_it_reads_tensor_memory(name):
+    """tcgen05.ld is an instruction of the whole warp, and lanes may leave a turn of the loop around it apart."""
+    body = DEVICE[name]
+    turn = body[body.index("for ("):]
+    assert 0 < turn.find("__syncwarp()") < turn.index("tmem_ld")
