@@ -483,12 +483,35 @@ __device__ __forceinline__ void ql_drain_wide(const QlKernelParams& p, const QlT
 // with while the one before it is drained.
 // ---------------------------------------------------------------------------
 
-// A wait whose loop holds one instruction: a try_wait comes back after 4 us at the latest, so many of them are 1.6 s.
-__device__ __forceinline__ bool mbar_wait_count(uint32_t bar, uint32_t parity) {
-  int tries = 0;
-  while (!mbar_try_wait(bar, parity))
-    if (++tries > 400000) return false;
-  return true;
+// A wait whose loop holds little. It gives up by the clock, which is looked at once in a thousand tries, however long one takes, and starts when
+// the kernel ahead is done: all roles but the first units' dequantisation depend on that one, and it may take long. In one piece, since a loop of
+// the compiler's took 28672 x 4096 at 1 and 32 rows from 16.1 and 16.9 us to 16.4 and 17.2, and with the rest in a function that is called to 16.4
+// and 17.0 (192 rows 36.7 -> 37.1).
+__device__ __forceinline__ bool ql_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;   // nanoseconds: 32 bits of them are 4.3 s
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t.reg .u32 tries, start, t;\n\t"
+      "mov.u32 tries, 0;\n\tmov.u32 start, 0;\n"
+      "AGAIN%=:\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "@p bra OVER%=;\n\t"
+      "add.u32 tries, tries, 1;\n\t"
+      "and.b32 t, tries, 1023;\n\t"
+      "setp.ne.u32 q, t, 0;\n\t"
+      "@q bra AGAIN%=;\n\t"
+      "griddepcontrol.wait;\n\t"
+      "mov.u32 t, %%globaltimer_lo;\n\t"
+      "setp.eq.u32 q, tries, 1024;\n\t"
+      "selp.u32 start, t, start, q;\n\t"
+      "sub.u32 t, t, start;\n\t"
+      "setp.le.u32 q, t, %4;\n\t"
+      "@q bra AGAIN%=;\n"
+      "OVER%=:\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(20000u), "n"((uint32_t)KC_SPIN_LIMIT_NS)
+      : "memory");
+  return ok != 0;
 }
 // What was asked for still lands in shared memory; it takes microseconds.
 __device__ __noinline__ void ql_gave_up(uint32_t* status, uint32_t wait) {
@@ -575,7 +598,7 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
         const uint8_t* src = first;
         auto copy = [&](int kbs) {
           const uint32_t full = raw_full + slot;
-          ok = mbar_wait_count(raw_empty + slot, phase);
+          ok = ql_wait(raw_empty + slot, phase);
           if (!ok) return;
           mbar_arrive_expect_tx(full, kbs * p.record_bytes);
           bulk_g2s(dst, src, p.record_bytes, full);
@@ -607,7 +630,7 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
         int x = t.kb0 * QL_KB;
         const int step = QL_KB * (CG == 1 ? UNIT : loops);
         auto copy = [&](int kbs) {
-          ok = mbar_wait_count(done + slot, phase);
+          ok = ql_wait(done + slot, phase);
           if (!ok) return;
           if (CG == 1 || side == 0) mbar_arrive_expect_tx(ready + slot, kbs * kb_bytes * CG);
           tma_load_2d_pair<CG>(dst, &map_rows, x, row, lead + slot);
@@ -641,11 +664,11 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
       QlTask t;
       while (ok && tasks.next(t)) {
        for (int c = 0; ok && c < loops; ++c) {
-        ok = mbar_wait_count(acc_free + 8 * buf, fphase);
+        ok = ql_wait(acc_free + 8 * buf, fphase);
         const uint32_t d = tmem_base + buf * acc_cols;
         uint32_t acc = tasks.goes_on(t) ? 1u : 0u;
         auto issue = [&](int kbs) {
-          ok = mbar_wait_count(ready + slot, phase);
+          ok = ql_wait(ready + slot, phase);
           if (!ok) return;
           tc_fence_after();   // the A operand was written with tcgen05.st by other threads
 #pragma unroll
@@ -690,14 +713,14 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
       uint32_t rec = d * r_bytes, raw = 8 * d, a_t = a0 + UNIT * 32 * d, bar = raw, phase = 0;
       uint32_t old = 8 * (p.b_slots - p.a_slots + d), freed = 1;   // barrier of the unit that had the A slot before; none at first
       for (int left = cuts->units - (int)d; left > 0; left -= DQ) {
-        ok = __all_sync(0xffffffffu, mbar_wait_count(raw_full + raw, phase));
+        ok = __all_sync(0xffffffffu, ql_wait(raw_full + raw, phase));
         if (!ok) break;
 #pragma unroll
         for (int k = 0; k < UNIT; ++k) {   // of half a unit at a task's end, the second half is what the slot held before: no MMA reads it
           uint32_t v[32];
           dequant_row<BITS, GPK>(row0 + rec + k * p.record_bytes, sb0 + rec + k * p.record_bytes, p.factors, v);
           if (k == 0) {
-            ok = __all_sync(0xffffffffu, mbar_wait_count(done + old, freed));
+            ok = __all_sync(0xffffffffu, ql_wait(done + old, freed));
             if (!ok) break;
             tc_fence_after();
           }

@@ -38,7 +38,9 @@ def test_peers_have_started_before_their_shared_memory_is_touched(name):
         assert barrier and barrier[0] < remote[0]
 
 
-DEVICE = {name: body for _, name, body in functions("__device__ __forceinline__")}
+DEVICE = {}
+for _, function, text in functions("__device__ __forceinline__"):
+    DEVICE[function] = DEVICE.get(function, "") + text     # overloads together
 
 
 def test_sums_between_teams_are_stored_as_they_are_polled():
@@ -58,3 +60,14 @@ def test_a_warp_is_whole_before_it_reads_tensor_memory(name):
     body = DEVICE[name]
     turn = body[body.index("for ("):]
     assert 0 < turn.find("__syncwarp()") < turn.index("tmem_ld")
+
+
+def test_the_waits_of_the_gemm_are_bounded_by_the_clock():
+    """A limit that counts tries is as long as a try happens to be, and one whose start is the kernel's own counts the kernel ahead of
+    it, which may itself wait for another GPU: the clock, from that kernel's end."""
+    wait = DEVICE["ql_wait"]
+    assert 0 < wait.index("griddepcontrol.wait") < wait.index("globaltimer") < wait.index("KC_SPIN_LIMIT_NS")
+    assert "KC_SPIN_LIMIT_NS" in DEVICE["mbar_wait"]
+    kernel = KERNELS["qlinear_umma_kernel"][1]
+    assert not set(re.findall(r"(\w*mbar_\w*wait\w*)\(", kernel)) - {"mbar_test_wait"}
+    assert kernel.index("pdl_wait()") < kernel.index("warp_wait(")
