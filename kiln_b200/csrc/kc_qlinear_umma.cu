@@ -109,7 +109,12 @@ __host__ __device__ constexpr int ql_unit(int cg) { return cg == 1 ? 2 : 1; }
 //   APART    a team a (pair, split, chunk of rows); the splits are left to the kernel that reads the result, or there is one
 //   RUNS     the k-blocks of all pairs, one after the other, in as many equal runs as the SMs have teams, each at least a pair's:
 //            where a run ends inside a pair, its sums so far go through global memory to the team with the pair's end, which goes
-//            on from them: the same chain of products as one team's
+//            on from them: the same chain of products as one team's. A team waits for the one before it only, having left its own sums
+//            first, so all that it takes is that CTAs start in the order of their indices, or that all are resident: then a waiting
+//            CTA's predecessor runs. CUDA promises neither; the hardware hands CTAs out in order, and a grid has one a SM. With both
+//            broken (another process's waiting kernel on the SMs that are missing) the wait gives up by its limit and the call fails.
+//            Numbers taken from a counter as CTAs start need no such order; they cost the start a round trip: 28672 x 4096 at 1 row 16.1
+//            -> 16.5 us, the one-row step of the 8B model 2025 -> 2053. A cooperative launch: 16.1 -> 20.0, 2025 -> 2143
 //   IN_TURN  a team takes a (pair, chunk) at a time, its splits one after the other, their sums in shared memory
 constexpr int QL_MAX_SPLITS = 16;
 constexpr uint32_t QL_NOTHING = 0xFFFFFFFFu;
