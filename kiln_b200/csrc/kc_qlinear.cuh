@@ -65,10 +65,9 @@ struct QLinearLaunch {
   const ActOperand* x;
   int row0;         // first activation row of this launch (x, y and partial are indexed from it)
   int M;            // live activation rows, at most qlinear_slab_rows
-  bf16* y;          // [M, ldy] bf16 when the weight has splits == 1 or qlinear_in_turn(w, M, summed) (else unused)
+  bf16* y;          // [M, ldy] bf16 when the weight has splits == 1 or qlinear_in_turn(w, M) (else unused)
   int ldy;
   float* partial;   // [splits][M][N] fp32 workspace when splits > 1 (rows relative to row0)
-  bool summed = false;   // partials, if there are any, are summed by the kernel that reads the result, not by one of their own
   // Workspace of qlinear_fix_bytes for what teams that share a weight's k-blocks leave for one another, all its bits set between
   // launches; without it they share whole pairs of tiles. Launches that have the same one run one after the other.
   float* fix = nullptr;
@@ -83,7 +82,6 @@ struct QLinearLaunch {
 };
 
 constexpr int QL_CHUNK_ROWS = 192;   // rows of a chunk, at most: two accumulators of them and four slots of dequantised weights are tensor memory's 512 columns
-constexpr int QL_SOLO_ROWS = 64;     // up to these rows the CTAs of a team read the activations each for itself
 constexpr int QL_FIX_CHUNKS = 3;     // chunks of rows that a launch of cut pairs keeps parts' sums for
 size_t qlinear_fix_bytes(int sm_count);
 
@@ -114,9 +112,8 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s);
 // has 65535 chunks of 96 rows or more, and looking for the best number of them is host time that a launch of a million rows
 // hides. Asked again for each launch, since what a large one leaves may go the other way.
 constexpr int QL_LAUNCH_ROWS = 1 << 20;
-// Whether a launch of M rows takes the splits of its weight one after the other and writes y, no partials. summed: see
-// QLinearLaunch; for at most QL_MAX_M rows only.
-bool qlinear_in_turn(const QWeight& w, int M, bool summed = false);
+// Whether a launch of M rows takes the splits of its weight one after the other and writes y, no partials.
+bool qlinear_in_turn(const QWeight& w, int M);
 inline int qlinear_slab_rows(const QWeight& w, int M) {
   const int all = M < QL_LAUNCH_ROWS ? M : QL_LAUNCH_ROWS;
   return all <= QL_MAX_M || w.splits == 1 || qlinear_in_turn(w, all) ? all : QL_MAX_M;

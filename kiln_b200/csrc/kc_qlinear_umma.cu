@@ -1,7 +1,7 @@
 // The affine-dequant GEMM on the tensor cores. See kc_qlinear.cuh for the data layout.
 //
 // qlinear_umma_kernel — teams of two CTAs. A team has a PAIR of neighbouring 128-row weight tiles at a time, one tile a CTA,
-// and the same k-blocks of both. Up to 64 activation rows its CTAs know nothing of each other; with more they are a cluster
+// and the same k-blocks of both. Up to solo_rows activation rows its CTAs know nothing of each other; with more they are a cluster
 // whose two SMs work on one M = 256 product (tcgen05 cta_group::2), each holding half of the activations. 20 warps:
 //   warp 0        bulk-copies the weight records (cp.async.bulk, mbarrier tx)
 //   warp 1        TMA-loads the activation k-blocks (cp.async.bulk.tensor, 128B swizzle), of a cluster its CTA's half of the rows
@@ -100,14 +100,13 @@ constexpr int QL_GROUP0 = 4;                                   // first warp of 
 constexpr int QL_GROUPS = 4;
 constexpr int QL_THREADS = (QL_GROUP0 + 4 * QL_GROUPS) * 32;   // 20 warps
 constexpr int QL_STAGE_BYTES = 1280;                           // a warp's buffer on the way out: 16 rows of 32 bf16, or 8 of fp32, with padding
-constexpr int QL_SUM_ROWS = 160;                               // rows of a chunk whose parts' sums lie in shared memory, at most
 // k-blocks of a unit: two where a unit's products take few cycles a k-block, one where two accumulators of many rows leave tensor
 // memory for four k-blocks only.
 __host__ __device__ constexpr int ql_unit(int cg) { return cg == 1 ? 2 : 1; }
 
 // How a launch's teams share the work:
 //   APART    a team a (pair, split, chunk of rows); the splits are left to the kernel that reads the result, or there is one
-//   RUNS     the k-blocks of all pairs, one after the other, in as many equal runs as the SMs have teams, each at least a pair's:
+//   RUNS     (of one chain) the k-blocks of all pairs, one after the other, in as many equal runs as the SMs have teams, each at least a pair's:
 //            where a run ends inside a pair, its sums so far go through global memory to the team with the pair's end, which goes
 //            on from them: the same chain of products as one team's. A team waits for the one before it only, having left its own sums
 //            first, so all that it takes is that CTAs start in the order of their indices, or that all are resident: then a waiting
@@ -139,7 +138,7 @@ struct QlKernelParams {
   int vec;               // rows of y, or of the partials, start on 16 bytes, and whole groups of 8 (4) features
   bf16* y; int ldy;
   float* partial;        // APART with several splits: [splits][M][N]
-  uint4* fix;            // RUNS: [chunk][chain][team][CTA][m_pad / 4][128], see ql_fix_slot
+  uint4* fix;            // RUNS: [chunk][team][CTA][m_pad / 4][128], see ql_fix_slot
   uint32_t* status;
 };
 
@@ -222,15 +221,15 @@ struct QlTasks {
   // A task that goes on from another team's sums.
   __device__ bool goes_on(const QlTask& t) const { return p.way == QL_RUNS && !t.first; }
   // The part has an odd k-block: a second chain that is no chain of nothing.
-  __device__ bool second(const QlTask& t) const { return p.chains == 2 && (p.way == QL_RUNS ? p.kblocks : t.nkb) > 1; }
+  __device__ bool second(const QlTask& t) const { return p.chains == 2 && t.nkb > 1; }
 };
 
 // The sums that a run leaves of a pair whose end it does not hold: [row / 4][128][4], of a CTA. Between launches every word is
 // QL_NOTHING, and a word that is something else is there: the reader polls the sums themselves and puts QL_NOTHING back. A word
 // that says so needs a fence before it, which took 4 us beside the copies that are under way. Relaxed accesses on both sides: a plain store beside
 // a load of the same word would be a race.
-__device__ __forceinline__ uint4* ql_fix_slot(const QlKernelParams& p, int chunk, int chain, int team, int row) {
-  return p.fix + (((size_t)(chunk * p.chains + chain) * p.teams + team) * 2 + (blockIdx.x & 1)) * (p.m_pad / 4) * QL_TILE_N + row;
+__device__ __forceinline__ uint4* ql_fix_slot(const QlKernelParams& p, int chunk, int team, int row) {
+  return p.fix + (((size_t)chunk * p.teams + team) * 2 + (blockIdx.x & 1)) * (p.m_pad / 4) * QL_TILE_N + row;
 }
 __device__ __forceinline__ bool ql_fix_load(const uint4* src, uint4& v) {
   asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(src) : "memory");
@@ -241,9 +240,9 @@ __device__ __forceinline__ void ql_fix_store(uint4* dst, uint4 v) {
   asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-// Puts another team's sums of a chain into a task's accumulator: one group's warps, a lane quarter each.
-__device__ __forceinline__ bool ql_go_on(const QlKernelParams& p, const QlTask& t, int chain, uint32_t acc, int q, int lane) {
-  uint4* src = ql_fix_slot(p, t.chunk, chain, (blockIdx.x >> 1) - 1, q * 32 + lane);
+// Puts another team's sums into a task's accumulator: one group's warps, a lane quarter each.
+__device__ __forceinline__ bool ql_go_on(const QlKernelParams& p, const QlTask& t, uint32_t acc, int q, int lane) {
+  uint4* src = ql_fix_slot(p, t.chunk, (blockIdx.x >> 1) - 1, q * 32 + lane);
   const uint4 nothing = make_uint4(QL_NOTHING, QL_NOTHING, QL_NOTHING, QL_NOTHING);
   const int last = p.m_pad / 4 - 1;
   for (int s = 0; s < p.m_pad; s += 32) {   // a round trip to L2 each; the last 16 rows may be past the chunk's, in columns that nothing else has
@@ -273,9 +272,9 @@ __device__ __forceinline__ bool ql_go_on(const QlKernelParams& p, const QlTask& 
   return true;
 }
 
-// Leaves a run's sums of a chain of a pair for the team that has its end: one group's warps, a lane quarter each.
-__device__ __forceinline__ void ql_leave(const QlKernelParams& p, const QlTask& t, int chain, uint32_t acc, int q, int lane) {
-  uint4* dst = ql_fix_slot(p, t.chunk, chain, blockIdx.x >> 1, q * 32 + lane);
+// Leaves a run's sums of a pair for the team that has its end: one group's warps, a lane quarter each.
+__device__ __forceinline__ void ql_leave(const QlKernelParams& p, const QlTask& t, uint32_t acc, int q, int lane) {
+  uint4* dst = ql_fix_slot(p, t.chunk, blockIdx.x >> 1, q * 32 + lane);
   for (int s = 0; s < p.m_pad; s += 16, dst += 4 * QL_TILE_N) {
     uint32_t e[16];
     tmem_ld16_issue(acc + s, e);
@@ -483,7 +482,7 @@ __device__ __forceinline__ void ql_drain_wide(const QlKernelParams& p, const QlT
 // weights 2c and 2c + 1), so the MMAs read only the activation k-block from shared memory.
 //
 // TMEM columns: [accs accumulators of round32(m_pad)] [a_slots x unit x 32 columns of bf16 pairs]. With two chains an accumulator is two
-// beside each other up to 64 rows: a unit has a k-block of each. A cluster takes a task's even k-blocks first, then the odd ones, and each
+// beside each other where CTAs work alone: a unit has a k-block of each. A cluster takes a task's even k-blocks first, then the odd ones, and each
 // chain has an accumulator with a barrier of its own: three of 128 rows are as many as tensor memory holds, and the third is what a task starts
 // with while the one before it is drained.
 // ---------------------------------------------------------------------------
@@ -767,22 +766,20 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
           if (ahead.goes_on(fresh)) {
             // Where the task before it is the one that leaves sums for another team, whichever of the two can go first goes first:
             // if all teams waited to go on they would wait for one another in a row.
-            if (prepared > chain && cuts->segments == 2) {
-              const uint4* first = ql_fix_slot(p, fresh.chunk, chain, (blockIdx.x >> 1) - 1, q * 32 + lane);
-              const uint32_t before = loops == 2 ? turn(acc) : acc;
+            if (prepared > 0 && cuts->segments == 2) {
+              const uint4* first = ql_fix_slot(p, fresh.chunk, (blockIdx.x >> 1) - 1, q * 32 + lane);
               if (!released) { pdl_wait(); released = true; }
               bool there = false, over = !ok;
               const unsigned long long t0 = globaltimer_ns();
               while (!there && !over) {
                 uint4 v;
                 there = __all_sync(0xffffffffu, ql_fix_load(first, v));
-                over = __all_sync(0xffffffffu, mbar_test_wait(acc_full + 8 * (before & 3), before >> 2)) || __any_sync(0xffffffffu, globaltimer_ns() - t0 > KC_SPIN_LIMIT_NS);
+                over = __all_sync(0xffffffffu, mbar_test_wait(acc_full + 8 * (acc & 3), acc >> 2)) || __any_sync(0xffffffffu, globaltimer_ns() - t0 > KC_SPIN_LIMIT_NS);
               }
               if (!there) break;
             }
             if (!released) { pdl_wait(); released = true; }
-            if (ok) ok = ql_go_on(p, fresh, chain, at(facc), q, lane);
-            if (CG == 1 && p.chains == 2 && ok) ok = ql_go_on(p, fresh, 1, at(facc) + cs, q, lane);
+            if (ok) ok = ql_go_on(p, fresh, at(facc), q, lane);
           }
           tc_fence_before();
           __syncwarp();
@@ -809,8 +806,7 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
       tc_fence_after();
       const uint32_t acc0 = at(t.acc), acc1 = CG == 1 ? acc0 + cs : at(t.acc1);
       if (p.way == QL_RUNS && !t.last) {   // never the last task: a run starts with it
-        if (ok) ql_leave(p, t, 0, acc0, q, lane);
-        if (ok && p.chains == 2) ql_leave(p, t, 1, acc1, q, lane);
+        if (ok) ql_leave(p, t, acc0, q, lane);
       } else if (ok) {
         if (CG == 1) ql_drain(p, t, acc0, tasks.second(t), acc1, group, last ? QL_GROUPS : 1, sums, stage, q, lane);
         else ql_drain_wide(p, t, acc0, tasks.second(t), acc1, group, last ? QL_GROUPS : 1, sums, stage, q, lane);
@@ -869,83 +865,81 @@ static bool plan_rings(UmmaPlan* t, const QWeight& w, bool several_tasks, bool s
   return true;
 }
 
-// Rows of a chunk for a weight that is split along K, its parts apart. All chunks are one launch, CTAs of the next filling the
-// SMs that the last wave of one leaves idle; the chunk size is the one whose waves take the least time, counted in
-// cycles that were fitted to this choice's launches: a unit of 128 x 64 weights 2 per row, not less than 184, and a CTA about 6000
-// around them. Chunks of fewer than 96 rows are not looked at: a unit takes no less time then, so more chunks are only more waves.
+// Rows of one or two chunks up to which the CTAs of a team read the activations each for itself. Alone and in pairs, us: 65 rows 4096 x 14336 15.7 and
+// 18.4, 28672 x 4096 22.1 and 24.7; 96 rows 17.0 and 19.1, 24.6 and 26.9; 128 rows 19.6 and 20.2, 30.1 and 30.8; 200 rows 26.5 and 30.2, 53.6 and 58.1. Records
+// of 9216 bytes leave too little shared memory for units of so many activations: 3584 x 18944 of 8 bits 96 rows 21.8 and 22.4, 112 rows 25.3 and 23.0.
+static int solo_rows(const QWeight& w) { return w.record_bytes > 5120 ? 96 : 128; }
+
+// What launches of a weight that is split along K take, in nanoseconds, by the rows of a chunk (96, 128, 160, 192): fitted to 17 weights of 8 to
+// 72 tiles, 32 to 448 k-blocks, 4 and 8 bits, at 20 row counts from 193 to 3000. A team's k-block takes what its dequantisation does up to 128 rows,
+// then its products' two cycles a row; 160 and 192 rows leave no accumulator to start the next split with while one is drained.
+constexpr int QL_APART_NS[2][4] = {{200, 205, 250, 285}, {225, 225, 285, 325}};   // a k-block, of records up to 5120 bytes and of larger ones
+constexpr int QL_TURN_NS[2][4] = {{167, 168, 227, 274}, {176, 179, 263, 340}};
+constexpr int QL_TURN_END_NS[4] = {1600, 2200, 3000, 3400};                         // a split's end, in turn; half more where there are more than eight
+constexpr int QL_APART_START_NS = 6000, QL_TURN_START_NS = 3000;                    // a CTA's start and end: of each wave; of a launch
+
+static long long waves_of(long long tasks, const QWeight& w) { const int teams = std::max(1, w.sm_count / 2); return (tasks + teams - 1) / teams; }
+static int chunk_rows(int M, int chunks) { return ((M + chunks - 1) / chunks + 31) & ~31; }
+static long long apart_ns(const QWeight& w, int M, int per) {
+  const int at = std::max(96, per) / 32 - 3;
+  return waves_of((long long)pairs_of(w) * w.splits * ((M + per - 1) / per), w) * ((long long)w.kblocks * QL_APART_NS[w.record_bytes > 5120][at] / w.splits + QL_APART_START_NS);
+}
+static long long turn_ns(const QWeight& w, int M, int per) {
+  const int at = per / 32 - 3;
+  return waves_of((long long)pairs_of(w) * ((M + per - 1) / per), w) * ((long long)w.kblocks * QL_TURN_NS[w.record_bytes > 5120][at] + (long long)w.splits * QL_TURN_END_NS[at] * (w.splits > 8 ? 3 : 2) / 2) + QL_TURN_START_NS;
+}
+
+// Rows of a chunk where splits are apart. All chunks are one launch; smaller ones than 96 rows take no less time and are only more of them. Of
+// 153 launches of 193 to 512 rows that chunks of all four sizes were timed for, the choice takes the fastest but for 3 % in one.
 static int plan_apart_rows(const QWeight& w, int M) {
-  const int ctas = w.n_tiles * w.splits;
-  const long long units = (long long)w.kblocks / w.splits;
   int best = 0;
-  long long best_cost = 0;
   for (int chunks = (M + QL_CHUNK_ROWS - 1) / QL_CHUNK_ROWS; best == 0 || chunks * 96 <= M; ++chunks) {
-    const int per = ((M + chunks - 1) / chunks + 15) & ~15;
-    const int n = (M + per - 1) / per;
-    const long long waves = ((long long)ctas * n + w.sm_count - 1) / w.sm_count;
-    const long long cost = waves * (units * std::max(184, 2 * per) + 6000);
-    if (best == 0 || cost < best_cost) { best = per; best_cost = cost; }
+    const int per = chunk_rows(M, chunks);
+    if (best == 0 || apart_ns(w, M, per) < apart_ns(w, M, best) * 98 / 100) best = per;
   }
   return best;
 }
 
-constexpr int QL_ROWS_MIN = 257;   // below, a chunk or two of rows never fill the SMs
-// With more k-blocks all splits in turn were the slower way at most row counts with one CTA a tile: 7000 x 28672 (448) 499 -> 564 us at
-// 1200 rows. 3584 x 18944 (296), apart and in turn: 320 rows 43 and 62 us, 1024 rows 137 and 119.
-constexpr int QL_ROWS_MAX_KBLOCKS = 300;
-// Whether the rows of a weight that is split along K take its splits in turn, and how many a chunk: 0 where splits apart take about as
-// long or less. Apart (with the reduction behind it) and in turn, us: 4096 x 14336 264 rows 40.5 and 48.0, 320 41.7 and 48.1, 513 80.5
-// and 51.6, 1024 133 and 91, 2048 263 and 160; 4096 x 4096 320 rows 25.7 and 21.6 (the reduction is 5 of the first, which a step does not
-// have), 1024 77 and 38, 2048 153 and 61; 6144 x 4096 1024 rows 91 and 52; 2048 x 8192 513 rows 43.6 and 41.9, 2048 140 and 74. The line
-// is drawn in cycles, fitted to launches of 264 to 2048 rows against eight weights of 16 to 64 tiles and 56 to 448 k-blocks with one CTA a
-// tile; teams gain on both sides, and it still takes the faster one but where both are within a fifth: a k-block there takes 330 and 1.55 a row, a CTA's start and end 9500; here 330 and 1.9 a row, 2.3
-// where two stages of activations only have room, a segment's end 600. A reduction of their own costs partials 2150 bytes a
-// cycle over all SMs where there are more than QL_MAX_M rows, else 6500. Summed by the kernel that reads the result anyway
-// they cost that next to nothing, and of the two ways the one with a launch of its own size has to be faster by a seventh.
-static int plan_in_turn_rows(const QWeight& w, int M, bool summed) {
+constexpr int QL_ROWS_MIN = 257;           // below, a chunk or two of rows never fill the SMs
+constexpr int QL_ROWS_MAX_KBLOCKS = 300;   // above, apart and in turn, us: 8192 x 28672 1500 rows 680 and 605, 1024 rows 475 and 391, 7000 x 28672 level
+// Whether the rows of a weight that is split along K take its splits in turn, and how many a chunk: 0 where they stay apart. In turn has to be the
+// faster way by a fifth in these figures: at rows near the line the calls keep the way they had. Apart, with the reduction behind it, and
+// in turn, us: 4096 x 14336 320 rows 41.2 and 42.8, 513 82 and 59, 1024 132 and 94, 2048 271 and 183; 4096 x 4096 366 rows 27.9 and 20.1 (the reduction
+// is 7 of the first, which a step does not have), 1024 77 and 42, 2048 153 and 80; 2048 x 8192 513 rows 43.5 and 37.7, 2048 140 and 85. The
+// reduction of more rows than QL_MAX_M, whose slabs do not stay in L2, goes at 3060 GB/s over the partials and the result; of fewer rows it is not counted, so
+// that a call has the way of the step, where the kernel that reads the result sums the partials at next to no cost. More than eight
+// splits are short ones, whose ends lie less under the next one's start.
+// Against the other way and all chunk sizes, in turn's chunk is 0.3 % behind the fastest on the mean of 340 points, 11 % at most.
+static int plan_in_turn_rows(const QWeight& w, int M) {
   if (w.splits == 1 || M < QL_ROWS_MIN || w.kblocks > QL_ROWS_MAX_KBLOCKS) return 0;
-  auto apart_cost = [&](int rows) -> long long {
-    if (rows == 0) return 0;
-    const int per = plan_apart_rows(w, rows);
-    const long long ctas = (long long)w.n_tiles * w.splits * ((rows + per - 1) / per), waves = (ctas + w.sm_count - 1) / w.sm_count;
-    const long long values = (long long)rows * w.N;
-    return waves * (w.kblocks * (330 + per * 31 / 20) / w.splits + 9500) +
-           (summed ? 0 : M > QL_MAX_M ? values * (4 * w.splits + 2) / 2150 : values * 4 * w.splits / 6500);
-  };
-  const long long apart = M / QL_MAX_M * apart_cost(QL_MAX_M) + apart_cost(M % QL_MAX_M);
+  auto slab = [&](int rows) { return rows ? apart_ns(w, rows, plan_apart_rows(w, rows)) : 0; };
+  long long most = M / QL_MAX_M * slab(M >= QL_MAX_M ? QL_MAX_M : 0) + slab(M % QL_MAX_M);
+  if (M > QL_MAX_M) most += (long long)M * w.N * (4 * w.splits + 2) * 100 / 306000;
+  most = most * 80 / 100;
   int best = 0;
-  long long best_cost = apart / 100 * (summed ? 86 : 92);
-  const int ends = w.splits * (w.splits > 8 ? 900 : 600);
-  if (w.kblocks * (330 + 96 * 19 / 10) + ends + 8000 >= best_cost) return 0;   // one wave of the smallest chunks
-  for (int per = 192; per >= 96; per -= 16) {
-    const int row_cost = w.record_bytes > 5120 && per > 144 ? 23 : per > 160 ? 23 : 19;
-    const long long items = (long long)w.n_tiles * ((M + per - 1) / per), waves = (items + w.sm_count - 1) / w.sm_count;
-    const long long cost = waves * (w.kblocks * (330 + per * row_cost / 10) + ends) + 8000;
-    if (cost < best_cost) { best = per; best_cost = cost; }
-  }
+  for (int per = 96; per <= QL_CHUNK_ROWS; per += 32)
+    if (turn_ns(w, M, per) < (best ? turn_ns(w, M, best) : most)) best = per;
   return best;
 }
-bool qlinear_in_turn(const QWeight& w, int M, bool summed) { return plan_in_turn_rows(w, M, summed) > 0; }
+bool qlinear_in_turn(const QWeight& w, int M) { return plan_in_turn_rows(w, M) > 0; }
 
-// Rows of a chunk for a weight that is not split along K, and whether its teams share the work by runs: the choice whose products
-// take the least time, 2 cycles a row and k-block and not less than 256, larger chunks where two are level. Runs leave no team idle and
-// cost a cut pair's way through global memory, counted as 8 k-blocks a chunk; fix: chunks that they may have.
-// Whole pairs and runs, us: 28672 x 4096 (112 pairs, 74 teams) 1 row 17.4 and 16.5, 32 rows 18.1 and 17.4, 192 rows 37.2 and 37.0 alone, in a step
-// 44.7 and 42.3; where the difference is smaller the way through memory counts for more than that: 320 rows 57.2 and 60.3, the head's
-// 501 pairs 138 and 142 at 192 rows.
+// Rows of a chunk for a weight that is not split along K, and whether its teams share the work by runs: the choice whose products take the least
+// time. With two chains, turn_ns of one part; runs would hand on two sums of a cut pair, and lose: 26000 x 2048 at 33 rows, whole pairs and runs,
+// 14.3 and 21.1 us, 22016 x 4096 at 192 rows 40.8 and 44.0. With one chain 2 cycles a row and k-block and not less than 300, larger chunks where two
+// are level. Runs leave no team idle and cost a cut pair's way through global memory, counted as 20 k-blocks a chunk; fix: chunks that
+// they may have. Whole pairs and runs, us: 28672 x 4096 (112 pairs, 74 teams) 1 row 19.0 and 17.8, 33 rows 18.9 and 18.5, 192 rows 43.1 and 40.0, 384
+// rows 81.6 and 77.3, 512 rows 96.6 and 108.6; the head's 501 pairs 138 and 142 at 192 rows.
 static int plan_whole_rows(const QWeight& w, int M, int fix, bool* runs) {
-  const int teams = w.sm_count / 2, pairs = pairs_of(w);
+  const int teams = std::max(1, w.sm_count / 2), pairs = pairs_of(w);
   if (pairs < teams) fix = 0;   // a run holds a whole pair's k-blocks at least
   int best = 0;
   double best_cost = 0;
-  for (int per = QL_CHUNK_ROWS; per >= 16; per -= per > QL_SOLO_ROWS ? 32 : 16) {
-    if (per < 96 && M > QL_SOLO_ROWS) break;
-    if (per - 32 >= M && per > QL_SOLO_ROWS) continue;
-    if (per - 16 >= M && per <= QL_SOLO_ROWS) continue;
+  for (int per = QL_CHUNK_ROWS; per >= 96; per -= 32) {
+    if (per - 32 >= M && per > 96) continue;
     const int chunks = (M + per - 1) / per;
-    if (chunks > 1 && per <= QL_SOLO_ROWS) break;
-    const double whole = (double)((pairs * (long long)chunks + teams - 1) / teams) * w.kblocks, cut = ((double)pairs * w.kblocks / teams + 8) * chunks;
-    const bool r = chunks * per * w.chains <= fix * QL_CHUNK_ROWS && cut < whole;
-    const double cost = (r ? cut : whole) * (std::max(256, 2 * per) + 20);
+    const double whole = (double)waves_of((long long)pairs * chunks, w) * w.kblocks, cut = ((double)pairs * w.kblocks / teams + 20) * chunks;
+    const bool r = w.chains == 1 && chunks <= fix && cut < whole;
+    const double cost = w.chains == 2 ? (double)turn_ns(w, M, per) : (r ? cut : whole) * (std::max(300, 2 * per) + 20);
     if (best == 0 || cost < best_cost * 0.995) { best = per; best_cost = cost; *runs = r; }
   }
   return best;
@@ -982,7 +976,7 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   UmmaPlan t{};
   const int pairs = pairs_of(w), all_teams = std::max(1, w.sm_count / 2);
   if (w.splits > 1) {
-    const int turn = plan_in_turn_rows(w, l.M, l.summed);
+    const int turn = plan_in_turn_rows(w, l.M);
     t.way = turn ? QL_IN_TURN : QL_APART;
     t.m_pad = turn ? turn : plan_apart_rows(w, l.M);
   } else {
@@ -990,13 +984,17 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
     t.m_pad = plan_whole_rows(w, l.M, l.fix ? QL_FIX_CHUNKS : 0, &runs);
     t.way = runs ? QL_RUNS : QL_IN_TURN;
   }
-  t.cg = t.m_pad > QL_SOLO_ROWS ? 2 : 1;
-  if (t.cg == 2) t.m_pad = (t.m_pad + 31) & ~31;
-  if (t.way == QL_IN_TURN && w.splits > 1) t.m_pad = std::min(t.m_pad, QL_SUM_ROWS);
-  t.chunks = (l.M + t.m_pad - 1) / t.m_pad;
-  t.teams = t.way == QL_IN_TURN ? (int)std::min<long long>((long long)pairs * t.chunks, all_teams) : all_teams;
-  const bool sums = t.way == QL_IN_TURN && w.splits > 1, several = t.way == QL_RUNS || (t.way == QL_IN_TURN && (sums || (long long)pairs * t.chunks > t.teams));
-  if (!plan_rings(&t, w, several, sums)) return cudaErrorInvalidValue;
+  const bool sums = t.way == QL_IN_TURN && w.splits > 1;
+  // with two chains and several tasks a team, tensor memory has room for the accumulators of 64 rows of a CTA alone
+  const int rows = t.m_pad, chunks = (l.M + rows - 1) / rows, alone = ((l.M + chunks - 1) / chunks + 15) & ~15;
+  for (t.cg = !sums && chunks <= 2 && alone <= solo_rows(w) ? 1 : 2;; t.cg = 2) {
+    t.m_pad = t.cg == 1 ? alone : rows;
+    t.chunks = (l.M + t.m_pad - 1) / t.m_pad;
+    t.teams = t.way == QL_IN_TURN ? (int)std::min<long long>((long long)pairs * t.chunks, all_teams) : all_teams;
+    const bool several = t.way == QL_RUNS || (t.way == QL_IN_TURN && (sums || (long long)pairs * t.chunks > t.teams));
+    if (plan_rings(&t, w, several, sums)) break;
+    if (t.cg == 2) return cudaErrorInvalidValue;
+  }
   QlKernelParams p;
   p.records = w.records; p.record_bytes = w.record_bytes;
   p.N = w.N; p.kblocks = w.kblocks; p.n_pairs = pairs; p.splits = w.splits; p.chains = w.chains; p.teams = t.teams;

@@ -272,3 +272,18 @@ ok(L.lib().kc_forward_step(model._h, pool._h, p.ids_p, p.n, p.seq_arr, p.n_seqs,
 threads = [s.split(":")[0] for s in fake.fake_shapes().decode().split()]
 assert [t for t in threads if t in ("384", "768")] == ["{threads}"], threads
 """, first="import torch")
+
+
+def test_a_launch_has_the_chunks_that_were_weighed(fake):
+    """Rows of 4096 x 14336 that are taken with all splits in turn: four chunks of at most 192 rows are one task for each of 64 teams of two
+    SMs. Chunks of fewer rows than the choice was made for would be 80 tasks, two rounds of the 74 teams."""
+    run(fake, """
+w = C.c_void_p()
+src = C.create_string_buffer(4096 * 14336 // 2)
+ok(lib.kc_qweight_create(ctx, C.addressof(src), C.addressof(src), C.addressof(src), 4096, 14336, 4, 64, 0, C.byref(w)))
+fake.fake_shapes.restype = C.c_char_p
+for m in (641, 672, 704, 768):
+    fake.fake_reset()
+    ok(lib.kc_quantized_matmul(ctx, w, at, m, at))
+    assert fake.fake_shapes().decode().split() == ["640:128x1x1"], (m, fake.fake_shapes())
+""")
