@@ -337,6 +337,18 @@ __device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& 
 #pragma unroll
     for (int j = 0; j < 8; ++j) buf[j * 36 + lane] = v[j];
     __syncwarp();
+    if (!p.vec) {                        // a lane a feature, row by row
+      const bool apart = p.way == QL_APART && p.splits > 1;
+      const int first = m - r;
+#pragma unroll 1
+      for (int j = 0; j < 8 && first + j < p.M; ++j) {
+        const float x = buf[j * 36 + lane];
+        if (n0 + lane >= p.N) continue;
+        if (apart) p.partial[((size_t)t.split * p.M + first + j) * p.N + n0 + lane] = x;
+        else p.y[(size_t)(p.row0 + first + j) * p.ldy + n0 + lane] = __float2bfloat16_rn(x);
+      }
+      continue;
+    }
     if (m >= p.M) continue;
     if (p.glu) {                         // four features of a row: gate at 32 of a warp's k .., up 16 further
       const int c = (lane & 3) * 4;
@@ -348,21 +360,11 @@ __device__ __forceinline__ void ql_drain(const QlKernelParams& p, const QlTask& 
     const float4 a = *reinterpret_cast<const float4*>(buf + r * 36 + f), b = *reinterpret_cast<const float4*>(buf + r * 36 + f + 4);
     if (p.way == QL_APART && p.splits > 1) {
       float* dst = p.partial + ((size_t)t.split * p.M + m) * p.N + n;
-      if (p.vec && n < p.N) {
-        *reinterpret_cast<float4*>(dst) = a;
-        if (n + 4 < p.N) *reinterpret_cast<float4*>(dst + 4) = b;
-      } else {
-#pragma unroll 1
-        for (int j = 0; j < 8 && n + j < p.N; ++j) dst[j] = buf[r * 36 + f + j];
-      }
+      if (n < p.N) *reinterpret_cast<float4*>(dst) = a;
+      if (n + 4 < p.N) *reinterpret_cast<float4*>(dst + 4) = b;
     } else {
       bf16* dst = p.y + (size_t)(p.row0 + m) * p.ldy + n;
-      if (p.vec && n < p.N) {
-        *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf162(a.x, a.y), pack_bf162(a.z, a.w), pack_bf162(b.x, b.y), pack_bf162(b.z, b.w));
-      } else {
-#pragma unroll 1
-        for (int j = 0; j < 8 && n + j < p.N; ++j) dst[j] = __float2bfloat16_rn(buf[r * 36 + f + j]);
-      }
+      if (n < p.N) *reinterpret_cast<uint4*>(dst) = make_uint4(pack_bf162(a.x, a.y), pack_bf162(a.z, a.w), pack_bf162(b.x, b.y), pack_bf162(b.z, b.w));
     }
   }
 }
@@ -1006,7 +1008,7 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   p.back0 = ldexpf(1.f, std::min(w.shift, 127)); p.back1 = ldexpf(1.f, w.shift - std::min(w.shift, 127));
   p.glu = glu ? l.glu : 0; p.act = l.act; p.ld_act = l.ld_act;
   p.y = l.y; p.ldy = l.ldy; p.partial = l.partial;
-  p.vec = t.way == QL_APART && w.splits > 1 ? (w.N & 3) == 0 && (reinterpret_cast<uintptr_t>(l.partial) & 15) == 0
+  p.vec = glu ? 1 : t.way == QL_APART && w.splits > 1 ? (w.N & 3) == 0 && (reinterpret_cast<uintptr_t>(l.partial) & 15) == 0
                                             : (w.N & 7) == 0 && (l.ldy & 7) == 0 && (reinterpret_cast<uintptr_t>(l.y) & 15) == 0;
   p.fix = reinterpret_cast<uint4*>(l.fix); p.status = l.status;
   if (w.bits == 4) return w.gpk == 2 ? launch_umma_cg<4, 2>(l, t, p, s) : launch_umma_cg<4, 1>(l, t, p, s);

@@ -332,3 +332,18 @@ def test_even_and_odd_k_blocks_are_sums_of_their_own(ctx, n, k, bits, group):
     for m in (1, 17, 64, 65, 130, 192, 320, 1100):
         assert torch.equal(qw.matmul(x[:m]).cpu().float(), want[:m].expand(m, n)), m
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("n,k", [(301, 512), (300, 1024), (4099, 4096), (9500, 256), (19501, 512)])
+def test_rows_that_are_not_aligned_match_aligned_ones(ctx, n, k):
+    """Widths that are no multiple of eight leave value by value, as y and as partials of splits: the same bits as the aligned weight that
+    the rows are the first ones of, in lone CTAs and in pairs."""
+    wide = (n + 127) // 128 * 128       # as many tiles, so the same splits and chains
+    p, s, b = make(wide, k, 4, 64, 61)
+    aligned = api.QuantizedWeight(ctx, p.cuda(), s.cuda(), b.cuda(), 4, 64)
+    ragged = api.QuantizedWeight(ctx, p[:n].contiguous().cuda(), s[:n].contiguous().cuda(), b[:n].contiguous().cuda(), 4, 64)
+    x = acts(321, k, 62).cuda()
+    for m in (1, 9, 64, 121, 150, 250, 321):
+        want, got = aligned.matmul(x[:m])[:, :n], ragged.matmul(x[:m])
+        assert torch.equal(got.view(torch.int16), want.contiguous().view(torch.int16)), m
+    assert ctx.device_status() == 0
