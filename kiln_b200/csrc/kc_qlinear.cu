@@ -16,8 +16,8 @@ namespace kc {
 __global__ void qweight_retile_kernel(uint8_t* __restrict__ records, const uint32_t* __restrict__ w,
                                       const bf16* __restrict__ scales, const bf16* __restrict__ biases,
                                       int N, int K, int bits, int group, int n_tiles, int kblocks,
-                                      int alternate, int gpk, uint32_t packed_bytes, uint32_t record_bytes, int* __restrict__ top) {
-  int exponent = 0;   // the largest of a finite scale that this thread has met, biased
+                                      int alternate, int gpk, uint32_t packed_bytes, uint32_t record_bytes, int* __restrict__ exponents) {
+  int largest = 0, smallest = 0;   // exponents, biased, that this thread has met: of finite scales; from 255, of scales and biases that are not 0
   // alternate: the source has N / 2 gate rows, then N / 2 up rows; 16 of each take turns
   auto source = [&](int n) { return alternate ? (n >> 5 << 4) + (n & 15) + (n & 16 ? N / 2 : 0) : n; };
   const int words_per_row_kb = QL_KB * bits / 32;  // 8 (w4) or 16 (w8)
@@ -63,14 +63,20 @@ __global__ void qweight_retile_kernel(uint8_t* __restrict__ records, const uint3
         const int g = (kb * QL_KB + gi * group) / group;
         sb.x = scales[(long long)source(n) * groups_per_row + g];
         sb.y = biases[(long long)source(n) * groups_per_row + g];
-        const int e = (int)(__bfloat16_as_ushort(sb.x) >> 7) & 0xFF;
-        if (e < 255) exponent = max(exponent, e);
+        const int scale = __bfloat16_as_ushort(sb.x) & 0x7FFF, bias = __bfloat16_as_ushort(sb.y) & 0x7FFF;
+        if (scale >> 7 < 255) largest = max(largest, scale >> 7);
+        if (scale) smallest = max(smallest, 255 - (scale >> 7));
+        if (bias) smallest = max(smallest, 255 - (bias >> 7));
       }
       reinterpret_cast<bf162*>(base + packed_bytes)[e2] = sb;
     }
   }
-  exponent = __reduce_max_sync(0xffffffffu, exponent);   // all threads are here
-  if (exponent && (threadIdx.x & 31) == 0) atomicMax(top, exponent);
+  largest = __reduce_max_sync(0xffffffffu, largest);   // all threads are here
+  smallest = __reduce_max_sync(0xffffffffu, smallest);
+  if ((threadIdx.x & 31) == 0) {
+    if (largest) atomicMax(exponents, largest);
+    if (smallest) atomicMax(exponents + 1, smallest);
+  }
 }
 
 int qlinear_plan_splits(int n_tiles, int kblocks, int sm_count) {
@@ -96,18 +102,18 @@ cudaError_t qweight_build(QWeight* out, const uint32_t* w, const bf16* scales, c
   q.splits = qlinear_plan_splits(q.n_tiles, q.kblocks, sm_count);
   q.chains = qlinear_plan_chains(q.n_tiles, q.splits, sm_count);
   q.sm_count = sm_count;
-  // one allocation: the records, then the largest exponent of a scale, which the re-tiling finds
+  // one allocation: the records, then the exponents that the re-tiling finds
   cudaError_t e = cudaMalloc(&q.records, q.bytes() + 16);
   if (e != cudaSuccess) return e;
-  q.top = reinterpret_cast<int*>(q.records + q.bytes());
-  e = cudaMemsetAsync(q.top, 0, 16, s);
+  q.exponents = reinterpret_cast<int*>(q.records + q.bytes());
+  e = cudaMemsetAsync(q.exponents, 0, 16, s);
   if (e != cudaSuccess) { cudaFree(q.records); return e; }
   const long long total = (long long)(q.bytes() / 4);
   const int threads = 256;
   const int blocks = (int)std::min<long long>((total + threads - 1) / threads, 148LL * 16);
   qweight_retile_kernel<<<blocks, threads, 0, s>>>(q.records, w, scales, biases, N, K, bits, group,
                                                    q.n_tiles, q.kblocks, alternate ? 1 : 0, q.gpk, q.packed_bytes,
-                                                   q.record_bytes, q.top);
+                                                   q.record_bytes, q.exponents);
   e = cudaGetLastError();
   if (e != cudaSuccess) { cudaFree(q.records); return e; }
   *out = q;
@@ -115,9 +121,13 @@ cudaError_t qweight_build(QWeight* out, const uint32_t* w, const bf16* scales, c
 }
 
 cudaError_t qweight_finish(QWeight* w) {
-  int exponent = 0;
-  cudaError_t e = cudaMemcpy(&exponent, w->top, sizeof(int), cudaMemcpyDeviceToHost);
-  w->shift = std::max(0, exponent - 121);   // scale * 2^(133 - shift) < 2^(exponent - 126 + 133 - shift) <= 2^128
+  int exponents[2] = {0, 0};
+  cudaError_t e = cudaMemcpy(exponents, w->exponents, sizeof exponents, cudaMemcpyDeviceToHost);
+  w->shift = std::max(0, exponents[0] - 121);   // scale * 2^(133 - shift) < 2^(exponent - 126 + 133 - shift) <= 2^128
+  // A weight is a multiple of the last place of its scale or bias, and rounded as the shifted one is unless that falls below 2^-126; its product
+  // with an activation of 2^-32 or more, and all bits of it, stay above that too where no scale or bias is shifted below 2^-63.
+  w->wide = w->shift > 0 && 255 - exponents[1] - w->shift < 127 - 63;
+  if (w->wide) w->shift = 0;
   return e;
 }
 

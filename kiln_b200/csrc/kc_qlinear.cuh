@@ -42,8 +42,9 @@ struct QWeight {
   int splits = 1;              // fixed function of (N, K): never of M
   int chains = 1;              // .. and chains of products a split has (qlinear_plan_chains)
   int sm_count = 148;
-  int* top = nullptr;          // the re-tiling's largest exponent of a scale (inside the records' allocation)
-  int shift = 0;               // from it, read once at load: the GEMM takes the weights times 2^-shift
+  int* exponents = nullptr;    // the re-tiling's largest exponent of a scale and (from 255) smallest of a scale or bias (inside the records' allocation)
+  int shift = 0;               // from them, read once at load: the GEMM takes the weights times 2^-shift
+  bool wide = false;           // .. or, where that would not be exact, converts the integers
   size_t bytes() const { return (size_t)((n_tiles + QL_TILE_GROUP - 1) / QL_TILE_GROUP) * QL_TILE_GROUP * kblocks * record_bytes; }
   // Algorithmic bytes of the mlx tensors this weight was built from.
   size_t mlx_bytes() const { return (size_t)N * K * bits / 8 + (size_t)2 * N * (K / group) * 2; }

@@ -34,7 +34,9 @@ namespace kc {
 // powers of two) gives q * scale + bias rounded once — the value that converting q first gives. 9 instructions for 8 weights
 // of 4 bits (two nibbles of a half-word in place, two behind one shift), 4 for 4 of 8 bits. The scaled scale must stay below
 // 2^128: a weight with larger scales (2^-5 and more) is taken at 2^-shift of its size, QWeight::shift, and its sums are
-// multiplied back, both exact.
+// multiplied back, both exact as long as nothing falls below the normal numbers on the way. Where scales are so far apart that
+// something would (2^57 and more between the smallest and 2^-6 of the largest), WIDE brings the integers to size instead, two
+// multiplications a pair.
 // ---------------------------------------------------------------------------
 
 __device__ __forceinline__ bf162 bf2_bits(uint32_t u) { return *reinterpret_cast<const bf162*>(&u); }
@@ -42,6 +44,7 @@ __device__ __forceinline__ uint32_t bf2_fma(uint32_t a, bf162 s, bf162 b) {
   const bf162 r = __hfma2(*reinterpret_cast<const bf162*>(&a), s, b);
   return *reinterpret_cast<const uint32_t*>(&r);
 }
+__device__ __forceinline__ uint32_t bf2_raw(bf162 v) { return *reinterpret_cast<const uint32_t*>(&v); }
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
@@ -52,7 +55,12 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 struct QlFactors { uint32_t s0, s1, b; };
 
 // Packed words of a row (16-byte chunk c at row + c * QL_TILE_N * 16), its scale and bias pairs at sb -> v[32].
-template <int BITS, int GPK>
+template <bool WIDE>
+__device__ __forceinline__ uint32_t dequant_pair(uint32_t q, uint32_t size, bf162 s, bf162 b) {   // size: 2^-127 of what makes q the integers
+  if (!WIDE) return bf2_fma(q, s, b);
+  return bf2_fma(bf2_raw(__hmul2(__hmul2(bf2_bits(q), bf2_bits(0x7F007F00u)), bf2_bits(size))), s, b);
+}
+template <int BITS, int GPK, bool WIDE>
 __device__ __forceinline__ void dequant_row(uint32_t row, uint32_t sb, const QlFactors& f, uint32_t (&v)[32]) {
   constexpr int CHUNKS = BITS / 2;
   bf162 s_lo[GPK], s_hi[GPK], bias[GPK];
@@ -65,9 +73,13 @@ __device__ __forceinline__ void dequant_row(uint32_t row, uint32_t sb, const QlF
 #pragma unroll
   for (int g = 0; g < GPK; ++g) {
     const bf162 pair = bf2_bits(raw[g]);
-    s_lo[g] = __hmul2(__hmul2(__bfloat162bfloat162(pair.x), bf2_bits(f.s0)), bf2_bits(f.s1));
-    if (BITS == 4) s_hi[g] = __hmul2(s_lo[g], bf2_bits(0x3D803D80u));   // 2^-4
-    bias[g] = __hmul2(__bfloat162bfloat162(pair.y), bf2_bits(f.b));
+    s_lo[g] = __bfloat162bfloat162(pair.x);
+    bias[g] = __bfloat162bfloat162(pair.y);
+    if (!WIDE) {
+      s_lo[g] = __hmul2(__hmul2(s_lo[g], bf2_bits(f.s0)), bf2_bits(f.s1));
+      bias[g] = __hmul2(bias[g], bf2_bits(f.b));
+    }
+    if (BITS == 4) s_hi[g] = WIDE ? s_lo[g] : __hmul2(s_lo[g], bf2_bits(0x3D803D80u));   // 2^-4
   }
 #pragma unroll
   for (int h = 0; h < CHUNKS; ++h) {
@@ -79,14 +91,14 @@ __device__ __forceinline__ void dequant_row(uint32_t row, uint32_t sb, const QlF
         // the record's nibble order: element 2j at bits 4j, element 2j + 1 at bits 16 + 4j
         uint32_t* o = v + (h * 4 + c) * 4;
         const uint32_t up = word[c] >> 8;
-        o[0] = bf2_fma(word[c] & 0x000F000Fu, s_lo[g], bias[g]);
-        o[1] = bf2_fma(word[c] & 0x00F000F0u, s_hi[g], bias[g]);
-        o[2] = bf2_fma(up & 0x000F000Fu, s_lo[g], bias[g]);
-        o[3] = bf2_fma(up & 0x00F000F0u, s_hi[g], bias[g]);
+        o[0] = dequant_pair<WIDE>(word[c] & 0x000F000Fu, 0x42804280u, s_lo[g], bias[g]);   // 2^6
+        o[1] = dequant_pair<WIDE>(word[c] & 0x00F000F0u, 0x40804080u, s_hi[g], bias[g]);   // 2^2
+        o[2] = dequant_pair<WIDE>(up & 0x000F000Fu, 0x42804280u, s_lo[g], bias[g]);
+        o[3] = dequant_pair<WIDE>(up & 0x00F000F0u, 0x40804080u, s_hi[g], bias[g]);
       } else {
         uint32_t* o = v + (h * 4 + c) * 2;
-        o[0] = bf2_fma(__byte_perm(word[c], 0u, 0x4140u), s_lo[g], bias[g]);
-        o[1] = bf2_fma(__byte_perm(word[c], 0u, 0x4342u), s_lo[g], bias[g]);
+        o[0] = dequant_pair<WIDE>(__byte_perm(word[c], 0u, 0x4140u), 0x42804280u, s_lo[g], bias[g]);
+        o[1] = dequant_pair<WIDE>(__byte_perm(word[c], 0u, 0x4342u), 0x42804280u, s_lo[g], bias[g]);
       }
     }
   }
@@ -537,7 +549,7 @@ __device__ __forceinline__ void ql_commit(uint32_t bar) {
   else umma_commit_pair(bar);
 }
 
-template <int BITS, int GPK, int CG>
+template <int BITS, int GPK, int CG, bool WIDE>
 __global__ void __launch_bounds__(QL_THREADS, 1)
 qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_constant__ QlKernelParams p) {
   constexpr uint32_t PACKED = QL_TILE_N * (QL_KB * BITS / 8);
@@ -724,7 +736,7 @@ qlinear_umma_kernel(const __grid_constant__ CUtensorMap map_rows, const __grid_c
 #pragma unroll
         for (int k = 0; k < UNIT; ++k) {   // of half a unit at a task's end, the second half is what the slot held before: no MMA reads it
           uint32_t v[32];
-          dequant_row<BITS, GPK>(row0 + rec + k * p.record_bytes, sb0 + rec + k * p.record_bytes, p.factors, v);
+          dequant_row<BITS, GPK, WIDE>(row0 + rec + k * p.record_bytes, sb0 + rec + k * p.record_bytes, p.factors, v);
           if (k == 0) {
             ok = __all_sync(0xffffffffu, ql_wait(done + old, freed));
             if (!ok) break;
@@ -947,21 +959,22 @@ static int plan_whole_rows(const QWeight& w, int M, int fix, bool* runs) {
   return best;
 }
 
-template <int BITS, int GPK, int CG>
+template <int BITS, int GPK, int CG, bool WIDE>
 static cudaError_t launch_umma(const QLinearLaunch& l, const UmmaPlan& t, const QlKernelParams& p, cudaStream_t s) {
   static DeviceOnce configured;   // the attribute belongs to the device's copy of the kernel
   if (configured.first_on_current_device()) {
-    cudaError_t e = cudaFuncSetAttribute(qlinear_umma_kernel<BITS, GPK, CG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(qlinear_umma_kernel<BITS, GPK, CG, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) { configured.forget_current_device(); return e; }
   }
   const CUtensorMap* rows = act_operand_rows_map(l.x, p.m_pad / CG);
   if (!rows) return cudaErrorInvalidValue;
   const dim3 grid = p.way == QL_APART ? dim3(CG == 2 ? 2 * p.n_pairs : l.w->n_tiles, p.splits, p.chunks) : dim3(2 * t.teams);
-  return launch_k_cluster(CG, qlinear_umma_kernel<BITS, GPK, CG>, grid, dim3(QL_THREADS), t.smem, s, *rows, p);
+  return launch_k_cluster(CG, qlinear_umma_kernel<BITS, GPK, CG, WIDE>, grid, dim3(QL_THREADS), t.smem, s, *rows, p);
 }
 template <int BITS, int GPK>
 static cudaError_t launch_umma_cg(const QLinearLaunch& l, const UmmaPlan& t, const QlKernelParams& p, cudaStream_t s) {
-  return t.cg == 2 ? launch_umma<BITS, GPK, 2>(l, t, p, s) : launch_umma<BITS, GPK, 1>(l, t, p, s);
+  if (l.w->wide) return t.cg == 2 ? launch_umma<BITS, GPK, 2, true>(l, t, p, s) : launch_umma<BITS, GPK, 1, true>(l, t, p, s);
+  return t.cg == 2 ? launch_umma<BITS, GPK, 2, false>(l, t, p, s) : launch_umma<BITS, GPK, 1, false>(l, t, p, s);
 }
 
 static uint32_t bf16_twice(int exponent) {   // 2^exponent as a pair of bf16, subnormals included

@@ -347,3 +347,27 @@ def test_rows_that_are_not_aligned_match_aligned_ones(ctx, n, k):
         want, got = aligned.matmul(x[:m])[:, :n], ragged.matmul(x[:m])
         assert torch.equal(got.view(torch.int16), want.contiguous().view(torch.int16)), m
     assert ctx.device_status() == 0
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("large,small", [(100, -30), (20, -40), (30, -39), (127, -126), (-4, -120), (-4, -40)])
+def test_scales_far_apart_are_exact(ctx, bits, large, small):
+    """A weight with large scales is taken at a power of two less only where that is exact: rows of the largest and of far smaller scales
+    and biases come out as q * scale + bias rounded once. Exact: one-hot rows bring the weights out as they are."""
+    n, k = 256, 128
+    g = torch.Generator().manual_seed(71)
+    q = torch.randint(0, 2 ** bits, (n, k), generator=g)
+    per = 32 // bits
+    packed = (q.reshape(n, -1, per) << (torch.arange(per) * bits)).sum(-1)
+    packed = torch.where(packed >= 2 ** 31, packed - 2 ** 32, packed).to(torch.int32)
+    power = torch.full((n, 1), float(small), dtype=torch.float64)
+    power[::7] = large - bits                                            # the largest product stays a bf16 number
+    s = (torch.exp2(power) * (129 / 128)).expand(n, 2).to(torch.bfloat16).contiguous()
+    b = (torch.exp2(power) * torch.where(torch.arange(n).reshape(n, 1) % 2 == 0, -5.0, 3.0)).expand(n, 2).to(torch.bfloat16).contiguous()
+    exact = q.double() * s.double().repeat_interleave(64, 1) + b.double().repeat_interleave(64, 1)
+    ulp = torch.exp2(torch.floor(torch.log2(exact.abs().clamp_min(2.0 ** -126))) - 7)
+    want = (torch.round(exact / ulp) * ulp).float()                      # half to even, of the exact value
+    qw = api.QuantizedWeight(ctx, packed.cuda(), s.cuda(), b.cuda(), bits, 64)
+    got = qw.matmul(torch.eye(k).to(torch.bfloat16).cuda()).cpu().float().T
+    assert torch.equal(got, want)
+    assert ctx.device_status() == 0
