@@ -304,11 +304,13 @@ __device__ __forceinline__ float tanh_any(float y, float near) {
 // Mlp::forward activation (nn.rs:284-294): silu(gate) * up with the three bf16 roundings of the composed ops, or
 // gelu_approx(gate) * up op for op (nn.rs:221-235). g and u are bf16 values held in fp32; so is the result.
 // 1 / (1 + e^-g), the reciprocal by the hardware's estimate and one step of Newton's iteration, r + r (1 - d r): within 0.501 units
-// of fp32's last place of the quotient, which is what a division gives, and without a division's branches, which cost a warp 100
-// cycles each where others compute. An infinite denominator is a zero.
+// of fp32's last place of the quotient, where a division is within 0.5, and without a division's branches, which cost a warp 100
+// cycles each where others compute; rounded to bf16 it is the quotient's for every bf16 gate. The denominator is taken at 2^-32 of its
+// size, so that the reciprocal of a large one (a gate below -87.3) is no subnormal number, which the estimate would flush. An
+// infinite denominator is a zero.
 __device__ __forceinline__ float act_sigmoid(float g) {
-  const float d = 1.f + __expf(-g), r = rcp_approx(d), n = fmaf(r, fmaf(-d, r, 1.f), r);
-  return d > 1e37f ? r : n;
+  const float d = fmaf(__expf(-g), 0x1p-32f, 0x1p-32f), r = rcp_approx(d), n = fmaf(r, fmaf(-d, r, 1.f), r);
+  return (d > 1e37f ? r : n) * 0x1p-32f;
 }
 __device__ __forceinline__ float act_silu_mul(float g, float u) {
   const float s = bf16_round(act_sigmoid(g));
