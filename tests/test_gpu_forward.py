@@ -470,3 +470,24 @@ def test_live_object_counter_returns_to_baseline(ctx):
     kv.close()
     m.close()
     assert api.live_objects() == base
+
+
+@pytest.mark.parametrize("name,gain", [("tiny-llama-wide", 1.0), ("tiny-llama-wide", 64.0), ("tiny-gemma2", 1.0)])
+def test_gated_activation_of_cut_pairs(ctx, name, gain):
+    """The gated activation where teams cut pairs of gate_up's tiles between them, also of a weight with large scales: 104 pairs of 40
+    k-blocks are cut at 5 rows and whole at 530, in three chunks. A sequence's logits have the same bits in both steps."""
+    cfg = dataclasses.replace(PRESETS[name], num_hidden_layers=1, hidden_size=2560, intermediate_size=13312)
+    ck = synth_checkpoint(cfg, seed=0, std=0.01)
+    for part in ("scales", "biases"):
+        w = ck[f"model.layers.0.mlp.up_proj.{part}"]
+        w.copy_((w.float() * gain).to(w.dtype))
+    model = api.CudaModel(ctx, cfg, ck, max_step_tokens=544, max_step_seqs=16)
+    kv = api.PagedKv(ctx, model.kv_spec(48, BS))
+    first, other = prompts(cfg, [5, 525], 1)
+    alone = model.forward_step(api.StepBatch(first, [api.SeqStep(5, 0, 5, [0])]), kv).clone()
+    ctx.sync()
+    both = model.forward_step(api.StepBatch(first + other, [api.SeqStep(5, 0, 5, [1]), api.SeqStep(525, 0, 1, list(range(2, 35)))]), kv)
+    ctx.sync()
+    assert torch.equal(alone.view(torch.int16), both[:5].view(torch.int16))
+    assert bool(torch.isfinite(alone.float()).all()) and float(alone.float().abs().max()) > 0
+    assert ctx.device_status() == 0

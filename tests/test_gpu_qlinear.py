@@ -41,9 +41,9 @@ CASES = [
     (256, 512, 8, 32, 48),         # 8-bit
     (256, 448, 8, 64, 7),          # K = 7 k-blocks
     (1024, 4096, 4, 64, 192),      # the 8B attention-output shape at verify width: split-K engaged
-    (2048, 2048, 4, 64, 320),      # two accumulator tiles (M > 256)
+    (2048, 2048, 4, 64, 320),      # two chunks of rows
     (512, 2048, 4, 64, 1),         # decode row
-    (53248, 256, 8, 32, 100),      # 416 tiles of 8-bit records at 100 rows: four tiles per CTA do not fit shared memory
+    (53248, 256, 8, 32, 100),      # 416 tiles of 8-bit records at 100 rows
 ]
 
 
@@ -184,18 +184,18 @@ def test_stream_lane_rows_do_not_depend_on_row_count(ctx):
 
 
 @pytest.mark.parametrize("n,k,bits,group,m,gain", [
-    (26700, 192, 4, 64, 33, 1.0),     # 209 tiles, two per CTA: the last CTA owns one; three k-blocks
-    (26700, 64, 8, 64, 192, 1.0),     # one k-block: the second issuer has nothing to do
-    (384, 1088, 4, 32, 192, 1.0),     # one tile per CTA, the most rows of one chunk, splits of 8 and 9 k-blocks: stages with one k-block
+    (26700, 192, 4, 64, 33, 1.0),     # 209 tiles: the last team's second CTA has none; three k-blocks
+    (26700, 64, 8, 64, 192, 1.0),     # one k-block
+    (384, 1088, 4, 32, 192, 1.0),     # the most rows of one chunk, splits of 8 and 9 k-blocks: an odd number of them
     (384, 1088, 4, 32, 256, 1.0),     # the same in two chunks
     (384, 1088, 8, 32, 177, 1.0),     # 8-bit, rows past the activations' end inside the last group of 16
-    (300, 512, 4, 64, 20, 200.0),     # scales of 0.5 and more: integers converted before the multiply-add
+    (300, 512, 4, 64, 20, 200.0),     # scales of 0.5 and more: taken at 2^-shift of their size
     (300, 512, 8, 64, 20, 300.0),     # the same for 8 bits (scales of 1/32 and more)
     (300, 512, 4, 64, 20, 1e-30),     # scales near the smallest normal numbers
 ])
 def test_stage_edges_and_scale_range(ctx, n, k, bits, group, m, gain):
-    """The places where the pipeline's stages end unevenly, and the range of scales on both sides of the one where the
-    dequantisation changes form. Bound: the GEMM's bar for outputs of order one; with another gain the outputs scale
+    """The places where the pipeline's stages end unevenly, and the range of scales on both sides of the one from which on
+    weights are taken at 2^-shift of their size. Bound: the GEMM's bar for outputs of order one; with another gain the outputs scale
     with it, so the inputs are scaled back by a power of two and the same bar holds."""
     g = torch.Generator().manual_seed(31)
     w = torch.empty(n, k).normal_(0, 0.02 * gain, generator=g)
@@ -221,9 +221,9 @@ def test_stage_edges_and_scale_range(ctx, n, k, bits, group, m, gain):
 
 
 @pytest.mark.parametrize("n,k,bits,group,m", [
-    (26700, 320, 4, 64, 193),     # two tiles per CTA, two chunks, the last accumulator tile missing
+    (26700, 320, 4, 64, 193),     # two chunks, the last team's second tile missing
     (26700, 384, 4, 128, 1001),   # a last chunk of fewer rows than the others
-    (384, 1088, 4, 32, 257),      # one tile per CTA, split along K
+    (384, 1088, 4, 32, 257),      # split along K
     (300, 512, 8, 64, 700),       # more rows than a slab of the split-K workspace
 ])
 def test_row_chunks_carry_the_bits_of_few_rows(ctx, n, k, bits, group, m):
@@ -241,7 +241,7 @@ def test_row_chunks_carry_the_bits_of_few_rows(ctx, n, k, bits, group, m):
 @pytest.mark.parametrize("n,k,bits,group,m,gain", [
     (384, 1088, 4, 32, 1201, 1.0),    # three tiles, splits of 8 and 9 k-blocks, a last chunk of few rows
     (4100, 2176, 4, 128, 1300, 1.0),  # several items a CTA, splits of 8 and 9 k-blocks, a ragged last tile
-    (300, 1024, 4, 64, 1000, 200.0),  # integers converted before the multiply-add
+    (300, 1024, 4, 64, 1000, 200.0),  # scales of 0.5 and more: taken at 2^-shift of their size
     (4608, 3584, 8, 32, 1111, 1.0),
     (6144, 4096, 4, 64, 700, 1.0),    # three splits
     (1000, 1024, 8, 64, 5003, 1.0),
@@ -261,7 +261,7 @@ def test_many_rows_carry_the_bits_of_few(ctx, n, k, bits, group, m, gain):
 
 
 @pytest.mark.parametrize("bits", [4, 8])
-@pytest.mark.parametrize("scale", [129 / 2 ** 10, 129 / 2 ** 8])     # below and above the line where the integers are converted first
+@pytest.mark.parametrize("scale", [129 / 2 ** 10, 129 / 2 ** 8])     # below and above the line from which on weights are taken at 2^-shift of their size
 def test_weights_are_rounded_once(ctx, bits, scale):
     """A weight is q * scale + bias rounded to bf16 once: with a bias far below the last bit of a product that lies half way
     between two bf16 numbers, a rounding to fp32 in between loses it and the half way goes to the even one. Exact: one-hot
@@ -288,21 +288,42 @@ def test_weights_are_rounded_once(ctx, bits, scale):
     assert ctx.device_status() == 0
 
 
-@pytest.mark.parametrize("n,k,bits,group", [
-    (19000, 1024, 4, 64),         # 75 pairs of tiles (the last tile missing) for 74 teams: runs that end inside a pair
-    (19000, 1088, 4, 32),         # 17 k-blocks: units of one at a pair's end
-    (28672, 448, 8, 32),          # runs of a pair and a half
+def chunks_of_cut_pairs(n, k, m):
+    """The library's rule for a weight of one chain of products, restated: the chunks of rows of a launch whose teams cut pairs of weight tiles
+    between them, 0 where they have whole pairs."""
+    teams, pairs, blocks = 74, (-(-n // 128) + 1) // 2, k // 64
+    assert pairs * 10 >= 148 * 7
+    best = None
+    for per in (192, 160, 128, 96):
+        if per - 32 >= m and per > 96:
+            continue
+        chunks = -(-m // per)
+        whole, cut = -(-pairs * chunks // teams) * blocks, (pairs * blocks / teams + 20) * chunks
+        cuts = chunks <= 3 and cut < whole
+        cost = (cut if cuts else whole) * (max(300, 2 * per) + 20)
+        if best is None or cost < best[0] * 0.995:
+            best = cost, chunks if cuts else 0
+    return best[1]
+
+
+@pytest.mark.parametrize("n,k,bits,group,gain,cuts", [
+    (28672, 4096, 4, 64, 1.0, {1: 1, 17: 1, 64: 1, 65: 1, 128: 1, 192: 1, 384: 2, 577: 0}),    # a pair and a half a team: two and three pairs of a run
+    (28672, 4096, 8, 32, 300.0, {1: 1, 96: 1, 97: 1, 384: 2}),                                # .. at 2^-shift of its size
+    (28665, 4160, 4, 32, 200.0, {5: 1, 80: 1, 150: 1, 383: 2}),                               # 65 k-blocks; rows that leave value by value
+    (31744, 8192, 4, 64, 1.0, {33: 1, 576: 3}),                                               # all chunks that the workspace has room for
 ])
-def test_teams_that_share_a_pair_carry_its_bits(ctx, n, k, bits, group):
+def test_teams_that_share_a_pair_carry_its_bits(ctx, n, k, bits, group, gain, cuts):
     """A team that has the end of a pair of weight tiles goes on from the sums of the one that has its start: one chain of products,
-    whoever has it. The entry point without that workspace has whole pairs only; few rows, rows of a cluster, and two to five chunks."""
-    p, s, b = make(n, k, bits, group, 51)
-    qw = api.QuantizedWeight(ctx, p.cuda(), s.cuda(), b.cuda(), bits, group)
-    x = acts(800, k, 52).cuda()
-    want = torch.empty(800, n, dtype=torch.bfloat16, device="cuda")
-    qw.matmul_static(x, 800, want)
+    whoever has it. The entry point without that workspace has whole pairs only; few rows, rows of a cluster, and two and three chunks."""
+    g = torch.Generator(device="cuda").manual_seed(51)
+    p, s, b = quantize_affine(torch.empty(n, k, device="cuda").normal_(0, 0.02 * gain, generator=g), bits, group)
+    qw = api.QuantizedWeight(ctx, p, s, b, bits, group)
+    x = acts(max(cuts), k, 52).cuda()
+    want = torch.empty(max(cuts), n, dtype=torch.bfloat16, device="cuda")
+    qw.matmul_static(torch.cat([x, x[:16]]), max(cuts), want)
     ctx.sync()
-    for m in (1, 17, 64, 65, 192, 193, 385, 576, 800, 1):
+    for m, chunks in list(cuts.items()) + [(min(cuts), 1)]:
+        assert chunks_of_cut_pairs(n, k, m) == chunks
         y = qw.matmul(x[:m])
         assert torch.equal(y.view(torch.int16), want[:m].view(torch.int16)), m
     assert ctx.device_status() == 0
@@ -312,7 +333,7 @@ def test_teams_that_share_a_pair_carry_its_bits(ctx, n, k, bits, group):
     (384, 1088, 4, 32),           # splits of 8 and 9 k-blocks
     (4096, 2048, 8, 32),          # four splits, apart and in turn
     (11000, 256, 4, 64),          # not split
-    (19000, 1088, 4, 64),         # not split, pairs of tiles cut between teams
+    (19000, 1088, 4, 64),         # not split, more pairs of tiles than teams
 ])
 def test_even_and_odd_k_blocks_are_sums_of_their_own(ctx, n, k, bits, group):
     """Weights of fewer than 207 tiles: a split is two chains of products, its even and its odd k-blocks, half as long as one. Exact:
