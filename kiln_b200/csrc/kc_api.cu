@@ -309,14 +309,15 @@ extern "C" void kc_ctx_destroy(kc_ctx_t c) {
 static void clear_gemm_fix(kc_ctx* c) {
   if (c->gemm_fix) cudaMemsetAsync(c->gemm_fix, 0xFF, qlinear_fix_bytes(c->sm_count), c->stream);
 }
-// The workspace, with the first weight that has a use for it: a team's share is a pair of tiles at least.
-static int ensure_gemm_fix(kc_ctx* c, const QWeight& w) {
-  if (w.n_tiles < c->sm_count || c->gemm_fix) return KC_OK;
-  const size_t bytes = qlinear_fix_bytes(c->sm_count);
-  cudaError_t e = cudaMalloc(&c->gemm_fix, bytes);
-  if (e != cudaSuccess) { c->gemm_fix = nullptr; return fail(KC_ERR_OOM, "GEMM workspace of %zu bytes: %s", bytes, cudaGetErrorString(e)); }
+// The workspace, with the first weight that has a use for it (plan_whole_rows). Where there is no room for it launches do without.
+static void ensure_gemm_fix(kc_ctx* c, const QWeight& w) {
+  if (w.splits > 1 || w.chains > 1 || c->gemm_fix) return;
+  if (cudaMalloc(&c->gemm_fix, qlinear_fix_bytes(c->sm_count)) != cudaSuccess) {
+    c->gemm_fix = nullptr;
+    cudaGetLastError();
+    return;
+  }
   clear_gemm_fix(c);
-  return KC_OK;
 }
 
 // Read after a synchronisation. A bounded wait that gave up never passes as success: every entry point that
@@ -604,8 +605,8 @@ extern "C" int kc_qweight_create(kc_ctx_t c, const uint32_t* w, const void* scal
   cudaStreamSynchronize(c->stream);
   if (e == cudaSuccess) e = qweight_finish(&q->w);
   cudaFree(dw); cudaFree(ds); cudaFree(db);
-  if (e == cudaSuccess && (rc = ensure_gemm_fix(c, q->w))) { cudaFree(q->partial); qweight_free(&q->w); delete q; return rc; }
   if (e != cudaSuccess) { qweight_free(&q->w); delete q; return fail(KC_ERR_CUDA, "kc_qweight_create: %s", cudaGetErrorString(e)); }
+  ensure_gemm_fix(c, q->w);
   g_live++;
   *out = q;
   return KC_OK;
@@ -757,7 +758,8 @@ int build_linear(kc_model* m, TensorIndex& idx, const std::vector<Part>& parts, 
   cudaFree(dw); cudaFree(ds); cudaFree(db);
   if (e != cudaSuccess) return fail(e == cudaErrorMemoryAllocation ? KC_ERR_OOM : KC_ERR_CUDA, "re-tiling %s: %s", parts[0].prefix.c_str(), cudaGetErrorString(e));
   m->weight_bytes += (int64_t)out->mlx_bytes();
-  return ensure_gemm_fix(c, *out);
+  ensure_gemm_fix(c, *out);
+  return KC_OK;
 }
 
 // Norm weight [H] bf16; Gemma's 1 + w is folded in at load (NormStyle::OnePlus, nn.rs:241-257).

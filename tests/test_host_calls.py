@@ -287,3 +287,18 @@ for m in (641, 672, 704, 768):
     ok(lib.kc_quantized_matmul(ctx, w, at, m, at))
     assert fake.fake_shapes().decode().split() == ["640:128x1x1"], (m, fake.fake_shapes())
 """)
+
+
+def test_a_weight_loads_without_room_for_what_teams_leave(fake):
+    """A wide weight's launches cut its pairs of tiles between teams, which takes a workspace of 44 MB: a weight that fits the device's
+    memory without it loads, and its launches have whole pairs."""
+    run(fake, """
+w = C.c_void_p()
+src = C.create_string_buffer(26700 * 2304 // 2 + 256)
+fake.fake_fail_above(41 << 20)
+ok(lib.kc_qweight_create(ctx, C.addressof(src), C.addressof(src), C.addressof(src), 26700, 2304, 4, 64, 0, C.byref(w)))
+fake.fake_fail_above(2 ** 62)
+fake.fake_reset()
+ok(lib.kc_quantized_matmul(ctx, w, at, 5, at))
+assert [c for c in calls() if c != "sync"] == ["launch early"]
+""")
