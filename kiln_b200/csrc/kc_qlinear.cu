@@ -80,8 +80,8 @@ __global__ void qweight_retile_kernel(uint8_t* __restrict__ records, const uint3
 }
 
 int qlinear_plan_splits(int n_tiles, int kblocks, int sm_count) {
-  // As many k-splits as fill the SMs with one-tile CTAs, each keeping at least 8 k-blocks; none when two-tile CTAs
-  // already fill them. Splits need not divide the k-blocks evenly (the kernel cuts [K s / S, K (s + 1) / S)).
+  // As many k-splits as fill the SMs with a CTA a tile and split, each keeping at least 8 k-blocks; none where the tiles alone keep
+  // half of the SMs busy. Splits need not divide the k-blocks evenly (the kernel cuts [K s / S, K (s + 1) / S)).
   if (n_tiles * 2 >= sm_count) return 1;
   int s = sm_count / n_tiles;
   s = std::min(s, std::min(16, kblocks / 8));
