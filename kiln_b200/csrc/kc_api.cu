@@ -502,15 +502,15 @@ extern "C" int kc_kv_write_block(kc_kv_t kv, uint32_t block, const void* src, si
 // through memory less). More rows than one 512-row slab go through the reduction kernel, or take the splits in turn.
 static int run_qlinear(kc_ctx* c, const QWeight& w, const ActOperand& x, int M, bf16* y, int ldy, float* partial,
                        SublayerOut* fused = nullptr) {
-  const bool defer = fused && w.splits > 1 && M <= QL_MAX_M && !qlinear_in_turn(w, M);
+  const bool summed = fused && w.splits > 1 && M <= QL_MAX_M, defer = summed && !qlinear_in_turn(w, M, true);
   for (int row0 = 0, rows; row0 < M; row0 += rows) {
     rows = qlinear_slab_rows(w, M - row0);
     QLinearLaunch l;
     l.w = &w; l.x = &x; l.row0 = row0; l.M = rows;
-    l.y = y; l.ldy = ldy; l.partial = partial; l.status = c->status;
+    l.y = y; l.ldy = ldy; l.partial = partial; l.summed = summed; l.status = c->status;
     l.fix = c->gemm_fix;
     LAUNCH(c, KC_PROF_GEMM, 1, qlinear_umma(l, c->stream));
-    if (w.splits > 1 && !defer && !qlinear_in_turn(w, l.M))
+    if (w.splits > 1 && !defer && !qlinear_in_turn(w, l.M, summed))
       LAUNCH(c, KC_PROF_GEMM_REDUCE, 1, qlinear_reduce_splits(partial, w.splits, l.M, w.N, y + (size_t)row0 * ldy, ldy, c->stream));
   }
   if (fused) *fused = defer ? SublayerOut::partials(partial, w.splits, (size_t)M, w.N) : SublayerOut::dense(y, ldy);

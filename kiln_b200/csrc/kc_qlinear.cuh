@@ -66,12 +66,13 @@ struct QLinearLaunch {
   const ActOperand* x;
   int row0;         // first activation row of this launch (x, y and partial are indexed from it)
   int M;            // live activation rows, at most qlinear_slab_rows
-  bf16* y;          // [M, ldy] bf16 when the weight has splits == 1 or qlinear_in_turn(w, M) (else unused)
+  bf16* y;          // [M, ldy] bf16 when the weight has splits == 1 or qlinear_in_turn(w, M, summed) (else unused)
   int ldy;
   float* partial;   // [splits][M][N] fp32 workspace when splits > 1 (rows relative to row0)
   // Workspace of qlinear_fix_bytes for what teams that share a weight's k-blocks leave for one another, all its bits set between
   // launches; without it they share whole pairs of tiles. Launches that have the same one run one after the other.
   float* fix = nullptr;
+  bool summed = false;   // partials, if there are any, are summed by the kernel that reads the result, not by one of their own
   uint32_t* status; // device status word
   // Optional fused gated activation for a weight whose rows are 16 gate and 16 up rows in turn: glu = 1 (silu) or 2 (gelu_approx)
   // asks the kernel to write act[M, N / 2] = activation(gate) * up instead of y. Honoured only when K is not split
@@ -113,8 +114,9 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s);
 // has 65535 chunks of 96 rows or more, and looking for the best number of them is host time that a launch of a million rows
 // hides. Asked again for each launch, since what a large one leaves may go the other way.
 constexpr int QL_LAUNCH_ROWS = 1 << 20;
-// Whether a launch of M rows takes the splits of its weight one after the other and writes y, no partials.
-bool qlinear_in_turn(const QWeight& w, int M);
+// Whether a launch of M rows takes the splits of its weight one after the other and writes y, no partials. summed: see
+// QLinearLaunch; for at most QL_MAX_M rows only.
+bool qlinear_in_turn(const QWeight& w, int M, bool summed = false);
 inline int qlinear_slab_rows(const QWeight& w, int M) {
   const int all = M < QL_LAUNCH_ROWS ? M : QL_LAUNCH_ROWS;
   return all <= QL_MAX_M || w.splits == 1 || qlinear_in_turn(w, all) ? all : QL_MAX_M;

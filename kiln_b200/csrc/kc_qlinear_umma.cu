@@ -7,9 +7,9 @@
 //   warp 1        TMA-loads the activation k-blocks (cp.async.bulk.tensor, 128B swizzle), of a cluster its CTA's half of the rows
 //   warp 2        allocates TMEM; issues tcgen05.mma (weights = A/M side from TENSOR MEMORY, activations = B/N side from shared
 //                 memory), of a cluster the first CTA's for both
-//   warps 4-19    four groups of four warps. Dequantisers unpack the 4/8-bit words, apply scale and bias in registers and write
-//                 the bf16 A operand into tensor memory (tcgen05.st); of a cluster the first group drains accumulators
-//                 (tcgen05.ld) under the next task's products instead.
+//   warps 4-19    four groups of four warps. Three dequantise: they unpack the 4/8-bit words, apply scale and bias in registers and
+//                 write the bf16 A operand into tensor memory (tcgen05.st). The first drains accumulators (tcgen05.ld) under the
+//                 next task's products; the last task is drained by all.
 // The accumulator D[n, m] lives in TMEM: lane = weight row n, column = activation row m.
 //
 // Every output element depends only on its own activation row and on an order of sums fixed by (N, K) and the SM count: a
@@ -917,25 +917,27 @@ static int plan_apart_rows(const QWeight& w, int M) {
 constexpr int QL_ROWS_MIN = 257;           // below, a chunk or two of rows never fill the SMs
 constexpr int QL_ROWS_MAX_KBLOCKS = 300;   // above, apart and in turn, us: 8192 x 28672 1500 rows 680 and 605, 1024 rows 475 and 391, 7000 x 28672 level
 // Whether the rows of a weight that is split along K take its splits in turn, and how many a chunk: 0 where they stay apart. In turn has to be the
-// faster way by a fifth in these figures: at rows near the line the calls keep the way they had. Apart, with the reduction behind it, and
-// in turn, us: 4096 x 14336 320 rows 41.2 and 42.8, 513 82 and 59, 1024 132 and 94, 2048 271 and 183; 4096 x 4096 366 rows 27.9 and 20.1 (the reduction
-// is 7 of the first, which a step does not have), 1024 77 and 42, 2048 153 and 80; 2048 x 8192 513 rows 43.5 and 37.7, 2048 140 and 85. The
-// reduction of more rows than QL_MAX_M, whose slabs do not stay in L2, goes at 3060 GB/s over the partials and the result; of fewer rows it is not counted, so
-// that a call has the way of the step, where the kernel that reads the result sums the partials at next to no cost. More than eight
-// splits are short ones, whose ends lie less under the next one's start.
+// faster way by a fifth in these figures, a call of up to QL_MAX_M rows with a reduction of its own by a third: at rows near the line the
+// calls keep the way they had. Apart, with the reduction behind it, and in turn, us: 4096 x 14336 320 rows 41.2 and 42.8, 513 82 and 59, 1024 132 and 94,
+// 2048 271 and 183; 4096 x 4096 366 rows 27.9 and 20.1 (the reduction is 7 of the first, which a step does not have), 1024 77 and 42, 2048 153
+// and 80; 6144 x 4096 512 rows 46.6 and 28.9; 2048 x 8192 513 rows 43.5 and 37.7, 2048 140 and 85. The reduction takes 2 us and 4570 GB/s over the
+// partials and the result, of more rows than QL_MAX_M, whose slabs do not stay in L2, 3060. Summed by the kernel that reads the
+// result anyway they cost next to nothing. More than eight splits are short ones, whose ends lie less under the next one's start.
 // Against the other way and all chunk sizes, in turn's chunk is 0.3 % behind the fastest on the mean of 340 points, 11 % at most.
-static int plan_in_turn_rows(const QWeight& w, int M) {
+static int plan_in_turn_rows(const QWeight& w, int M, bool summed) {
   if (w.splits == 1 || M < QL_ROWS_MIN || w.kblocks > QL_ROWS_MAX_KBLOCKS) return 0;
   auto slab = [&](int rows) { return rows ? apart_ns(w, rows, plan_apart_rows(w, rows)) : 0; };
   long long most = M / QL_MAX_M * slab(M >= QL_MAX_M ? QL_MAX_M : 0) + slab(M % QL_MAX_M);
-  if (M > QL_MAX_M) most += (long long)M * w.N * (4 * w.splits + 2) * 100 / 306000;
-  most = most * 80 / 100;
+  const long long bytes = (long long)M * w.N * (4 * w.splits + 2);
+  if (M > QL_MAX_M) most += bytes * 100 / 306000;
+  else if (!summed) most += 2100 + bytes * 100 / 457000;
+  most = most * (M > QL_MAX_M || summed ? 80 : 66) / 100;
   int best = 0;
   for (int per = 96; per <= QL_CHUNK_ROWS; per += 32)
     if (turn_ns(w, M, per) < (best ? turn_ns(w, M, best) : most)) best = per;
   return best;
 }
-bool qlinear_in_turn(const QWeight& w, int M) { return plan_in_turn_rows(w, M) > 0; }
+bool qlinear_in_turn(const QWeight& w, int M, bool summed) { return plan_in_turn_rows(w, M, summed) > 0; }
 
 // Rows of a chunk for a weight that is not split along K, and whether its teams share the work by runs: the choice whose products take the least
 // time. With two chains, turn_ns of one part; runs would hand on two sums of a cut pair, and lose: 26000 x 2048 at 33 rows, whole pairs and runs,
@@ -991,7 +993,7 @@ cudaError_t qlinear_umma(const QLinearLaunch& l, cudaStream_t s) {
   UmmaPlan t{};
   const int pairs = pairs_of(w), all_teams = std::max(1, w.sm_count / 2);
   if (w.splits > 1) {
-    const int turn = plan_in_turn_rows(w, l.M);
+    const int turn = plan_in_turn_rows(w, l.M, l.summed);
     t.way = turn ? QL_IN_TURN : QL_APART;
     t.m_pad = turn ? turn : plan_apart_rows(w, l.M);
   } else {
