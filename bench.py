@@ -194,9 +194,9 @@ def algorithmic(cfg, batch, k, mean_ctx):
 
 # DRAM traffic of the dominant kernel (the quantised GEMM) relative to its algorithmic weight bytes, from ncu captures of
 # single launches at 192 rows (summary committed under profiles/): dram__bytes_read.sum + dram__bytes_write.sum = 69.0 MB +
-# 3.2 MB for the 66.1 MB of records of a layer's gate_up and 311.3 MB + 47.6 MB for the 295.5 MB of the head. Weighted by the step's bytes (the head is 0.07 of them); the per-launch figure reported
+# 3.2 MB for the 66.1 MB of records of a layer's gate_up and 297.2 MB + 33.2 MB for the 295.5 MB of the head. Weighted by the step's bytes (the head is 0.07 of them); the per-launch figure reported
 # is this ratio times the mean algorithmic weight bytes per GEMM launch of the step.
-GEMM_DRAM_TRAFFIC_PER_WEIGHT_BYTE = 0.93 * (69.0 + 3.2) / 66.1 + 0.07 * (311.3 + 47.6) / 295.5
+GEMM_DRAM_TRAFFIC_PER_WEIGHT_BYTE = 0.93 * (69.0 + 3.2) / 66.1 + 0.07 * (297.2 + 33.2) / 295.5
 
 # --------------------------------------------------------------------------------------
 # GPU arm
